@@ -1,0 +1,88 @@
+"""The 32-bit path's product and attention where their kernels change hands: edges of tiles, a few rows against many, short runs
+against long ones.  Every form does the same operations in the same order, so a row's bits do not depend on what stands beside it."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def ops():
+    from mimirmind_b200.kernels import ops as o
+    return o
+
+
+@pytest.mark.parametrize("N,K", [(8, 4), (131, 260), (896, 4864), (4736, 72), (37888, 68), (200, 67)])
+@pytest.mark.parametrize("M", [1, 2, 4, 5, 8, 9, 16, 17, 33, 130])
+def test_product(M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(M * N + K)
+    a, w, b = (torch.randn(s, generator=g, device=DEV) for s in ((M, K), (N, K), (N,)))
+    out = torch.empty((M, N), device=DEV)
+    ops().gemm_simt(a, w, b, out)
+    ref, size = a.double() @ w.double().T + b.double(), a.double().abs() @ w.double().abs().T + b.double().abs()
+    # K products added one after the other and a bias: each addition rounds by at most 2^-24 of what has been added up
+    assert ((out - ref).abs() <= (K + 1) * 2.0 ** -24 * size).all()
+    for m in {0, M // 2, M - 1}:                # alone: the kernel for a few rows
+        one = torch.empty((1, N), device=DEV)
+        ops().gemm_simt(a[m:m + 1].contiguous(), w, b, one)
+        assert torch.equal(one[0], out[m])
+
+
+@pytest.mark.parametrize("M,N,K", [(3, 70, 96), (40, 130, 100), (300, 257, 36)])
+@pytest.mark.parametrize("ta,tw,tc", [(torch.bfloat16, torch.float32, torch.bfloat16), (torch.float32, torch.bfloat16, torch.float32)])
+def test_product_of_mixed_types(M, N, K, ta, tw, tc):
+    g = torch.Generator(device=DEV).manual_seed(M)
+    a, w = torch.randn((M, K), generator=g, device=DEV).to(ta), torch.randn((N, K), generator=g, device=DEV).to(tw)
+    out = torch.empty((M, N), dtype=tc, device=DEV)
+    ops().gemm_simt(a, w, None, out)
+    wide = torch.empty((M, N), device=DEV)
+    ops().gemm_simt(a.float(), w.float(), None, wide)
+    assert torch.equal(out, wide.to(tc))        # the same products of the same numbers
+
+
+@pytest.mark.parametrize("hd,H,G", [(64, 6, 2), (128, 4, 4)])
+@pytest.mark.parametrize("window", [0, 40])
+@pytest.mark.parametrize("runs", [[(0, 1)], [(0, 100), (70, 3), (300, 1), (31, 33), (0, 4)], [(5, 1), (260, 1), (127, 1), (128, 1), (1000, 2)]])
+def test_attention(hd, H, G, window, runs):
+    """runs: (first position, tokens) of the requests of a step, their earlier keys in the cache."""
+    page = 16
+    g = torch.Generator(device=DEV).manual_seed(hd + window + len(runs))
+    width = -(-max(p + n for p, n in runs) // page)
+    pages = len(runs) * width
+    k, v = (torch.randn((pages, G, page, hd), generator=g, device=DEV) for _ in range(2))
+    table = torch.randperm(pages, generator=g, device=DEV).to(torch.int32).view(len(runs), width)
+    n = sum(c for _, c in runs)
+    q = torch.randn((n, H * hd), generator=g, device=DEV) * 2
+    pos = torch.cat([torch.arange(p, p + c, dtype=torch.int32, device=DEV) for p, c in runs])
+    req = torch.cat([torch.full((c,), r, dtype=torch.int32, device=DEV) for r, (_, c) in enumerate(runs)])
+    for r, (p, c) in enumerate(runs):           # what lies behind a request's last token is nobody's: it must not be touched
+        for j in range(p + c, width * page):
+            k[table[r, j // page], :, j % page] = float("nan")
+            v[table[r, j // page], :, j % page] = float("nan")
+    out = ops().attention_generic(q, k, v, torch.empty_like(q), pos, req, table, page, H, G, hd, window, 0.1)
+    at = 0
+    for r, (p, c) in enumerate(runs):
+        kk, vv = (t[table[r].long()].transpose(1, 2).reshape(width * page, G, hd).double() for t in (k, v))
+        for i in {0, c // 2, c - 1}:
+            hi = p + i + 1
+            lo = max(0, hi - window) if window else 0
+            for h in range(H):
+                s = kk[lo:hi, h * G // H] @ q[at + i].view(H, hd)[h].double() * 0.1
+                want = torch.softmax(s, 0) @ vv[lo:hi, h * G // H]
+                # scores of up to 128 products of size ~2, weights and a sum over the keys in 32 bits
+                assert (out[at + i].view(H, hd)[h] - want).abs().max() <= 2e-5 * max(1.0, vv[lo:hi].abs().max())
+            one = ops().attention_generic(q[at + i:at + i + 1].contiguous(), k, v, torch.empty((1, H * hd), device=DEV), pos[at + i:at + i + 1].contiguous(),
+                                          req[at + i:at + i + 1].contiguous(), table, page, H, G, hd, window, 0.1)
+            assert torch.equal(one[0], out[at + i])          # as a single token, bit for bit
+        at += c
+
+
+def test_attention_skips_infinite_values_that_a_row_does_not_see():
+    page, hd = 16, 64
+    g = torch.Generator(device=DEV).manual_seed(1)
+    k, v, q = (torch.randn(s, generator=g, device=DEV) for s in ((3, 1, page, hd), (3, 1, page, hd), (40, hd)))
+    v[2, 0, 5] = float("inf")                   # the value of token 37
+    table = torch.arange(3, dtype=torch.int32, device=DEV).view(1, 3)
+    pos, req = torch.arange(40, dtype=torch.int32, device=DEV), torch.zeros(40, dtype=torch.int32, device=DEV)
+    out = ops().attention_generic(q, k, v, torch.empty_like(q), pos, req, table, page, 1, 1, hd, 0, 0.125)
+    assert torch.isfinite(out[:37]).all() and torch.isinf(out[37:]).all()
