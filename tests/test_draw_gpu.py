@@ -1,0 +1,81 @@
+"""The draw of tokens where the search for an element changes its way: flat rows (more elements in a bin than its list holds, then equal
+ones), rows that hold few finite logits, a NaN, very low and very high temperatures, every number of CTAs per row."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+import plain_qwen2 as plain
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def rows_of(kind, R, V, rng):
+    if kind == "flat":
+        return np.full((R, V), 1.25, dtype=np.float32)
+    if kind == "nearly flat":
+        return (1e-5 * rng.randn(R, V)).astype(np.float32)
+    if kind == "few values":
+        return rng.choice([-1.0, 0.0, 0.0, 0.5, 3.0], size=(R, V)).astype(np.float32)
+    if kind == "mostly -inf":
+        x = np.full((R, V), -np.inf, dtype=np.float32)
+        for r in range(R):
+            x[r, rng.choice(V, 9, replace=False)] = rng.randn(9) * 2
+        return x
+    return (3 * rng.randn(R, V)).astype(np.float32)
+
+
+def check(row, T, k, p, u, token):
+    """The token's share of the kept mass holds u, up to what 32-bit weights (relative error below 4e-6: exponents up to 28 in
+    32 bits) can move a boundary."""
+    order = np.lexsort((np.arange(row.size), -row.astype(np.float64)))
+    x = row[order].astype(np.float64)
+    kept = np.ones(row.size, dtype=bool) if not (0 < k < row.size) else x >= x[k - 1]
+    with np.errstate(over="ignore", invalid="ignore"):
+        w = np.where(kept, np.exp((x - x[0]) / T), 0.0)
+    w[w < 2.0 ** -40] = 0.0
+    cum, slack = np.cumsum(w), 4e-6
+    lo = hi = cum[-1]
+    if 0.0 < p < 1.0:           # the cut keeps equal logits together; a cut within the slack may fall on either side
+        lo, hi = (cum[np.searchsorted(x[0] - x, x[0] - x[min(row.size - 1, np.searchsorted(cum, q * cum[-1]))], side="right") - 1]
+                  for q in (max(0.0, p - slack), min(1.0, p + slack)))
+    at = int(np.nonzero(order == token)[0][0])
+    before = cum[at] - w[at]
+    assert before <= u * hi + slack * cum[-1] and cum[at] >= u * lo - slack * cum[-1], (T, k, p, u, before / cum[-1], cum[at] / cum[-1])
+
+
+@pytest.mark.parametrize("kind", ["flat", "nearly flat", "few values", "mostly -inf", "normal"])
+@pytest.mark.parametrize("R,V", [(2, 300), (8, 9001), (16, 40000), (5, 152064), (70, 65536), (150, 33000)])
+def test_draws(kind, R, V):
+    from mimirmind_b200.kernels import ops
+    rng = np.random.RandomState(V % 997 + R)
+    logits = rows_of(kind, R, V, rng)
+    temps = rng.choice([0.02, 0.3, 0.8, 1.5, 50.0], size=R).astype(np.float32)
+    ks = rng.choice([0, 0, 2, 40, 5000], size=R).astype(np.int32)
+    ps = rng.choice([1.0, 0.95, 0.5, 0.05], size=R).astype(np.float32)
+    seeds, counters = rng.randint(1, 2 ** 31, size=R), rng.randint(0, 1000, size=R)
+    t = lambda a, dt: torch.tensor(a, dtype=dt, device=DEV)                  # noqa: E731
+    args = [t(temps, torch.float32), t(ks, torch.int32), t(ps, torch.float32), t(seeds, torch.int64), t(counters, torch.int64)]
+    got = ops.sample_rows(t(logits, torch.float32), *args).cpu().tolist()
+    for r in list(range(R))[:24]:
+        u = plain.uniform_from(int(seeds[r]), int(counters[r]))
+        check(logits[r], float(temps[r]), int(ks[r]), float(ps[r]), u, got[r])
+    # a row alone is shared by another number of CTAs and draws the same token
+    for r in (0, R - 1):
+        one = ops.sample_rows(t(logits[r:r + 1], torch.float32), *[a[r:r + 1].contiguous() for a in args]).item()
+        assert one == got[r]
+
+
+def test_a_row_with_a_nan_or_an_infinite_logit_leaves_the_others_alone():
+    from mimirmind_b200.kernels import ops
+    rng = np.random.RandomState(4)
+    x = torch.tensor(rng.randn(4, 20000), dtype=torch.float32, device=DEV)
+    full = lambda v, dt: torch.full((4,), v, dtype=dt, device=DEV)           # noqa: E731
+    args = [full(0.9, torch.float32), full(30, torch.int32), full(0.9, torch.float32), full(5, torch.int64), torch.arange(4, device=DEV)]
+    want = ops.sample_rows(x, *args).cpu().tolist()
+    x[1, 77] = math.nan
+    x[2, 5] = math.inf
+    got = ops.sample_rows(x, *args).cpu().tolist()
+    assert got[0] == want[0] and got[3] == want[3] and all(0 <= v < 20000 for v in got)
