@@ -94,43 +94,72 @@ __global__ void causal_conv_tokens_kernel(const float* __restrict__ x, int ld, i
     y[(size_t)t * ldy + c] = act ? ls_silu(acc) : acc;
 }
 
-// The same per (token, 4 consecutive channels): a block owns 8 consecutive tokens x 128 channels, so the rows that
-// neighbouring tokens share are read from DRAM once and from L1 after that; 16-byte loads and stores.  A channel's
-// products are summed in the same order as above, so both forms give the same bits.
+// The same four channels at a time: a warp owns 128 channels of CONV_RUN consecutive tokens and slides over them with the last K
+// inputs and the taps in registers, so a row is loaded K - 1 times extra per CONV_RUN tokens instead of K times per token, and
+// all rows of a run are on their way at once.  Where a run holds the start of a portion (whose earlier inputs are the state's), each
+// token fetches its own inputs.  A channel's products are summed in the same order as above, so all forms give the same bits.
+// Bound by memory: 4,096 x 3,072 with 4 taps (100 MB) 103 us with a thread per (token, four channels), 30 us so.
+#define CONV_RUN 8
 template <int K>
 __global__ void __launch_bounds__(256) causal_conv_tokens4_kernel(
     const float* __restrict__ x, int ld, int C, const float* __restrict__ taps, const float* __restrict__ tail,
     long long tail_stride, float* __restrict__ y, int ldy, const int32_t* __restrict__ token_req, const int32_t* __restrict__ req_meta,
     const int32_t* __restrict__ slots, const int32_t* __restrict__ positions, int act, int n_tokens) {
     const int c = (blockIdx.x * 32 + (threadIdx.x & 31)) * 4;
-    const int t = blockIdx.y * 8 + (threadIdx.x >> 5);
-    if (c >= C || t >= n_tokens) return;
-    const int r = token_req[t];
-    const int o = t - (req_meta ? req_meta[4 * r] : t);       // the token's place in its portion
-    const int pos = positions[t];
-    const float* tl = tail + (size_t)slots[r] * tail_stride;
-    float4 in[K];                                              // every load is issued before the first product
+    const int t0 = (blockIdx.y * 8 + (threadIdx.x >> 5)) * CONV_RUN;
+    if (c >= C || t0 >= n_tokens) return;
+    const int cnt = min(CONV_RUN, n_tokens - t0), r0 = token_req[t0];
+    const bool inside = token_req[t0 + cnt - 1] == r0 && t0 - (req_meta ? req_meta[4 * r0] : t0) >= K - 1;      // no token looks beyond its portion
+    float w[4][K];                                             // w[.][j] multiplies the input j tokens back
 #pragma unroll
-    for (int j = 0; j < K; ++j) {
-        in[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);           // before the sequence's start: zeros (a product with zero adds nothing)
-        if (pos - j >= 0)
-            in[j] = (o - j >= 0) ? *reinterpret_cast<const float4*>(x + (size_t)(t - j) * ld + c)
-                                 : *reinterpret_cast<const float4*>(tl + (size_t)(j - o - 1) * C + c);
-    }
-    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int e = 0; e < 4; ++e)
 #pragma unroll
-    for (int j = 0; j < K; ++j) {
-        const float* w = taps + (size_t)c * K + (K - 1 - j);
-        acc[0] = fmaf(w[0], in[j].x, acc[0]);
-        acc[1] = fmaf(w[K], in[j].y, acc[1]);
-        acc[2] = fmaf(w[2 * K], in[j].z, acc[2]);
-        acc[3] = fmaf(w[3 * K], in[j].w, acc[3]);
-    }
-    if (act) {
+        for (int j = 0; j < K; ++j) w[e][j] = taps[(size_t)(c + e) * K + (K - 1 - j)];
+    auto put = [&](int t, const float4* in) {                   // in[j]: the input j tokens back
+        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[e] = ls_silu(acc[e]);
+        for (int j = 0; j < K; ++j) {
+            acc[0] = fmaf(w[0][j], in[j].x, acc[0]);
+            acc[1] = fmaf(w[1][j], in[j].y, acc[1]);
+            acc[2] = fmaf(w[2][j], in[j].z, acc[2]);
+            acc[3] = fmaf(w[3][j], in[j].w, acc[3]);
+        }
+        if (act) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[e] = ls_silu(acc[e]);
+        }
+        *reinterpret_cast<float4*>(y + (size_t)t * ldy + c) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    };
+    if (inside) {
+        float4 row[CONV_RUN + K - 1];                          // rows t0 - (K - 1) ..
+#pragma unroll
+        for (int i = 0; i < CONV_RUN + K - 1; ++i)
+            row[i] = i - (K - 1) < cnt ? *reinterpret_cast<const float4*>(x + (size_t)(t0 + i - (K - 1)) * ld + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int i = 0; i < CONV_RUN; ++i) {
+            if (i >= cnt) break;
+            float4 in[K];
+#pragma unroll
+            for (int j = 0; j < K; ++j) in[j] = row[i + K - 1 - j];
+            put(t0 + i, in);
+        }
+        return;
     }
-    *reinterpret_cast<float4*>(y + (size_t)t * ldy + c) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    for (int t = t0; t < t0 + cnt; ++t) {
+        const int r = token_req[t];
+        const int o = t - (req_meta ? req_meta[4 * r] : t);       // the token's place in its portion
+        const int pos = positions[t];
+        const float* tl = tail + (size_t)slots[r] * tail_stride;
+        float4 in[K];
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+            in[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);           // before the sequence's start: zeros (a product with zero adds nothing)
+            if (pos - j >= 0)
+                in[j] = (o - j >= 0) ? *reinterpret_cast<const float4*>(x + (size_t)(t - j) * ld + c)
+                                     : *reinterpret_cast<const float4*>(tl + (size_t)(j - o - 1) * C + c);
+        }
+        put(t, in);
+    }
 }
 
 __global__ void causal_conv_tail_kernel(const float* __restrict__ x, int ld, int C, int K, float* __restrict__ tail, long long tail_stride,
@@ -161,12 +190,12 @@ MM_EXPORT int mm_causal_conv_tokens(const void* x, int ld, int C, const void* ta
     MM_REQUIRE((tail != nullptr || K == 1) && slots != nullptr && positions != nullptr && token_req != nullptr && y != nullptr && y != x,
                "causal conv: the state, the positions, the tokens' requests and a result buffer of its own are needed");
     if (n_tokens <= 0 || n_requests <= 0) return MM_OK;
-    const bool by4 = C % 4 == 0 && ld % 4 == 0 && ldy % 4 == 0 && tail_stride % 4 == 0 && ceil_div(n_tokens, 8) <= 65535 &&
+    const bool by4 = C % 4 == 0 && ld % 4 == 0 && ldy % 4 == 0 && tail_stride % 4 == 0 && ceil_div(n_tokens, 8 * CONV_RUN) <= 65535 &&
                      (((uintptr_t)x | (uintptr_t)y | (uintptr_t)tail) & 15) == 0;
     if (by4) {
 #define CONV4_CASE(KK)                                                                                                                  \
     case KK:                                                                                                                            \
-        mm_launch(causal_conv_tokens4_kernel<KK>, dim3(ceil_div(C, 128), ceil_div(n_tokens, 8)), dim3(256), 0, (cudaStream_t)stream,     \
+        mm_launch(causal_conv_tokens4_kernel<KK>, dim3(ceil_div(C, 128), ceil_div(n_tokens, 8 * CONV_RUN)), dim3(256), 0, (cudaStream_t)stream,     \
                   (const float*)x, ld, C, (const float*)taps, (const float*)tail, tail_stride, (float*)y, ldy, (const int32_t*)token_req, \
                   (const int32_t*)req_meta, (const int32_t*)slots, (const int32_t*)positions, act, n_tokens);                            \
         break;
@@ -636,10 +665,43 @@ __global__ void forget_gate_prep_kernel(float* __restrict__ x, int ld, long long
     row[f_off + c] = l + (1.0f - l) * ls_sigmoid(row[f_off + c] + (bias ? bias[c] : 0.0f));
 }
 
+// The same four numbers at a time.  Bound by memory: 2,048 tokens x 2,048 + 2,048 (67 MB) 26 us one by one, 14 us so.
+__global__ void __launch_bounds__(256) forget_gate_prep4_kernel(float* __restrict__ x, int ld, int n_tokens, int q_off, int f_off, int n_qf, int act_q,
+                                                                const float* __restrict__ bias, const float* __restrict__ lower) {
+    const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
+    if (c >= n_qf) return;
+    const float4 b = bias ? *reinterpret_cast<const float4*>(bias + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float4 l = lower ? *reinterpret_cast<const float4*>(lower + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const int t0 = blockIdx.y * 4, t1 = min(n_tokens, t0 + 4);
+    float4 f[4], q[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (t0 + i < t1) {
+            f[i] = *reinterpret_cast<const float4*>(x + (size_t)(t0 + i) * ld + f_off + c);
+            if (act_q) q[i] = *reinterpret_cast<const float4*>(x + (size_t)(t0 + i) * ld + q_off + c);
+        }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (t0 + i < t1) {
+            float* row = x + (size_t)(t0 + i) * ld;
+            if (act_q) *reinterpret_cast<float4*>(row + q_off + c) = make_float4(ls_silu(q[i].x), ls_silu(q[i].y), ls_silu(q[i].z), ls_silu(q[i].w));
+            *reinterpret_cast<float4*>(row + f_off + c) =
+                make_float4(l.x + (1.0f - l.x) * ls_sigmoid(f[i].x + b.x), l.y + (1.0f - l.y) * ls_sigmoid(f[i].y + b.y),
+                            l.z + (1.0f - l.z) * ls_sigmoid(f[i].z + b.z), l.w + (1.0f - l.w) * ls_sigmoid(f[i].w + b.w));
+        }
+}
+
 MM_EXPORT int mm_forget_gate_prep(void* x, int ld, int n_tokens, int q_off, int f_off, int n_qf, int act_q, const void* bias, const void* lower,
                                   void* stream) {
     MM_REQUIRE(n_tokens >= 0 && n_qf > 0 && q_off >= 0 && f_off >= 0 && q_off + n_qf <= ld && f_off + n_qf <= ld, "forget gate: columns outside the row");
     if (n_tokens == 0) return MM_OK;
+    if (n_qf % 4 == 0 && ld % 4 == 0 && q_off % 4 == 0 && f_off % 4 == 0 && ceil_div(n_tokens, 4) <= 65535 &&
+        (((uintptr_t)x | (uintptr_t)bias | (uintptr_t)lower) & 15) == 0) {
+        mm_launch(forget_gate_prep4_kernel, dim3(ceil_div(n_qf / 4, 256), ceil_div(n_tokens, 4)), dim3(256), 0, (cudaStream_t)stream, (float*)x, ld,
+                  n_tokens, q_off, f_off, n_qf, act_q, (const float*)bias, (const float*)lower);
+        MM_CHECK_LAUNCH();
+        return MM_OK;
+    }
     const long long total = (long long)n_tokens * n_qf;
     mm_launch(forget_gate_prep_kernel, dim3(ceil_div(total, 256)), dim3(256), 0, (cudaStream_t)stream, (float*)x, ld, total, q_off, f_off, n_qf, act_q,
               (const float*)bias, (const float*)lower);

