@@ -1,4 +1,4 @@
-// Paged causal prefill attention on the tcgen05 tensor cores, head sizes 64 and 128, bfloat16.
+// Paged causal prefill attention on the tcgen05 tensor cores, key and value sizes 64 and 128 in any pairing, bfloat16.
 //
 // One CTA per (tile of up to 128 query tokens of one request, query head).  Q stays in shared
 // memory; keys and values stream in tiles of 128 keys, fetched page by page with TMA straight
@@ -66,31 +66,30 @@ struct AttCtl {
 };
 
 // tiles: int32 [n_tiles, 4] = (request index, first token row, rows in the tile (<= 128), position of the first row)
-template <int HD>
+template <int HDK, int HDV, bool CAP>
 __global__ void __launch_bounds__(ATT_TC_THREADS, 1)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                            const __grid_constant__ CUtensorMap tmV, __nv_bfloat16* __restrict__ out,
+                            const __grid_constant__ CUtensorMap tmV, void* __restrict__ out, int out_f32,
                             const int32_t* __restrict__ tiles, const int32_t* __restrict__ block_table, int table_width,
-                            int page_size, int H, int G, KeyMask mask, float scale_log2, int sink, const float* __restrict__ gate, int gate_ld,
-                            int* __restrict__ err) {
+                            int page_size, int H, int G, int Gv, KeyMask mask, float scale_log2, float cap_in, int sink,
+                            const float* __restrict__ sink_logit, const float* __restrict__ gate, int gate_ld, int* __restrict__ err) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];   // 128-byte swizzle wants 1024-byte aligned tiles
     if ((smem_u32(smem_raw) & 1023u) != 0) {                      // never seen; without the alignment nothing below is valid
         if (threadIdx.x == 0 && err != nullptr) atomicExch(err, 3);
         return;
     }
-    constexpr int HALVES = HD / 64;                             // 64-column halves of a row of Q, K or V
-    constexpr int HEAD_TILE_BYTES = HALVES * HALF_BYTES;        // [128 rows x head size]: a tile of Q, of keys or of values
-    unsigned char* sQ = smem_raw;                               // HEAD_TILE_BYTES
-    unsigned char* sP = sQ + HEAD_TILE_BYTES;                   // 2 * TILE_BYTES
-    unsigned char* sK = sP + 2 * TILE_BYTES;                    // KV_STAGES * HEAD_TILE_BYTES
-    unsigned char* sV = sK + KV_STAGES * HEAD_TILE_BYTES;       // KV_STAGES * HEAD_TILE_BYTES
-    AttCtl* ctl = reinterpret_cast<AttCtl*>(sV + KV_STAGES * HEAD_TILE_BYTES);
+    constexpr int K_TILE_BYTES = HDK / 64 * HALF_BYTES, V_TILE_BYTES = HDV / 64 * HALF_BYTES;      // a tile of Q or keys, of values: [128 rows x size] as 64-column halves
+    unsigned char* sQ = smem_raw;                               // K_TILE_BYTES
+    unsigned char* sP = sQ + K_TILE_BYTES;                      // 2 * TILE_BYTES
+    unsigned char* sK = sP + 2 * TILE_BYTES;                    // KV_STAGES * K_TILE_BYTES
+    unsigned char* sV = sK + KV_STAGES * K_TILE_BYTES;          // KV_STAGES * V_TILE_BYTES
+    AttCtl* ctl = reinterpret_cast<AttCtl*>(sV + KV_STAGES * V_TILE_BYTES);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     volatile int* abort_flag = &ctl->abort_flag;
 
     // heads fastest, later (longer) tiles first: the longest tiles of every head start in the first wave
     const int tile = gridDim.y - 1 - blockIdx.y, h = blockIdx.x;
-    const int g = (h * G) / H;
+    const int g = (h * G) / H, gv = g % Gv;                      // key head, value head
     const int req = tiles[tile * 4 + 0], row0 = tiles[tile * 4 + 1], n_rows = tiles[tile * 4 + 2], pos0 = tiles[tile * 4 + 3];
     const int32_t* table = block_table + (size_t)req * table_width;
     const int hi_all = pos0 + n_rows;
@@ -106,7 +105,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
     // ---- what the TMA producers need: warp 0 keys (and Q), warp 10 values; lane = (page of the tile, column half) ----
     const int pages_per_tile = BN / page_size;
     const uint32_t page_bytes = (uint32_t)page_size * 128u;           // one column half of a page
-    const int pj = lane / HALVES, phf = lane % HALVES;                // this lane's page and half
+    const int halves = warp == V_PRODUCER_WARP ? HDV / 64 : HDK / 64;
+    const int pj = lane / halves, phf = lane % halves;                // this lane's page and half
     // pages of a tile that hold keys some row of the tile may see.  The ids are read a few tiles ahead: the load
     // from the block table would otherwise sit, with its full latency, between every two tiles.
     auto page_of = [&](int kt) -> int {
@@ -133,8 +133,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         }
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (ok && pid >= 0)
-            tma_load_2d(smem_u32((for_k ? sK : sV) + s * HEAD_TILE_BYTES) + phf * HALF_BYTES + (uint32_t)pj * page_bytes, for_k ? &tmK : &tmV,
-                        phf * 64, (pid * G + g) * page_size, full);
+            tma_load_2d(smem_u32(for_k ? sK + s * K_TILE_BYTES : sV + s * V_TILE_BYTES) + phf * HALF_BYTES + (uint32_t)pj * page_bytes,
+                        for_k ? &tmK : &tmV, phf * 64, (for_k ? pid * G + g : pid * Gv + gv) * page_size, full);
         return ok;
     };
     if (warp == 0 || warp == V_PRODUCER_WARP) {
@@ -162,15 +162,15 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             // Q and the first tile of keys need nobody else: their copies go out before the CTA has set itself up
             const uint32_t qbar = smem_u32(&ctl->q_full);
-            mbar_expect_tx(qbar, HEAD_TILE_BYTES);
+            mbar_expect_tx(qbar, K_TILE_BYTES);
 #pragma unroll
-            for (int hf = 0; hf < HALVES; ++hf) tma_load_2d(smem_u32(sQ) + hf * HALF_BYTES, &tmQ, h * HD + hf * 64, row0, qbar);
+            for (int hf = 0; hf < HDK / 64; ++hf) tma_load_2d(smem_u32(sQ) + hf * HALF_BYTES, &tmQ, h * HDK + hf * 64, row0, qbar);
         }
         __syncwarp();
         if (kt_begin < kt_end) produce(true, kt_begin, 0, false);
     }
     // Value tiles must never hold non-finite leftovers: rows of a page that was not fetched are multiplied by P = 0.
-    for (int i = threadIdx.x; i < KV_STAGES * HEAD_TILE_BYTES / 16; i += ATT_TC_THREADS) reinterpret_cast<uint4*>(sV)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = threadIdx.x; i < KV_STAGES * V_TILE_BYTES / 16; i += ATT_TC_THREADS) reinterpret_cast<uint4*>(sV)[i] = make_uint4(0, 0, 0, 0);
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(TMEM_COLS_ATT) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -201,9 +201,9 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
                 if (!mbar_wait(smem_u32(&ctl->s_free[b]), (u & 1) ^ 1, abort_flag)) return false;
                 if (!mbar_wait(smem_u32(&ctl->k_full[s]), (it / KV_STAGES) & 1, abort_flag)) return false;
                 tc_fence_after();
-                const uint32_t k_addr = smem_u32(sK + s * HEAD_TILE_BYTES);
+                const uint32_t k_addr = smem_u32(sK + s * K_TILE_BYTES);
 #pragma unroll
-                for (int k = 0; k < HD / 16; ++k) {
+                for (int k = 0; k < HDK / 16; ++k) {
                     const uint32_t off = (k >> 2) * HALF_BYTES + (k & 3) * 32;      // 16 columns = 32 bytes inside the swizzled row
                     umma_bf16(tmem_base + b * 128, smem_desc_sw128(q_addr + off, 16, 1024), smem_desc_sw128(k_addr + off, 16, 1024), IDESC_QK, k ? 1u : 0u);
                 }
@@ -218,7 +218,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
     } else if (warp == PV_ISSUER_WARP) {
         if (lane == 0) {
             // ---- P V issuer ----
-            constexpr uint32_t IDESC_PV = idesc_bf16(BM, HD, true);
+            constexpr uint32_t IDESC_PV = idesc_bf16(BM, HDV, true);
             const int n_tiles_k = kt_end - kt_begin;
             for (uint32_t it = 0; (int)it < n_tiles_k; ++it) {
                 const int s = it % KV_STAGES;
@@ -226,12 +226,12 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
                 if (!mbar_wait(smem_u32(&ctl->p_full[b]), u & 1, abort_flag)) break;       // P is there, O is rescaled
                 if (!mbar_wait(smem_u32(&ctl->v_full[s]), (it / KV_STAGES) & 1, abort_flag)) break;
                 tc_fence_after();
-                const uint32_t p_addr = smem_u32(sP + b * TILE_BYTES), v_addr = smem_u32(sV + s * HEAD_TILE_BYTES);
+                const uint32_t p_addr = smem_u32(sP + b * TILE_BYTES), v_addr = smem_u32(sV + s * V_TILE_BYTES);
 #pragma unroll
                 for (int k = 0; k < BN / 16; ++k) {
                     const uint32_t a_off = (k >> 2) * HALF_BYTES + (k & 3) * 32;    // P: K-major over the keys
                     const uint32_t b_off = (uint32_t)k * 16 * 128;                  // V: 16 key rows of 128 bytes further
-                    umma_bf16(tmem_base + 256 + b * HD, smem_desc_sw128(p_addr + a_off, 16, 1024), smem_desc_sw128(v_addr + b_off, HALF_BYTES, 1024), IDESC_PV, (u | (uint32_t)k) ? 1u : 0u);
+                    umma_bf16(tmem_base + 256 + b * HDV, smem_desc_sw128(p_addr + a_off, 16, 1024), smem_desc_sw128(v_addr + b_off, HALF_BYTES, 1024), IDESC_PV, (u | (uint32_t)k) ? 1u : 0u);
                 }
                 umma_commit(smem_u32(&ctl->pv_done[b]));
                 umma_commit(smem_u32(&ctl->v_empty[s]));
@@ -247,7 +247,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         const bool row_valid = row < n_rows;
         const int wlo = mask_low(mask, pos);
         const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
-        const uint32_t s_addr = lane_addr + g * 128, o_addr = lane_addr + 256 + g * HD;
+        const uint32_t s_addr = lane_addr + g * 128, o_addr = lane_addr + 256 + g * HDV;
         float m_ref = -INFINITY;           // the maximum the group's probabilities (and its O) are taken relative to
         float l = 0.0f;                    // the group's sum for this row, relative to m_ref
         const int n_tiles_k = kt_end - kt_begin;
@@ -256,8 +256,8 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         uint32_t sreg[128];
         const SoftmaxBars bars = {smem_u32(&ctl->s_full[g]), smem_u32(&ctl->s_free[g]), smem_u32(&ctl->p_full[g]), smem_u32(&ctl->pv_done[g])};
         for (uint32_t it = g; (int)it < n_tiles_k && ok; it += 2, ++done) {
-            ok = softmax_tile<HD>(bars, abort_flag, s_addr, o_addr, sP + g * TILE_BYTES, HALF_BYTES, row, lane, row_valid, pos, wlo,
-                                  walk.real(kt_begin + (int)it) * BN, it >> 1, done == 0, scale_log2, sreg, m_ref, l, keep);
+            ok = softmax_tile<HDV, CAP>(bars, abort_flag, s_addr, o_addr, sP + g * TILE_BYTES, HALF_BYTES, row, lane, row_valid, pos, wlo,
+                                  walk.real(kt_begin + (int)it) * BN, it >> 1, done == 0, scale_log2, sreg, m_ref, l, keep, cap_in);
         }
         // Merge the two groups: every thread posts its row's (reference, sum); the row's output is
         // (O0 f0 + O1 f1) / (l0 f0 + l1 f1) with f = 2^((m_g - m) scale); group g writes its half of the output columns.
@@ -270,33 +270,40 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         const float m = fmaxf(m0, m1);
         const float f0 = (m0 == -INFINITY) ? 0.0f : fast_exp2((m0 - m) * scale_log2);
         const float f1 = (m1 == -INFINITY) ? 0.0f : fast_exp2((m1 - m) * scale_log2);
-        // a softmax sink (a key of score 0 without a value) only adds its weight, 2^(-m scale), to the row's sum
-        const float total = l0 * f0 + l1 * f1 + (sink ? fast_exp2(-m * scale_log2) : 0.0f);
+        // a softmax sink (a key without a value, of score 0 or the head's logit) only adds its weight, 2^(-m scale), to the row's sum
+        const float sink_log2 = sink_logit != nullptr ? sink_logit[h] * 1.4426950408889634f : 0.0f;
+        const float total = l0 * f0 + l1 * f1 + (sink ? fast_exp2(fmaf(-m, scale_log2, sink_log2)) : 0.0f);
         // O of both groups is complete when their last P V is done (a group without tiles has no O)
         const int tiles0 = (n_tiles_k + 1) / 2, tiles1 = n_tiles_k / 2;
         if (ok && tiles0 > 0) ok = mbar_wait(smem_u32(&ctl->pv_done[0]), (uint32_t)(tiles0 - 1) & 1, abort_flag);
         if (ok && tiles1 > 0) ok = mbar_wait(smem_u32(&ctl->pv_done[1]), (uint32_t)(tiles1 - 1) & 1, abort_flag);
         tc_fence_after();
         const float inv = (total > 0.0f ? 1.0f / total : 0.0f) * (row_valid ? head_gate(gate, gate_ld, row0 + row, h) : 0.0f);
-        __nv_bfloat16* orow = out + ((size_t)(row0 + row) * H + h) * HD + g * (HD / 2);
+        const size_t at = ((size_t)(row0 + row) * H + h) * HDV + g * (HDV / 2);
 #pragma unroll 1
-        for (int c = 0; c < HD / 64; ++c) {                        // 32 output columns at a time
+        for (int c = 0; c < HDV / 64; ++c) {                        // 32 output columns at a time
             float acc[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) acc[i] = 0.0f;
             if (ok && tiles0 > 0) {                                // uniform over the CTA
-                tmem_ld32_nowait(lane_addr + 256 + g * (HD / 2) + c * 32, sreg);
+                tmem_ld32_nowait(lane_addr + 256 + g * (HDV / 2) + c * 32, sreg);
                 tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < 32; ++i) acc[i] = __uint_as_float(sreg[i]) * f0;
             }
             if (ok && tiles1 > 0) {
-                tmem_ld32_nowait(lane_addr + 256 + HD + g * (HD / 2) + c * 32, sreg);
+                tmem_ld32_nowait(lane_addr + 256 + HDV + g * (HDV / 2) + c * 32, sreg);
                 tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < 32; ++i) acc[i] = fmaf(__uint_as_float(sreg[i]), f1, acc[i]);
             }
-            if (ok && row_valid) {
+            if (ok && row_valid && out_f32) {
+                float* orow = static_cast<float*>(out) + at;
+#pragma unroll
+                for (int i = 0; i < 32; i += 4)
+                    *reinterpret_cast<float4*>(orow + c * 32 + i) = make_float4(acc[i] * inv, acc[i + 1] * inv, acc[i + 2] * inv, acc[i + 3] * inv);
+            } else if (ok && row_valid) {
+                __nv_bfloat16* orow = static_cast<__nv_bfloat16*>(out) + at;
 #pragma unroll
                 for (int i = 0; i < 32; i += 8)
                     *reinterpret_cast<uint4*>(orow + c * 32 + i) = make_uint4(pack_bf16x2(acc[i] * inv, acc[i + 1] * inv), pack_bf16x2(acc[i + 2] * inv, acc[i + 3] * inv),
@@ -320,69 +327,81 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
 
 }  // namespace
 
-// q, out: [n_tokens, H*hd] bf16; k_pages, v_pages: [num_pages, G, page_size, hd] bf16 of one layer (hd 64 or 128);
-// tiles: int32 [n_tiles, 4] (request, first row, rows <= 128, first position).  `err`: device int set to 2 when a
-// bounded wait ran out (may be null).
-static int attention_prefill_tcgen05_launch(const void* q, const void* k_pages, const void* v_pages, void* out,
-                                            const void* tiles, int n_tiles, const void* block_table, int table_width,
-                                            int page_size, int num_pages, int n_tokens, int H, int G, int hd, KeyMask mask,
-                                            float scale, int sink, const void* gate, int gate_ld, void* err, void* stream) {
-    MM_REQUIRE(hd == 128 || hd == 64, "attention_prefill_tcgen05: built for head sizes 64 and 128");
-    MM_REQUIRE(n_tiles >= 0 && H > 0 && G > 0 && H % G == 0 && n_tokens > 0 && num_pages > 0, "attention_prefill_tcgen05: bad sizes");
-    MM_REQUIRE(page_size >= 8 && page_size <= 128 && (128 % page_size) == 0, "attention_prefill_tcgen05: page_size must be 8, 16, 32, 64 or 128");
-    MM_REQUIRE(table_width > 0 && mask.window >= 0 && mask.chunk >= 0 && mask.keep >= 0, "attention_prefill_tcgen05: bad table or mask");
-    MM_REQUIRE(gate == nullptr || gate_ld >= H, "attention_prefill_tcgen05: one gate per head");
-    if (n_tiles == 0) return MM_OK;
+struct PrefillArgs {
+    const void *q, *k_pages, *v_pages, *tiles, *block_table, *gate, *sink_logit;
+    void *out, *err;
+    int n_tiles, table_width, page_size, num_pages, n_tokens, H, G, Gv, out_f32, sink, gate_ld;
+    KeyMask mask;
+    float scale, softcap;
+};
+
+template <int HDK, int HDV, bool CAP>
+static int attention_prefill_launch_as(const PrefillArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, cudaStream_t s) {
+    constexpr size_t smem = (size_t)(HDK / 64 + 4 + KV_STAGES * (HDK / 64 + HDV / 64)) * HALF_BYTES + sizeof(AttCtl);
+    if (cudaFuncSetAttribute(attention_prefill_tc_kernel<HDK, HDV, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        mm_set_last_error("attention_prefill_tcgen05: cannot reserve shared memory");
+        return MM_ERR_LAUNCH;
+    }
+    const float LOG2E = 1.4426950408889634f;
+    attention_prefill_tc_kernel<HDK, HDV, CAP><<<dim3(a.H, a.n_tiles), ATT_TC_THREADS, smem, s>>>(
+        tq, tk, tv, a.out, a.out_f32, (const int32_t*)a.tiles, (const int32_t*)a.block_table, a.table_width, a.page_size, a.H, a.G, a.Gv, a.mask,
+        (CAP ? a.softcap : a.scale) * LOG2E, CAP ? a.scale / a.softcap : 0.0f, a.sink, (const float*)a.sink_logit, (const float*)a.gate, a.gate_ld,
+        (int*)a.err);
+    MM_CHECK_LAUNCH();
+    return MM_OK;
+}
+
+// q: [n_tokens, H*dk] bf16; k_pages [num_pages, G, page_size, dk], v_pages [num_pages, Gv, page_size, dv] bf16 of one layer (dk and dv 64 or
+// 128; key head g reads value head g % Gv); out [n_tokens, H*dv], bf16 or fp32; tiles: int32 [n_tiles, 4] (request, first row,
+// rows <= 128, first position).  `err`: device int set to 2 when a bounded wait ran out (may be null).
+static int attention_prefill_tcgen05_launch(const PrefillArgs& a, int dk, int dv, void* stream) {
+    MM_REQUIRE((dk == 128 || dk == 64) && (dv == 128 || dv == 64), "attention_prefill_tcgen05: built for key and value sizes 64 and 128");
+    MM_REQUIRE(a.n_tiles >= 0 && a.H > 0 && a.G > 0 && a.H % a.G == 0 && a.n_tokens > 0 && a.num_pages > 0, "attention_prefill_tcgen05: bad sizes");
+    MM_REQUIRE(a.Gv > 0 && a.G % a.Gv == 0, "attention_prefill_tcgen05: the value heads are a divisor of the key heads");
+    MM_REQUIRE(a.page_size >= 8 && a.page_size <= 128 && (128 % a.page_size) == 0, "attention_prefill_tcgen05: page_size must be 8, 16, 32, 64 or 128");
+    MM_REQUIRE(a.table_width > 0 && a.mask.window >= 0 && a.mask.chunk >= 0 && a.mask.keep >= 0, "attention_prefill_tcgen05: bad table or mask");
+    MM_REQUIRE(a.gate == nullptr || a.gate_ld >= a.H, "attention_prefill_tcgen05: one gate per head");
+    if (a.n_tiles == 0) return MM_OK;
     CUtensorMap tq, tk, tv;
-    const long long pool_rows = (long long)num_pages * G * page_size;
-    if (!tc::make_map_bf16(&tq, q, n_tokens, H * hd, (long long)H * hd, 128) ||
-        !tc::make_map_bf16(&tk, k_pages, pool_rows, hd, hd, page_size) ||
-        !tc::make_map_bf16(&tv, v_pages, pool_rows, hd, hd, page_size)) {
+    const long long pages = (long long)a.num_pages * a.page_size;
+    if (!tc::make_map_bf16(&tq, a.q, a.n_tokens, a.H * dk, (long long)a.H * dk, 128) ||
+        !tc::make_map_bf16(&tk, a.k_pages, pages * a.G, dk, dk, a.page_size) ||
+        !tc::make_map_bf16(&tv, a.v_pages, pages * a.Gv, dv, dv, a.page_size)) {
         mm_set_last_error("attention_prefill_tcgen05: cuTensorMapEncodeTiled failed or is not available");
         return MM_ERR_DRIVER;
     }
-    const int halves = hd / 64;
-    const size_t smem = (size_t)(halves + 4 + 2 * KV_STAGES * halves) * HALF_BYTES + sizeof(AttCtl);
-    static bool configured[2] = {false, false};
-    if (!configured[halves - 1]) {
-        const cudaError_t e = hd == 128 ? cudaFuncSetAttribute(attention_prefill_tc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                                        : cudaFuncSetAttribute(attention_prefill_tc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) {
-            mm_set_last_error("attention_prefill_tcgen05: cannot reserve shared memory");
-            return MM_ERR_LAUNCH;
-        }
-        configured[halves - 1] = true;
-    }
-    const float LOG2E = 1.4426950408889634f;
-    MM_REQUIRE(n_tiles <= 65535, "attention_prefill_tcgen05: more than 65535 tiles in one launch");
-    dim3 grid(H, n_tiles);
-    if (hd == 128)
-        attention_prefill_tc_kernel<128><<<grid, ATT_TC_THREADS, smem, (cudaStream_t)stream>>>(
-            tq, tk, tv, (__nv_bfloat16*)out, (const int32_t*)tiles, (const int32_t*)block_table, table_width, page_size, H, G,
-            mask, scale * LOG2E, sink, (const float*)gate, gate_ld, (int*)err);
-    else
-        attention_prefill_tc_kernel<64><<<grid, ATT_TC_THREADS, smem, (cudaStream_t)stream>>>(
-            tq, tk, tv, (__nv_bfloat16*)out, (const int32_t*)tiles, (const int32_t*)block_table, table_width, page_size, H, G,
-            mask, scale * LOG2E, sink, (const float*)gate, gate_ld, (int*)err);
-    MM_CHECK_LAUNCH();
-    return MM_OK;
+    MM_REQUIRE(a.n_tiles <= 65535, "attention_prefill_tcgen05: more than 65535 tiles in one launch");
+    cudaStream_t s = (cudaStream_t)stream;
+#define PREFILL_AS(K, V)                                                     \
+    if (dk == K && dv == V)                                                  \
+        return a.softcap > 0.0f ? attention_prefill_launch_as<K, V, true>(a, tq, tk, tv, s) : attention_prefill_launch_as<K, V, false>(a, tq, tk, tv, s)
+    PREFILL_AS(128, 128);
+    PREFILL_AS(64, 64);
+    PREFILL_AS(128, 64);
+    PREFILL_AS(64, 128);
+#undef PREFILL_AS
+    return MM_ERR_UNSUPPORTED;
 }
 
 MM_EXPORT int mm_attention_prefill_tcgen05(const void* q, const void* k_pages, const void* v_pages, void* out,
                                            const void* tiles, int n_tiles, const void* block_table, int table_width,
                                            int page_size, int num_pages, int n_tokens, int H, int G, int hd, int window,
                                            float scale, void* err, void* stream) {
-    return attention_prefill_tcgen05_launch(q, k_pages, v_pages, out, tiles, n_tiles, block_table, table_width, page_size, num_pages,
-                                            n_tokens, H, G, hd, KeyMask{window, 0, 0}, scale, 0, nullptr, 0, err, stream);
+    const PrefillArgs a = {q, k_pages, v_pages, tiles, block_table, nullptr, nullptr, out, err, n_tiles, table_width, page_size, num_pages, n_tokens,
+                           H, G, G, 0, 0, 0, KeyMask{window, 0, 0}, scale, 0.0f};
+    return attention_prefill_tcgen05_launch(a, hd, hd, stream);
 }
 
-// The same with a softmax sink (one is added to every row's denominator; scale must be positive), any mask and a gate per head
-// (fp32 [n_tokens, gate_ld] or null).
+// The same with keys and values of different sizes, a softmax sink (one, or exp of a logit per head, fp32 [H], is added to every row's
+// denominator; scale must be positive), any mask, a gate per head (fp32 [n_tokens, gate_ld] or null), a cap on the scores (0: none),
+// value heads shared by key heads, and a result in fp32.
 MM_EXPORT int mm_attention_prefill_tcgen05_sink(const void* q, const void* k_pages, const void* v_pages, void* out,
                                                 const void* tiles, int n_tiles, const void* block_table, int table_width,
-                                                int page_size, int num_pages, int n_tokens, int H, int G, int hd, int window, int chunk,
-                                                int keep, float scale, int sink, const void* gate, int gate_ld, void* err, void* stream) {
-    MM_REQUIRE(scale > 0.0f, "attention_prefill_tcgen05: the scale must be positive");
-    return attention_prefill_tcgen05_launch(q, k_pages, v_pages, out, tiles, n_tiles, block_table, table_width, page_size, num_pages,
-                                            n_tokens, H, G, hd, KeyMask{window, chunk, keep}, scale, sink, gate, gate_ld, err, stream);
+                                                int page_size, int num_pages, int n_tokens, int H, int G, int Gv, int dk, int dv, int window,
+                                                int chunk, int keep, float scale, float softcap, int sink, const void* sink_logit,
+                                                const void* gate, int gate_ld, int out_f32, void* err, void* stream) {
+    MM_REQUIRE(scale > 0.0f && softcap >= 0.0f, "attention_prefill_tcgen05: the scale must be positive, the cap not negative");
+    const PrefillArgs a = {q, k_pages, v_pages, tiles, block_table, gate, sink_logit, out, err, n_tiles, table_width, page_size, num_pages, n_tokens,
+                           H, G, Gv, out_f32, sink, gate_ld, KeyMask{window, chunk, keep}, scale, softcap};
+    return attention_prefill_tcgen05_launch(a, dk, dv, stream);
 }

@@ -45,6 +45,38 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
+// tanh of a row's numbers in place.  Scores are mostly small against their cap: where no number of the warp exceeds 0.35 the odd
+// polynomial of the Taylor series up to y^11 (relative error below 4e-9) spares the special-function unit, which the softmax
+// keeps busy; else 1 - 2 / (1 + e^(2y)) (absolute error below 2e-7).
+template <int N>
+__device__ __forceinline__ void tanh_row(uint32_t (&x)[N], float scale) {
+    float tops[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const float y = __uint_as_float(x[i]) * scale;
+        x[i] = __float_as_uint(y);
+        tops[i & 3] = fmaxf(tops[i & 3], fabsf(y));
+    }
+    const float top = fmaxf(fmaxf(tops[0], tops[1]), fmaxf(tops[2], tops[3]));
+    if (__all_sync(0xffffffffu, top <= 0.35f)) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const float y = __uint_as_float(x[i]), z = y * y;
+            float p = fmaf(z, -1382.0f / 155925.0f, 62.0f / 2835.0f);
+            p = fmaf(z, p, -17.0f / 315.0f);
+            p = fmaf(z, p, 2.0f / 15.0f);
+            p = fmaf(z, p, -1.0f / 3.0f);
+            x[i] = __float_as_uint(fmaf(y * z, p, y));
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const float e = fast_exp2(__uint_as_float(x[i]) * 2.8853900817779268f);      // e^(2y)
+            x[i] = __float_as_uint(1.0f - __fdividef(2.0f, 1.0f + fminf(e, 1e30f)));
+        }
+    }
+}
+
 // Every lane has done its part (and its fences); one lane arrives for the warp.
 __device__ __forceinline__ void warp_arrive(uint32_t bar, int lane) {
     __syncwarp();
@@ -62,11 +94,11 @@ struct SoftmaxBars {
 // One thread's row of one tile of 128 keys, the group's tile number `u` (`first`: its first): S from tensor memory into `sreg`,
 // masked by position, O (O_COLS columns at o_addr) rescaled when the row's maximum has outgrown its reference by RESCALE_STEP,
 // P rounded to bf16 into p_tile (two halves of 64 keys, 128-byte swizzle), the row's sum added to l.  The row sees keys wlo .. pos and
-// the first `keep` ones.  False: a wait ran out.
-template <int O_COLS>
+// the first `keep` ones.  CAP: a score s becomes tanh(s cap_in) first (scale_log2 is then the cap's).  False: a wait ran out.
+template <int O_COLS, bool CAP = false>
 __device__ __forceinline__ bool softmax_tile(const SoftmaxBars& bars, volatile int* abort_flag, uint32_t s_addr, uint32_t o_addr, unsigned char* p_tile,
                                              uint32_t half_bytes, int row, int lane, bool row_valid, int pos, int wlo, int key0, uint32_t u, bool first,
-                                             float scale_log2, uint32_t (&sreg)[128], float& m_ref, float& l, int keep = 0) {
+                                             float scale_log2, uint32_t (&sreg)[128], float& m_ref, float& l, int keep = 0, float cap_in = 0.0f) {
     constexpr int BN = 128;
     if (!mbar_wait(bars.s_full, u & 1, abort_flag)) return false;
     tc_fence_after();
@@ -75,27 +107,30 @@ __device__ __forceinline__ bool softmax_tile(const SoftmaxBars& bars, volatile i
     tmem_ld_wait();
     tc_fence_before();
     warp_arrive(bars.s_free, lane);                // S of this tile is in registers
+    if constexpr (CAP) tanh_row(sreg, cap_in);
     // a tile every key of which this row sees needs no mask
     const bool interior = row_valid && key0 + BN - 1 <= pos && key0 >= wlo;
-    float mx = -INFINITY;
+    // (four chains each for the maximum and the sum: one would have every thread wait 128 times for its own last result)
+    float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
     if (interior) {
 #pragma unroll
-        for (int i = 0; i < BN; ++i) mx = fmaxf(mx, __uint_as_float(sreg[i]));
+        for (int i = 0; i < BN; ++i) top[i & 3] = fmaxf(top[i & 3], __uint_as_float(sreg[i]));
     } else if (key0 < keep) {                      // a tile with kept tokens (uniform over the CTA)
 #pragma unroll
         for (int i = 0; i < BN; ++i) {
             const int key = key0 + i;
             if (!(row_valid && key <= pos && (key >= wlo || key < keep))) sreg[i] = 0xff800000u;
-            mx = fmaxf(mx, __uint_as_float(sreg[i]));
+            top[i & 3] = fmaxf(top[i & 3], __uint_as_float(sreg[i]));
         }
     } else {
 #pragma unroll
         for (int i = 0; i < BN; ++i) {
             const int key = key0 + i;
             if (!(row_valid && key <= pos && key >= wlo)) sreg[i] = 0xff800000u;      // -inf
-            mx = fmaxf(mx, __uint_as_float(sreg[i]));
+            top[i & 3] = fmaxf(top[i & 3], __uint_as_float(sreg[i]));
         }
     }
+    const float mx = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
     // P V of the group's previous tile is done: its P buffer is free and its O is at rest until this tile's P is published
     if (!first && !mbar_wait(bars.pv_done, (u - 1) & 1, abort_flag)) return false;
     // Move the reference only when the maximum has outgrown it by RESCALE_STEP (or there was none).  O of a row without a
@@ -121,7 +156,7 @@ __device__ __forceinline__ bool softmax_tile(const SoftmaxBars& bars, volatile i
     const float use = (m_ref == -INFINITY) ? 0.0f : m_ref * scale_log2;
     // probabilities, rounded to bf16 as the tensor core will read them: the row of P is two halves of 64 keys, each 8 chunks
     // of 16 bytes, chunk index xor-ed with row % 8
-    float sum = 0.0f;
+    float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) {
         unsigned char* prow = p_tile + hf * half_bytes + row * 128;
@@ -132,13 +167,13 @@ __device__ __forceinline__ bool softmax_tile(const SoftmaxBars& bars, volatile i
             for (int i = 0; i < 4; ++i) {
                 const float p0 = fast_exp2(fmaf(__uint_as_float(sreg[hf * 64 + ch * 8 + 2 * i]), scale_log2, -use));
                 const float p1 = fast_exp2(fmaf(__uint_as_float(sreg[hf * 64 + ch * 8 + 2 * i + 1]), scale_log2, -use));
-                sum += p0 + p1;
+                sum[i] += p0 + p1;
                 packed[i] = pack_bf16x2(p0, p1);
             }
             *reinterpret_cast<uint4*>(prow + ((ch ^ (row & 7)) << 4)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
         }
     }
-    l += sum;
+    l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // P is read by the tensor core (async proxy)
     tc_fence_before();                                                // ... and O, if it was rescaled, is in tensor memory
     warp_arrive(bars.p_full, lane);

@@ -44,7 +44,7 @@ def _sink_lib():
         _lib.declare("mm_attention_sink_prefill_bf16", [P, P, P, P, P, I, P, I, I, I, I, I, I, I, I, I, F, I, P, P, I, F, I, P, I, I, P])
         _lib.declare("mm_attention_sink_decode_bf16", [P, P, P, P, P, P, I, P, I, P, P, P, I, I, I, I, I, I, I, I, I, F, I, P, P, I, F, I, P, I, I, P])
         _lib.declare("mm_attention_decode_tma_bf16_sink", [P, P, P, P, P, I, P, P, P, I, I, I, I, I, I, I, I, I, F, I, I, I, P, I, P, P])
-        _lib.declare("mm_attention_prefill_tcgen05_sink", [P, P, P, P, P, I, P, I, I, I, I, I, I, I, I, I, I, F, I, P, I, P, P])
+        _lib.declare("mm_attention_prefill_tcgen05_sink", [P, P, P, P, P, I, P, I, I, I, I, I, I, I, I, I, I, I, I, F, F, I, P, P, I, I, P, P])
         _sink_declared = True
     return _lib.load()
 
@@ -124,24 +124,25 @@ def paged_sink_attention(q, cache, out, ctx, num_heads: int, num_kv_heads: int, 
             and _sink_lib().mm_attention_sink_supported(key_dim, value_dim)):
         from .lib import check
         lib = _sink_lib()
-        # equal key and value sizes of 64 or 128: the tcgen05 prefill kernel of the plain attention, told of the sink
+        # key and value sizes of 64 or 128 without a distance bias: the tcgen05 prefill kernel of the plain attention, told of the rest
         from . import attention_bf16
-        # a learned sink or a distance bias: the mma.sync kernels take them, the tcgen05 and TMA kernels do not
+        # a learned sink, a distance bias, a cap, shared value heads or an fp32 result: the mma.sync kernels take them, the TMA decode kernel does not
         out_f32 = int(out.dtype == torch.float32)
         extended = sink_logit is not None or dist_bias is not None or softcap > 0 or value_heads != num_kv_heads or bool(out_f32)
         sink_ptr = sink_logit.data_ptr() if sink_logit is not None else None
         bias_ptr = dist_bias.data_ptr() if dist_bias is not None else None
         dist_max = dist_bias.shape[1] - 1 if dist_bias is not None else 0
         gate_ptr, gate_ld = ops.gate_args(gate, q.shape[0], num_heads)
-        tensor_memory = (USE_SINK_TCGEN05 and not extended and key_dim == value_dim
-                         and attention_bf16.tcgen05_prefill_usable(key_dim, cache.page_size))
+        tensor_memory = (USE_SINK_TCGEN05 and dist_bias is None and attention_bf16.tcgen05_prefill_usable(key_dim, cache.page_size)
+                         and attention_bf16.tcgen05_prefill_usable(value_dim, cache.page_size))
         tiles, n_tiles, items, n_items = sink_plan(ctx, q.shape[0], attention_bf16.TILE_ROWS_TC if tensor_memory else SINK_TILE_ROWS)
         stream = ops._stream()
         if n_tiles and tensor_memory:
             check(lib.mm_attention_prefill_tcgen05_sink(q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), out.data_ptr(), tiles.data_ptr(),
                                                         n_tiles, table.data_ptr(), table.shape[1], cache.page_size, k_pages.shape[0],
-                                                        q.shape[0], num_heads, num_kv_heads, key_dim, int(window), int(chunk), int(keep), float(scale),
-                                                        int(bool(sink)), gate_ptr, gate_ld, ops.tcgen05_error_flag(q.device).data_ptr(), stream),
+                                                        q.shape[0], num_heads, num_kv_heads, value_heads, key_dim, value_dim, int(window), int(chunk),
+                                                        int(keep), float(scale), float(softcap), int(bool(sink)), sink_ptr, gate_ptr, gate_ld, out_f32,
+                                                        ops.tcgen05_error_flag(q.device).data_ptr(), stream),
                   "attention_prefill_tcgen05_sink")
         elif n_tiles:
             check(lib.mm_attention_sink_prefill_bf16(q.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), out.data_ptr(), tiles.data_ptr(),
