@@ -1,0 +1,1000 @@
+// The matrix-state recurrence (csrc/linear_state.cu) over long portions as products of matrices, 64 tokens at a time.
+//
+// Within a chunk, with gamma_t the product of the decays up to token t and S the state before it ([dk, dv]),
+//
+//   o_t = gamma_t S^T q_t + sum_(s <= t) (gamma_t / gamma_s) (q_t . k_s) u_s,      S' = gamma_C S + sum_s (gamma_C / gamma_s) k_s u_s^T,
+//
+// where u = v without the delta rule.  With it, u = beta (v - g S^T k) is the solution of a unit triangular system,
+//
+//   (I + L) U = diag(beta) (V - diag(gamma) K S),      L[t, s] = beta_t (gamma_t / gamma_s) (k_t . k_s) for s < t,
+//
+// so with T = (I + L)^-1, W = T diag(beta gamma) K and U0 = T diag(beta) V it is U = U0 - W S: only that product and S' have to
+// wait for the chunk before.  The launches:
+//   plain:  lc_state (what each chunk adds), lc_carry over the chunks per number of the state, lc_output;
+//   delta:  lc_delta_prepare (T, W, U0 per chunk), lc_delta_carry (U and S', chunk after chunk), lc_output with u for v.
+// A token costs dk dv multiply-adds three to four times as in the token-by-token walk, but as tiles of 16 x 8 x 8 on the tensor
+// cores: every operand is split into two tf32 numbers (11 bits each, both rounded to nearest), the product is the sum of the
+// three larger of the four partial products, added up in 32 bits: 22 bits of every factor enter, and the error against 64 bits stays
+// that of the 32-bit walk (measured over random and correlated keys, see the tests).  mma.sync gives 92 TFLOP/s that way, the FMA
+// units, whose tiles are held up by shared-memory reads, 40 to 45.
+// Ratios of decays are exponentials of differences of the logarithms' sums, which are kept in 64 bits: quotients of products of
+// the decays themselves would underflow within a chunk (0.2 a token), differences of 32-bit sums lose what lies close together.
+#include "common.cuh"
+
+#include <type_traits>
+
+#define LC_C 64              // tokens per chunk
+#define LC_LD 136            // floats per row of a [tokens, 128] tile: rows 8 banks apart
+#define LC_LP 68             // floats per row of a [64, 64] tile that is read along its rows: rows 4 banks apart
+
+__device__ __forceinline__ void lc_cp16(void* smem, const void* gmem, bool in) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem);
+    const int bytes = in ? 16 : 0;               // 0: zeros
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gmem), "r"(bytes));
+}
+__device__ __forceinline__ void lc_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+template <int N>
+__device__ __forceinline__ void lc_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
+
+// rows [0, 64) x columns [0, COLS) of a matrix of `rows` x `cols` numbers (row stride ld) into shared memory, zeros beyond
+template <int COLS, int LD, int THREADS = 256>
+__device__ __forceinline__ void lc_load(float* s, const float* __restrict__ p, size_t ld, int rows, int cols) {
+    constexpr int Q = COLS / 4;
+#pragma unroll
+    for (int e = 0; e < 64 * Q / THREADS; ++e) {
+        const int idx = threadIdx.x + e * THREADS, r = idx / Q, c = (idx % Q) * 4;
+        const bool in = r < rows && c < cols;
+        lc_cp16(s + r * LD + c, p + (in ? (size_t)r * ld + c : 0), in);
+    }
+}
+
+// x = hi + lo + (less than 2^-22 of x): two tf32 numbers (the tensor core reads the upper 19 bits)
+struct LcSplit {
+    uint32_t hi, lo;
+};
+__device__ __forceinline__ LcSplit lc_split(float x) {
+    LcSplit r;
+    r.hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+    r.lo = __float_as_uint(x - __uint_as_float(r.hi)) + 0x1000u;
+    return r;
+}
+struct LcA {
+    LcSplit x[4];
+};
+struct LcB {
+    LcSplit x[2];
+};
+__device__ __forceinline__ void lc_mma(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void lc_mma_first(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
+}
+// acc[i][j] += A_i B_j for eight k.  The tensor core cuts its sums off instead of rounding them, so a long chain of them drifts (1e-6 over
+// 128 k).  Eight k are added up there, from zero and the small terms first; the accumulators are added to by the FMA units, which
+// round to nearest.  The three steps go over all tiles in turn: one tile's next step would wait for its last.
+template <int NI, int NJ>
+__device__ __forceinline__ void lc_products(float (*acc)[NJ][4], const LcA* a, const LcB* b) {
+    float t[NI][NJ][4];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int i = 0; i < NI; ++i) lc_mma_first(t[i][j], a[i].x[0].lo, a[i].x[1].lo, a[i].x[2].lo, a[i].x[3].lo, b[j].x[0].hi, b[j].x[1].hi);
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int i = 0; i < NI; ++i) lc_mma(t[i][j], a[i].x[0].hi, a[i].x[1].hi, a[i].x[2].hi, a[i].x[3].hi, b[j].x[0].lo, b[j].x[1].lo);
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int i = 0; i < NI; ++i) lc_mma(t[i][j], a[i].x[0].hi, a[i].x[1].hi, a[i].x[2].hi, a[i].x[3].hi, b[j].x[0].hi, b[j].x[1].hi);
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) acc[i][j][x] += t[i][j][x];
+}
+// Fragments of eight k.  "rows": the operand stands as [m or n][k]; a thread takes k 2t and 2t + 1 for its two places (any order
+// of k will do, as long as both operands have the same), as one 8-byte word.  "rows4": the same in the order t, t + 4, for a
+// product whose other operand stands as [k][n].  "cols": the operand stands as [k][m or n], order t, t + 4.
+__device__ __forceinline__ LcA lc_a_rows(const float* p, int ld) {
+    const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    const float2 x = *reinterpret_cast<const float2*>(p + g * ld + 2 * t), y = *reinterpret_cast<const float2*>(p + (g + 8) * ld + 2 * t);
+    return LcA{{lc_split(x.x), lc_split(y.x), lc_split(x.y), lc_split(y.y)}};
+}
+// "rows" with a factor per k: scale points at the first of the eight
+__device__ __forceinline__ LcA lc_a_rows_scaled(const float* p, int ld, const float* scale) {
+    const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    const float2 x = *reinterpret_cast<const float2*>(p + g * ld + 2 * t), y = *reinterpret_cast<const float2*>(p + (g + 8) * ld + 2 * t);
+    const float2 f = *reinterpret_cast<const float2*>(scale + 2 * t);
+    return LcA{{lc_split(x.x * f.x), lc_split(y.x * f.x), lc_split(x.y * f.y), lc_split(y.y * f.y)}};
+}
+__device__ __forceinline__ LcB lc_b_rows(const float* p, int ld) {
+    const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    const float2 x = *reinterpret_cast<const float2*>(p + g * ld + 2 * t);
+    return LcB{{lc_split(x.x), lc_split(x.y)}};
+}
+// s0, s1: factors of the numbers at k = t and k = t + 4
+__device__ __forceinline__ LcA lc_a_rows4(const float* p, int ld, float s0, float s1) {
+    const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    return LcA{{lc_split(p[g * ld + t] * s0), lc_split(p[(g + 8) * ld + t] * s0), lc_split(p[g * ld + t + 4] * s1),
+                lc_split(p[(g + 8) * ld + t + 4] * s1)}};
+}
+__device__ __forceinline__ LcA lc_a_cols(const float* p, int ld, float s0, float s1) {
+    const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    return LcA{{lc_split(p[t * ld + g] * s0), lc_split(p[t * ld + g + 8] * s0), lc_split(p[(t + 4) * ld + g] * s1),
+                lc_split(p[(t + 4) * ld + g + 8] * s1)}};
+}
+__device__ __forceinline__ LcB lc_b_cols(const float* p, int ld) {
+    const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    return LcB{{lc_split(p[t * ld + g]), lc_split(p[(t + 4) * ld + g])}};
+}
+
+// The sums of the decays' logarithms over the chunk's tokens, sb[t] = log gamma_t, by the first two warps; tokens beyond the
+// chunk add nothing.  A decay of 0 counts as exp(-200), which no 32-bit number can tell from it.
+__device__ __forceinline__ void lc_decays(const float* __restrict__ gate, const float* __restrict__ head_decay, int t0, int cnt, int H, int h,
+                                          double* sb) {
+    __shared__ double first_half;
+    double x = 0.0;
+    const int t = threadIdx.x, lane = t & 31;
+    if (t < LC_C) {
+        if (t < cnt) x = (double)fmaxf(logf(gate ? gate[(size_t)(t0 + t) * H + h] : head_decay[h]), -200.0f);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double up = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += up;
+        }
+        if (t == 31) first_half = x;
+    }
+    __syncthreads();
+    if (t < LC_C) sb[t] = t >= 32 ? x + first_half : x;
+    __syncthreads();
+}
+__device__ __forceinline__ float lc_exp(double x) { return expf((float)x); }
+
+struct LcArgs {
+    const float *q, *k, *v, *gate, *beta, *head_decay;
+    int ldq, ldk, ldv;
+    float *out, *state;
+    long long state_stride;
+    const int32_t *chunk_meta, *req_chunks, *slots, *positions;
+    int n_chunks, H, G, dk, dv;
+    float *states;       // [chunks, H, dv, dk]: what a chunk adds, then what it starts from
+    float *gain;         // [chunks, H]: gamma_C
+    float *ratio;        // [chunks, H, 64]: gamma_C / gamma_t (delta rule)
+    float *w, *u;        // [tokens, H dk], [tokens, H dv] (delta rule)
+};
+
+// V^T diag(sr) K of a chunk, [dv, dk], to its place in `states`; k and v stand in shared memory.
+template <int DK, int DV>
+__device__ __forceinline__ void lc_add_up(const LcArgs& a, int h, int c, const float* sk, const float* sv, const float* sr) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int WM = DV / 32, WN = 8 / WM, NT = DK / WN / 8;      // warps along dv (32 rows each) and dk; tiles of 8 columns per warp
+    const int m0 = (warp % WM) * 32, n0 = (warp / WM) * (DK / WN);
+    float acc[NT / 2][2][2][4];                  // [pair of column tiles][16 rows][column tile]
+#pragma unroll
+    for (int x = 0; x < NT * 8; ++x) (&acc[0][0][0][0])[x] = 0.0f;
+    const int t = lane & 3, g = lane >> 2;
+#pragma unroll 2
+    for (int k0 = 0; k0 < LC_C; k0 += 8) {
+        const float s0 = sr[k0 + t], s1 = sr[k0 + t + 4];
+        LcA fa[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) fa[i] = lc_a_cols(sv + k0 * LC_LD + m0 + 16 * i, LC_LD, s0, s1);
+#pragma unroll
+        for (int j = 0; j < NT / 2; ++j) {
+            const float* p = sk + k0 * LC_LD + n0 + 16 * j;
+            const LcB fb[2] = {lc_b_cols(p, LC_LD), lc_b_cols(p + 8, LC_LD)};
+            lc_products<2, 2>(acc[j], fa, fb);
+        }
+    }
+    float* o = a.states + ((size_t)c * a.H + h) * a.dv * a.dk;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+            const int n = n0 + 8 * j + 2 * t;
+            if (n >= a.dk) continue;
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int m = m0 + 16 * i + g + 8 * half;
+                if (m < a.dv) *reinterpret_cast<float2*>(o + (size_t)m * a.dk + n) = make_float2(acc[j >> 1][i][j & 1][2 * half], acc[j >> 1][i][j & 1][2 * half + 1]);
+            }
+        }
+}
+
+// ---- what a chunk adds to the state, as [dv, dk]: V^T diag(gamma_C / gamma) K -------------------------------------------------
+// Bound by the tensor cores and, with 64 KB of result per 64 tokens and head, by writing it.
+template <int DK, int DV>
+__global__ void __launch_bounds__(256, 2) lc_state_kernel(LcArgs a) {
+    extern __shared__ __align__(16) float lc_smem[];
+    float* sk = lc_smem;                         // [64][LC_LD]
+    float* sv = sk + LC_C * LC_LD;               // [64][LC_LD]
+    __shared__ double sb[LC_C];
+    __shared__ float sr[LC_C];
+    const int h = blockIdx.x, c = blockIdx.y;
+    const int t0 = a.chunk_meta[4 * c], cnt = a.chunk_meta[4 * c + 1];
+    const int kh = h / (a.H / a.G);
+    lc_load<DK, LC_LD>(sk, a.k + (size_t)t0 * a.ldk + (size_t)kh * a.dk, a.ldk, cnt, a.dk);
+    lc_load<DV, LC_LD>(sv, a.v + (size_t)t0 * a.ldv + (size_t)h * a.dv, a.ldv, cnt, a.dv);
+    lc_commit();
+    lc_decays(a.gate, a.head_decay, t0, cnt, a.H, h, sb);
+    if (threadIdx.x < LC_C) sr[threadIdx.x] = lc_exp(sb[LC_C - 1] - sb[threadIdx.x]);
+    if (threadIdx.x == 0) a.gain[(size_t)c * a.H + h] = lc_exp(sb[LC_C - 1]);
+    lc_wait<0>();
+    __syncthreads();
+    lc_add_up<DK, DV>(a, h, c, sk, sv, sr);
+}
+
+// The carry over the chunks, a thread per number of the state: gain [chunks, H], or with a factor per key channel [chunks, H, dk].
+template <bool CHANNEL>
+__global__ void __launch_bounds__(256) lc_carry_kernel(LcArgs a) {
+    const long long size = (long long)a.H * a.dv * a.dk, i = (long long)blockIdx.x * 256 + threadIdx.x;
+    const int r = blockIdx.y;
+    if (i >= size) return;
+    const int h = (int)(i / (a.dv * a.dk)), first = a.req_chunks[2 * r], count = a.req_chunks[2 * r + 1];
+    if (count <= 0) return;
+    float* __restrict__ states = a.states + i;
+    const float* __restrict__ gain = a.gain + (CHANNEL ? (size_t)h * a.dk + i % a.dk : (size_t)h);
+    const size_t step = CHANNEL ? (size_t)a.H * a.dk : (size_t)a.H;
+    float* st = a.state + (size_t)a.slots[r] * a.state_stride + i;
+    float S = a.positions[a.chunk_meta[4 * first]] == 0 ? 0.0f : *st;
+    for (int c0 = first; c0 < first + count; c0 += 8) {          // eight chunks' loads in flight: they do not depend on the carried value
+        float add[8], gn[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const bool in = c0 + j < first + count;
+            add[j] = in ? states[(size_t)(c0 + j) * size] : 0.0f;
+            gn[j] = in ? gain[(size_t)(c0 + j) * step] : 1.0f;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (c0 + j < first + count) {
+                states[(size_t)(c0 + j) * size] = S;
+                S = fmaf(gn[j], S, add[j]);
+            }
+        }
+    }
+    *st = S;
+}
+
+// ---- the outputs of a chunk: diag(gamma) Q S + (Q K^T, decayed and masked) U --------------------------------------------------
+// Two blocks per SM (104 KB each): q, and two buffers through which half of S, the other half, k (then the decayed scores) and u
+// pass, each on its way while the one before it is multiplied.  Bound by the tensor cores.
+template <int DK, int DV>
+__global__ void __launch_bounds__(256, 2) lc_output_kernel(LcArgs a, const float* __restrict__ values, size_t ldu) {
+    extern __shared__ __align__(16) float lc_smem[];
+    float* sq = lc_smem;                         // [64][LC_LD]
+    float* sa = sq + LC_C * LC_LD;               // S's first 64 rows (of dv), then k, then the scores [64][LC_LP]
+    float* su = sa + LC_C * LC_LD;               // S's other rows, then u
+    __shared__ double sb[LC_C];
+    const int h = blockIdx.x, c = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t0 = a.chunk_meta[4 * c], cnt = a.chunk_meta[4 * c + 1];
+    const int kh = h / (a.H / a.G);
+    const float* S = a.states + ((size_t)c * a.H + h) * a.dv * a.dk;
+    const float* up = values + (size_t)t0 * ldu + (size_t)h * a.dv;
+    lc_load<DK, LC_LD>(sq, a.q + (size_t)t0 * a.ldq + (size_t)kh * a.dk, a.ldq, cnt, a.dk);
+    lc_load<DK, LC_LD>(sa, S, a.dk, min(64, a.dv), a.dk);
+    lc_commit();
+    if (DV > 64) lc_load<DK, LC_LD>(su, a.dv > 64 ? S + (size_t)64 * a.dk : S, a.dk, a.dv - 64, a.dk);
+    else lc_load<DV, LC_LD>(su, up, ldu, cnt, a.dv);
+    lc_commit();
+    lc_decays(a.gate, a.head_decay, t0, cnt, a.H, h, sb);
+    const int m0 = (warp & 1) * 32, wn = warp >> 1, t = lane & 3, g = lane >> 2;
+    constexpr int HALVES = DV / 64;
+    float acc[HALVES][2][2][4];                  // [half of dv][16 rows][8 columns]
+#pragma unroll
+    for (int x = 0; x < HALVES * 16; ++x) (&acc[0][0][0][0])[x] = 0.0f;
+    auto times_state = [&](const float* s, float (*o)[2][4]) {
+#pragma unroll 2
+        for (int k0 = 0; k0 < DK; k0 += 8) {
+            LcA fa[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows(sq + (m0 + 16 * i) * LC_LD + k0, LC_LD);
+            const LcB fb[2] = {lc_b_rows(s + wn * 16 * LC_LD + k0, LC_LD), lc_b_rows(s + (wn * 16 + 8) * LC_LD + k0, LC_LD)};
+            lc_products<2, 2>(o, fa, fb);
+        }
+    };
+    lc_wait<1>();
+    __syncthreads();
+    times_state(sa, acc[0]);
+    __syncthreads();
+    lc_load<DK, LC_LD>(sa, a.k + (size_t)t0 * a.ldk + (size_t)kh * a.dk, a.ldk, cnt, a.dk);
+    lc_commit();
+    if (DV > 64) {
+        lc_wait<1>();
+        __syncthreads();
+        times_state(su, acc[HALVES - 1]);
+        __syncthreads();
+        lc_load<DV, LC_LD>(su, up, ldu, cnt, a.dv);
+        lc_commit();
+        lc_wait<1>();
+    } else {
+        lc_wait<0>();
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const float g0 = lc_exp(sb[m0 + 16 * i + g]), g1 = lc_exp(sb[m0 + 16 * i + g + 8]);
+#pragma unroll
+        for (int b = 0; b < HALVES; ++b)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                acc[b][i][j][0] *= g0;
+                acc[b][i][j][1] *= g0;
+                acc[b][i][j][2] *= g1;
+                acc[b][i][j][3] *= g1;
+            }
+    }
+    {   // scores of the rows m0.. and keys 16 wn..: nothing to do above the diagonal
+        float s[2][2][4];
+#pragma unroll
+        for (int x = 0; x < 16; ++x) (&s[0][0][0])[x] = 0.0f;
+        if (wn * 16 <= m0 + 31) {
+#pragma unroll 2
+            for (int k0 = 0; k0 < DK; k0 += 8) {
+                LcA fa[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows(sq + (m0 + 16 * i) * LC_LD + k0, LC_LD);
+                const LcB fb[2] = {lc_b_rows(sa + wn * 16 * LC_LD + k0, LC_LD), lc_b_rows(sa + (wn * 16 + 8) * LC_LD + k0, LC_LD)};
+                lc_products<2, 2>(s, fa, fb);
+            }
+        }
+        __syncthreads();                         // every warp is through with k
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    const int m = m0 + 16 * i + g + 8 * (x >> 1), n = wn * 16 + 8 * j + 2 * t + (x & 1);
+                    sa[m * LC_LP + n] = n <= m ? s[i][j][x] * lc_exp(sb[m] - sb[n]) : 0.0f;
+                }
+    }
+    lc_wait<0>();
+    __syncthreads();
+    for (int k0 = 0; k0 < m0 + 32; k0 += 8) {
+        LcA fa[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows4(sa + (m0 + 16 * i) * LC_LP + k0, LC_LP, 1.0f, 1.0f);
+#pragma unroll
+        for (int b = 0; b < HALVES; ++b) {
+            const float* p = su + k0 * LC_LD + 64 * b + wn * 16;
+            const LcB fb[2] = {lc_b_cols(p, LC_LD), lc_b_cols(p + 8, LC_LD)};
+            lc_products<2, 2>(acc[b], fa, fb);
+        }
+    }
+#pragma unroll
+    for (int b = 0; b < HALVES; ++b)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int n = 64 * b + wn * 16 + 8 * j + 2 * t;
+                if (n >= a.dv) continue;
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int m = m0 + 16 * i + g + 8 * half;
+                    if (m < cnt)
+                        *reinterpret_cast<float2*>(a.out + ((size_t)(t0 + m) * a.H + h) * a.dv + n) =
+                            make_float2(acc[b][i][j][2 * half], acc[b][i][j][2 * half + 1]);
+                }
+            }
+}
+
+// ---- the delta rule ---------------------------------------------------------------------------------------------------------
+// T = (I + L)^-1 by blocks: the four 16 x 16 blocks on the diagonal by substitution, a column per thread; then twice the inverse of a
+// matrix of two by two blocks, [A 0; B D]^-1 = [A^-1 0; -D^-1 B A^-1, D^-1].  The part of T above its diagonal blocks is scratch.
+__device__ __forceinline__ void lc_invert(const float* __restrict__ L, float* __restrict__ T) {
+    const int tid = threadIdx.x;
+    if (tid < 64) {
+        const int b = (tid >> 4) * 16, j = tid & 15;
+        float x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            float s = i == j ? 1.0f : 0.0f;
+#pragma unroll
+            for (int p = 0; p < i; ++p) s = fmaf(-L[(b + i) * LC_LP + b + p], x[p], s);
+            x[i] = s;
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) T[(b + i) * LC_LP + b + j] = x[i];
+    }
+    __syncthreads();
+    // pairs of 16: blocks (1, 0) and (3, 2); the product in between goes to blocks (0, 1) and (2, 3)
+    const int b16 = (tid >> 7) * 32, r16 = (tid & 127) >> 3, c16 = (tid & 7) * 2;
+    {
+        float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll
+        for (int p = 0; p < 16; ++p) {
+            const float x = L[(b16 + 16 + r16) * LC_LP + b16 + p];
+            s0 = fmaf(x, T[(b16 + p) * LC_LP + b16 + c16], s0);
+            s1 = fmaf(x, T[(b16 + p) * LC_LP + b16 + c16 + 1], s1);
+        }
+        T[(b16 + r16) * LC_LP + b16 + 16 + c16] = s0;
+        T[(b16 + r16) * LC_LP + b16 + 16 + c16 + 1] = s1;
+    }
+    __syncthreads();
+    {
+        float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll
+        for (int p = 0; p < 16; ++p) {
+            const float x = T[(b16 + 16 + r16) * LC_LP + b16 + 16 + p];
+            s0 = fmaf(-x, T[(b16 + p) * LC_LP + b16 + 16 + c16], s0);
+            s1 = fmaf(-x, T[(b16 + p) * LC_LP + b16 + 16 + c16 + 1], s1);
+        }
+        T[(b16 + 16 + r16) * LC_LP + b16 + c16] = s0;
+        T[(b16 + 16 + r16) * LC_LP + b16 + c16 + 1] = s1;
+    }
+    __syncthreads();
+    // the pair of 32: T[32.., 0..] = -T[32.., 32..] L[32.., 0..] T[0.., 0..]; both triangles' upper blocks are scratch by now and count as zero
+    const int r = tid >> 3, c = (tid & 7) * 4;
+    {
+        float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        const int from = c & 16;                 // T[0..32, 0..32] is zero above its diagonal blocks
+        for (int p = from; p < 32; ++p) {
+            const float x = L[(32 + r) * LC_LP + p];
+            const float4 y = *reinterpret_cast<const float4*>(T + p * LC_LP + c);
+            s[0] = fmaf(x, y.x, s[0]);
+            s[1] = fmaf(x, y.y, s[1]);
+            s[2] = fmaf(x, y.z, s[2]);
+            s[3] = fmaf(x, y.w, s[3]);
+        }
+        *reinterpret_cast<float4*>(T + r * LC_LP + 32 + c) = make_float4(s[0], s[1], s[2], s[3]);
+    }
+    __syncthreads();
+    {
+        float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        const int to = (r & 16) + 16;
+        for (int p = 0; p < to; ++p) {
+            const float x = T[(32 + r) * LC_LP + 32 + p];
+            const float4 y = *reinterpret_cast<const float4*>(T + p * LC_LP + 32 + c);
+            s[0] = fmaf(-x, y.x, s[0]);
+            s[1] = fmaf(-x, y.y, s[1]);
+            s[2] = fmaf(-x, y.z, s[2]);
+            s[3] = fmaf(-x, y.w, s[3]);
+        }
+        *reinterpret_cast<float4*>(T + (32 + r) * LC_LP + c) = make_float4(s[0], s[1], s[2], s[3]);
+    }
+    __syncthreads();
+}
+
+// W = T diag(beta gamma) K, U0 = T diag(beta) V of a chunk, and the decays that the carry needs.  Bound by the tensor cores.
+template <int DK, int DV>
+__global__ void __launch_bounds__(256, 2) lc_delta_prepare_kernel(LcArgs a) {
+    extern __shared__ __align__(16) float lc_smem[];
+    float* sk = lc_smem;                         // [64][LC_LD]
+    float* sv = sk + LC_C * LC_LD;               // [64][LC_LD]
+    float* sL = sv + LC_C * LC_LD;               // [64][LC_LP]
+    float* sT = sL + LC_C * LC_LP;               // [64][LC_LP]
+    __shared__ double sb[LC_C];
+    __shared__ float sbeta[LC_C], sbg[LC_C];
+    const int h = blockIdx.x, c = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t0 = a.chunk_meta[4 * c], cnt = a.chunk_meta[4 * c + 1];
+    const int kh = h / (a.H / a.G);
+    lc_load<DK, LC_LD>(sk, a.k + (size_t)t0 * a.ldk + (size_t)kh * a.dk, a.ldk, cnt, a.dk);
+    lc_commit();
+    lc_load<DV, LC_LD>(sv, a.v + (size_t)t0 * a.ldv + (size_t)h * a.dv, a.ldv, cnt, a.dv);
+    lc_commit();
+    lc_decays(a.gate, a.head_decay, t0, cnt, a.H, h, sb);
+    if (threadIdx.x < LC_C) {
+        const int t = threadIdx.x;
+        const float b = t < cnt ? a.beta[(size_t)(t0 + t) * a.H + h] : 0.0f;
+        sbeta[t] = b;
+        sbg[t] = b * lc_exp(sb[t]);
+        a.ratio[((size_t)c * a.H + h) * LC_C + t] = lc_exp(sb[LC_C - 1] - sb[t]);
+        if (t == 0) a.gain[(size_t)c * a.H + h] = lc_exp(sb[LC_C - 1]);
+    }
+    const int m0 = (warp & 1) * 32, wn = warp >> 1, t = lane & 3, g = lane >> 2;
+    lc_wait<1>();
+    __syncthreads();
+    {
+        float s[2][2][4];
+#pragma unroll
+        for (int x = 0; x < 16; ++x) (&s[0][0][0])[x] = 0.0f;
+        if (wn * 16 <= m0 + 31) {
+#pragma unroll 2
+            for (int k0 = 0; k0 < DK; k0 += 8) {
+                LcA fa[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows(sk + (m0 + 16 * i) * LC_LD + k0, LC_LD);
+                const LcB fb[2] = {lc_b_rows(sk + wn * 16 * LC_LD + k0, LC_LD), lc_b_rows(sk + (wn * 16 + 8) * LC_LD + k0, LC_LD)};
+                lc_products<2, 2>(s, fa, fb);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    const int m = m0 + 16 * i + g + 8 * (x >> 1), n = wn * 16 + 8 * j + 2 * t + (x & 1);
+                    sL[m * LC_LP + n] = n < m ? s[i][j][x] * sbeta[m] * lc_exp(sb[m] - sb[n]) : 0.0f;
+                }
+    }
+    lc_wait<0>();
+    __syncthreads();
+    lc_invert(sL, sT);
+    // both products: rows m0 + 16 i (32 per warp pair), columns wn * (COLS / 4)..; T has nothing to the right of its diagonal blocks
+    auto product = [&](const float* s, const float* scale, int cols, int width, float* o, size_t ld, auto tiles) {
+        constexpr int NT = decltype(tiles)::value;
+        float acc[NT / 2][2][2][4];
+#pragma unroll
+        for (int x = 0; x < NT * 8; ++x) (&acc[0][0][0][0])[x] = 0.0f;
+        for (int k0 = 0; k0 < m0 + 32; k0 += 8) {
+            const float s0 = scale[k0 + t], s1 = scale[k0 + t + 4];
+            LcA fa[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const bool right = k0 >= m0 + 16 * i + 16;       // scratch: counts as zero
+                fa[i] = right ? LcA{} : lc_a_rows4(sT + (m0 + 16 * i) * LC_LP + k0, LC_LP, s0, s1);
+            }
+#pragma unroll
+            for (int j = 0; j < NT / 2; ++j) {
+                const float* p = s + k0 * LC_LD + wn * width + 16 * j;
+                const LcB fb[2] = {lc_b_cols(p, LC_LD), lc_b_cols(p + 8, LC_LD)};
+                lc_products<2, 2>(acc[j], fa, fb);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+                const int n = wn * width + 8 * j + 2 * t;
+                if (n >= cols) continue;
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int m = m0 + 16 * i + g + 8 * half;
+                    if (m < cnt) *reinterpret_cast<float2*>(o + (size_t)m * ld + n) = make_float2(acc[j >> 1][i][j & 1][2 * half], acc[j >> 1][i][j & 1][2 * half + 1]);
+                }
+            }
+    };
+    product(sk, sbg, a.dk, DK / 4, a.w + ((size_t)t0 * a.H + h) * a.dk, (size_t)a.H * a.dk, std::integral_constant<int, DK / 32>{});
+    product(sv, sbeta, a.dv, DV / 4, a.u + ((size_t)t0 * a.H + h) * a.dv, (size_t)a.H * a.dv, std::integral_constant<int, DV / 32>{});
+}
+
+// U = U0 - W S and S' = gamma_C S + K^T diag(gamma_C / gamma) U, chunk after chunk, for NS columns of one head's S per block.
+// Bound by the chain of the two products and three barriers a chunk, so 16 warps share each product: in the first, warp w and w + 8 have one
+// tile of U and half of the key channels each (their halves meet when U is read), in the second a warp has 16 rows of dk and
+// half of the columns.  S stands in the accumulators and, for the first product, in shared memory; the next chunk's W, k and U0 arrive
+// under the current one's products.
+#define LC_CARRY_THREADS 512
+template <int DK, int NS>
+__global__ void __launch_bounds__(LC_CARRY_THREADS) lc_delta_carry_kernel(LcArgs a) {
+    constexpr int LU = NS + 8, TILE = 2 * LC_C * LC_LD + LC_C * LU + LC_C + 4, NT = NS / 16;      // column tiles of a warp
+    extern __shared__ __align__(16) float lc_smem[];
+    float* sS = lc_smem + 2 * TILE;              // [NS][LC_LD]
+    float* sp = sS + NS * LC_LD;                 // [64][LU]: the second half's part of W S
+    const int h = blockIdx.y, r = blockIdx.z, n_base = blockIdx.x * NS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t = lane & 3, g = lane >> 2, kh = h / (a.H / a.G), side = warp >> 3;
+    const int first = a.req_chunks[2 * r], count = a.req_chunks[2 * r + 1];
+    if (count <= 0) return;
+    const int cols = min(NS, a.dv - n_base);
+    auto fill = [&](int i) {
+        const int c = first + i, t0 = a.chunk_meta[4 * c], cnt = a.chunk_meta[4 * c + 1];
+        float* sw = lc_smem + (i & 1) * TILE;
+        float* sk = sw + LC_C * LC_LD;
+        float* su = sk + LC_C * LC_LD;
+        float* sr = su + LC_C * LU;
+        lc_load<DK, LC_LD, LC_CARRY_THREADS>(sw, a.w + ((size_t)t0 * a.H + h) * a.dk, (size_t)a.H * a.dk, cnt, a.dk);
+        lc_load<DK, LC_LD, LC_CARRY_THREADS>(sk, a.k + (size_t)t0 * a.ldk + (size_t)kh * a.dk, a.ldk, cnt, a.dk);
+        for (int idx = threadIdx.x; idx < LC_C * (NS / 4); idx += LC_CARRY_THREADS) {
+            const int row = idx / (NS / 4), col = (idx % (NS / 4)) * 4;
+            const bool in = row < cnt && col < cols;
+            lc_cp16(su + row * LU + col, a.u + (in ? ((size_t)(t0 + row) * a.H + h) * a.dv + n_base + col : 0), in);
+        }
+        if (threadIdx.x < LC_C / 4) lc_cp16(sr + 4 * threadIdx.x, a.ratio + ((size_t)c * a.H + h) * LC_C + 4 * threadIdx.x, true);
+        lc_commit();
+    };
+    // the warp's part of S: rows 16 (warp % 8).. of dk (if there are so many), columns 8 side + 16 j..
+    const int s_row = (warp & 7) * 16;
+    const bool has_rows = s_row < DK;
+    float S[NT][4];
+    {
+        const bool fresh = a.positions[a.chunk_meta[4 * first]] == 0;
+        const float* st = a.state + (size_t)a.slots[r] * a.state_stride + (size_t)h * a.dv * a.dk;
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const int m = s_row + g + 8 * (x >> 1), n = n_base + 8 * side + 16 * j + 2 * t + (x & 1);
+                S[j][x] = (!fresh && has_rows && m < a.dk && n < a.dv) ? st[(size_t)n * a.dk + m] : 0.0f;
+            }
+    }
+    auto publish = [&](float* __restrict__ to, bool local) {     // S to global memory and, if another chunk follows, to shared memory
+        if (!has_rows) return;
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const int m = s_row + g + 8 * (x >> 1), n = 8 * side + 16 * j + 2 * t + (x & 1);
+                if (local) sS[n * LC_LD + m] = S[j][x];
+                if (m < a.dk && n_base + n < a.dv) to[(size_t)(n_base + n) * a.dk + m] = S[j][x];
+            }
+    };
+    fill(0);
+    publish(a.states + ((size_t)first * a.H + h) * a.dv * a.dk, true);
+    for (int i = 0; i < count; ++i) {
+        const int c = first + i, t0 = a.chunk_meta[4 * c], cnt = a.chunk_meta[4 * c + 1];
+        const float gain = a.gain[(size_t)c * a.H + h];
+        if (i + 1 < count) {
+            fill(i + 1);
+            lc_wait<1>();
+        } else {
+            lc_wait<0>();
+        }
+        __syncthreads();                         // this chunk's tiles and S
+        const float* sw = lc_smem + (i & 1) * TILE;
+        const float* sk = sw + LC_C * LC_LD;
+        float* su = const_cast<float*>(sk) + LC_C * LC_LD;
+        const float* sr = su + LC_C * LU;
+        {   // rows 16 (warp % 4) of the chunk, columns 8 (warp / 4 % 2) + 16 j, channels DK / 2 side..
+            const int m0 = (warp & 3) * 16, n0 = ((warp >> 2) & 1) * 8;
+            float p[1][NT][4];
+#pragma unroll
+            for (int x = 0; x < NT * 4; ++x) (&p[0][0][0])[x] = 0.0f;
+#pragma unroll
+            for (int k = 0; k < DK / 2; k += 8) {
+                const int k0 = side * (DK / 2) + k;
+                const LcA fa = lc_a_rows(sw + m0 * LC_LD + k0, LC_LD);
+                LcB fb[NT];
+#pragma unroll
+                for (int j = 0; j < NT; ++j) fb[j] = lc_b_rows(sS + (n0 + 16 * j) * LC_LD + k0, LC_LD);
+                lc_products<1, NT>(p, &fa, fb);
+            }
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    const int at = (m0 + g + 8 * (x >> 1)) * LU + n0 + 16 * j + 2 * t + (x & 1);
+                    if (side == 0) su[at] -= p[0][j][x];
+                    else sp[at] = p[0][j][x];
+                }
+        }
+        __syncthreads();
+        if (has_rows) {
+            float p[1][NT][4];
+#pragma unroll
+            for (int x = 0; x < NT * 4; ++x) (&p[0][0][0])[x] = 0.0f;
+#pragma unroll
+            for (int k0 = 0; k0 < LC_C; k0 += 8) {
+                const LcA fa = lc_a_cols(sk + k0 * LC_LD + s_row, LC_LD, sr[k0 + t], sr[k0 + t + 4]);
+                LcB fb[NT];
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    const int at = (k0 + t) * LU + 8 * side + 16 * j + g;
+                    fb[j] = LcB{{lc_split(su[at] - sp[at]), lc_split(su[at + 4 * LU] - sp[at + 4 * LU])}};
+                }
+                lc_products<1, NT>(p, &fa, fb);
+            }
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) S[j][x] = fmaf(gain, S[j][x], p[0][j][x]);
+        }
+        for (int idx = threadIdx.x; idx < LC_C * NS; idx += LC_CARRY_THREADS) {
+            const int m = idx / NS, n = idx % NS;
+            if (m < cnt && n < cols) a.u[((size_t)(t0 + m) * a.H + h) * a.dv + n_base + n] = su[m * LU + n] - sp[m * LU + n];
+        }
+        if (i + 1 < count) publish(a.states + ((size_t)(c + 1) * a.H + h) * a.dv * a.dk, true);
+        __syncthreads();                         // the tiles may be filled again, S is whole
+    }
+    publish(a.state + (size_t)a.slots[r] * a.state_stride + (size_t)h * a.dv * a.dk, false);
+}
+
+// ---- a forget gate per key channel (csrc/linear_state.cu): k_t = 1 - f_t, S_t = diag(f_t) S_(t-1) + k_t v_t^T -------------------------
+// The ratio of two tokens' decays is a product of gates per channel, so it rides on q and k.  A chunk is cut into four runs of
+// 16 tokens, and every product of gates is made forward or backward inside a run (F: over a whole run), so none is a quotient and
+// none exceeds 1:
+//   q'_t = q_t prod(u <= t in t's run) f_u,     k'_s = k_s prod(u > s in s's run) f_u;
+//   scores between runs i > j: q'_t diag(prod of F between j and i) k'_s;    from the state: q'_t diag(prod of F before i) S;
+//   to the state: k'_s diag(prod of F behind j);    inside a run, where the product would have to be taken apart, token by token.
+#define LC_RUN 16
+
+template <int DK, int DV>
+__global__ void __launch_bounds__(256, 2) lc_forget_state_kernel(LcArgs a) {
+    extern __shared__ __align__(16) float lc_smem[];
+    float* sf = lc_smem;                         // [64][LC_LD]: f, then what k becomes
+    float* sv = sf + LC_C * LC_LD;               // [64][LC_LD]
+    __shared__ float sF[4][DK], sr[LC_C];
+    const int h = blockIdx.x, c = blockIdx.y;
+    const int t0 = a.chunk_meta[4 * c], cnt = a.chunk_meta[4 * c + 1];
+    lc_load<DK, LC_LD>(sf, a.k + (size_t)t0 * a.ldk + (size_t)h * a.dk, a.ldk, cnt, a.dk);
+    lc_load<DV, LC_LD>(sv, a.v + (size_t)t0 * a.ldv + (size_t)h * a.dv, a.ldv, cnt, a.dv);
+    lc_commit();
+    if (threadIdx.x < LC_C) sr[threadIdx.x] = 1.0f;
+    lc_wait<0>();
+    __syncthreads();
+    constexpr int PER = DK / 64;                 // runs per thread; a thread owns one channel
+    const int ch = threadIdx.x % DK, first = threadIdx.x / DK * PER;
+    float kk[PER][LC_RUN];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+        float r = 1.0f;
+#pragma unroll
+        for (int s = LC_RUN - 1; s >= 0; --s) {
+            const int t = (first + u) * LC_RUN + s;
+            const bool in = t < cnt && ch < a.dk;
+            const float f = in ? sf[t * LC_LD + ch] : 1.0f;
+            kk[u][s] = in ? (1.0f - f) * r : 0.0f;
+            r *= f;
+        }
+        sF[first + u][ch] = r;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+        float behind = 1.0f;
+        for (int m = first + u + 1; m < 4; ++m) behind *= sF[m][ch];
+#pragma unroll
+        for (int s = 0; s < LC_RUN; ++s) sf[((first + u) * LC_RUN + s) * LC_LD + ch] = kk[u][s] * behind;
+    }
+    if (first == 0 && ch < a.dk) a.gain[((size_t)c * a.H + h) * a.dk + ch] = sF[0][ch] * sF[1][ch] * sF[2][ch] * sF[3][ch];
+    __syncthreads();
+    lc_add_up<DK, DV>(a, h, c, sf, sv, sr);
+}
+
+// Two blocks per SM: q (then q', then the scores), f (then k'), and a buffer for S's halves and then v.
+template <int DK, int DV>
+__global__ void __launch_bounds__(256, 2) lc_forget_output_kernel(LcArgs a) {
+    extern __shared__ __align__(16) float lc_smem[];
+    float* sq = lc_smem;
+    float* sf = sq + LC_C * LC_LD;
+    float* sx = sf + LC_C * LC_LD;
+    __shared__ __align__(16) float sF[4][DK], sbefore[4][DK], sone[DK], smid[DK];      // a run's product; of the runs before one; 1; of runs 1 and 2
+    const int h = blockIdx.x, c = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t0 = a.chunk_meta[4 * c], cnt = a.chunk_meta[4 * c + 1];
+    const float* S = a.states + ((size_t)c * a.H + h) * a.dv * a.dk;
+    lc_load<DK, LC_LD>(sq, a.q + (size_t)t0 * a.ldq + (size_t)h * a.dk, a.ldq, cnt, a.dk);
+    lc_load<DK, LC_LD>(sf, a.k + (size_t)t0 * a.ldk + (size_t)h * a.dk, a.ldk, cnt, a.dk);
+    lc_commit();
+    lc_load<DK, LC_LD>(sx, S, a.dk, min(64, a.dv), a.dk);
+    lc_commit();
+    lc_wait<1>();
+    __syncthreads();
+    // inside the runs: thread (run, s, channels 4 cl.. of every 16) carries k_s through the tokens t >= s
+    const int run = threadIdx.x >> 6, ds = (threadIdx.x & 63) >> 2, cl = threadIdx.x & 3;
+    float inner[LC_RUN];
+#pragma unroll
+    for (int t = 0; t < LC_RUN; ++t) inner[t] = 0.0f;
+#pragma unroll 1
+    for (int e = 0; e < DK; e += 16) {
+        const float* fq = sq + run * LC_RUN * LC_LD + e + 4 * cl;
+        const float* ff = sf + run * LC_RUN * LC_LD + e + 4 * cl;
+        float4 r = *reinterpret_cast<const float4*>(ff + ds * LC_LD);
+        r = make_float4(1.0f - r.x, 1.0f - r.y, 1.0f - r.z, 1.0f - r.w);
+#pragma unroll
+        for (int t = 0; t < LC_RUN; ++t) {
+            const float4 qv = *reinterpret_cast<const float4*>(fq + t * LC_LD), fv = *reinterpret_cast<const float4*>(ff + t * LC_LD);
+            if (t > ds) r = make_float4(r.x * fv.x, r.y * fv.y, r.z * fv.z, r.w * fv.w);
+            if (t >= ds) inner[t] = fmaf(qv.x, r.x, fmaf(qv.y, r.y, fmaf(qv.z, r.z, fmaf(qv.w, r.w, inner[t]))));
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < LC_RUN; ++t) {
+        inner[t] += __shfl_xor_sync(0xffffffffu, inner[t], 1);
+        inner[t] += __shfl_xor_sync(0xffffffffu, inner[t], 2);
+    }
+    __syncthreads();
+    {   // q' and k' in place: a thread owns one channel of DK / 64 runs
+        constexpr int PER = DK / 64;
+        const int ch = threadIdx.x % DK, first = threadIdx.x / DK * PER;
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            float f[LC_RUN];
+            float* pq = sq + (first + u) * LC_RUN * LC_LD + ch;
+            float* pf = sf + (first + u) * LC_RUN * LC_LD + ch;
+            float r = 1.0f;
+#pragma unroll
+            for (int s = 0; s < LC_RUN; ++s) {
+                const bool in = (first + u) * LC_RUN + s < cnt && ch < a.dk;
+                f[s] = in ? pf[s * LC_LD] : 1.0f;
+                r *= f[s];
+                pq[s * LC_LD] *= r;
+            }
+            sF[first + u][ch] = r;
+            r = 1.0f;
+#pragma unroll
+            for (int s = LC_RUN - 1; s >= 0; --s) {
+                pf[s * LC_LD] = (1.0f - f[s]) * r;
+                r *= f[s];
+            }
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < DK) {
+        const int ch = threadIdx.x;
+        sone[ch] = sbefore[0][ch] = 1.0f;
+        float r = 1.0f;
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            r *= sF[m][ch];
+            sbefore[m + 1][ch] = r;
+        }
+        smid[ch] = sF[1][ch] * sF[2][ch];
+    }
+    const int m0 = (warp & 1) * 32, wn = warp >> 1, t = lane & 3, g = lane >> 2;
+    constexpr int HALVES = DV / 64;
+    float acc[HALVES][2][2][4];
+#pragma unroll
+    for (int x = 0; x < HALVES * 16; ++x) (&acc[0][0][0][0])[x] = 0.0f;
+#pragma unroll
+    for (int b = 0; b < HALVES; ++b) {
+        lc_wait<0>();
+        __syncthreads();
+#pragma unroll 2
+        for (int k0 = 0; k0 < DK; k0 += 8) {
+            LcA fa[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows_scaled(sq + (m0 + 16 * i) * LC_LD + k0, LC_LD, &sbefore[m0 / 16 + i][k0]);
+            const LcB fb[2] = {lc_b_rows(sx + wn * 16 * LC_LD + k0, LC_LD), lc_b_rows(sx + (wn * 16 + 8) * LC_LD + k0, LC_LD)};
+            lc_products<2, 2>(acc[b], fa, fb);
+        }
+        __syncthreads();
+        if (b + 1 < HALVES) lc_load<DK, LC_LD>(sx, a.dv > 64 ? S + (size_t)64 * a.dk : S, a.dk, a.dv - 64, a.dk);
+        else lc_load<DV, LC_LD>(sx, a.v + (size_t)t0 * a.ldv + (size_t)h * a.dv, a.ldv, cnt, a.dv);
+        lc_commit();
+    }
+    // between the runs: warp w < 6 takes one of the blocks (1,0) (2,0) (2,1) (3,0) (3,1) (3,2)
+    float cross[2][4];
+#pragma unroll
+    for (int x = 0; x < 8; ++x) (&cross[0][0])[x] = 0.0f;
+    const int bi = warp == 0 ? 1 : warp < 3 ? 2 : 3, bj = warp == 0 ? 0 : warp < 3 ? warp - 1 : warp - 3;
+    if (warp < 6) {
+        const float* between = bi - bj == 1 ? sone : bi - bj == 2 ? sF[bi - 1] : smid;
+#pragma unroll 4
+        for (int k0 = 0; k0 < DK; k0 += 8) {
+            const LcA fa = lc_a_rows_scaled(sq + bi * LC_RUN * LC_LD + k0, LC_LD, between + k0);
+            const float* p = sf + bj * LC_RUN * LC_LD + k0;
+            const LcB fb[2] = {lc_b_rows(p, LC_LD), lc_b_rows(p + 8 * LC_LD, LC_LD)};
+            lc_products<1, 2>(&cross, &fa, fb);
+        }
+    }
+    __syncthreads();                             // every warp is through with q': the scores take its place
+#pragma unroll
+    for (int x = 0; x < LC_RUN; ++x)
+        if ((x & 3) == cl) sq[(run * LC_RUN + x) * LC_LP + run * LC_RUN + ds] = x >= ds ? inner[x] : 0.0f;
+    if (warp < 6) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) sq[(bi * LC_RUN + g + 8 * (x >> 1)) * LC_LP + bj * LC_RUN + 8 * j + 2 * t + (x & 1)] = cross[j][x];
+    }
+    lc_wait<0>();
+    __syncthreads();
+    for (int k0 = 0; k0 < m0 + 32; k0 += 8) {
+        LcA fa[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)              // nothing stands to the right of a row's own run
+            fa[i] = k0 >= m0 + 16 * i + 16 ? LcA{} : lc_a_rows4(sq + (m0 + 16 * i) * LC_LP + k0, LC_LP, 1.0f, 1.0f);
+#pragma unroll
+        for (int b = 0; b < HALVES; ++b) {
+            const float* p = sx + k0 * LC_LD + 64 * b + wn * 16;
+            const LcB fb[2] = {lc_b_cols(p, LC_LD), lc_b_cols(p + 8, LC_LD)};
+            lc_products<2, 2>(acc[b], fa, fb);
+        }
+    }
+#pragma unroll
+    for (int b = 0; b < HALVES; ++b)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int n = 64 * b + wn * 16 + 8 * j + 2 * t;
+                if (n >= a.dv) continue;
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int m = m0 + 16 * i + g + 8 * half;
+                    if (m < cnt)
+                        *reinterpret_cast<float2*>(a.out + ((size_t)(t0 + m) * a.H + h) * a.dv + n) =
+                            make_float2(acc[b][i][j][2 * half], acc[b][i][j][2 * half + 1]);
+                }
+            }
+}
+
+template <typename... A>
+static int lc_launch(void (*kernel)(A...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        mm_set_last_error("linear state chunks: cannot reserve shared memory");
+        return MM_ERR_LAUNCH;
+    }
+    mm_launch(kernel, grid, dim3(threads), smem, s, args...);
+    MM_CHECK_LAUNCH();
+    return MM_OK;
+}
+
+template <int DK, int DV>
+static int lc_run(const LcArgs& a, int n_requests, cudaStream_t s) {
+    const dim3 chunks(a.H, a.n_chunks);
+    const size_t tile = LC_C * LC_LD * sizeof(float), square = LC_C * LC_LP * sizeof(float);
+    if (a.beta == nullptr) {
+        if (const int rc = lc_launch(lc_state_kernel<DK, DV>, chunks, 256, 2 * tile, s, a)) return rc;
+        const long long size = (long long)a.H * a.dv * a.dk;
+        if (const int rc = lc_launch(lc_carry_kernel<false>, dim3(ceil_div(size, 256), n_requests), 256, 0, s, a)) return rc;
+        return lc_launch(lc_output_kernel<DK, DV>, chunks, 256, 3 * tile, s, a, a.v, (size_t)a.ldv);
+    }
+    if (const int rc = lc_launch(lc_delta_prepare_kernel<DK, DV>, chunks, 256, 2 * tile + 2 * square, s, a)) return rc;
+    // columns of S per block: 16 while the blocks then fit the SMs (one each: 166 KB), else 32, whose chain is a little longer
+    const bool wide = (long long)ceil_div(a.dv, 16) * a.H * n_requests > 148 && a.dv > 16;
+#define LC_CARRY(NS)                                                                                                                       \
+    lc_launch(lc_delta_carry_kernel<DK, NS>, dim3(ceil_div(a.dv, NS), a.H, n_requests), LC_CARRY_THREADS,                                   \
+              (size_t)(2 * (2 * LC_C * LC_LD + LC_C * (NS + 8) + LC_C + 4) + NS * LC_LD + LC_C * (NS + 8)) * sizeof(float), s, a)
+    if (const int rc = wide ? LC_CARRY(32) : LC_CARRY(16)) return rc;
+#undef LC_CARRY
+    return lc_launch(lc_output_kernel<DK, DV>, chunks, 256, 3 * tile, s, a, (const float*)a.u, (size_t)a.H * a.dv);
+}
+
+// 1 if the products take these sizes and pointers: heads of up to 128 numbers that are multiples of 4, rows and heads on 16-byte boundaries
+MM_EXPORT int mm_linear_chunk_supported(const void* q, const void* k, const void* v, int ldq, int ldk, int ldv, const void* state,
+                                        long long state_stride, int dk, int dv) {
+    return dk > 0 && dv > 0 && dk <= 128 && dv <= 128 && dk % 4 == 0 && dv % 4 == 0 && ldq % 4 == 0 && ldk % 4 == 0 && ldv % 4 == 0 &&
+           (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v) & 15) == 0 && state != nullptr && state_stride > 0;
+}
+
+// q, k, v, gate, beta (null: no delta rule), head_decay, out, state as for the walk (decays positive or zero); chunk_meta [chunks, 4] =
+// (first token, tokens <= 64, request, .), req_chunks [requests, 2] = (first chunk, chunks).  Scratch, fp32: states [chunks, H, dv, dk], gain
+// [chunks, H], and with beta ratio [chunks, H, 64], w [tokens, H, dk], u [tokens, H, dv].
+MM_EXPORT int mm_linear_chunk(const void* q, const void* k, const void* v, int ldq, int ldk, int ldv, const void* gate, const void* beta,
+                              const void* head_decay, void* out, void* state, long long state_stride, const void* chunk_meta,
+                              const void* req_chunks, const void* slots, const void* positions, int n_requests, int n_chunks, int H, int Gq,
+                              int dk, int dv, void* states, void* gain, void* ratio, void* w, void* u, void* stream) {
+    MM_REQUIRE(H > 0 && Gq > 0 && H % Gq == 0, "linear state chunks: heads must be a positive multiple of the q/k heads");
+    MM_REQUIRE(mm_linear_chunk_supported(q, k, v, ldq, ldk, ldv, state, state_stride, dk, dv), "linear state chunks: sizes or pointers that the products do not take");
+    MM_REQUIRE(gate != nullptr || head_decay != nullptr, "linear state: a decay per token or per head is needed");
+    MM_REQUIRE(out && slots && positions && chunk_meta && req_chunks && states && gain, "linear state chunks: the lists and the scratch are needed");
+    MM_REQUIRE(beta == nullptr || (ratio && w && u), "linear state chunks: the delta rule needs its scratch");
+    MM_REQUIRE((((uintptr_t)out | (uintptr_t)states | (uintptr_t)ratio | (uintptr_t)w | (uintptr_t)u) & 15) == 0, "linear state chunks: the scratch starts on 16-byte boundaries");
+    MM_REQUIRE(n_chunks <= 65535 && n_requests <= 65535, "linear state chunks: too many chunks or requests");
+    if (n_requests <= 0 || n_chunks <= 0) return MM_OK;
+    LcArgs a;
+    a.q = (const float*)q; a.k = (const float*)k; a.v = (const float*)v;
+    a.gate = (const float*)gate; a.beta = (const float*)beta; a.head_decay = (const float*)head_decay;
+    a.ldq = ldq; a.ldk = ldk; a.ldv = ldv;
+    a.out = (float*)out; a.state = (float*)state; a.state_stride = state_stride;
+    a.chunk_meta = (const int32_t*)chunk_meta; a.req_chunks = (const int32_t*)req_chunks;
+    a.slots = (const int32_t*)slots; a.positions = (const int32_t*)positions;
+    a.n_chunks = n_chunks; a.H = H; a.G = Gq; a.dk = dk; a.dv = dv;
+    a.states = (float*)states; a.gain = (float*)gain; a.ratio = (float*)ratio; a.w = (float*)w; a.u = (float*)u;
+    cudaStream_t s = (cudaStream_t)stream;
+    if (dk <= 64) return dv <= 64 ? lc_run<64, 64>(a, n_requests, s) : lc_run<64, 128>(a, n_requests, s);
+    return dv <= 64 ? lc_run<128, 64>(a, n_requests, s) : lc_run<128, 128>(a, n_requests, s);
+}
+
+template <int DK, int DV>
+static int lc_run_forget(const LcArgs& a, int n_requests, cudaStream_t s) {
+    const dim3 chunks(a.H, a.n_chunks);
+    const size_t tile = LC_C * LC_LD * sizeof(float);
+    if (const int rc = lc_launch(lc_forget_state_kernel<DK, DV>, chunks, 256, 2 * tile, s, a)) return rc;
+    const long long size = (long long)a.H * a.dv * a.dk;
+    if (const int rc = lc_launch(lc_carry_kernel<true>, dim3(ceil_div(size, 256), n_requests), 256, 0, s, a)) return rc;
+    return lc_launch(lc_forget_output_kernel<DK, DV>, chunks, 256, 3 * tile, s, a);
+}
+
+// The recurrence with a forget gate per key channel: f [tokens, H dk] beside q; gain fp32 [chunks, H, dk]; the rest as above.
+MM_EXPORT int mm_forget_gate_chunk(const void* q, const void* f, const void* v, int ldq, int ldf, int ldv, void* out, void* state,
+                                   long long state_stride, const void* chunk_meta, const void* req_chunks, const void* slots,
+                                   const void* positions, int n_requests, int n_chunks, int H, int dk, int dv, void* states, void* gain,
+                                   void* stream) {
+    MM_REQUIRE(H > 0, "forget gate chunks: bad sizes");
+    MM_REQUIRE(mm_linear_chunk_supported(q, f, v, ldq, ldf, ldv, state, state_stride, dk, dv), "forget gate chunks: sizes or pointers that the products do not take");
+    MM_REQUIRE(out && slots && positions && chunk_meta && req_chunks && states && gain, "forget gate chunks: the lists and the scratch are needed");
+    MM_REQUIRE((((uintptr_t)out | (uintptr_t)states | (uintptr_t)gain) & 15) == 0, "forget gate chunks: the scratch starts on 16-byte boundaries");
+    MM_REQUIRE(n_chunks <= 65535 && n_requests <= 65535, "forget gate chunks: too many chunks or requests");
+    if (n_requests <= 0 || n_chunks <= 0) return MM_OK;
+    LcArgs a = {};
+    a.q = (const float*)q; a.k = (const float*)f; a.v = (const float*)v;
+    a.ldq = ldq; a.ldk = ldf; a.ldv = ldv;
+    a.out = (float*)out; a.state = (float*)state; a.state_stride = state_stride;
+    a.chunk_meta = (const int32_t*)chunk_meta; a.req_chunks = (const int32_t*)req_chunks;
+    a.slots = (const int32_t*)slots; a.positions = (const int32_t*)positions;
+    a.n_chunks = n_chunks; a.H = a.G = H; a.dk = dk; a.dv = dv;
+    a.states = (float*)states; a.gain = (float*)gain;
+    cudaStream_t s = (cudaStream_t)stream;
+    if (dk <= 64) return dv <= 64 ? lc_run_forget<64, 64>(a, n_requests, s) : lc_run_forget<64, 128>(a, n_requests, s);
+    return dv <= 64 ? lc_run_forget<128, 64>(a, n_requests, s) : lc_run_forget<128, 128>(a, n_requests, s);
+}

@@ -1121,6 +1121,57 @@ def linear_state_chunked(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, stat
     return out
 
 
+LINEAR_CHUNK = 64      # tokens per chunk of linear_state_products
+
+
+def linear_state_products_supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, dk: int, dv: int) -> bool:
+    """True if ``linear_state_products`` takes these rows: heads of up to 128 numbers in multiples of 4, 16-byte boundaries."""
+    return bool(_lib.load().mm_linear_chunk_supported(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0),
+                                                      state.data_ptr(), state.stride(0), int(dk), int(dv)))
+
+
+def linear_state_products(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, chunk_meta: torch.Tensor,
+                          req_chunks: torch.Tensor, slots: torch.Tensor, positions: torch.Tensor, heads: int, qk_heads: int, dk: int, dv: int,
+                          gate: Optional[torch.Tensor] = None, beta: Optional[torch.Tensor] = None,
+                          head_decay: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """The recurrence of ``linear_state_walk`` (with or without the delta rule) for long portions, as products of matrices over
+    chunks of at most ``LINEAR_CHUNK`` tokens.  ``chunk_meta`` [chunks, 4] = (first token, tokens, request, .), ``req_chunks``
+    [requests, 2] = (first chunk, chunks); the decays are 0 or positive."""
+    for t, what in ((q, "q"), (k, "k"), (v, "v")):
+        if t.dtype != torch.float32 or not t.is_cuda or t.stride(1) != 1:
+            raise KernelError(f"linear state {what}: fp32 rows with unit column stride are needed")
+    n = q.shape[0]
+    if q.shape[1] != qk_heads * dk or k.shape != q.shape or v.shape != (n, heads * dv):
+        raise KernelError("linear state: shape mismatch")
+    if state.dtype != torch.float32 or state.stride(-1) != 1 or state.shape[1] < heads * dv * dk:
+        raise KernelError("linear state: the state is fp32 [slots, >= heads * dv * dk]")
+    for t, what in ((gate, "gate"), (beta, "beta")):
+        if t is not None:
+            _need(t, what, torch.float32)
+            if t.shape != (n, heads):
+                raise KernelError(f"linear state {what}: wrong shape")
+    if head_decay is not None:
+        _need(head_decay, "head decay", torch.float32)
+        if head_decay.numel() != heads:
+            raise KernelError("linear state: a decay per head is needed")
+    for t, what in ((chunk_meta, "chunk_meta"), (req_chunks, "req_chunks"), (slots, "state slots"), (positions, "positions")):
+        _need(t, what, torch.int32)
+    n_chunks, n_req = chunk_meta.shape[0], req_chunks.shape[0]
+    out = torch.empty((n, heads * dv), dtype=torch.float32, device=q.device)
+    states = torch.empty((max(1, n_chunks), heads * dv * dk), dtype=torch.float32, device=q.device)
+    gain = torch.empty((max(1, n_chunks), heads), dtype=torch.float32, device=q.device)
+    ratio = w = u = None
+    if beta is not None:
+        ratio = torch.empty((max(1, n_chunks), heads, LINEAR_CHUNK), dtype=torch.float32, device=q.device)
+        w = torch.empty((n, heads * dk), dtype=torch.float32, device=q.device)
+        u = torch.empty((n, heads * dv), dtype=torch.float32, device=q.device)
+    check(_lib.load().mm_linear_chunk(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0), _ptr(gate), _ptr(beta),
+                                      _ptr(head_decay), out.data_ptr(), state.data_ptr(), state.stride(0), chunk_meta.data_ptr(),
+                                      req_chunks.data_ptr(), slots.data_ptr(), positions.data_ptr(), n_req, n_chunks, heads, qk_heads, dk, dv,
+                                      states.data_ptr(), gain.data_ptr(), _ptr(ratio), _ptr(w), _ptr(u), _stream()), "linear_chunk")
+    return out
+
+
 GATE_ACTIVATIONS = {"silu": 1, "sigmoid": 2}
 
 
@@ -1668,6 +1719,31 @@ def forget_gate_chunked(q: torch.Tensor, f: torch.Tensor, v: torch.Tensor, state
                                              state.data_ptr(), state.stride(0), chunk_meta.data_ptr(), req_chunks.data_ptr(), slots.data_ptr(),
                                              positions.data_ptr(), n_req, n_chunks, int(heads), int(dk), int(dv), scratch.data_ptr(), gain.data_ptr(),
                                              _stream()), "forget_gate_chunked")
+    return out
+
+
+def forget_gate_products(q: torch.Tensor, f: torch.Tensor, v: torch.Tensor, state: torch.Tensor, chunk_meta: torch.Tensor, req_chunks: torch.Tensor,
+                         slots: torch.Tensor, positions: torch.Tensor, heads: int, dk: int, dv: int) -> torch.Tensor:
+    """The same for long portions as products of matrices over chunks of at most ``LINEAR_CHUNK`` tokens (what
+    ``linear_state_products_supported`` says of q, f and v)."""
+    for t, what in ((q, "q"), (f, "f"), (v, "v")):
+        if t.dtype != torch.float32 or not t.is_cuda or t.stride(1) != 1:
+            raise KernelError(f"forget gate products {what}: fp32 rows with unit column stride are needed")
+    n = q.shape[0]
+    if q.shape[1] != heads * dk or f.shape != q.shape or v.shape != (n, heads * dv):
+        raise KernelError("forget gate products: shape mismatch")
+    if state.dtype != torch.float32 or state.stride(-1) != 1 or state.shape[1] < heads * dv * dk:
+        raise KernelError("forget gate products: the state is fp32 [slots, >= heads * dv * dk]")
+    for t, what in ((chunk_meta, "chunk_meta"), (req_chunks, "req_chunks"), (slots, "state slots"), (positions, "positions")):
+        _need(t, what, torch.int32)
+    n_chunks, n_req = chunk_meta.shape[0], req_chunks.shape[0]
+    out = torch.empty((n, heads * dv), dtype=torch.float32, device=q.device)
+    states = torch.empty((max(1, n_chunks), heads * dv * dk), dtype=torch.float32, device=q.device)
+    gain = torch.empty((max(1, n_chunks), heads * dk), dtype=torch.float32, device=q.device)
+    check(_lib.load().mm_forget_gate_chunk(q.data_ptr(), f.data_ptr(), v.data_ptr(), q.stride(0), f.stride(0), v.stride(0), out.data_ptr(),
+                                           state.data_ptr(), state.stride(0), chunk_meta.data_ptr(), req_chunks.data_ptr(), slots.data_ptr(),
+                                           positions.data_ptr(), n_req, n_chunks, int(heads), int(dk), int(dv), states.data_ptr(), gain.data_ptr(),
+                                           _stream()), "forget_gate_chunk")
     return out
 
 

@@ -25,9 +25,9 @@ One class covers the family; what differs between its members is a parameter:
   ``heads * value_dim`` (``all``) numbers, or None; ``gate_activation``: ``silu`` or ``sigmoid`` on ``W_g h``.
 
 All input projections are one product with an fp32 result; everything between it and the output projection is fp32
-(``csrc/linear_state.cu``, ``csrc/norm_gated.cu``).  A request's tokens are walked in order from its slot's state; long
-portions without the delta rule (whose update is a scaling and an addition) are cut into chunks that are walked side by
-side, except in float32 runs, which keep one order of operations whatever the cutting.  q and k have ``qk_heads`` heads; head h reads q/k head ``h // (heads / qk_heads)``.
+(``csrc/linear_state.cu``, ``csrc/linear_chunk.cu``, ``csrc/norm_gated.cu``).  A request's tokens are walked in order from its slot's
+state; long portions are cut into chunks whose outputs and states are products of matrices (head sizes these do not take: chunks that are
+walked side by side, with the delta rule the walk), except in float32 runs, which keep one order of operations whatever the cutting.  q and k have ``qk_heads`` heads; head h reads q/k head ``h // (heads / qk_heads)``.
 """
 from __future__ import annotations
 
@@ -44,7 +44,8 @@ from .linear import linear
 
 
 CHUNK = 64                   # tokens per chunk of the three-pass walk
-CHUNKED_FROM = 256           # a step whose longest portion has at least this many tokens walks its chunks side by side (not in float32)
+CHUNKED_FROM = 256           # a step whose longest portion has at least this many tokens goes chunk by chunk (not in float32)
+DELTA_CHUNKED_FROM = 128     # the same with the delta rule, whose walk is the slower one
 CONV_BY_TOKEN_FROM = 32      # a step whose longest portion has at least this many tokens runs the convolution per (token, channel)
 
 
@@ -129,6 +130,8 @@ class LinearStateMixer(Mixer):
             if len(spec["decay"]) != H:
                 raise ValueError(f"linear state: {len(spec['decay'])} decay constants for {H} heads")
             self.head_decay = torch.tensor([float(x) for x in spec["decay"]], dtype=torch.float32, device=rt.device)
+        # the products over chunks take logarithms of the decays
+        self.decays_by_logarithm = self.learned_decay or (not self.forget_gate and all(float(x) >= 0.0 for x in spec["decay"]))
         rot = spec.get("rotary")
         self.rot_dims, self.freq, self.rot_key = 0, None, None
         if rot and int(rot["dims"]):
@@ -162,7 +165,10 @@ class LinearStateMixer(Mixer):
             ops.forget_gate_prep(a, self.q_off, self.k_off, H * dk, self.f_bias, self.lower, silu_q=self.activation == "silu")
             qs, fs, vs = a[:, self.q_off:self.q_off + H * dk], a[:, self.k_off:self.k_off + H * dk], a[:, self.v_off:self.v_off + H * dv]
             # the 32-bit path keeps one order of operations whatever the cutting: it always walks token by token
-            if ctx.max_q_len >= CHUNKED_FROM and self.rt.dtype != torch.float32:
+            if ctx.max_q_len >= CHUNKED_FROM and self.rt.dtype != torch.float32 and ops.linear_state_products_supported(qs, fs, vs, state, dk, dv):
+                chunk_meta, req_chunks = token_chunks(ctx, ops.LINEAR_CHUNK)
+                o = ops.forget_gate_products(qs, fs, vs, state, chunk_meta, req_chunks, ctx.state_slots, ctx.positions, H, dk, dv)
+            elif ctx.max_q_len >= CHUNKED_FROM and self.rt.dtype != torch.float32:
                 chunk_meta, req_chunks = token_chunks(ctx, CHUNK)
                 o = ops.forget_gate_chunked(qs, fs, vs, state, chunk_meta, req_chunks, ctx.state_slots, ctx.positions, H, dk, dv)
             else:
@@ -186,9 +192,13 @@ class LinearStateMixer(Mixer):
             k_scale=self.k_scale, a_off=self.a_off if self.learned_decay else -1, b_off=self.b_off, heads=H, A_log=self.A_log,
             dt_bias=self.dt_bias, gate_rows=gate_rows)
         qs, ks_, vs = qkv[:, self.q_off:self.q_off + G * dk], qkv[:, self.k_off:self.k_off + G * dk], qkv[:, self.v_off:self.v_off + H * dv]
-        # the 32-bit path keeps one order of operations whatever the cutting: it always walks; so does the delta rule,
-        # whose update of the state is not a scaling and an addition
-        if not self.delta and ctx.max_q_len >= CHUNKED_FROM and self.rt.dtype != torch.float32:
+        # the 32-bit path keeps one order of operations whatever the cutting: it always walks
+        long = ctx.max_q_len >= (DELTA_CHUNKED_FROM if self.delta else CHUNKED_FROM) and self.rt.dtype != torch.float32
+        if long and self.decays_by_logarithm and ops.linear_state_products_supported(qs, ks_, vs, state, dk, dv):
+            chunk_meta, req_chunks = token_chunks(ctx, ops.LINEAR_CHUNK)
+            o = ops.linear_state_products(qs, ks_, vs, state, chunk_meta, req_chunks, ctx.state_slots, ctx.positions, H, G, dk, dv,
+                                          gate=gate, beta=beta, head_decay=self.head_decay)
+        elif long and not self.delta:
             chunk_meta, req_chunks = token_chunks(ctx, CHUNK)
             o = ops.linear_state_chunked(qs, ks_, vs, state, chunk_meta, req_chunks, ctx.state_slots, ctx.positions, H, G, dk, dv,
                                          gate=gate, head_decay=self.head_decay)

@@ -1,0 +1,111 @@
+"""The matrix-state recurrence as products over chunks against 64 bits and against the token-by-token walk: edges of chunks, requests of
+unequal length, heads narrower than a tile, decays that underflow within a chunk, correlated keys, a state carried on."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def plain(q, k, v, decay, beta, S):
+    """In 64 bits; q, k [n, H, dk], v [n, H, dv], decay [n, H], S [H, dk, dv]."""
+    out = torch.empty_like(v)
+    for t in range(q.shape[0]):
+        S = S * decay[t][:, None, None]
+        u = v[t] if beta is None else beta[t][:, None] * (v[t] - torch.einsum("hkv,hk->hv", S, k[t]))
+        S = S + k[t][:, :, None] * u[:, None]
+        out[t] = torch.einsum("hkv,hk->hv", S, q[t])
+    return out, S
+
+
+@pytest.mark.parametrize("H,G,dk,dv", [(4, 2, 128, 128), (3, 3, 64, 128), (2, 1, 128, 64), (6, 2, 24, 36), (20, 5, 100, 128)])
+@pytest.mark.parametrize("delta", [False, True])
+@pytest.mark.parametrize("decay", ["near 1", "strong", "constant", "zero"])
+def test_products(H, G, dk, dv, delta, decay):
+    from mimirmind_b200.kernels import ops
+    if decay == "constant" and delta:
+        pytest.skip("the delta rule's decay is learned")
+    gen = torch.Generator(device=DEV).manual_seed(H * dk + dv + delta)
+    lens, begin, slots = [200, 1, 64, 129], [0, 5, 70, 0], [2, 0, 3, 4]
+    n = sum(lens)
+    rnd = lambda *s: torch.randn(s, generator=gen, device=DEV)                       # noqa: E731
+    ld = 2 * G * dk + H * dv + 4
+    row = rnd(n, ld)
+    q, k, v = row[:, :G * dk], row[:, G * dk:2 * G * dk], row[:, 2 * G * dk + 4:]
+    q *= dk ** -0.5
+    if delta:           # unit keys, neighbouring ones alike
+        kk = k.reshape(n, G, dk) + 2.0 * rnd(1, G, dk)
+        k.copy_((kk / kk.norm(dim=-1, keepdim=True)).reshape(n, G * dk))
+    else:
+        k *= dk ** -0.5
+    gate = {"near 1": 0.9 + 0.1 * torch.rand((n, H), generator=gen, device=DEV), "strong": 0.02 + 0.3 * torch.rand((n, H), generator=gen, device=DEV),
+            "constant": None, "zero": (torch.rand((n, H), generator=gen, device=DEV) > 0.1).float()}[decay]
+    head = torch.linspace(0.5, 0.9995, H, device=DEV) if gate is None else None
+    beta = torch.rand((n, H), generator=gen, device=DEV) if delta else None
+    state = rnd(5, H * dv * dk + 8)
+    before = state.clone()
+    starts = [sum(lens[:i]) for i in range(4)]
+    meta, per = [], []
+    for r, (s, m) in enumerate(zip(starts, lens)):
+        per.append([len(meta), -(-m // 64)])
+        meta += [[s + o, min(64, m - o), r, 0] for o in range(0, m, 64)]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)                   # noqa: E731
+    pos = torch.cat([torch.arange(b, b + m, dtype=torch.int32, device=DEV) for b, m in zip(begin, lens)])
+    assert ops.linear_state_products_supported(q, k, v, state, dk, dv)
+    walked = before.clone()
+    got = ops.linear_state_products(q, k, v, state, i32(meta), i32(per), i32(slots), pos, H, G, dk, dv, gate=gate, beta=beta, head_decay=head)
+    walk = ops.linear_state_walk(q, k, v, walked, i32([[s, m, b + m, x] for s, m, b, x in zip(starts, lens, begin, slots)]), i32(slots), pos, 4, H, G,
+                                 dk, dv, gate=gate, beta=beta, head_decay=head)
+    assert torch.equal(state[1], before[1]) and torch.equal(state[:, H * dv * dk:], before[:, H * dv * dk:])      # nobody else's
+    for r, (s, m) in enumerate(zip(starts, lens)):
+        rep = lambda t, w: t[s:s + m].reshape(m, G, w).repeat_interleave(H // G, dim=1).double()                  # noqa: E731
+        S = torch.zeros(H, dk, dv, dtype=torch.float64, device=DEV) if begin[r] == 0 else \
+            before[slots[r], :H * dv * dk].view(H, dv, dk).transpose(1, 2).double()
+        g = (gate[s:s + m] if gate is not None else head.expand(m, H)).double()
+        want, S = plain(rep(q, dk), rep(k, dk), v[s:s + m].reshape(m, H, dv).double(), g, None if beta is None else beta[s:s + m].double(), S)
+        kept = S.transpose(1, 2).reshape(-1)
+        for mine, old, ref in ((got[s:s + m], walk[s:s + m], want.reshape(m, -1)), (state[slots[r], :H * dv * dk], walked[slots[r], :H * dv * dk], kept)):
+            scale = ref.norm()
+            err, was = ((mine - ref).norm() / scale).item(), ((old - ref).norm() / scale).item()
+            print(f"err {err:.2e} walk {was:.2e}")
+            # 22 bits of every factor of up to 64 + 128 + 128 products one after the other, each rounded like the walk's: a few 2^-22
+            assert err <= max(5e-7, 1.5 * was), (r, err, was)
+
+
+@pytest.mark.parametrize("H,dk,dv", [(4, 128, 64), (2, 128, 128), (3, 64, 64), (5, 36, 100)])
+@pytest.mark.parametrize("gates", ["near 1", "wide", "near 0"])
+def test_forget_gate_products(H, dk, dv, gates):
+    from mimirmind_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(H * dk + dv)
+    lens, begin, slots = [150, 17, 64, 81], [0, 5, 70, 0], [2, 0, 3, 4]
+    n = sum(lens)
+    rnd = lambda *s: torch.randn(s, generator=gen, device=DEV)                       # noqa: E731
+    row = rnd(n, 2 * H * dk + H * dv + 4)
+    q, f, v = row[:, :H * dk], row[:, H * dk:2 * H * dk], row[:, 2 * H * dk + 4:]
+    f.copy_({"near 1": 0.9 + 0.1 * torch.sigmoid(f), "wide": torch.sigmoid(4 * f), "near 0": 1e-6 + 0.05 * torch.sigmoid(f)}[gates])
+    state = rnd(5, H * dv * dk + 8)
+    before, walked = state.clone(), state.clone()
+    starts = [sum(lens[:i]) for i in range(4)]
+    meta, per = [], []
+    for r, (s, m) in enumerate(zip(starts, lens)):
+        per.append([len(meta), -(-m // 64)])
+        meta += [[s + o, min(64, m - o), r, 0] for o in range(0, m, 64)]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)                   # noqa: E731
+    pos = torch.cat([torch.arange(b, b + m, dtype=torch.int32, device=DEV) for b, m in zip(begin, lens)])
+    got = ops.forget_gate_products(q, f, v, state, i32(meta), i32(per), i32(slots), pos, H, dk, dv)
+    walk = ops.forget_gate_walk(q, f, v, walked, i32([[s, m, b + m, x] for s, m, b, x in zip(starts, lens, begin, slots)]), i32(slots), pos, 4, H, dk, dv)
+    assert torch.equal(state[1], before[1]) and torch.equal(state[:, H * dv * dk:], before[:, H * dv * dk:])
+    for r, (s, m) in enumerate(zip(starts, lens)):
+        S = torch.zeros(H, dk, dv, dtype=torch.float64, device=DEV) if begin[r] == 0 else \
+            before[slots[r], :H * dv * dk].view(H, dv, dk).transpose(1, 2).double()
+        qq, ff, vv = (t[s:s + m].reshape(m, H, -1).double() for t in (q, f, v))
+        want = torch.empty_like(vv)
+        for t in range(m):
+            S = S * ff[t][:, :, None] + (1.0 - ff[t])[:, :, None] * vv[t][:, None]
+            want[t] = torch.einsum("hkv,hk->hv", S, qq[t])
+        for mine, old, ref in ((got[s:s + m], walk[s:s + m], want.reshape(m, -1)),
+                               (state[slots[r], :H * dv * dk], walked[slots[r], :H * dv * dk], S.transpose(1, 2).reshape(-1))):
+            scale = ref.norm()
+            err, was = ((mine - ref).norm() / scale).item(), ((old - ref).norm() / scale).item()
+            print(f"err {err:.2e} walk {was:.2e}")
+            assert err <= max(5e-7, 1.5 * was), (r, err, was)      # as above
