@@ -13,7 +13,7 @@
 //   plain:  lc_state (what each chunk adds), lc_carry over the chunks per number of the state, lc_output;
 //   delta:  lc_delta_prepare (T, W, U0 per chunk), lc_delta_carry (U and S', chunk after chunk), lc_output with u for v.
 // A token costs dk dv multiply-adds three to four times as in the token-by-token walk, but as tiles of 16 x 8 x 8 on the tensor
-// cores: every operand is split into two tf32 numbers (11 bits each, both rounded to nearest), the product is the sum of the
+// cores: every operand is split into two tf32 numbers (11 bits each), the product is the sum of the
 // three larger of the four partial products, added up in 32 bits: 22 bits of every factor enter, and the error against 64 bits stays
 // that of the 32-bit walk (measured over random and correlated keys, see the tests).  mma.sync gives 92 TFLOP/s that way, the FMA
 // units, whose tiles are held up by shared-memory reads, 40 to 45.
@@ -48,14 +48,16 @@ __device__ __forceinline__ void lc_load(float* s, const float* __restrict__ p, s
     }
 }
 
-// x = hi + lo + (less than 2^-22 of x): two tf32 numbers (the tensor core reads the upper 19 bits)
+// x = hi + lo: hi is x rounded to 11 bits (Veltkamp's split, with the FMA units; masks and integer additions take twice as
+// long), lo the rest, of which the tensor core reads the upper 11 bits.
 struct LcSplit {
     uint32_t hi, lo;
 };
 __device__ __forceinline__ LcSplit lc_split(float x) {
+    const float c = __fmul_rn(x, 8193.0f), hi = __fsub_rn(c, __fsub_rn(c, x));
     LcSplit r;
-    r.hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-    r.lo = __float_as_uint(x - __uint_as_float(r.hi)) + 0x1000u;
+    r.hi = __float_as_uint(hi);
+    r.lo = __float_as_uint(__fsub_rn(x, hi));
     return r;
 }
 struct LcA {
@@ -231,36 +233,44 @@ __global__ void __launch_bounds__(256, 2) lc_state_kernel(LcArgs a) {
     lc_add_up<DK, DV>(a, h, c, sk, sv, sr);
 }
 
-// The carry over the chunks, a thread per number of the state: gain [chunks, H], or with a factor per key channel [chunks, H, dk].
+// The carry over the chunks, a thread per four numbers of the state: gain [chunks, H], or with a factor per key channel [chunks, H, dk].
+// Bound by memory; 48 states of 2 MB, more than L2 holds beside what it still writes back: 55 us (a number per thread 74).
 template <bool CHANNEL>
 __global__ void __launch_bounds__(256) lc_carry_kernel(LcArgs a) {
-    const long long size = (long long)a.H * a.dv * a.dk, i = (long long)blockIdx.x * 256 + threadIdx.x;
+    const long long size = (long long)a.H * a.dv * a.dk, i = 4 * ((long long)blockIdx.x * 256 + threadIdx.x);
     const int r = blockIdx.y;
     if (i >= size) return;
     const int h = (int)(i / (a.dv * a.dk)), first = a.req_chunks[2 * r], count = a.req_chunks[2 * r + 1];
     if (count <= 0) return;
-    float* __restrict__ states = a.states + i;
-    const float* __restrict__ gain = a.gain + (CHANNEL ? (size_t)h * a.dk + i % a.dk : (size_t)h);
-    const size_t step = CHANNEL ? (size_t)a.H * a.dk : (size_t)a.H;
+    float* base = a.states + (size_t)first * size + i;
+    const float* gain = a.gain + (CHANNEL ? ((size_t)first * a.H + h) * a.dk + i % a.dk : (size_t)first * a.H + h);
+    const int step = CHANNEL ? a.H * a.dk : a.H;
     float* st = a.state + (size_t)a.slots[r] * a.state_stride + i;
-    float S = a.positions[a.chunk_meta[4 * first]] == 0 ? 0.0f : *st;
-    for (int c0 = first; c0 < first + count; c0 += 8) {          // eight chunks' loads in flight: they do not depend on the carried value
-        float add[8], gn[8];
+    const bool fresh = a.positions[a.chunk_meta[4 * first]] == 0;
+    float4 S = fresh ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : make_float4(st[0], st[1], st[2], st[3]);
+    for (int c0 = 0; c0 < count; c0 += 8) {      // eight chunks' loads in flight: they do not depend on the carried value
+        float4 add[8], g[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const bool in = c0 + j < first + count;
-            add[j] = in ? states[(size_t)(c0 + j) * size] : 0.0f;
-            gn[j] = in ? gain[(size_t)(c0 + j) * step] : 1.0f;
+            const bool in = c0 + j < count;
+            add[j] = in ? *reinterpret_cast<const float4*>(base + (size_t)(c0 + j) * size) : S;
+            if (CHANNEL) g[j] = in ? *reinterpret_cast<const float4*>(gain + (size_t)(c0 + j) * step) : S;
+            else g[j].x = in ? gain[(size_t)(c0 + j) * step] : 1.0f;
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            if (c0 + j < first + count) {
-                states[(size_t)(c0 + j) * size] = S;
-                S = fmaf(gn[j], S, add[j]);
+        for (int j = 0; j < 8; ++j)
+            if (c0 + j < count) {
+                *reinterpret_cast<float4*>(base + (size_t)(c0 + j) * size) = S;
+                S.x = fmaf(g[j].x, S.x, add[j].x);
+                S.y = fmaf(CHANNEL ? g[j].y : g[j].x, S.y, add[j].y);
+                S.z = fmaf(CHANNEL ? g[j].z : g[j].x, S.z, add[j].z);
+                S.w = fmaf(CHANNEL ? g[j].w : g[j].x, S.w, add[j].w);
             }
-        }
     }
-    *st = S;
+    st[0] = S.x;
+    st[1] = S.y;
+    st[2] = S.z;
+    st[3] = S.w;
 }
 
 // ---- the outputs of a chunk: diag(gamma) Q S + (Q K^T, decayed and masked) U --------------------------------------------------
@@ -559,39 +569,39 @@ __global__ void __launch_bounds__(256, 2) lc_delta_prepare_kernel(LcArgs a) {
 }
 
 // U = U0 - W S and S' = gamma_C S + K^T diag(gamma_C / gamma) U, chunk after chunk, for NS columns of one head's S per block.
-// Bound by the chain of the two products and three barriers a chunk, so 16 warps share each product: in the first, warp w and w + 8 have one
-// tile of U and half of the key channels each (their halves meet when U is read), in the second a warp has 16 rows of dk and
-// half of the columns.  S stands in the accumulators and, for the first product, in shared memory; the next chunk's W, k and U0 arrive
-// under the current one's products.
+// Bound by the chain of the two products and its barriers, and within it by issuing instructions (splitting the operands is most of
+// them), so 16 warps share the k of each product and a warp makes as many tiles as use its fragments: in the first, warp w has rows
+// 16 (w % 4) of U and a quarter of the key channels, in the second rows 16 (w % 8) of dk and half of the tokens; both have all
+// NS columns.  The quarters meet in a pass over U, the halves never: S is kept as the sum of two, each carried by its own warps.
+// The next chunk's W, k and U0 arrive under the current one's products.  64 chunks: 229 us (254 with a tile and half of the k per warp).
 #define LC_CARRY_THREADS 512
 template <int DK, int NS>
 __global__ void __launch_bounds__(LC_CARRY_THREADS) lc_delta_carry_kernel(LcArgs a) {
-    constexpr int LU = NS + 8, TILE = 2 * LC_C * LC_LD + LC_C * LU + LC_C + 4, NT = NS / 16;      // column tiles of a warp
+    constexpr int LU = NS + 8, LQ = NS + 4, TILE = 2 * LC_C * LC_LD + LC_C * LU + LC_C + 4, NT = NS / 8;
     extern __shared__ __align__(16) float lc_smem[];
-    float* sS = lc_smem + 2 * TILE;              // [NS][LC_LD]
-    float* sp = sS + NS * LC_LD;                 // [64][LU]: the second half's part of W S
+    float* sS = lc_smem + 2 * TILE;              // [2][NS][LC_LD]: the two parts of S
+    float* sp = sS + 2 * NS * LC_LD;             // [4][64][LQ]: the quarters of W S
     const int h = blockIdx.y, r = blockIdx.z, n_base = blockIdx.x * NS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = lane & 3, g = lane >> 2, kh = h / (a.H / a.G), side = warp >> 3;
     const int first = a.req_chunks[2 * r], count = a.req_chunks[2 * r + 1];
     if (count <= 0) return;
     const int cols = min(NS, a.dv - n_base);
-    auto fill = [&](int i) {
-        const int c = first + i, t0 = a.chunk_meta[4 * c], cnt = a.chunk_meta[4 * c + 1];
+    auto fill = [&](int i, int t0, int cnt) {
         float* sw = lc_smem + (i & 1) * TILE;
         float* sk = sw + LC_C * LC_LD;
         float* su = sk + LC_C * LC_LD;
         float* sr = su + LC_C * LU;
         lc_load<DK, LC_LD, LC_CARRY_THREADS>(sw, a.w + ((size_t)t0 * a.H + h) * a.dk, (size_t)a.H * a.dk, cnt, a.dk);
         lc_load<DK, LC_LD, LC_CARRY_THREADS>(sk, a.k + (size_t)t0 * a.ldk + (size_t)kh * a.dk, a.ldk, cnt, a.dk);
-        for (int idx = threadIdx.x; idx < LC_C * (NS / 4); idx += LC_CARRY_THREADS) {
-            const int row = idx / (NS / 4), col = (idx % (NS / 4)) * 4;
+        if (threadIdx.x < LC_C * (NS / 4)) {     // (NS <= 32)
+            const int row = threadIdx.x / (NS / 4), col = (threadIdx.x % (NS / 4)) * 4;
             const bool in = row < cnt && col < cols;
             lc_cp16(su + row * LU + col, a.u + (in ? ((size_t)(t0 + row) * a.H + h) * a.dv + n_base + col : 0), in);
         }
-        if (threadIdx.x < LC_C / 4) lc_cp16(sr + 4 * threadIdx.x, a.ratio + ((size_t)c * a.H + h) * LC_C + 4 * threadIdx.x, true);
+        if (threadIdx.x < LC_C / 4) lc_cp16(sr + 4 * threadIdx.x, a.ratio + ((size_t)(first + i) * a.H + h) * LC_C + 4 * threadIdx.x, true);
         lc_commit();
     };
-    // the warp's part of S: rows 16 (warp % 8).. of dk (if there are so many), columns 8 side + 16 j..
+    // the warp's part of S: rows 16 (warp % 8).. of dk (if there are so many), all columns; the second half's part starts from zero
     const int s_row = (warp & 7) * 16;
     const bool has_rows = s_row < DK;
     float S[NT][4];
@@ -602,59 +612,90 @@ __global__ void __launch_bounds__(LC_CARRY_THREADS) lc_delta_carry_kernel(LcArgs
         for (int j = 0; j < NT; ++j)
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
-                const int m = s_row + g + 8 * (x >> 1), n = n_base + 8 * side + 16 * j + 2 * t + (x & 1);
-                S[j][x] = (!fresh && has_rows && m < a.dk && n < a.dv) ? st[(size_t)n * a.dk + m] : 0.0f;
+                const int m = s_row + g + 8 * (x >> 1), n = n_base + 8 * j + 2 * t + (x & 1);
+                S[j][x] = (side == 0 && !fresh && has_rows && m < a.dk && n < a.dv) ? st[(size_t)n * a.dk + m] : 0.0f;
             }
     }
-    auto publish = [&](float* __restrict__ to, bool local) {     // S to global memory and, if another chunk follows, to shared memory
+    auto to_shared = [&]() {
         if (!has_rows) return;
 #pragma unroll
         for (int j = 0; j < NT; ++j)
 #pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                const int m = s_row + g + 8 * (x >> 1), n = 8 * side + 16 * j + 2 * t + (x & 1);
-                if (local) sS[n * LC_LD + m] = S[j][x];
-                if (m < a.dk && n_base + n < a.dv) to[(size_t)(n_base + n) * a.dk + m] = S[j][x];
-            }
+            for (int x = 0; x < 4; ++x) sS[(side * NS + 8 * j + 2 * t + (x & 1)) * LC_LD + s_row + g + 8 * (x >> 1)] = S[j][x];
     };
-    fill(0);
-    publish(a.states + ((size_t)first * a.H + h) * a.dv * a.dk, true);
-    for (int i = 0; i < count; ++i) {
-        const int c = first + i, t0 = a.chunk_meta[4 * c], cnt = a.chunk_meta[4 * c + 1];
-        const float gain = a.gain[(size_t)c * a.H + h];
-        if (i + 1 < count) {
-            fill(i + 1);
-            lc_wait<1>();
-        } else {
-            lc_wait<0>();
+    auto to_global = [&](float* __restrict__ to, bool vec) {     // the sum of the two parts, as [dv, dk]
+        for (int idx = threadIdx.x; idx < NS * (DK / 4); idx += LC_CARRY_THREADS) {
+            const int n = idx / (DK / 4), m = (idx % (DK / 4)) * 4;
+            if (n >= cols || m >= a.dk) continue;
+            const float4 x = *reinterpret_cast<const float4*>(sS + n * LC_LD + m), y = *reinterpret_cast<const float4*>(sS + (NS + n) * LC_LD + m);
+            float* p = to + (size_t)(n_base + n) * a.dk + m;
+            if (vec) {
+                *reinterpret_cast<float4*>(p) = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
+            } else {
+                p[0] = x.x + y.x;
+                p[1] = x.y + y.y;
+                p[2] = x.z + y.z;
+                p[3] = x.w + y.w;
+            }
         }
-        __syncthreads();                         // this chunk's tiles and S
+    };
+    int t0 = a.chunk_meta[4 * first], cnt = a.chunk_meta[4 * first + 1];
+    float gain = a.gain[(size_t)first * a.H + h];
+    fill(0, t0, cnt);
+    to_shared();
+    for (int i = 0; i < count; ++i) {
+        const int c = first + i;
+        int next_t0 = 0, next_cnt = 0;
+        float next_gain = 0.0f;
+        if (i + 1 < count) {
+            next_t0 = a.chunk_meta[4 * (c + 1)];
+            next_cnt = a.chunk_meta[4 * (c + 1) + 1];
+            next_gain = a.gain[(size_t)(c + 1) * a.H + h];
+        }
+        lc_wait<0>();                            // the chunk's tiles, on their way since the chunk before
+        __syncthreads();                         // ... and S; nobody still reads the other tiles
+        if (i + 1 < count) fill(i + 1, next_t0, next_cnt);
         const float* sw = lc_smem + (i & 1) * TILE;
         const float* sk = sw + LC_C * LC_LD;
         float* su = const_cast<float*>(sk) + LC_C * LC_LD;
         const float* sr = su + LC_C * LU;
-        {   // rows 16 (warp % 4) of the chunk, columns 8 (warp / 4 % 2) + 16 j, channels DK / 2 side..
-            const int m0 = (warp & 3) * 16, n0 = ((warp >> 2) & 1) * 8;
+        {
+            const int m0 = (warp & 3) * 16, part = warp >> 2;
             float p[1][NT][4];
 #pragma unroll
             for (int x = 0; x < NT * 4; ++x) (&p[0][0][0])[x] = 0.0f;
 #pragma unroll
-            for (int k = 0; k < DK / 2; k += 8) {
-                const int k0 = side * (DK / 2) + k;
+            for (int k = 0; k < DK / 4; k += 8) {
+                const int k0 = part * (DK / 4) + k;
                 const LcA fa = lc_a_rows(sw + m0 * LC_LD + k0, LC_LD);
                 LcB fb[NT];
 #pragma unroll
-                for (int j = 0; j < NT; ++j) fb[j] = lc_b_rows(sS + (n0 + 16 * j) * LC_LD + k0, LC_LD);
+                for (int j = 0; j < NT; ++j) {
+                    const float2 x = *reinterpret_cast<const float2*>(sS + (8 * j + g) * LC_LD + k0 + 2 * t);
+                    const float2 y = *reinterpret_cast<const float2*>(sS + (NS + 8 * j + g) * LC_LD + k0 + 2 * t);
+                    fb[j] = LcB{{lc_split(x.x + y.x), lc_split(x.y + y.y)}};
+                }
                 lc_products<1, NT>(p, &fa, fb);
             }
 #pragma unroll
             for (int j = 0; j < NT; ++j)
 #pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                    const int at = (m0 + g + 8 * (x >> 1)) * LU + n0 + 16 * j + 2 * t + (x & 1);
-                    if (side == 0) su[at] -= p[0][j][x];
-                    else sp[at] = p[0][j][x];
-                }
+                for (int half = 0; half < 2; ++half)
+                    *reinterpret_cast<float2*>(sp + (part * LC_C + m0 + g + 8 * half) * LQ + 8 * j + 2 * t) =
+                        make_float2(p[0][j][2 * half], p[0][j][2 * half + 1]);
+        }
+        to_global(a.states + ((size_t)c * a.H + h) * a.dv * a.dk, true);
+        __syncthreads();
+        if (threadIdx.x < LC_C * (NS / 4)) {
+            const int row = threadIdx.x / (NS / 4), col = (threadIdx.x % (NS / 4)) * 4;
+            float4 u = *reinterpret_cast<const float4*>(su + row * LU + col);
+#pragma unroll
+            for (int part = 0; part < 4; ++part) {
+                const float4 x = *reinterpret_cast<const float4*>(sp + (part * LC_C + row) * LQ + col);
+                u = make_float4(u.x - x.x, u.y - x.y, u.z - x.z, u.w - x.w);
+            }
+            *reinterpret_cast<float4*>(su + row * LU + col) = u;
+            if (row < cnt && col < cols) *reinterpret_cast<float4*>(a.u + ((size_t)(t0 + row) * a.H + h) * a.dv + n_base + col) = u;
         }
         __syncthreads();
         if (has_rows) {
@@ -662,14 +703,12 @@ __global__ void __launch_bounds__(LC_CARRY_THREADS) lc_delta_carry_kernel(LcArgs
 #pragma unroll
             for (int x = 0; x < NT * 4; ++x) (&p[0][0][0])[x] = 0.0f;
 #pragma unroll
-            for (int k0 = 0; k0 < LC_C; k0 += 8) {
+            for (int k = 0; k < LC_C / 2; k += 8) {
+                const int k0 = side * (LC_C / 2) + k;
                 const LcA fa = lc_a_cols(sk + k0 * LC_LD + s_row, LC_LD, sr[k0 + t], sr[k0 + t + 4]);
                 LcB fb[NT];
 #pragma unroll
-                for (int j = 0; j < NT; ++j) {
-                    const int at = (k0 + t) * LU + 8 * side + 16 * j + g;
-                    fb[j] = LcB{{lc_split(su[at] - sp[at]), lc_split(su[at + 4 * LU] - sp[at + 4 * LU])}};
-                }
+                for (int j = 0; j < NT; ++j) fb[j] = lc_b_cols(su + k0 * LU + 8 * j, LU);
                 lc_products<1, NT>(p, &fa, fb);
             }
 #pragma unroll
@@ -677,14 +716,14 @@ __global__ void __launch_bounds__(LC_CARRY_THREADS) lc_delta_carry_kernel(LcArgs
 #pragma unroll
                 for (int x = 0; x < 4; ++x) S[j][x] = fmaf(gain, S[j][x], p[0][j][x]);
         }
-        for (int idx = threadIdx.x; idx < LC_C * NS; idx += LC_CARRY_THREADS) {
-            const int m = idx / NS, n = idx % NS;
-            if (m < cnt && n < cols) a.u[((size_t)(t0 + m) * a.H + h) * a.dv + n_base + n] = su[m * LU + n] - sp[m * LU + n];
-        }
-        if (i + 1 < count) publish(a.states + ((size_t)(c + 1) * a.H + h) * a.dv * a.dk, true);
-        __syncthreads();                         // the tiles may be filled again, S is whole
+        to_shared();                             // read by everyone before the pass over U
+        t0 = next_t0;
+        cnt = next_cnt;
+        gain = next_gain;
     }
-    publish(a.state + (size_t)a.slots[r] * a.state_stride + (size_t)h * a.dv * a.dk, false);
+    __syncthreads();
+    float* st = a.state + (size_t)a.slots[r] * a.state_stride + (size_t)h * a.dv * a.dk;
+    to_global(st, ((uintptr_t)st & 15) == 0);
 }
 
 // ---- a forget gate per key channel (csrc/linear_state.cu): k_t = 1 - f_t, S_t = diag(f_t) S_(t-1) + k_t v_t^T -------------------------
@@ -915,15 +954,15 @@ static int lc_run(const LcArgs& a, int n_requests, cudaStream_t s) {
     if (a.beta == nullptr) {
         if (const int rc = lc_launch(lc_state_kernel<DK, DV>, chunks, 256, 2 * tile, s, a)) return rc;
         const long long size = (long long)a.H * a.dv * a.dk;
-        if (const int rc = lc_launch(lc_carry_kernel<false>, dim3(ceil_div(size, 256), n_requests), 256, 0, s, a)) return rc;
+        if (const int rc = lc_launch(lc_carry_kernel<false>, dim3(ceil_div(size / 4, 256), n_requests), 256, 0, s, a)) return rc;
         return lc_launch(lc_output_kernel<DK, DV>, chunks, 256, 3 * tile, s, a, a.v, (size_t)a.ldv);
     }
     if (const int rc = lc_launch(lc_delta_prepare_kernel<DK, DV>, chunks, 256, 2 * tile + 2 * square, s, a)) return rc;
-    // columns of S per block: 16 while the blocks then fit the SMs (one each: 166 KB), else 32, whose chain is a little longer
+    // columns of S per block: 16 while the blocks then fit the SMs (one each: 186 KB), else 32, whose chain is a little longer
     const bool wide = (long long)ceil_div(a.dv, 16) * a.H * n_requests > 148 && a.dv > 16;
 #define LC_CARRY(NS)                                                                                                                       \
     lc_launch(lc_delta_carry_kernel<DK, NS>, dim3(ceil_div(a.dv, NS), a.H, n_requests), LC_CARRY_THREADS,                                   \
-              (size_t)(2 * (2 * LC_C * LC_LD + LC_C * (NS + 8) + LC_C + 4) + NS * LC_LD + LC_C * (NS + 8)) * sizeof(float), s, a)
+              (size_t)(2 * (2 * LC_C * LC_LD + LC_C * (NS + 8) + LC_C + 4) + 2 * NS * LC_LD + 4 * LC_C * (NS + 4)) * sizeof(float), s, a)
     if (const int rc = wide ? LC_CARRY(32) : LC_CARRY(16)) return rc;
 #undef LC_CARRY
     return lc_launch(lc_output_kernel<DK, DV>, chunks, 256, 3 * tile, s, a, (const float*)a.u, (size_t)a.H * a.dv);
@@ -971,7 +1010,7 @@ static int lc_run_forget(const LcArgs& a, int n_requests, cudaStream_t s) {
     const size_t tile = LC_C * LC_LD * sizeof(float);
     if (const int rc = lc_launch(lc_forget_state_kernel<DK, DV>, chunks, 256, 2 * tile, s, a)) return rc;
     const long long size = (long long)a.H * a.dv * a.dk;
-    if (const int rc = lc_launch(lc_carry_kernel<true>, dim3(ceil_div(size, 256), n_requests), 256, 0, s, a)) return rc;
+    if (const int rc = lc_launch(lc_carry_kernel<true>, dim3(ceil_div(size / 4, 256), n_requests), 256, 0, s, a)) return rc;
     return lc_launch(lc_forget_output_kernel<DK, DV>, chunks, 256, 3 * tile, s, a);
 }
 
