@@ -274,8 +274,8 @@ __global__ void __launch_bounds__(256) lc_carry_kernel(LcArgs a) {
 }
 
 // ---- the outputs of a chunk: diag(gamma) Q S + (Q K^T, decayed and masked) U --------------------------------------------------
-// Two blocks per SM (104 KB each): q, and two buffers through which half of S, the other half, k (then the decayed scores) and u
-// pass, each on its way while the one before it is multiplied.  Bound by the tensor cores.
+// Two blocks per SM (104 KB each): q, and two buffers, first for the halves of S, then for k (later the decayed scores) and u.  Bound by the
+// tensor cores and by issuing what splits their operands.
 template <int DK, int DV>
 __global__ void __launch_bounds__(256, 2) lc_output_kernel(LcArgs a, const float* __restrict__ values, size_t ldu) {
     extern __shared__ __align__(16) float lc_smem[];
@@ -300,27 +300,25 @@ __global__ void __launch_bounds__(256, 2) lc_output_kernel(LcArgs a, const float
     float acc[HALVES][2][2][4];                  // [half of dv][16 rows][8 columns]
 #pragma unroll
     for (int x = 0; x < HALVES * 16; ++x) (&acc[0][0][0][0])[x] = 0.0f;
-    auto times_state = [&](const float* s, float (*o)[2][4]) {
-#pragma unroll 2
-        for (int k0 = 0; k0 < DK; k0 += 8) {
-            LcA fa[2];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows(sq + (m0 + 16 * i) * LC_LD + k0, LC_LD);
-            const LcB fb[2] = {lc_b_rows(s + wn * 16 * LC_LD + k0, LC_LD), lc_b_rows(s + (wn * 16 + 8) * LC_LD + k0, LC_LD)};
-            lc_products<2, 2>(o, fa, fb);
-        }
-    };
-    lc_wait<1>();
+    if (DV > 64) lc_wait<0>();
+    else lc_wait<1>();
     __syncthreads();
-    times_state(sa, acc[0]);
+#pragma unroll 2
+    for (int k0 = 0; k0 < DK; k0 += 8) {         // (both halves of S with one reading of q)
+        LcA fa[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows(sq + (m0 + 16 * i) * LC_LD + k0, LC_LD);
+#pragma unroll
+        for (int b = 0; b < HALVES; ++b) {
+            const float* p = (b == 0 ? sa : su) + wn * 16 * LC_LD + k0;
+            const LcB fb[2] = {lc_b_rows(p, LC_LD), lc_b_rows(p + 8 * LC_LD, LC_LD)};
+            lc_products<2, 2>(acc[b], fa, fb);
+        }
+    }
     __syncthreads();
     lc_load<DK, LC_LD>(sa, a.k + (size_t)t0 * a.ldk + (size_t)kh * a.dk, a.ldk, cnt, a.dk);
     lc_commit();
     if (DV > 64) {
-        lc_wait<1>();
-        __syncthreads();
-        times_state(su, acc[HALVES - 1]);
-        __syncthreads();
         lc_load<DV, LC_LD>(su, up, ldu, cnt, a.dv);
         lc_commit();
         lc_wait<1>();

@@ -271,6 +271,82 @@ __global__ void linear_state_prep_kernel(float* __restrict__ x, int ld, int q_of
     }
 }
 
+// The same for heads of 64 or 128 numbers that are turned whole or not at all: a head is four numbers per lane of LANES lanes, the other half
+// of a pair LANES / 2 lanes away, and a warp has four times 32 / LANES heads on their way at once.  Bound by memory: 3,000 tokens, 2 x 32
+// heads of 128 turned (196 MB) 54 us through shared memory one number at a time, 28 us so.  A block has as many tokens as fill
+// its four rounds: with one token of 2 x 4 heads per block (4,096 tokens, 33 MB) the latency of a round is all there is, 18.5 us, now 13.
+// (ONE: a block's only token's angles are read once.)
+#define PREP_RUN 4
+template <int LANES, bool ONE>
+__global__ void __launch_bounds__(256) linear_state_prep4_kernel(float* __restrict__ x, int ld, int n_tokens, int tokens, int q_off, int k_off, int v_off, int Gq, int n_v, int act,
+                                                                 const float2* __restrict__ rot, int unit, float unit_eps, float q_scale,
+                                                                 float k_scale, const float* __restrict__ gx, int gld, int a_off, int b_off, int H,
+                                                                 const float* __restrict__ A_log, const float* __restrict__ dt_bias,
+                                                                 float* __restrict__ gate, float* __restrict__ beta) {
+    constexpr int DK = 4 * LANES, SLOTS = 8 * (32 / LANES), RUN = PREP_RUN;      // heads that the block's warps have at a time; how many times
+    const int lane = threadIdx.x % LANES, slot = threadIdx.x / LANES, t0 = blockIdx.x * tokens, n = min(tokens, n_tokens - t0);
+    const float side = lane < LANES / 2 ? -1.0f : 1.0f;
+    constexpr int ANGLES = ONE ? 1 : RUN;
+    float4 c0[ANGLES], c1[ANGLES];                                        // (cos, sin) of the lane's four pairs
+    c0[0] = c1[0] = make_float4(1.0f, 0.0f, 1.0f, 0.0f);
+    if (ONE && rot) {
+        const float4* cs = reinterpret_cast<const float4*>(rot + (size_t)t0 * (DK / 2) + (lane % (LANES / 2)) * 4);
+        c0[0] = cs[0];
+        c1[0] = cs[1];
+    }
+    for (int base = 0; base < n * 2 * Gq; base += RUN * SLOTS) {
+        float4 v[RUN];
+        float* at[RUN];
+        bool query[RUN];
+#pragma unroll
+        for (int u = 0; u < RUN; ++u) {
+            const int item = base + u * SLOTS + slot, t = ONE ? 0 : item / (2 * Gq), vec = item - t * 2 * Gq;
+            query[u] = vec < Gq;
+            at[u] = item < n * 2 * Gq ? x + (size_t)(t0 + t) * ld + (query[u] ? q_off + vec * DK : k_off + (vec - Gq) * DK) + lane * 4 : nullptr;
+            v[u] = at[u] != nullptr ? *reinterpret_cast<const float4*>(at[u]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (!ONE && rot && at[u] != nullptr) {
+                const float4* cs = reinterpret_cast<const float4*>(rot + (size_t)(t0 + t) * (DK / 2) + (lane % (LANES / 2)) * 4);
+                c0[ONE ? 0 : u] = cs[0];
+                c1[ONE ? 0 : u] = cs[1];
+            } else if (!ONE) {
+                c0[ONE ? 0 : u] = c1[ONE ? 0 : u] = make_float4(1.0f, 0.0f, 1.0f, 0.0f);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < RUN; ++u) {
+            float4 y = v[u];
+            if (act) y = make_float4(ls_silu(y.x), ls_silu(y.y), ls_silu(y.z), ls_silu(y.w));
+            if (rot) {
+                const float px = __shfl_xor_sync(0xffffffffu, y.x, LANES / 2), py = __shfl_xor_sync(0xffffffffu, y.y, LANES / 2);
+                const float pz = __shfl_xor_sync(0xffffffffu, y.z, LANES / 2), pw = __shfl_xor_sync(0xffffffffu, y.w, LANES / 2);
+                y = make_float4(y.x * c0[ONE ? 0 : u].x + side * px * c0[ONE ? 0 : u].y, y.y * c0[ONE ? 0 : u].z + side * py * c0[ONE ? 0 : u].w, y.z * c1[ONE ? 0 : u].x + side * pz * c1[ONE ? 0 : u].y,
+                                y.w * c1[ONE ? 0 : u].z + side * pw * c1[ONE ? 0 : u].w);
+            }
+            float f = query[u] ? q_scale : k_scale;
+            if (unit) {
+                float ss = fmaf(y.x, y.x, y.y * y.y) + fmaf(y.z, y.z, y.w * y.w);
+#pragma unroll
+                for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                f *= 1.0f / sqrtf(ss + unit_eps);
+            }
+            if (at[u] != nullptr) *reinterpret_cast<float4*>(at[u]) = make_float4(y.x * f, y.y * f, y.z * f, y.w * f);
+        }
+    }
+    if (act)
+        for (int t = t0; t < t0 + n; ++t)
+            for (int d = threadIdx.x * 4; d < n_v; d += 1024) {
+                float4* p = reinterpret_cast<float4*>(x + (size_t)t * ld + v_off + d);
+                const float4 y = *p;
+                *p = make_float4(ls_silu(y.x), ls_silu(y.y), ls_silu(y.z), ls_silu(y.w));
+            }
+    for (int i = threadIdx.x; i < n * H; i += 256) {
+        const int t = t0 + i / H, h = i % H;
+        const float* grow = gx + (size_t)t * gld;
+        if (a_off >= 0) gate[(size_t)t * H + h] = expf(-expf(A_log[h]) * ls_softplus(grow[a_off + h] + dt_bias[h]));
+        if (b_off >= 0) beta[(size_t)t * H + h] = ls_sigmoid(grow[b_off + h]);
+    }
+}
+
 MM_EXPORT int mm_linear_state_prep(void* x, int ld, int n_tokens, int q_off, int k_off, int v_off, int Gq, int dk, int n_v, int act,
                                    const void* rot, int rot_dims, int unit, float unit_eps, float q_scale, float k_scale, const void* gx,
                                    int gld, int a_off, int b_off, int H, const void* A_log, const void* dt_bias, void* gate, void* beta,
@@ -286,6 +362,17 @@ MM_EXPORT int mm_linear_state_prep(void* x, int ld, int n_tokens, int q_off, int
     if (a_off < 0 && b_off < 0) H = 0;
     if (n_tokens == 0) return MM_OK;
     MM_REQUIRE(dk <= 1024, "linear state prep: key sizes above 1024 are not supported");
+    if ((dk == 64 || dk == 128) && (rot_dims == 0 || rot_dims == dk) && ld % 4 == 0 && q_off % 4 == 0 && k_off % 4 == 0 && v_off % 4 == 0 && n_v % 4 == 0 &&
+        (((uintptr_t)x | (uintptr_t)rot) & 15) == 0) {
+        const int heads = PREP_RUN * (dk == 64 ? 16 : 8), tokens = heads / (2 * Gq) > 1 ? heads / (2 * Gq) : 1;
+        auto kernel = dk == 64 ? (tokens == 1 ? linear_state_prep4_kernel<16, true> : linear_state_prep4_kernel<16, false>)
+                               : (tokens == 1 ? linear_state_prep4_kernel<32, true> : linear_state_prep4_kernel<32, false>);
+        mm_launch(kernel, dim3(ceil_div(n_tokens, tokens)), dim3(256), 0,
+                  (cudaStream_t)stream, (float*)x, ld, n_tokens, tokens, q_off, k_off, v_off, Gq, n_v, act, rot_dims ? (const float2*)rot : (const float2*)nullptr, unit, unit_eps, q_scale, k_scale, (const float*)gx,
+                  gld, a_off, b_off, H, (const float*)A_log, (const float*)dt_bias, (float*)gate, (float*)beta);
+        MM_CHECK_LAUNCH();
+        return MM_OK;
+    }
     mm_launch(linear_state_prep_kernel, dim3(n_tokens), dim3(256), (size_t)8 * dk * sizeof(float), (cudaStream_t)stream, (float*)x, ld, q_off, k_off, v_off, Gq, dk, n_v, act,
               (const float2*)rot, rot_dims, unit, unit_eps, q_scale, k_scale, (const float*)gx, gld, a_off, b_off, H, (const float*)A_log,
               (const float*)dt_bias,

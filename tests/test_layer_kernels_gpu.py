@@ -116,3 +116,76 @@ def test_weighted_sum_of_experts(d, top, weighed):
     rows = y[place.long()].double().view(n, top, d)
     want = (rows * (w.double()[:, :, None] if weighed else 1.0)).sum(1)
     assert (got.double() - want).abs().max() <= 2.0 ** -8 * want.abs().max()
+
+
+@pytest.mark.parametrize("dk", [64, 128, 72])
+@pytest.mark.parametrize("Gq", [1, 3, 40])
+@pytest.mark.parametrize("rot,act,unit", [(True, False, False), (False, True, True), (True, True, True)])
+def test_preparation_of_a_matrix_state(dk, Gq, rot, act, unit):
+    from mimirmind_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(dk + Gq)
+    n, H, n_v = 5, 6, 36
+    q_off, k_off, v_off = 4, 4 + Gq * dk, 4 + 2 * Gq * dk
+    a_off, b_off = v_off + n_v, v_off + n_v + H
+    x = torch.randn((n, b_off + H + 4), generator=gen, device=DEV)
+    before = x.double()
+    angles = torch.randn((n, dk // 2), generator=gen, device=DEV) * 3
+    table = torch.stack([angles.cos(), angles.sin()], dim=-1).contiguous()
+    A, dt = torch.randn(H, generator=gen, device=DEV), torch.randn(H, generator=gen, device=DEV)
+    gate, beta = ops.linear_state_prep(x, q_off, k_off, v_off, Gq, dk, n_v, silu=act, rot=table if rot else None, rot_dims=dk if rot else 0, unit=unit,
+                                       unit_eps=1e-6, q_scale=0.3, k_scale=2.0, a_off=a_off, b_off=b_off, heads=H, A_log=A, dt_bias=dt)
+    f = torch.nn.functional.silu if act else (lambda t: t)
+    want = before.clone()
+    for off, scale in ((q_off, 0.3), (k_off, 2.0)):
+        y = f(before[:, off:off + Gq * dk]).view(n, Gq, dk)
+        if rot:
+            a, b = y.chunk(2, dim=-1)
+            c, s = table[:, None, :, 0].double(), table[:, None, :, 1].double()
+            y = torch.cat([a * c - b * s, b * c + a * s], dim=-1)
+        if unit:
+            y = y / torch.sqrt((y * y).sum(-1, keepdim=True) + 1e-6)
+        want[:, off:off + Gq * dk] = (y * scale).reshape(n, -1)
+    want[:, v_off:v_off + n_v] = f(before[:, v_off:v_off + n_v])
+    # a dozen roundings of 2^-24 on numbers up to the largest
+    assert (x - want).abs().max() <= 2e-6 * want.abs().max()
+    assert torch.allclose(gate.double(), torch.exp(-A.double().exp() * torch.nn.functional.softplus(before[:, a_off:a_off + H] + dt.double())), rtol=3e-6, atol=1e-7)
+    assert torch.allclose(beta.double(), torch.sigmoid(before[:, b_off:b_off + H]), rtol=1e-6, atol=1e-7)
+
+
+@pytest.mark.parametrize("dk,dv", [(64, 128), (128, 64), (36, 20), (10, 6)])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_rows_cut_into_queries_keys_and_values(dk, dv, dt):
+    from mimirmind_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(dk)
+    n, Hq, Gk, Gv, page = 21, 12, 4, 2, 8
+    x = torch.randn((n, Hq * dk + Gk * dk + Gv * dv + 4), generator=gen, device=DEV)
+    q_off, k_off, v_off = 4, 4 + Hq * dk, 4 + (Hq + Gk) * dk
+    slots = torch.randperm(64, generator=gen, device=DEV)[:n].to(torch.int32)
+    slots[3] = -1
+    q = torch.empty((n, Hq * dk), dtype=dt, device=DEV)
+    k, v = torch.zeros((8, Gk, page, dk), dtype=dt, device=DEV), torch.zeros((8, Gv, page, dv), dtype=dt, device=DEV)
+    ops.qkv_split_post(x, q_off, k_off, v_off, q, k, v, slots, page, Hq, Gk, dk, Gv, dv)
+    assert torch.equal(q, x[:, q_off:k_off].to(dt))
+    wk, wv = torch.zeros_like(k), torch.zeros_like(v)
+    for t, s in enumerate(slots.tolist()):
+        if s >= 0:
+            wk[s // page, :, s % page] = x[t, k_off:v_off].to(dt).view(Gk, dk)
+            wv[s // page, :, s % page] = x[t, v_off:v_off + Gv * dv].to(dt).view(Gv, dv)
+    assert torch.equal(k, wk) and torch.equal(v, wv)
+
+
+@pytest.mark.parametrize("dv", [64, 128, 256, 96])
+@pytest.mark.parametrize("pair,gated,out", [(True, True, torch.bfloat16), (False, False, torch.float32), (True, False, torch.float32)])
+def test_heads_finished(dv, pair, gated, out):
+    from mimirmind_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(dv)
+    n, H = 13, 5
+    att = torch.randn((n, (2 if pair else 1) * H * dv), generator=gen, device=DEV)
+    gate = torch.randn((n, H + 3), generator=gen, device=DEV)[:, 1:1 + H] if gated else None
+    got = ops.head_finish(att, H, dv, pair=pair, lam=0.37, eps=1e-5, post=0.5, gate=gate, out_dtype=out)
+    x = att.double().view(n, -1, dv)
+    o = x[:, :H] - (0.37 * x[:, H:] if pair else 0.0)
+    o = 0.5 * o / torch.sqrt((o * o).mean(-1, keepdim=True) + 1e-5)
+    if gated:
+        o = o * torch.sigmoid(gate.double())[:, :, None]
+    assert (got.double() - o.reshape(n, -1)).abs().max() <= (2.0 ** -8 if out == torch.bfloat16 else 3e-6) * o.abs().max()
