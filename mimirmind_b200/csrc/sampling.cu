@@ -804,7 +804,9 @@ sample_rows_kernel(const float* __restrict__ logits, int32_t* __restrict__ out, 
     const float max_logit = logit_of_key((uint32_t)(best >> 32));
     const float inv_t = 1.0f / T;
     const float max_scaled = max_logit * inv_t;
-    const bool plain = cluster_combine(c, has_nan ? 1ull : 0ull, true) == 0ull && isfinite(max_scaled) && isfinite(inv_t) && inv_t > 0.0f;
+    // At or beyond 2^16 the rounding of max_scaled lets weights of the largest logits exceed FIXED_ONE by more than the 32-bit sums
+    // of the histograms have room for; NaN and infinities are not below it.
+    const bool plain = cluster_combine(c, has_nan ? 1ull : 0ull, true) == 0ull && fabsf(max_scaled) < 65536.0f && isfinite(inv_t) && inv_t > 0.0f;
     const DrawBins bins{inv_t, max_scaled};
 
     // top-k: everything at or above the k-th largest logit stays

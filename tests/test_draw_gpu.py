@@ -79,3 +79,20 @@ def test_a_row_with_a_nan_or_an_infinite_logit_leaves_the_others_alone():
     x[2, 5] = math.inf
     got = ops.sample_rows(x, *args).cpu().tolist()
     assert got[0] == want[0] and got[3] == want[3] and all(0 <= v < 20000 for v in got)
+
+
+@pytest.mark.parametrize("T", [1e-3, 1e-5, 1e-6])
+@pytest.mark.parametrize("R,V", [(150, 33000), (5, 152064)])
+def test_equal_logits_at_a_very_low_temperature(R, V, T):
+    """logit / T - max / T is then off zero by its rounding: every weight is above one, and their sums have to hold them.  (At 1e-6 the
+    rounding is at most 1, V e 2^40 < 2^59; at 1e-7 it may be 8, and 33000 e^8 2^40 is beyond the 64 bits of the total.)"""
+    from mimirmind_b200.kernels import ops
+    rng = np.random.RandomState(11)
+    logits = np.repeat(rng.uniform(1.0, 20.0, size=(R, 1)).astype(np.float32), V, axis=1)
+    seeds, counters = rng.randint(1, 2 ** 31, size=R), rng.randint(0, 1000, size=R)
+    t = lambda a, dt: torch.tensor(a, dtype=dt, device=DEV)                  # noqa: E731
+    got = ops.sample_rows(t(logits, torch.float32), torch.full((R,), T, device=DEV), torch.zeros(R, dtype=torch.int32, device=DEV),
+                          torch.ones(R, device=DEV), t(seeds, torch.int64), t(counters, torch.int64)).cpu().tolist()
+    for r in range(R):          # equal weights: the share of token i is [i, i+1) / V; u has 24 or more bits, the product rounds once
+        u = plain.uniform_from(int(seeds[r]), int(counters[r]))
+        assert abs(got[r] - u * V) <= 1.0 + 1e-6 * V, (r, T, got[r], u * V)
