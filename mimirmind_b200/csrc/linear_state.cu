@@ -457,6 +457,7 @@ __global__ void __launch_bounds__(128) linear_state_walk_kernel(
     // MODE 1, 2: r is a chunk, req_meta the chunk list (first token, tokens, ., .), state the scratch with one matrix set per chunk
     const int t0 = req_meta ? req_meta[4 * r] : r;
     const int n = req_meta ? req_meta[4 * r + 1] : 1;
+    if (n <= 0) return;                            // (another kernel takes this request)
     float* st[CPT];
 #pragma unroll
     for (int c = 0; c < CPT; ++c)
@@ -829,6 +830,7 @@ __global__ void __launch_bounds__(256) forget_gate_walk_kernel(const float* __re
     const bool col_ok = col < dv;
     const int t0 = req_meta ? req_meta[4 * r] : r;
     const int n = req_meta ? req_meta[4 * r + 1] : 1;
+    if (n <= 0) return;                            // (another kernel takes this request)
     const bool fresh = MODE == 1 || (MODE == 0 && positions[t0] == 0);
     // MODE 1, 2: r is a chunk, req_meta the chunk list, state the scratch with one set of matrices per chunk
     float* st = state + (size_t)(MODE == 0 ? slots[r] : r) * state_stride + ((size_t)h * dv + (col_ok ? col : 0)) * dk;

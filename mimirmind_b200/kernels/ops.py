@@ -1055,14 +1055,35 @@ def linear_state_prep(x: torch.Tensor, q_off: int, k_off: int, v_off: int, qk_he
     return gate, beta
 
 
+def _rows_for(out: Optional[torch.Tensor], n: int, width: int, like: torch.Tensor) -> torch.Tensor:
+    """``out`` checked, or new fp32 rows [n, width]."""
+    if out is None:
+        return torch.empty((n, width), dtype=torch.float32, device=like.device)
+    _need(out, "out", torch.float32)
+    if out.shape != (n, width):
+        raise KernelError("out: shape mismatch")
+    return out
+
+
+def _scratch(sizes, device):
+    """One fp32 allocation for arrays of ``sizes`` numbers: (tensor, address of each, on 16-byte boundaries)."""
+    starts, total = [], 0
+    for size in sizes:
+        starts.append(4 * total)
+        total += (size + 3) // 4 * 4
+    t = torch.empty(max(4, total), dtype=torch.float32, device=device)
+    base = t.data_ptr()
+    return t, [base + s for s in starts]
+
+
 def linear_state_walk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, req_meta: Optional[torch.Tensor],
                       slots: torch.Tensor, positions: torch.Tensor, n_requests: int, heads: int, qk_heads: int, dk: int, dv: int,
                       gate: Optional[torch.Tensor] = None, beta: Optional[torch.Tensor] = None,
-                      head_decay: Optional[torch.Tensor] = None) -> torch.Tensor:
+                      head_decay: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Per head ``S <- g S; u = v`` (or ``beta (v - S^T k)`` when ``beta`` is given); ``S <- S + k u^T; o = S^T q`` over each
     request's tokens in order.  q, k: fp32 column slices [n, qk_heads * dk], v [n, heads * dv] (any row stride);
     ``gate`` [n, heads] or ``head_decay`` [heads]; ``state`` [slots, stride] fp32 holds S as [heads, dv, dk] at its start
-    and is left updated.  Returns o fp32 [n, heads * dv]."""
+    and is left updated.  Returns o fp32 [n, heads * dv], or fills ``out``; a request of 0 tokens is left alone."""
     for t, what in ((q, "q"), (k, "k"), (v, "v")):
         if t.dtype != torch.float32 or not t.is_cuda or t.stride(1) != 1:
             raise KernelError(f"linear state {what}: fp32 rows with unit column stride are needed")
@@ -1080,7 +1101,7 @@ def linear_state_walk(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: 
         _need(head_decay, "head decay", torch.float32)
     _need(slots, "state slots", torch.int32)
     _need(positions, "positions", torch.int32)
-    out = torch.empty((n, heads * dv), dtype=torch.float32, device=q.device)
+    out = _rows_for(out, n, heads * dv, q)
     check(_lib.load().mm_linear_state_walk(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0), _ptr(gate),
                                            _ptr(beta), _ptr(head_decay), out.data_ptr(), state.data_ptr(), state.stride(0), _ptr(req_meta),
                                            slots.data_ptr(), positions.data_ptr(), int(n_requests), heads, qk_heads, dk, dv, _stream()),
@@ -1133,10 +1154,10 @@ def linear_state_products_supported(q: torch.Tensor, k: torch.Tensor, v: torch.T
 def linear_state_products(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, chunk_meta: torch.Tensor,
                           req_chunks: torch.Tensor, slots: torch.Tensor, positions: torch.Tensor, heads: int, qk_heads: int, dk: int, dv: int,
                           gate: Optional[torch.Tensor] = None, beta: Optional[torch.Tensor] = None,
-                          head_decay: Optional[torch.Tensor] = None) -> torch.Tensor:
+                          head_decay: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The recurrence of ``linear_state_walk`` (with or without the delta rule) for long portions, as products of matrices over
     chunks of at most ``LINEAR_CHUNK`` tokens.  ``chunk_meta`` [chunks, 4] = (first token, tokens, request, .), ``req_chunks``
-    [requests, 2] = (first chunk, chunks); the decays are 0 or positive."""
+    [requests, 2] = (first chunk, chunks), 0 chunks for a request that is left alone; the decays are 0 or positive."""
     for t, what in ((q, "q"), (k, "k"), (v, "v")):
         if t.dtype != torch.float32 or not t.is_cuda or t.stride(1) != 1:
             raise KernelError(f"linear state {what}: fp32 rows with unit column stride are needed")
@@ -1157,18 +1178,17 @@ def linear_state_products(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, sta
     for t, what in ((chunk_meta, "chunk_meta"), (req_chunks, "req_chunks"), (slots, "state slots"), (positions, "positions")):
         _need(t, what, torch.int32)
     n_chunks, n_req = chunk_meta.shape[0], req_chunks.shape[0]
-    out = torch.empty((n, heads * dv), dtype=torch.float32, device=q.device)
-    states = torch.empty((max(1, n_chunks), heads * dv * dk), dtype=torch.float32, device=q.device)
-    gain = torch.empty((max(1, n_chunks), heads), dtype=torch.float32, device=q.device)
-    ratio = w = u = None
+    out = _rows_for(out, n, heads * dv, q)
+    # states [chunks, heads, dv, dk], gain [chunks, heads], with the delta rule ratio [chunks, heads, 64], w [n, heads, dk], u [n, heads, dv]
+    sizes = [n_chunks * heads * dv * dk, n_chunks * heads]
     if beta is not None:
-        ratio = torch.empty((max(1, n_chunks), heads, LINEAR_CHUNK), dtype=torch.float32, device=q.device)
-        w = torch.empty((n, heads * dk), dtype=torch.float32, device=q.device)
-        u = torch.empty((n, heads * dv), dtype=torch.float32, device=q.device)
+        sizes += [n_chunks * heads * LINEAR_CHUNK, n * heads * dk, n * heads * dv]
+    _kept, parts = _scratch(sizes, q.device)
+    states, gain, ratio, w, u = parts + [None] * (5 - len(parts))
     check(_lib.load().mm_linear_chunk(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0), _ptr(gate), _ptr(beta),
                                       _ptr(head_decay), out.data_ptr(), state.data_ptr(), state.stride(0), chunk_meta.data_ptr(),
                                       req_chunks.data_ptr(), slots.data_ptr(), positions.data_ptr(), n_req, n_chunks, heads, qk_heads, dk, dv,
-                                      states.data_ptr(), gain.data_ptr(), _ptr(ratio), _ptr(w), _ptr(u), _stream()), "linear_chunk")
+                                      states, gain, ratio, w, u, _stream()), "linear_chunk")
     return out
 
 
@@ -1673,10 +1693,11 @@ def forget_gate_prep(x: torch.Tensor, q_off: int, f_off: int, n_qf: int, bias: O
 
 
 def forget_gate_walk(q: torch.Tensor, f: torch.Tensor, v: torch.Tensor, state: torch.Tensor, req_meta: Optional[torch.Tensor],
-                     slots: torch.Tensor, positions: torch.Tensor, n_requests: int, heads: int, dk: int, dv: int) -> torch.Tensor:
+                     slots: torch.Tensor, positions: torch.Tensor, n_requests: int, heads: int, dk: int, dv: int,
+                     out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Per head ``S <- diag(f) S + (1 - f) v^T; o = S^T q`` over each request's tokens in order.  q, f: fp32 column slices
     [n, heads * dk], v [n, heads * dv] (any row stride); ``state`` [slots, stride] fp32 holds S as [heads, dv, dk] at its
-    start and is left updated.  Returns o fp32 [n, heads * dv]."""
+    start and is left updated.  Returns o fp32 [n, heads * dv], or fills ``out``; a request of 0 tokens is left alone."""
     for t, what in ((q, "q"), (f, "f"), (v, "v")):
         if t.dtype != torch.float32 or not t.is_cuda or t.stride(1) != 1:
             raise KernelError(f"forget gate walk {what}: fp32 rows with unit column stride are needed")
@@ -1687,7 +1708,7 @@ def forget_gate_walk(q: torch.Tensor, f: torch.Tensor, v: torch.Tensor, state: t
         raise KernelError("forget gate walk: the state is fp32 [slots, >= heads * dv * dk]")
     _need(slots, "state slots", torch.int32)
     _need(positions, "positions", torch.int32)
-    out = torch.empty((n, heads * dv), dtype=torch.float32, device=q.device)
+    out = _rows_for(out, n, heads * dv, q)
     check(_lib.load().mm_forget_gate_walk(q.data_ptr(), f.data_ptr(), v.data_ptr(), q.stride(0), f.stride(0), v.stride(0), out.data_ptr(),
                                           state.data_ptr(), state.stride(0), _ptr(req_meta), slots.data_ptr(), positions.data_ptr(),
                                           int(n_requests), int(heads), int(dk), int(dv), _stream()), "forget_gate_walk")
@@ -1723,7 +1744,8 @@ def forget_gate_chunked(q: torch.Tensor, f: torch.Tensor, v: torch.Tensor, state
 
 
 def forget_gate_products(q: torch.Tensor, f: torch.Tensor, v: torch.Tensor, state: torch.Tensor, chunk_meta: torch.Tensor, req_chunks: torch.Tensor,
-                         slots: torch.Tensor, positions: torch.Tensor, heads: int, dk: int, dv: int) -> torch.Tensor:
+                         slots: torch.Tensor, positions: torch.Tensor, heads: int, dk: int, dv: int,
+                         out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The same for long portions as products of matrices over chunks of at most ``LINEAR_CHUNK`` tokens (what
     ``linear_state_products_supported`` says of q, f and v)."""
     for t, what in ((q, "q"), (f, "f"), (v, "v")):
@@ -1737,12 +1759,11 @@ def forget_gate_products(q: torch.Tensor, f: torch.Tensor, v: torch.Tensor, stat
     for t, what in ((chunk_meta, "chunk_meta"), (req_chunks, "req_chunks"), (slots, "state slots"), (positions, "positions")):
         _need(t, what, torch.int32)
     n_chunks, n_req = chunk_meta.shape[0], req_chunks.shape[0]
-    out = torch.empty((n, heads * dv), dtype=torch.float32, device=q.device)
-    states = torch.empty((max(1, n_chunks), heads * dv * dk), dtype=torch.float32, device=q.device)
-    gain = torch.empty((max(1, n_chunks), heads * dk), dtype=torch.float32, device=q.device)
+    out = _rows_for(out, n, heads * dv, q)
+    _kept, (states, gain) = _scratch([n_chunks * heads * dv * dk, n_chunks * heads * dk], q.device)
     check(_lib.load().mm_forget_gate_chunk(q.data_ptr(), f.data_ptr(), v.data_ptr(), q.stride(0), f.stride(0), v.stride(0), out.data_ptr(),
                                            state.data_ptr(), state.stride(0), chunk_meta.data_ptr(), req_chunks.data_ptr(), slots.data_ptr(),
-                                           positions.data_ptr(), n_req, n_chunks, int(heads), int(dk), int(dv), states.data_ptr(), gain.data_ptr(),
+                                           positions.data_ptr(), n_req, n_chunks, int(heads), int(dk), int(dv), states, gain,
                                            _stream()), "forget_gate_chunk")
     return out
 

@@ -27,7 +27,7 @@ One class covers the family; what differs between its members is a parameter:
 All input projections are one product with an fp32 result; everything between it and the output projection is fp32
 (``csrc/linear_state.cu``, ``csrc/linear_chunk.cu``, ``csrc/norm_gated.cu``).  A request's tokens are walked in order from its slot's
 state; long portions are cut into chunks whose outputs and states are products of matrices (head sizes these do not take: chunks that are
-walked side by side, with the delta rule the walk), except in float32 runs, which keep one order of operations whatever the cutting.  q and k have ``qk_heads`` heads; head h reads q/k head ``h // (heads / qk_heads)``.
+walked side by side, with the delta rule the walk; short portions beside long ones are walked), except in float32 runs, which keep one order of operations whatever the cutting.  q and k have ``qk_heads`` heads; head h reads q/k head ``h // (heads / qk_heads)``.
 """
 from __future__ import annotations
 
@@ -39,14 +39,35 @@ from ..config.spec import PartSpec, TensorSpec
 from ..kernels import ops
 from ..registry import MIXERS
 from .base import LayerCache, Mixer, Runtime, StateSpec, StepContext, WeightView
-from .chunks import token_chunks
+from .chunks import split_portions, token_chunks
 from .linear import linear
 
 
 CHUNK = 64                   # tokens per chunk of the three-pass walk
 CHUNKED_FROM = 256           # a step whose longest portion has at least this many tokens goes chunk by chunk (not in float32)
-DELTA_CHUNKED_FROM = 128     # the same with the delta rule, whose walk is the slower one
+# In such a step the portions of at least PRODUCTS_FROM tokens are cut into chunks for the products and the others are walked.  32 heads of
+# 128x128, us: 16 portions of 64 tokens 178 as products, 203 walked, of 128 tokens 330 and 370, one of 64 tokens 56 and 37; 200 portions of
+# one token 2600 and 250, which is why they are kept apart (a chunk costs the same whatever it holds).
+PRODUCTS_FROM = 128
 CONV_BY_TOKEN_FROM = 32      # a step whose longest portion has at least this many tokens runs the convolution per (token, channel)
+
+
+def delta_by_products(lens, heads: int, dk: int, dv: int) -> bool:
+    """Estimates, in us, from times measured with 8 to 64 heads of 64x64, 64x128 and 128x128 and 1 to 16 portions of 256 and 512 tokens:
+    a walk's token takes 0.22 (dk 64) to 0.30 (dk 128) after the one before it, and 0.0021, 0.0040 or 0.0064 per head of a full device
+    (a portion's state as much as six tokens); in the products it takes 0.0027, 0.0037 or 0.0053 per head.  One portion of 512 tokens, 32
+    heads of 128x128: 135 by products, 190 walked; 16 of 256: 717 and 811; of 64x64, 4 portions of 512: 199 and 182, so that is walked;
+    512 tokens beside 200 portions of one: about 385 and 361, walked.  Below 320 tokens and 8192 x 128 x 128 numbers the launches of the
+    products count for more: a layer with 16 heads took 165 by products for 256 tokens, 147 walked, one with 32 heads 147 and 171."""
+    inside = [n for n in lens if n >= CHUNKED_FROM]
+    if not inside or sum((n + ops.LINEAR_CHUNK - 1) // ops.LINEAR_CHUNK for n in inside) > 65535:
+        return False
+    if max(lens) < 320 and heads * sum(inside) * dk * dv < 8192 * 128 * 128:
+        return False
+    work = lambda part: heads * (sum(part) + 6 * len(part))                       # noqa: E731
+    per_walked, per_chunked = 6.7e-4 + 3.5e-7 * dk * dv, 1.84e-3 + 2.1e-7 * dk * dv
+    walk = max((0.14 + 0.00125 * dk) * max(lens), per_walked * work(lens))
+    return 25.0 + per_chunked * heads * sum(inside) + per_walked * work([n for n in lens if n < CHUNKED_FROM]) < walk
 
 
 @MIXERS.register("linear_state")
@@ -166,8 +187,10 @@ class LinearStateMixer(Mixer):
             qs, fs, vs = a[:, self.q_off:self.q_off + H * dk], a[:, self.k_off:self.k_off + H * dk], a[:, self.v_off:self.v_off + H * dv]
             # the 32-bit path keeps one order of operations whatever the cutting: it always walks token by token
             if ctx.max_q_len >= CHUNKED_FROM and self.rt.dtype != torch.float32 and ops.linear_state_products_supported(qs, fs, vs, state, dk, dv):
-                chunk_meta, req_chunks = token_chunks(ctx, ops.LINEAR_CHUNK)
+                chunk_meta, req_chunks, walked = split_portions(ctx, ops.LINEAR_CHUNK, PRODUCTS_FROM)
                 o = ops.forget_gate_products(qs, fs, vs, state, chunk_meta, req_chunks, ctx.state_slots, ctx.positions, H, dk, dv)
+                if walked is not None:
+                    ops.forget_gate_walk(qs, fs, vs, state, walked, ctx.state_slots, ctx.positions, ctx.n_requests, H, dk, dv, out=o)
             elif ctx.max_q_len >= CHUNKED_FROM and self.rt.dtype != torch.float32:
                 chunk_meta, req_chunks = token_chunks(ctx, CHUNK)
                 o = ops.forget_gate_chunked(qs, fs, vs, state, chunk_meta, req_chunks, ctx.state_slots, ctx.positions, H, dk, dv)
@@ -193,11 +216,15 @@ class LinearStateMixer(Mixer):
             dt_bias=self.dt_bias, gate_rows=gate_rows)
         qs, ks_, vs = qkv[:, self.q_off:self.q_off + G * dk], qkv[:, self.k_off:self.k_off + G * dk], qkv[:, self.v_off:self.v_off + H * dv]
         # the 32-bit path keeps one order of operations whatever the cutting: it always walks
-        long = ctx.max_q_len >= (DELTA_CHUNKED_FROM if self.delta else CHUNKED_FROM) and self.rt.dtype != torch.float32
-        if long and self.decays_by_logarithm and ops.linear_state_products_supported(qs, ks_, vs, state, dk, dv):
-            chunk_meta, req_chunks = token_chunks(ctx, ops.LINEAR_CHUNK)
+        long = ctx.max_q_len >= CHUNKED_FROM and self.rt.dtype != torch.float32
+        if long and self.decays_by_logarithm and (not self.delta or self._delta_by_products(ctx)) and \
+                ops.linear_state_products_supported(qs, ks_, vs, state, dk, dv):
+            chunk_meta, req_chunks, walked = split_portions(ctx, ops.LINEAR_CHUNK, CHUNKED_FROM if self.delta else PRODUCTS_FROM)
             o = ops.linear_state_products(qs, ks_, vs, state, chunk_meta, req_chunks, ctx.state_slots, ctx.positions, H, G, dk, dv,
                                           gate=gate, beta=beta, head_decay=self.head_decay)
+            if walked is not None:
+                ops.linear_state_walk(qs, ks_, vs, state, walked, ctx.state_slots, ctx.positions, ctx.n_requests, H, G, dk, dv,
+                                      gate=gate, beta=beta, head_decay=self.head_decay, out=o)
         elif long and not self.delta:
             chunk_meta, req_chunks = token_chunks(ctx, CHUNK)
             o = ops.linear_state_chunked(qs, ks_, vs, state, chunk_meta, req_chunks, ctx.state_slots, ctx.positions, H, G, dk, dv,
@@ -206,6 +233,14 @@ class LinearStateMixer(Mixer):
             o = ops.linear_state_walk(qs, ks_, vs, state, ctx.req_meta, ctx.state_slots, ctx.positions, ctx.n_requests, H, G, dk, dv,
                                       gate=gate, beta=beta, head_decay=self.head_decay)
         return self._finish(o, a)
+
+    def _delta_by_products(self, ctx: StepContext) -> bool:
+        """Whether the step's portions of at least CHUNKED_FROM tokens go to the products with the delta rule.  The walk takes as long as
+        its longest portion, or, with many heads and portions, as all of its work; the products' time follows their work alone."""
+        key = ("delta_by_products", self.heads, self.dk, self.dv)
+        if key not in ctx.derived:
+            ctx.derived[key] = delta_by_products(ctx.q_len, self.heads, self.dk, self.dv)
+        return ctx.derived[key]
 
     def _finish(self, o: torch.Tensor, a: torch.Tensor) -> torch.Tensor:
         """The norm behind the heads, the output gate (its columns stand in the projection's rows ``a``) and the output projection."""

@@ -109,3 +109,51 @@ def test_forget_gate_products(H, dk, dv, gates):
             err, was = ((mine - ref).norm() / scale).item(), ((old - ref).norm() / scale).item()
             print(f"err {err:.2e} walk {was:.2e}")
             assert err <= max(5e-7, 1.5 * was), (r, err, was)      # as above
+
+
+@pytest.mark.parametrize("kind", ["plain", "delta", "forget"])
+@pytest.mark.parametrize("lens", [[70, 1, 300, 127, 128], [256, 1], [1, 400, 3]])
+def test_short_portions_beside_long_ones_are_walked(kind, lens):
+    """Every request bit for bit what its own kernel makes of it, whatever stands beside it."""
+    from types import SimpleNamespace
+
+    from mimirmind_b200.kernels import ops
+    from mimirmind_b200.parts.chunks import split_portions
+    H, dk, dv, R, n = 3, 64, 128, len(lens), sum(lens)
+    gen = torch.Generator(device=DEV).manual_seed(n)
+    rnd = lambda *s: torch.randn(s, generator=gen, device=DEV)                       # noqa: E731
+    q, k, v = rnd(n, H * dk) * dk ** -0.5, rnd(n, H * dk) * dk ** -0.5, rnd(n, H * dv)
+    k = torch.sigmoid(k) if kind == "forget" else k
+    gate, beta = 0.9 + 0.1 * torch.rand((n, H), generator=gen, device=DEV), torch.rand((n, H), generator=gen, device=DEV)
+    more = {} if kind == "forget" else {"gate": gate, "beta": beta if kind == "delta" else None}
+    heads = (H,) if kind == "forget" else (H, H)
+    products, walk = (ops.forget_gate_products, ops.forget_gate_walk) if kind == "forget" else (ops.linear_state_products, ops.linear_state_walk)
+    starts = [sum(lens[:i]) for i in range(R)]
+    ctx = SimpleNamespace(q_start=starts, q_len=lens, kv_len=[m + 7 for m in lens], derived={}, token_ids=torch.zeros(1, device=DEV))
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)                   # noqa: E731
+    pos = torch.cat([torch.arange(7, 7 + m, dtype=torch.int32, device=DEV) for m in lens])
+    slots = i32(list(range(R))[::-1])
+    before = rnd(R, H * dv * dk)
+    chunk_meta, req_chunks, walked = split_portions(ctx, 64, 128)
+    state = before.clone()
+    out = products(q, k, v, state, chunk_meta, req_chunks, slots, pos, *heads, dk, dv, **more)
+    out = walk(q, k, v, state, walked, slots, pos, R, *heads, dk, dv, out=out, **more)
+    for r, (s, m) in enumerate(zip(starts, lens)):
+        lone = before.clone()
+        one = SimpleNamespace(q_start=[s], q_len=[m], kv_len=[m + 7], derived={}, token_ids=ctx.token_ids)
+        if m >= 128:
+            a, b, none = split_portions(one, 64, 128)
+            assert none is None
+            want = products(q, k, v, lone, a, b, slots[r:r + 1], pos, *heads, dk, dv, **more)
+        else:
+            want = walk(q, k, v, lone, i32([[s, m, m + 7, 0]]), slots[r:r + 1], pos, 1, *heads, dk, dv, **more)
+        assert torch.equal(out[s:s + m], want[s:s + m]) and torch.equal(state[R - 1 - r], lone[R - 1 - r])
+
+
+def test_which_steps_the_delta_rule_takes_to_the_products():
+    """As measured: long portions of wide heads; not what a walk over many portions does as fast."""
+    from mimirmind_b200.parts.linear_state import delta_by_products
+    for lens, heads, dk, dv in (([512], 8, 64, 64), ([4096], 32, 128, 128), ([256] * 16, 32, 128, 128), ([2048] + [1] * 200, 32, 128, 128)):
+        assert delta_by_products(lens, heads, dk, dv)
+    for lens, heads, dk, dv in (([255], 8, 128, 128), ([256], 16, 128, 128), ([512] * 4, 32, 64, 64), ([512] + [1] * 200, 32, 128, 128), ([128] * 16, 32, 128, 128)):
+        assert not delta_by_products(lens, heads, dk, dv)
