@@ -100,6 +100,14 @@ def sink_plan(ctx, n_tokens: int, tile_rows: int = SINK_TILE_ROWS):
     return plan
 
 
+def fills_tall_tiles(ctx) -> bool:
+    """Whether the step's portions fill at least half of the rows of 128-token tiles."""
+    if "fills_tall_tiles" not in ctx.plans:
+        inside = [n for n in ctx.q_len if n >= SINK_PREFILL_MIN]
+        ctx.plans["fills_tall_tiles"] = 2 * sum(inside) >= 128 * sum((n + 127) // 128 for n in inside)
+    return ctx.plans["fills_tall_tiles"]
+
+
 def paged_sink_attention(q, cache, out, ctx, num_heads: int, num_kv_heads: int, key_dim: int, value_dim: int, window: int,
                          scale: float, sink: bool, sink_logit=None, dist_bias=None, softcap: float = 0.0, value_heads=None,
                          k_pages=None, v_pages=None, value_row=None, chunk: int = 0, keep: int = 0, gate=None) -> torch.Tensor:
@@ -124,7 +132,10 @@ def paged_sink_attention(q, cache, out, ctx, num_heads: int, num_kv_heads: int, 
             and _sink_lib().mm_attention_sink_supported(key_dim, value_dim)):
         from .lib import check
         lib = _sink_lib()
-        # key and value sizes of 64 or 128 without a distance bias: the tcgen05 prefill kernel of the plain attention, told of the rest
+        # key and value sizes of 64 or 128 without a distance bias: the tcgen05 prefill kernel of the plain attention, told of the rest.  Unless
+        # sizes are equal and nothing is asked for beside the sink, short portions stay in 64-token tiles: 64 portions of 20 tokens, two maps
+        # of keys 64 / values 128 in 32 heads, took a layer 397 us in 128-token tiles and 235 in these, 8 of 33 tokens 120 and 100, 8 of 130
+        # (half filled) 214 and 220.
         from . import attention_bf16
         # a learned sink, a distance bias, a cap, shared value heads or an fp32 result: the mma.sync kernels take them, the TMA decode kernel does not
         out_f32 = int(out.dtype == torch.float32)
@@ -134,7 +145,8 @@ def paged_sink_attention(q, cache, out, ctx, num_heads: int, num_kv_heads: int, 
         dist_max = dist_bias.shape[1] - 1 if dist_bias is not None else 0
         gate_ptr, gate_ld = ops.gate_args(gate, q.shape[0], num_heads)
         tensor_memory = (USE_SINK_TCGEN05 and dist_bias is None and attention_bf16.tcgen05_prefill_usable(key_dim, cache.page_size)
-                         and attention_bf16.tcgen05_prefill_usable(value_dim, cache.page_size))
+                         and attention_bf16.tcgen05_prefill_usable(value_dim, cache.page_size)
+                         and ((not extended and key_dim == value_dim) or fills_tall_tiles(ctx)))
         tiles, n_tiles, items, n_items = sink_plan(ctx, q.shape[0], attention_bf16.TILE_ROWS_TC if tensor_memory else SINK_TILE_ROWS)
         stream = ops._stream()
         if n_tiles and tensor_memory:

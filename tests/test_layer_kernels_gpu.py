@@ -46,6 +46,14 @@ def test_prompt_attention_on_tensor_memory(dk, dv, what, monkeypatch):
     assert ((a - b).norm() / b.norm()).item() <= 2.0 ** -7 and (a - b).abs().max() <= 2.0 ** -5 * b.abs().max()
 
 
+@pytest.mark.parametrize("lens,tall", [([64], True), ([63], False), ([1, 1], True), ([20, 300], True), ([20] * 4 + [300], False), ([128, 15], True)])
+def test_short_portions_stay_in_short_tiles(lens, tall):
+    from types import SimpleNamespace
+
+    from mimirmind_b200.kernels.attention import fills_tall_tiles
+    assert fills_tall_tiles(SimpleNamespace(q_len=lens, plans={})) is tall
+
+
 @pytest.mark.parametrize("taps", [1, 2, 4, 8])
 @pytest.mark.parametrize("C", [128, 260])
 def test_convolution_in_runs_of_tokens(taps, C):
