@@ -83,6 +83,13 @@ __device__ __forceinline__ void epilogue_rows(uint32_t taddr, int m0, int n0, in
             tmem_ld32(taddr + c * 32, r);
             if (row >= M) continue;
             float* o = (float*)out + (size_t)row * ldo + col0;
+            if (bias == nullptr && col0 + 32 <= N && ((uintptr_t)o & 15) == 0) {
+#pragma unroll
+                for (int i = 0; i < 32; i += 4)
+                    *reinterpret_cast<float4*>(o + i) =
+                        make_float4(__uint_as_float(r[i]), __uint_as_float(r[i + 1]), __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
+                continue;
+            }
             for (int i = 0; i < 32 && col0 + i < N; ++i) {
                 float v = __uint_as_float(r[i]);
                 if (bias != nullptr) v += (bias_dtype == MM_F32) ? ((const float*)bias)[col0 + i] : __bfloat162float(((const __nv_bfloat16*)bias)[col0 + i]);
@@ -505,7 +512,7 @@ int launch_grouped(const CUtensorMap& a, const CUtensorMap& b, void* out, int M,
 // The grouped form: A [M, lda] bf16 holds the rows of `groups` groups side by side, W [groups * N, K] bf16 their weight
 // matrices one after the other; tile i of the device-made list `group_tiles` (3 ints each: first row, end row, group; at
 // most 128 rows, never across a group's border; `n_group_tiles` of them, at most `max_group_tiles`) is multiplied with
-// its group's matrix.  out [M, ldo]: bf16 [M, N], or with the SwiGLU epilogue bf16 [M, N/2].
+// its group's matrix.  out [M, ldo]: bf16 [M, N], fp32 [M, N], or with the SwiGLU epilogue bf16 [M, N/2].
 // glu, limit: another gated activation than silu(g) u in the SwiGLU epilogue (glu_act's kinds in common.cuh); with the bf16
 // epilogue `glu` is the activation of the product itself (unary_act's numbers).
 MM_EXPORT int mm_gemm_tcgen05_grouped_act(const void* A, const void* W, void* out, int epilogue, int M, int groups, int N, int K, int lda, int ldo,
@@ -515,7 +522,8 @@ MM_EXPORT int mm_gemm_tcgen05_grouped_act(const void* A, const void* W, void* ou
     MM_REQUIRE(M > 0 && N > 0 && K > 0 && groups > 0 && max_group_tiles > 0 && group_tiles && n_group_tiles, "gemm_tcgen05 grouped: bad sizes");
     MM_REQUIRE(K % 8 == 0 && lda % 8 == 0 && lda >= K, "gemm_tcgen05: K and the row stride of A must be multiples of 8 (16-byte TMA rows)");
     MM_REQUIRE(((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0 && ((uintptr_t)out & 15) == 0, "gemm_tcgen05: pointers must be 16-byte aligned");
-    MM_REQUIRE(epilogue == EPI_BF16 || epilogue == EPI_SWIGLU, "gemm_tcgen05 grouped: the epilogues are bf16 and SwiGLU");
+    MM_REQUIRE(epilogue == EPI_BF16 || epilogue == EPI_SWIGLU || (epilogue == EPI_F32 && glu == 0),
+               "gemm_tcgen05 grouped: the epilogues are bf16, SwiGLU and, without an activation, fp32");
     MM_REQUIRE(epilogue != EPI_SWIGLU || (N % 16 == 0 && ldo >= N / 2), "gemm_tcgen05: the SwiGLU epilogue needs N a multiple of 16");
     MM_REQUIRE(ldo % 8 == 0 && (epilogue == EPI_SWIGLU || ldo >= N), "gemm_tcgen05: the row stride of the output must be a multiple of 8 and at least N");
     CUtensorMap ta, tb;
@@ -530,6 +538,9 @@ MM_EXPORT int mm_gemm_tcgen05_grouped_act(const void* A, const void* W, void* ou
     if (epilogue == EPI_SWIGLU)
         return launch_grouped<EPI_SWIGLU>(ta, tb, out, M, N, K, ldo, (int*)err, sms, (const int32_t*)group_tiles, (const int32_t*)n_group_tiles,
                                           max_group_tiles, N, s, glu, limit);
+    if (epilogue == EPI_F32)
+        return launch_grouped<EPI_F32>(ta, tb, out, M, N, K, ldo, (int*)err, sms, (const int32_t*)group_tiles, (const int32_t*)n_group_tiles,
+                                       max_group_tiles, N, s);
     return launch_grouped<EPI_BF16>(ta, tb, out, M, N, K, ldo, (int*)err, sms, (const int32_t*)group_tiles, (const int32_t*)n_group_tiles,
                                     max_group_tiles, N, s, glu, 0.0f);
 }

@@ -1363,19 +1363,22 @@ def moe_gather_scaled(x: torch.Tensor, rows: ExpertRows, wts: Optional[torch.Ten
 
 
 def moe_gemm_grouped(a: torch.Tensor, w: torch.Tensor, rows: ExpertRows, swiglu: bool, activation: Optional[str] = "silu", limit: float = 0.0,
-                     single: bool = False) -> torch.Tensor:
+                     single: bool = False, out_dtype: torch.dtype = torch.bfloat16) -> torch.Tensor:
     """The grouped tensor-memory product: ``a`` [n_rows, K] bf16 in sorted order, ``w`` [E, N, K] bf16; every row tile of
     ``rows.tiles`` times its expert's matrix.  ``swiglu``: the matrix interleaves gate and up rows in blocks of 8 and the
     result is ``silu(gate) * up`` [n_rows, N/2] (or another gated ``activation``); else [n_rows, N], with ``single`` after ``activation``
-    (of ACTIVATIONS).  bf16, in sorted order."""
+    (of ACTIVATIONS).  In sorted order, bf16, or a plain product's fp32 (``out_dtype``)."""
     _need(a, "moe rows", torch.bfloat16)
     _need(w, "moe weights", torch.bfloat16)
     if rows.tiles is None:
         raise KernelError("moe gemm: the rows were sorted without their tile list")
     n_rows, K = a.shape
     E, N, _ = w.shape
-    out = torch.empty((n_rows, N // 2 if swiglu else N), dtype=torch.bfloat16, device=a.device)
-    check(_lib.load().mm_gemm_tcgen05_grouped_act(a.data_ptr(), w.data_ptr(), out.data_ptr(), 1 if swiglu else 0, n_rows, E, N, K, K, out.shape[1],
+    if out_dtype != torch.bfloat16 and (swiglu or single or out_dtype != torch.float32):
+        raise KernelError("moe gemm: the grouped product's result is bf16, or fp32 without an activation")
+    out = torch.empty((n_rows, N // 2 if swiglu else N), dtype=out_dtype, device=a.device)
+    epilogue = 1 if swiglu else (2 if out_dtype == torch.float32 else 0)
+    check(_lib.load().mm_gemm_tcgen05_grouped_act(a.data_ptr(), w.data_ptr(), out.data_ptr(), epilogue, n_rows, E, N, K, K, out.shape[1],
                                                   rows.tiles.data_ptr(), rows.n_tiles.data_ptr(), rows.max_tiles,
                                                   GLU_ACTIVATIONS[activation] if swiglu else (ACTIVATIONS[activation] + 1 if single else 0), float(limit),
                                                   tcgen05_error_flag(a.device).data_ptr(), _stream()), "gemm_tcgen05_grouped")

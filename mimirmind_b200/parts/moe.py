@@ -16,8 +16,8 @@ added to its score for the choice only (of runs and of experts), the weights are
 ``W_down act(W_up h)`` with a plain ``activation``.
 
 The experts' matrices are stacked at load (``[E, 2F, D]`` gate and up rows, ``[E, D, F]``).  A step routes on the
-device, puts the rows of every expert side by side, and runs two grouped products over them: for prompt-sized steps in
-bfloat16 the tcgen05 product over row tiles laid out on the device (``csrc/gemm_tcgen05.cu``, SwiGLU in its epilogue),
+device, puts the rows of every expert side by side, and runs two grouped products over them: for prompt-sized steps, and smaller ones
+of large experts, in bfloat16 the tcgen05 product over row tiles laid out on the device (``csrc/gemm_tcgen05.cu``, SwiGLU in its epilogue),
 otherwise the ``mma.sync`` or fp32 kernels of ``csrc/moe.cu``.  Nothing waits for the host, so a decode step with this
 feed-forward can be captured.
 """
@@ -35,6 +35,12 @@ from .linear import linear
 
 
 GROUPED_MIN_ROWS = 1024      # (token, choice) rows from which a step's expert products run on tensor memory
+# Below that, where what counts is how fast the experts' weights stream, steps of more than 16 tokens (up to which the mma.sync kernel has
+# tiles of 16 rows) run there too if the experts' second matrices together have at least this many numbers (the three 200 MB); the result
+# then stays fp32, as the other kernels leave it.  us of a layer, other kernels and this: 16 experts of 4096 x 2752, 17 to 200 tokens 411 to
+# 443 and 250 to 262, 16 tokens 236 and 250; 128 of 2048 x 768, 32 tokens 375 and 250; 16 of 2048 x 1408 156 and 131; 32 of 1024 x 512
+# (16.8 million numbers) 67 and 85, the two more launches.  A weight on the expert's input would be rounded with it, so that stays.
+GROUPED_MIN_WEIGHTS = 1 << 25
 
 
 def ctx_plain(ctx) -> bool:
@@ -144,8 +150,9 @@ class RoutedExperts(FeedForward):
         idx, wts, gate = chosen if self.shared_gated else chosen + (None,)
         n_rows = n * self.top
         on_input = self.weight_on == "input"
-        if self.tensor_memory and n_rows >= GROUPED_MIN_ROWS and not ctx_plain(ctx):
-            # prompt-sized: the rows are copied into sorted order once, and both products run on tensor memory over tiles of
+        grouped = n_rows >= GROUPED_MIN_ROWS or (n > 16 and not on_input and self.w_out.numel() >= GROUPED_MIN_WEIGHTS)
+        if self.tensor_memory and grouped and not ctx_plain(ctx):
+            # the rows are copied into sorted order once, and both products run on tensor memory over tiles of
             # 128 rows of one expert; the outputs stay in sorted order and the weighted sum fetches them by place
             rows = ops.moe_sort(idx, self.experts, with_tiles=True)
             if on_input:        # the weight rides on the copy: expert(w h) with w h rounded to the rows' dtype
@@ -155,7 +162,8 @@ class RoutedExperts(FeedForward):
                 ops.gather_rows(x, rows.row_token, sorted_x)
             hidden = ops.moe_gemm_grouped(sorted_x, self.w_in, rows, swiglu=self.gated, activation=self.activation, limit=self.limit,
                                           single=not self.gated)
-            y = ops.moe_gemm_grouped(hidden, self.w_out, rows, swiglu=False)
+            y = ops.moe_gemm_grouped(hidden, self.w_out, rows, swiglu=False,
+                                     out_dtype=torch.bfloat16 if n_rows >= GROUPED_MIN_ROWS else torch.float32)
             return y, (None if on_input else wts), rows.place, gate
         rows = ops.moe_sort(idx, self.experts)
         tc = self.rt.matmul != "simt"

@@ -54,6 +54,35 @@ def test_short_portions_stay_in_short_tiles(lens, tall):
     assert fills_tall_tiles(SimpleNamespace(q_len=lens, plans={})) is tall
 
 
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("n,d,ff,E,top", [(17, 64, 40, 6, 2), (100, 200, 136, 3, 3), (33, 2048, 256, 40, 8), (255, 72, 264, 5, 4)])
+def test_grouped_products_of_small_steps_stay_in_32_bits(n, d, ff, E, top, gated, monkeypatch):
+    from mimirmind_b200.config.spec import PartSpec
+    from mimirmind_b200.kernels import ops
+    from mimirmind_b200.parts import moe
+    from mimirmind_b200.parts.base import Runtime, WeightView
+    gen = torch.Generator(device=DEV).manual_seed(n + d)
+    rnd = lambda *s: torch.randn(s, generator=gen, device=DEV)                       # noqa: E731
+    w = {"router": rnd(E, d) * 4 * d ** -0.5}
+    for e in range(E):
+        w.update({f"e{e}.gate": rnd(ff, d) * d ** -0.5, f"e{e}.up": rnd(ff, d) * d ** -0.5, f"e{e}.down": rnd(d, ff) * ff ** -0.5})
+    spec = PartSpec("routed_experts", {"hidden": d, "ff": ff, "experts": E, "top": top, "router": "router", "expert": "e{}", "gated": gated,
+                                       "activation": "silu" if gated else "gelu_erf"})
+    part = moe.RoutedExperts(spec, WeightView({k: v.to(torch.bfloat16) for k, v in w.items()}), Runtime(torch.bfloat16, torch.device(DEV)))
+    x = rnd(n, d).to(torch.bfloat16)
+    got = {}
+    for least in (0, 1 << 40):
+        monkeypatch.setattr(moe, "GROUPED_MIN_WEIGHTS", least)
+        split, whole = part.forward_split(x, None), part.forward(x, None)
+        assert split.rows.dtype == torch.float32 and (split.place is None) == (least > 0)
+        y = split.rows if split.place is None else split.rows[split.place.long()]
+        assert torch.equal(whole, ops.moe_combine(split.rows, split.weights, torch.bfloat16, place=split.place, top=top))
+        got[least] = y
+    ops.check_tcgen05_errors(torch.device(DEV))
+    # the hidden rows are rounded to bf16 on both sides, mostly alike: 2^-9 each at most
+    assert ((got[0] - got[1 << 40]).norm() / got[1 << 40].norm()).item() <= 2.0 ** -8
+
+
 @pytest.mark.parametrize("taps", [1, 2, 4, 8])
 @pytest.mark.parametrize("C", [128, 260])
 def test_convolution_in_runs_of_tokens(taps, C):
