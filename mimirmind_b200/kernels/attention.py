@@ -13,13 +13,15 @@ from typing import Optional, Tuple
 
 import torch
 
+from . import attention_bf16
+from . import lib as _lib
 from . import ops
+from .lib import check
 
 
 def paged_attention(q, cache, out, ctx, num_heads: int, num_kv_heads: int, head_dim: int, window: int,
                     scale: float) -> torch.Tensor:
     if q.dtype == torch.bfloat16:
-        from . import attention_bf16
         if attention_bf16.supports(head_dim, num_heads, num_kv_heads):
             return attention_bf16.run(q, cache, out, ctx, num_heads, num_kv_heads, head_dim, window, scale)
     return ops.attention_generic(q, cache.k_pages, cache.v_pages, out, ctx.positions, ctx.token_req,
@@ -37,7 +39,6 @@ _sink_declared = False
 def _sink_lib():
     global _sink_declared
     from ctypes import c_float, c_int, c_void_p
-    from . import lib as _lib
     if not _sink_declared:
         P, I, F = c_void_p, c_int, c_float
         _lib.declare("mm_attention_sink_supported", [I, I])
@@ -128,15 +129,13 @@ def paged_sink_attention(q, cache, out, ctx, num_heads: int, num_kv_heads: int, 
     v_pages = cache.arrays["v"] if v_pages is None else v_pages
     value_heads = num_kv_heads if value_heads is None else int(value_heads)
     value_row = value_dim if value_row is None else int(value_row)
+    lib = _sink_lib()
     if (USE_SINK_MMA and value_row == value_dim and q.dtype == torch.bfloat16 and scale > 0 and num_heads // num_kv_heads <= 16
-            and _sink_lib().mm_attention_sink_supported(key_dim, value_dim)):
-        from .lib import check
-        lib = _sink_lib()
+            and lib.mm_attention_sink_supported(key_dim, value_dim)):
         # key and value sizes of 64 or 128 without a distance bias: the tcgen05 prefill kernel of the plain attention, told of the rest.  Unless
         # sizes are equal and nothing is asked for beside the sink, short portions stay in 64-token tiles: 64 portions of 20 tokens, two maps
         # of keys 64 / values 128 in 32 heads, took a layer 397 us in 128-token tiles and 235 in these, 8 of 33 tokens 120 and 100, 8 of 130
         # (half filled) 214 and 220.
-        from . import attention_bf16
         # a learned sink, a distance bias, a cap, shared value heads or an fp32 result: the mma.sync kernels take them, the TMA decode kernel does not
         out_f32 = int(out.dtype == torch.float32)
         extended = sink_logit is not None or dist_bias is not None or softcap > 0 or value_heads != num_kv_heads or bool(out_f32)
@@ -213,7 +212,6 @@ _latent_declared = False
 def _latent_lib():
     global _latent_declared
     from ctypes import c_float, c_int, c_void_p
-    from . import lib as _lib
     if not _latent_declared:
         P, I, F = c_void_p, c_int, c_float
         _lib.declare("mm_attention_latent_supported", [I, I])
@@ -264,7 +262,6 @@ _expanded_declared = False
 def _expanded_lib():
     global _expanded_declared
     from ctypes import c_float, c_int, c_void_p
-    from . import lib as _lib
     if not _expanded_declared:
         P, I, F = c_void_p, c_int, c_float
         _lib.declare("mm_attention_latent_tcgen05_supported", [I, I, I])
@@ -327,7 +324,6 @@ def latent_expanded_attention(plan: LatentExpandedPlan, q_wide, pages, cache, w_
     """The plan's requests: their cached latents side by side, every head's plain keys and values from them in one product
     (``w_kv`` [heads * (key_dim + value_dim), rank]), and the attention; writes those requests' rows of ``out`` [n, heads * value_dim]."""
     from ..parts.linear import linear
-    from .lib import check
     lib, dev = _expanded_lib(), q_wide.device
     c = torch.empty((plan.rows, rank), dtype=torch.bfloat16, device=dev)
     turned = torch.empty((plan.rows, rot_dim), dtype=torch.bfloat16, device=dev) if rot_dim else None
@@ -350,7 +346,6 @@ def paged_latent_attention(q, pages, cache, out, ctx, num_heads: int, wide: int,
     kernel is built for: that kernel, its key tiles shared out over several CTAs while the step has few query tiles;
     anything else: the fp32-arithmetic kernel.  ``without``: requests whose rows somebody else makes (they may be left unwritten)."""
     if USE_LATENT_MMA and q.dtype == torch.bfloat16 and scale > 0 and _latent_lib().mm_attention_latent_supported(wide, rank):
-        from .lib import check
         lib = _latent_lib()
         # portions of prompts: tiles of 64 rows (two 16-row tiles per warp, half the key traffic per row) where they fit
         tile_rows = 64 if USE_LATENT_WIDE_TILES and ctx.max_q_len * num_heads >= 64 and lib.mm_attention_latent_tile_rows(wide) == 64 else LATENT_TILE_ROWS
@@ -401,7 +396,6 @@ _talking_declared = False
 def _talking_lib():
     global _talking_declared
     from ctypes import c_float, c_int, c_void_p
-    from . import lib as _lib
     if not _talking_declared:
         P, I, F = c_void_p, c_int, c_float
         _lib.declare("mm_attention_talking_mma_supported", [I, I, I, I])
@@ -440,7 +434,6 @@ def paged_talking_attention(q, cache, out, ctx, num_heads: int, num_kv_heads: in
     k_pages, v_pages = cache.arrays["k"], cache.arrays["v"]
     if USE_TALKING_MMA and q.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and \
             _talking_lib().mm_attention_talking_mma_supported(num_heads, num_kv_heads, key_dim, value_dim):
-        from .lib import check
         lib = _talking_lib()
         tiles, n_tiles = talking_plan(ctx)
         keys = min(window, ctx.max_kv_len) if window > 0 else ctx.max_kv_len

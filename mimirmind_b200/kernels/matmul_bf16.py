@@ -16,12 +16,13 @@ from typing import Optional
 
 import torch
 
+from . import ops
+
 
 USE_LIBRARY_CALL = True       # False: the products of more than a few rows go through torch.mm (tests compare the two)
 
 
 def matmul_nt(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], out_dtype: torch.dtype) -> torch.Tensor:
-    from . import ops
     if ops.gemv_supported(x.shape[0], weight.shape[0], weight.shape[1]):
         return ops.gemv_bf16(x, weight, bias, out_dtype)          # a handful of rows: weight streaming
     if USE_LIBRARY_CALL and x.is_contiguous() and weight.is_contiguous() and out_dtype in (torch.float32, torch.bfloat16) \

@@ -23,6 +23,7 @@ from typing import List, Optional
 import torch
 
 from ..config.spec import PartSpec, TensorSpec
+from ..kernels import attention as attn_kernels
 from ..kernels import ops
 from ..registry import MIXERS
 from .base import CacheArray, KVCacheSpec, LayerCache, Mixer, Runtime, StateSpec, StepContext, WeightView
@@ -129,7 +130,6 @@ class DifferentialAttention(Mixer):
         ops.qkv_split_post(rows, 0, 2 * H * dk, 2 * (H + G) * dk, q, k_pages, v_pages, slots, cache.page_size, 2 * H, 2 * G, dk, G, dv)
         # both maps' results stay fp32: their difference is normed to unit size, which would magnify a rounding of the maps
         att = torch.empty((n, 2 * H * dv), dtype=torch.float32, device=a.device)
-        from ..kernels import attention as attn_kernels
         attn_kernels.paged_sink_attention(q, cache, att, ctx, 2 * H, 2 * G, dk, dv, self.window, self.scale, False,
                                           softcap=self.softcap, value_heads=G)
         o = ops.head_finish(att, H, dv, pair=True, lam=self.lam, eps=self.eps, post=1.0 - self.diff,

@@ -14,7 +14,7 @@ from typing import Optional
 
 import torch
 
-from ..kernels import ops
+from ..kernels import matmul_bf16, ops
 from .base import ElementwiseSink, Runtime
 
 
@@ -23,7 +23,6 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor], 
     out_dtype = out_dtype or x.dtype
     m, n = x.shape[0], weight.shape[0]
     if x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and rt.matmul != "simt":
-        from ..kernels import matmul_bf16
         return matmul_bf16.matmul_nt(x, weight, bias, out_dtype)
     out = torch.empty((m, n), dtype=out_dtype, device=x.device)
     return ops.gemm_simt(x, weight, bias, out)

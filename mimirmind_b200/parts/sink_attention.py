@@ -28,6 +28,7 @@ from typing import List, Optional
 import torch
 
 from ..config.spec import PartSpec, TensorSpec
+from ..kernels import attention as attn_kernels
 from ..kernels import ops
 from ..registry import MIXERS, POSITION_ENCODINGS
 from .base import CacheArray, KVCacheSpec, LayerCache, Mixer, Runtime, StepContext, WeightView
@@ -157,7 +158,6 @@ class SinkAttention(Mixer):
             slots = ctx.derived[skey]
         ops.qkv_pairs_post(qkv, q, k_pages, v_pages, v_first, rot, slots, cache.page_size, H, G, dk, dv, self.rot_dims, mode, self.mix)
         out = torch.empty((n, H * dv), dtype=self.rt.dtype, device=qkv.device)
-        from ..kernels import attention as attn_kernels
         attn_kernels.paged_sink_attention(q, cache, out, ctx, H, G, dk, dv, self.window, self.scale, self.sink,
                                           sink_logit=self.sink_logit, dist_bias=self.dist_bias)
         if self.w_gate is not None:
