@@ -76,6 +76,11 @@ def test_grouped_products_of_small_steps_stay_in_32_bits(n, d, ff, E, top, gated
         split, whole = part.forward_split(x, None), part.forward(x, None)
         assert split.rows.dtype == torch.float32 and (split.place is None) == (least > 0)
         y = split.rows if split.place is None else split.rows[split.place.long()]
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            replayed = part.forward(x, None)
+        graph.replay()
+        assert torch.equal(replayed, whole)
         assert torch.equal(whole, ops.moe_combine(split.rows, split.weights, torch.bfloat16, place=split.place, top=top))
         got[least] = y
     ops.check_tcgen05_errors(torch.device(DEV))
