@@ -45,9 +45,18 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
-// tanh of a row's numbers in place.  Scores are mostly small against their cap: where no number of the warp exceeds 0.35 the odd
-// polynomial of the Taylor series up to y^11 (relative error below 4e-9) spares the special-function unit, which the softmax
-// keeps busy; else 1 - 2 / (1 + e^(2y)) (absolute error below 2e-7).
+// tanh of a row's numbers in place, each number by itself: up to 0.35 the odd polynomial of the Taylor series up to y^11 (the next term is 1.2e-8
+// of the result there, the roundings add less than 1e-7), beyond it tanhf.  Scores are mostly small against their cap, so a warp none of
+// whose numbers is larger leaves out the second form, which takes the special-function unit that the softmax keeps busy.  That
+// only saves time: a number's result depends on neither the other columns, which may be keys that nobody sees, nor the other rows.
+__device__ __forceinline__ float tanh_small(float y) {
+    const float z = y * y;
+    float p = fmaf(z, -1382.0f / 155925.0f, 62.0f / 2835.0f);
+    p = fmaf(z, p, -17.0f / 315.0f);
+    p = fmaf(z, p, 2.0f / 15.0f);
+    p = fmaf(z, p, -1.0f / 3.0f);
+    return fmaf(y * z, p, y);
+}
 template <int N>
 __device__ __forceinline__ void tanh_row(uint32_t (&x)[N], float scale) {
     float tops[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -58,21 +67,16 @@ __device__ __forceinline__ void tanh_row(uint32_t (&x)[N], float scale) {
         tops[i & 3] = fmaxf(tops[i & 3], fabsf(y));
     }
     const float top = fmaxf(fmaxf(tops[0], tops[1]), fmaxf(tops[2], tops[3]));
-    if (__all_sync(0xffffffffu, top <= 0.35f)) {
+    if (__all_sync(0xffffffffu, top <= 0.35f)) {       // (a NaN goes through either form)
 #pragma unroll
-        for (int i = 0; i < N; ++i) {
-            const float y = __uint_as_float(x[i]), z = y * y;
-            float p = fmaf(z, -1382.0f / 155925.0f, 62.0f / 2835.0f);
-            p = fmaf(z, p, -17.0f / 315.0f);
-            p = fmaf(z, p, 2.0f / 15.0f);
-            p = fmaf(z, p, -1.0f / 3.0f);
-            x[i] = __float_as_uint(fmaf(y * z, p, y));
-        }
+        for (int i = 0; i < N; ++i) x[i] = __float_as_uint(tanh_small(__uint_as_float(x[i])));
     } else {
 #pragma unroll
         for (int i = 0; i < N; ++i) {
-            const float e = fast_exp2(__uint_as_float(x[i]) * 2.8853900817779268f);      // e^(2y)
-            x[i] = __float_as_uint(1.0f - __fdividef(2.0f, 1.0f + fminf(e, 1e30f)));
+            const float y = __uint_as_float(x[i]);
+            float r = tanh_small(y);
+            if (fabsf(y) > 0.35f) r = tanhf(y);
+            x[i] = __float_as_uint(r);
         }
     }
 }
