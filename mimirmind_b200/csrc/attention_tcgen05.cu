@@ -169,8 +169,6 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         __syncwarp();
         if (kt_begin < kt_end) produce(true, kt_begin, 0, false);
     }
-    // Value tiles must never hold non-finite leftovers: rows of a page that was not fetched are multiplied by P = 0.
-    for (int i = threadIdx.x; i < KV_STAGES * V_TILE_BYTES / 16; i += ATT_TC_THREADS) reinterpret_cast<uint4*>(sV)[i] = make_uint4(0, 0, 0, 0);
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)), "r"(TMEM_COLS_ATT) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -216,15 +214,34 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
             for (uint32_t it = 0; (int)it < n_tiles_k && ok; ++it) ok = issue_qk(it);
         }
     } else if (warp == PV_ISSUER_WARP) {
-        if (lane == 0) {
-            // ---- P V issuer ----
-            constexpr uint32_t IDESC_PV = idesc_bf16(BM, HDV, true);
-            const int n_tiles_k = kt_end - kt_begin;
-            for (uint32_t it = 0; (int)it < n_tiles_k; ++it) {
-                const int s = it % KV_STAGES;
+        // ---- P V issuer: one lane; the whole warp clears what stands in a tile for keys that none of the CTA's rows sees ----
+        constexpr uint32_t IDESC_PV = idesc_bf16(BM, HDV, true);
+        const int n_tiles_k = kt_end - kt_begin;
+        bool ok = true;
+        for (uint32_t it = 0; (int)it < n_tiles_k; ++it) {
+            const int s = it % KV_STAGES, key0 = walk.real(kt_begin + (int)it) * BN;
+            if (key0 + BN > hi_all || (key0 < lo_all && key0 + BN > keep)) {
+                // Such a key's probability is 0, but 0 times a NaN or an infinity is NaN: behind the last token stands what the page's owner
+                // before has left, in front of the window and in pages that were not fetched older tokens.  At most three tiles of a
+                // walk (its end, its window's start, the kept tokens' end), while the softmax still works on their scores.
+                __syncwarp();                                                       // lane 0 is through with the stage's tile before
+                if (mbar_wait(smem_u32(&ctl->v_full[s]), (it / KV_STAGES) & 1, abort_flag)) {
+                    for (int r = lane >> 3; r < BN; r += 4) {
+                        const int key = key0 + r;
+                        if (key < hi_all && (key >= lo_all || key < keep)) continue;
+#pragma unroll
+                        for (int hf = 0; hf < HDV / 64; ++hf)
+                            *reinterpret_cast<uint4*>(sV + s * V_TILE_BYTES + hf * HALF_BYTES + r * 128 + (lane & 7) * 16) = make_uint4(0, 0, 0, 0);
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // read by the tensor core
+                }
+                __syncwarp();
+            }
+            if (lane == 0 && ok) {
                 const uint32_t b = it & 1, u = it >> 1;
-                if (!mbar_wait(smem_u32(&ctl->p_full[b]), u & 1, abort_flag)) break;       // P is there, O is rescaled
-                if (!mbar_wait(smem_u32(&ctl->v_full[s]), (it / KV_STAGES) & 1, abort_flag)) break;
+                ok = mbar_wait(smem_u32(&ctl->p_full[b]), u & 1, abort_flag) &&         // P is there, O is rescaled
+                     mbar_wait(smem_u32(&ctl->v_full[s]), (it / KV_STAGES) & 1, abort_flag);
+                if (!ok) continue;
                 tc_fence_after();
                 const uint32_t p_addr = smem_u32(sP + b * TILE_BYTES), v_addr = smem_u32(sV + s * V_TILE_BYTES);
 #pragma unroll

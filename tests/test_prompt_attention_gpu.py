@@ -52,6 +52,20 @@ def unseen(form):
             yield r, j
 
 
+@pytest.mark.parametrize("dk,dv", [(128, 64), (64, 128), (64, 64), (128, 128)])
+@pytest.mark.parametrize("form", list(FORMS))
+def test_what_no_row_sees_does_not_count(dk, dv, form):
+    q, k, v, table = setting(dk, dv, form)
+    clean = attend(q, k, v, table, dk, dv, form)
+    assert torch.isfinite(clean).all()
+    for junk in (float("nan"), float("inf"), 200.0):          # what an earlier owner of the pages may have left there
+        kk, vv = k.clone(), v.clone()
+        for r, j in unseen(form):
+            kk[table[r, j // PAGE], :, j % PAGE] = junk
+            vv[table[r, j // PAGE], :, j % PAGE] = junk
+        assert torch.equal(attend(q, kk, vv, table, dk, dv, form), clean)
+
+
 @pytest.mark.parametrize("dk,dv", [(128, 64), (64, 128), (64, 64)])
 @pytest.mark.parametrize("form", ["cap", "hard cap", "capped window", "fp32"])
 def test_other_requests_of_the_step_do_not_count(dk, dv, form):
