@@ -66,7 +66,7 @@ struct AttCtl {
 };
 
 // tiles: int32 [n_tiles, 4] = (request index, first token row, rows in the tile (<= 128), position of the first row)
-template <int HDK, int HDV, bool CAP>
+template <int HDK, int HDV, bool CAP, bool FOLLOW>
 __global__ void __launch_bounds__(ATT_TC_THREADS, 1)
 attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                             const __grid_constant__ CUtensorMap tmV, void* __restrict__ out, int out_f32,
@@ -273,7 +273,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         uint32_t sreg[128];
         const SoftmaxBars bars = {smem_u32(&ctl->s_full[g]), smem_u32(&ctl->s_free[g]), smem_u32(&ctl->p_full[g]), smem_u32(&ctl->pv_done[g])};
         for (uint32_t it = g; (int)it < n_tiles_k && ok; it += 2, ++done) {
-            ok = softmax_tile<HDV, CAP>(bars, abort_flag, s_addr, o_addr, sP + g * TILE_BYTES, HALF_BYTES, row, lane, row_valid, pos, wlo,
+            ok = softmax_tile<HDV, CAP, FOLLOW>(bars, abort_flag, s_addr, o_addr, sP + g * TILE_BYTES, HALF_BYTES, row, lane, row_valid, pos, wlo,
                                   walk.real(kt_begin + (int)it) * BN, it >> 1, done == 0, scale_log2, sreg, m_ref, l, keep, cap_in);
         }
         // Merge the two groups: every thread posts its row's (reference, sum); the row's output is
@@ -352,15 +352,15 @@ struct PrefillArgs {
     float scale, softcap;
 };
 
-template <int HDK, int HDV, bool CAP>
+template <int HDK, int HDV, bool CAP, bool FOLLOW>
 static int attention_prefill_launch_as(const PrefillArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, cudaStream_t s) {
     constexpr size_t smem = (size_t)(HDK / 64 + 4 + KV_STAGES * (HDK / 64 + HDV / 64)) * HALF_BYTES + sizeof(AttCtl);
-    if (cudaFuncSetAttribute(attention_prefill_tc_kernel<HDK, HDV, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    if (cudaFuncSetAttribute(attention_prefill_tc_kernel<HDK, HDV, CAP, FOLLOW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
         mm_set_last_error("attention_prefill_tcgen05: cannot reserve shared memory");
         return MM_ERR_LAUNCH;
     }
     const float LOG2E = 1.4426950408889634f;
-    attention_prefill_tc_kernel<HDK, HDV, CAP><<<dim3(a.H, a.n_tiles), ATT_TC_THREADS, smem, s>>>(
+    attention_prefill_tc_kernel<HDK, HDV, CAP, FOLLOW><<<dim3(a.H, a.n_tiles), ATT_TC_THREADS, smem, s>>>(
         tq, tk, tv, a.out, a.out_f32, (const int32_t*)a.tiles, (const int32_t*)a.block_table, a.table_width, a.page_size, a.H, a.G, a.Gv, a.mask,
         (CAP ? a.softcap : a.scale) * LOG2E, CAP ? a.scale / a.softcap : 0.0f, a.sink, (const float*)a.sink_logit, (const float*)a.gate, a.gate_ld,
         (int*)a.err);
@@ -389,9 +389,13 @@ static int attention_prefill_tcgen05_launch(const PrefillArgs& a, int dk, int dv
     }
     MM_REQUIRE(a.n_tiles <= 65535, "attention_prefill_tcgen05: more than 65535 tiles in one launch");
     cudaStream_t s = (cudaStream_t)stream;
-#define PREFILL_AS(K, V)                                                     \
-    if (dk == K && dv == V)                                                  \
-        return a.softcap > 0.0f ? attention_prefill_launch_as<K, V, true>(a, tq, tk, tv, s) : attention_prefill_launch_as<K, V, false>(a, tq, tk, tv, s)
+    // Equal sizes without an option keep the lazy reference that they have always had; the other forms ran on mma.sync, whose reference follows every
+    // maximum, and are as close to 64 bits here.
+    const bool plain = dk == dv && a.softcap == 0.0f && a.Gv == a.G && a.sink_logit == nullptr && !a.out_f32;
+#define PREFILL_AS(K, V)                                                                                                                    \
+    if (dk == K && dv == V)                                                                                                                 \
+        return a.softcap > 0.0f ? attention_prefill_launch_as<K, V, true, true>(a, tq, tk, tv, s) : attention_prefill_launch_as<K, V, false, true>(a, tq, tk, tv, s)
+    if (plain) return dk == 128 ? attention_prefill_launch_as<128, 128, false, false>(a, tq, tk, tv, s) : attention_prefill_launch_as<64, 64, false, false>(a, tq, tk, tv, s);
     PREFILL_AS(128, 128);
     PREFILL_AS(64, 64);
     PREFILL_AS(128, 64);

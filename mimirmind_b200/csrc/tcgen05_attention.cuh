@@ -98,8 +98,10 @@ struct SoftmaxBars {
 // One thread's row of one tile of 128 keys, the group's tile number `u` (`first`: its first): S from tensor memory into `sreg`,
 // masked by position, O (O_COLS columns at o_addr) rescaled when the row's maximum has outgrown its reference by RESCALE_STEP,
 // P rounded to bf16 into p_tile (two halves of 64 keys, 128-byte swizzle), the row's sum added to l.  The row sees keys wlo .. pos and
-// the first `keep` ones.  CAP: a score s becomes tanh(s cap_in) first (scale_log2 is then the cap's).  False: a wait ran out.
-template <int O_COLS, bool CAP = false>
+// the first `keep` ones.  CAP: a score s becomes tanh(s cap_in) first (scale_log2 is then the cap's).  FOLLOW: the reference follows every new
+// maximum, so that the largest probability is 1, which bf16 holds exactly, as in a kernel that rescales on each tile; a row that few keys
+// dominate carries their rounding otherwise.  False: a wait ran out.
+template <int O_COLS, bool CAP = false, bool FOLLOW = false>
 __device__ __forceinline__ bool softmax_tile(const SoftmaxBars& bars, volatile int* abort_flag, uint32_t s_addr, uint32_t o_addr, unsigned char* p_tile,
                                              uint32_t half_bytes, int row, int lane, bool row_valid, int pos, int wlo, int key0, uint32_t u, bool first,
                                              float scale_log2, uint32_t (&sreg)[128], float& m_ref, float& l, int keep = 0, float cap_in = 0.0f) {
@@ -114,7 +116,7 @@ __device__ __forceinline__ bool softmax_tile(const SoftmaxBars& bars, volatile i
     if constexpr (CAP) tanh_row(sreg, cap_in);
     // a tile every key of which this row sees needs no mask
     const bool interior = row_valid && key0 + BN - 1 <= pos && key0 >= wlo;
-    // (four chains each for the maximum and the sum: one would have every thread wait 128 times for its own last result)
+    // (four chains for the maximum: one would have every thread wait 128 times for its own last result)
     float top[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
     if (interior) {
 #pragma unroll
@@ -139,7 +141,7 @@ __device__ __forceinline__ bool softmax_tile(const SoftmaxBars& bars, volatile i
     if (!first && !mbar_wait(bars.pv_done, (u - 1) & 1, abort_flag)) return false;
     // Move the reference only when the maximum has outgrown it by RESCALE_STEP (or there was none).  O of a row without a
     // reference is still zero.
-    const bool move = mx > m_ref && (m_ref == -INFINITY || (mx - m_ref) * scale_log2 > RESCALE_STEP);
+    const bool move = mx > m_ref && (FOLLOW || m_ref == -INFINITY || (mx - m_ref) * scale_log2 > RESCALE_STEP);
     const bool scale_o = move && m_ref != -INFINITY;
     if (__any_sync(0xffffffffu, scale_o)) {
         tc_fence_after();
@@ -160,7 +162,7 @@ __device__ __forceinline__ bool softmax_tile(const SoftmaxBars& bars, volatile i
     const float use = (m_ref == -INFINITY) ? 0.0f : m_ref * scale_log2;
     // probabilities, rounded to bf16 as the tensor core will read them: the row of P is two halves of 64 keys, each 8 chunks
     // of 16 bytes, chunk index xor-ed with row % 8
-    float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    float sum = 0.0f;
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) {
         unsigned char* prow = p_tile + hf * half_bytes + row * 128;
@@ -171,13 +173,13 @@ __device__ __forceinline__ bool softmax_tile(const SoftmaxBars& bars, volatile i
             for (int i = 0; i < 4; ++i) {
                 const float p0 = fast_exp2(fmaf(__uint_as_float(sreg[hf * 64 + ch * 8 + 2 * i]), scale_log2, -use));
                 const float p1 = fast_exp2(fmaf(__uint_as_float(sreg[hf * 64 + ch * 8 + 2 * i + 1]), scale_log2, -use));
-                sum[i] += p0 + p1;
+                sum += p0 + p1;
                 packed[i] = pack_bf16x2(p0, p1);
             }
             *reinterpret_cast<uint4*>(prow + ((ch ^ (row & 7)) << 4)) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
         }
     }
-    l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+    l += sum;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // P is read by the tensor core (async proxy)
     tc_fence_before();                                                // ... and O, if it was rescaled, is in tensor memory
     warp_arrive(bars.p_full, lane);

@@ -104,3 +104,31 @@ def test_capped_scores_against_64_bits(cap, spread):
     sizes = torch.einsum("nhd,mhd->hnm", q.view(n, H, dk).double().abs(), kk.abs()).amax() * dk ** -0.5
     score = 64 * 2.0 ** -23 * sizes + 2.0 ** -23 * cap
     assert ((out.double() - want).abs() <= 2 * (2.0 ** -9 + 1.01 * score) * size + 2.0 ** -9 * want.abs() + 1e-30).all()
+
+
+@pytest.mark.parametrize("dk,dv", [(128, 64), (64, 128), (128, 128), (64, 64)])
+@pytest.mark.parametrize("form,spread", [("fp32", 1.0), ("fp32", 4.0), ("capped fp32", 1.0), ("capped fp32", 4.0), ("shared values", 4.0)])
+def test_no_further_from_64_bits_than_the_kernel_before(dk, dv, form, spread, monkeypatch):
+    """Of the forms that came from the mma.sync kernel, whose reference follows every row's maximum: the largest weight is 1 before its division, exactly."""
+    from mimirmind_b200.kernels import attention
+    n = 700
+    gen = torch.Generator(device=DEV).manual_seed(dk + dv)
+    rnd = lambda *s: torch.randn(s, generator=gen, device=DEV).to(torch.bfloat16)     # noqa: E731
+    Gv = 2 if form == "shared values" else G
+    q, k, v = spread * rnd(n, H * dk), rnd(-(-n // PAGE), G, PAGE, dk), rnd(-(-n // PAGE), Gv, PAGE, dv)
+    table = torch.arange(k.shape[0], dtype=torch.int32, device=DEV).view(1, -1)
+    errs = []
+    kk, vv = (t.transpose(1, 2).reshape(-1, t.shape[1], t.shape[3])[:n].double() for t in (k, v))
+    s = torch.einsum("nhd,mhd->hnm", q.view(n, H, dk).double(), kk.repeat_interleave(H // G, dim=1)) * dk ** -0.5
+    s = 20.0 * torch.tanh(s / 20.0) if "cap" in form else s
+    s = s.masked_fill(torch.ones(n, n, device=DEV).triu(1).bool(), float("-inf"))
+    top = s.amax(dim=-1, keepdim=True).clamp_min(0.0)          # the sink's score
+    p = torch.exp(s - top) / (torch.exp(s - top).sum(dim=-1, keepdim=True) + torch.exp(-top))
+    heads = torch.arange(H, device=DEV) // (H // G) % Gv
+    want = torch.einsum("hnm,mhd->nhd", p, vv[:, heads]).flatten(1)
+    for tensor_memory in (True, False):
+        monkeypatch.setattr(attention, "USE_SINK_TCGEN05", tensor_memory)
+        out = attend(q, k, v, table, dk, dv, form, lens=[n], begin=[0])
+        errs.append(((out.double() - want).norm() / want.norm()).item())
+    print(form, spread, dk, dv, "%.3e %.3e" % tuple(errs))
+    assert errs[0] <= 1.002 * errs[1]
