@@ -289,7 +289,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __gri
         const float f1 = (m1 == -INFINITY) ? 0.0f : fast_exp2((m1 - m) * scale_log2);
         // a softmax sink (a key without a value, of score 0 or the head's logit) only adds its weight, 2^(-m scale), to the row's sum
         const float sink_log2 = sink_logit != nullptr ? sink_logit[h] * 1.4426950408889634f : 0.0f;
-        const float total = l0 * f0 + l1 * f1 + (sink ? fast_exp2(fmaf(-m, scale_log2, sink_log2)) : 0.0f);
+        const float total = l0 * f0 + l1 * f1 + (sink || sink_logit != nullptr ? fast_exp2(fmaf(-m, scale_log2, sink_log2)) : 0.0f);
         // O of both groups is complete when their last P V is done (a group without tiles has no O)
         const int tiles0 = (n_tiles_k + 1) / 2, tiles1 = n_tiles_k / 2;
         if (ok && tiles0 > 0) ok = mbar_wait(smem_u32(&ctl->pv_done[0]), (uint32_t)(tiles0 - 1) & 1, abort_flag);

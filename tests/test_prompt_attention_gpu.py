@@ -106,6 +106,12 @@ def test_capped_scores_against_64_bits(cap, spread):
     assert ((out.double() - want).abs() <= 2 * (2.0 ** -9 + 1.01 * score) * size + 2.0 ** -9 * want.abs() + 1e-30).all()
 
 
+@pytest.mark.parametrize("dk,dv", [(128, 64), (128, 128)])
+def test_a_learned_sink_needs_no_flag(dk, dv):
+    q, k, v, table = setting(dk, dv, "logits")
+    assert torch.equal(attend(q, k, v, table, dk, dv, "logits", sink=False), attend(q, k, v, table, dk, dv, "logits", sink=True))
+
+
 @pytest.mark.parametrize("dk,dv", [(128, 64), (64, 128), (128, 128), (64, 64)])
 @pytest.mark.parametrize("form,spread", [("fp32", 1.0), ("fp32", 4.0), ("capped fp32", 1.0), ("capped fp32", 4.0), ("shared values", 4.0)])
 def test_no_further_from_64_bits_than_the_kernel_before(dk, dv, form, spread, monkeypatch):
