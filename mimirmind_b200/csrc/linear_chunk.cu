@@ -12,11 +12,13 @@
 // wait for the chunk before.  The launches:
 //   plain:  lc_state (what each chunk adds), lc_carry over the chunks per number of the state, lc_output;
 //   delta:  lc_delta_prepare (T, W, U0 per chunk), lc_delta_carry (U and S', chunk after chunk), lc_output with u for v.
-// A token costs dk dv multiply-adds three to four times as in the token-by-token walk, but as tiles of 16 x 8 x 8 on the tensor
-// cores: every operand is split into two tf32 numbers (11 bits each), the product is the sum of the
-// three larger of the four partial products, added up in 32 bits: 22 bits of every factor enter, and the error against 64 bits stays
-// that of the 32-bit walk (measured over random and correlated keys, see the tests).  mma.sync gives 92 TFLOP/s that way, the FMA
-// units, whose tiles are held up by shared-memory reads, 40 to 45.
+// A token costs dk dv multiply-adds three to four times as in the token-by-token walk, but as tiles of 16 x 8 x 16 on the tensor
+// cores (mma.sync): every operand is split into three bf16 numbers, which hold all of its 24 bits, and the product is the sum of the six
+// larger of the nine partial products, added up in 32 bits.  Error against 64 bits, of outputs and states over 300 to 4,096 tokens: where many tokens
+// add up (decays near 1) 0.7e-7 to 1.4e-7, half of the 32-bit walk's; where a state forgets half of itself per token, so that the
+// walk has little left to round, 0.6e-7 to 1.2e-7 (the walk: 0.4e-7 to 0.9e-7).  With two tf32 numbers (22 bits) and three products it was
+// 1.0e-7 to 2.4e-7 in both, for kernels 5 to 8 % shorter (4,096 tokens with the delta rule: chain 219 us, now 238, preparation 82 and 87, outputs 99 and
+// 108).  The FMA units, whose tiles are held up by shared-memory reads, take twice as long.
 // Ratios of decays are exponentials of differences of the logarithms' sums, which are kept in 64 bits: quotients of products of
 // the decays themselves would underflow within a chunk (0.2 a token), differences of 32-bit sums lose what lies close together.
 #include "common.cuh"
@@ -48,16 +50,39 @@ __device__ __forceinline__ void lc_load(float* s, const float* __restrict__ p, s
     }
 }
 
-// x = hi + lo: hi is x rounded to 11 bits (Veltkamp's split, with the FMA units; masks and integer additions take twice as
-// long), lo the rest, of which the tensor core reads the upper 11 bits.
+// Two numbers as three bf16 pairs each, x = h + m + l: every part is the rest rounded to 8 bits, so the three hold all 24 bits of x
+// (from 3.4e38, bf16's largest number, on x counts as infinite).
 struct LcSplit {
-    uint32_t hi, lo;
+    uint32_t h, m, l;
 };
-__device__ __forceinline__ LcSplit lc_split(float x) {
-    const float c = __fmul_rn(x, 8193.0f), hi = __fsub_rn(c, __fsub_rn(c, x));
+__device__ __forceinline__ uint32_t lc_round2(float x, float y) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(y), "f"(x));
+    return r;
+}
+__device__ __forceinline__ LcSplit lc_split(float x, float y) {
     LcSplit r;
-    r.hi = __float_as_uint(hi);
-    r.lo = __float_as_uint(__fsub_rn(x, hi));
+    r.h = lc_round2(x, y);
+    x = __fsub_rn(x, __uint_as_float(r.h << 16));
+    y = __fsub_rn(y, __uint_as_float(r.h & 0xffff0000u));
+    r.m = lc_round2(x, y);
+    x = __fsub_rn(x, __uint_as_float(r.m << 16));
+    y = __fsub_rn(y, __uint_as_float(r.m & 0xffff0000u));
+    r.l = lc_round2(x, y);
+    return r;
+}
+// The same of x f and y e, whose roundings go into the last parts.
+__device__ __forceinline__ LcSplit lc_split(float x, float f, float y, float e) {
+    const float p = __fmul_rn(x, f), q = __fmul_rn(y, e);
+    const float dp = __fmaf_rn(x, f, -p), dq = __fmaf_rn(y, e, -q);
+    LcSplit r;
+    r.h = lc_round2(p, q);
+    x = __fsub_rn(p, __uint_as_float(r.h << 16));
+    y = __fsub_rn(q, __uint_as_float(r.h & 0xffff0000u));
+    r.m = lc_round2(x, y);
+    x = __fadd_rn(__fsub_rn(x, __uint_as_float(r.m << 16)), dp);
+    y = __fadd_rn(__fsub_rn(y, __uint_as_float(r.m & 0xffff0000u)), dq);
+    r.l = lc_round2(x, y);
     return r;
 }
 struct LcA {
@@ -67,74 +92,127 @@ struct LcB {
     LcSplit x[2];
 };
 __device__ __forceinline__ void lc_mma(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ void lc_mma_first(float* c, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
         : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
 }
-// acc[i][j] += A_i B_j for eight k.  The tensor core cuts its sums off instead of rounding them, so a long chain of them drifts (1e-6 over
-// 128 k).  Eight k are added up there, from zero and the small terms first; the accumulators are added to by the FMA units, which
-// round to nearest.  The three steps go over all tiles in turn: one tile's next step would wait for its last.
-template <int NI, int NJ>
-__device__ __forceinline__ void lc_products(float (*acc)[NJ][4], const LcA* a, const LcB* b) {
-    float t[NI][NJ][4];
-#pragma unroll
-    for (int j = 0; j < NJ; ++j)
-#pragma unroll
-        for (int i = 0; i < NI; ++i) lc_mma_first(t[i][j], a[i].x[0].lo, a[i].x[1].lo, a[i].x[2].lo, a[i].x[3].lo, b[j].x[0].hi, b[j].x[1].hi);
-#pragma unroll
-    for (int j = 0; j < NJ; ++j)
-#pragma unroll
-        for (int i = 0; i < NI; ++i) lc_mma(t[i][j], a[i].x[0].hi, a[i].x[1].hi, a[i].x[2].hi, a[i].x[3].hi, b[j].x[0].lo, b[j].x[1].lo);
-#pragma unroll
-    for (int j = 0; j < NJ; ++j)
-#pragma unroll
-        for (int i = 0; i < NI; ++i) lc_mma(t[i][j], a[i].x[0].hi, a[i].x[1].hi, a[i].x[2].hi, a[i].x[3].hi, b[j].x[0].hi, b[j].x[1].hi);
-#pragma unroll
-    for (int i = 0; i < NI; ++i)
-#pragma unroll
-        for (int j = 0; j < NJ; ++j)
-#pragma unroll
-            for (int x = 0; x < 4; ++x) acc[i][j][x] += t[i][j][x];
+__device__ __forceinline__ void lc_mma_half(float* c, uint32_t a0, uint32_t a1, uint32_t b0) {      // eight k, from zero
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};\n"
+        : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+        : "r"(a0), "r"(a1), "r"(b0), "f"(0.0f));
 }
-// Fragments of eight k.  "rows": the operand stands as [m or n][k]; a thread takes k 2t and 2t + 1 for its two places (any order
-// of k will do, as long as both operands have the same), as one 8-byte word.  "rows4": the same in the order t, t + 4, for a
-// product whose other operand stands as [k][n].  "cols": the operand stands as [k][m or n], order t, t + 4.
+// acc[i][j] += the largest partial products of A_i B_j over sixteen k, low[i][j] += the next five (the three below 2^-25 of the whole are left out).
+// The tensor core shifts the products of a sum to the place of the largest and cuts off what falls below 2^-24 of it instead of rounding, so a
+// chain of sums of full 24-bit numbers drifts.  The largest products have 16 bits each: sixteen of them, from zero, lose little, and
+// the FMA units, which round to nearest, add that on.  What is cut off the others, 2^-8 of them, is as much smaller, so they
+// stay on the tensor core for all of k.  The result is acc + low: one rounding, where a chain of FMAs has one per k.  The steps go over
+// all tiles in turn: one tile's next step would wait for its last.
+// EIGHT: the largest products eight k at a time, for sums whose terms span many binades (the forget gate's states are off by 5.3e-8 of them so
+// instead of 6.3e-8; 2,048 tokens in 20.4 us instead of 19.5; elsewhere it costs 4 to 11 % and gains something only under strong decays).
+template <int NI, int NJ, bool EIGHT = false>
+__device__ __forceinline__ void lc_products(float (*acc)[NJ][4], float (*low)[NJ][4], const LcA* a, const LcB* b) {
+    constexpr int PARTS = EIGHT ? 2 : 1;
+    float t[PARTS][NI][NJ][4];
+#define LC_TILES                                   \
+    _Pragma("unroll") for (int j = 0; j < NJ; ++j) \
+    _Pragma("unroll") for (int i = 0; i < NI; ++i)
+#define LC_PART(MMA, TO, PA, PB) \
+    LC_TILES MMA(TO[i][j], a[i].x[0].PA, a[i].x[1].PA, a[i].x[2].PA, a[i].x[3].PA, b[j].x[0].PB, b[j].x[1].PB)
+    if constexpr (EIGHT) {
+#pragma unroll
+        for (int p = 0; p < PARTS; ++p) LC_TILES lc_mma_half(t[p][i][j], a[i].x[2 * p].h, a[i].x[2 * p + 1].h, b[j].x[p].h);
+    } else {
+        LC_PART(lc_mma_first, t[0], h, h);
+    }
+    LC_PART(lc_mma, low, l, h);
+    LC_PART(lc_mma, low, h, l);
+    LC_PART(lc_mma, low, m, m);
+    LC_PART(lc_mma, low, m, h);
+    LC_PART(lc_mma, low, h, m);
+#pragma unroll
+    for (int p = 0; p < PARTS; ++p)
+        LC_TILES
+#pragma unroll
+        for (int x = 0; x < 4; ++x) acc[i][j][x] += t[p][i][j][x];
+#undef LC_PART
+#undef LC_TILES
+}
+// The same for one column tile and 32 rows, acc[16 rows].
+template <bool EIGHT = false>
+__device__ __forceinline__ void lc_one(float (*acc)[4], float (*low)[4], const LcA* a, const LcB& b) {
+    lc_products<2, 1, EIGHT>(reinterpret_cast<float(*)[1][4]>(acc), reinterpret_cast<float(*)[1][4]>(low), a, &b);
+}
+template <int N>
+__device__ __forceinline__ void lc_zero(float* v) {
+#pragma unroll
+    for (int x = 0; x < N; ++x) v[x] = 0.0f;
+}
+template <int N>
+__device__ __forceinline__ void lc_add(float* v, const float* w) {
+#pragma unroll
+    for (int x = 0; x < N; ++x) v[x] += w[x];
+}
+// Fragments of sixteen k.  "rows": the operand stands as [m or n][k]; a thread takes k 2t, 2t + 1, 2t + 8 and 2t + 9 for its four places (any order
+// of k will do, as long as both operands have the same), as two 8-byte words.  "rows4": the same in the order t, t + 4, t + 8, t + 12, for a
+// product whose other operand stands as [k][n].  "cols": the operand stands as [k][m or n], order t, t + 4, t + 8, t + 12.
+__device__ __forceinline__ float2 lc_pair(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ LcA lc_a_rows(const float* p, int ld) {
     const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
-    const float2 x = *reinterpret_cast<const float2*>(p + g * ld + 2 * t), y = *reinterpret_cast<const float2*>(p + (g + 8) * ld + 2 * t);
-    return LcA{{lc_split(x.x), lc_split(y.x), lc_split(x.y), lc_split(y.y)}};
+    const float* lo = p + g * ld + 2 * t;
+    const float* hi = lo + 8 * ld;
+    const float2 w = lc_pair(lo), x = lc_pair(hi), y = lc_pair(lo + 8), z = lc_pair(hi + 8);
+    return LcA{{lc_split(w.x, w.y), lc_split(x.x, x.y), lc_split(y.x, y.y), lc_split(z.x, z.y)}};
 }
-// "rows" with a factor per k: scale points at the first of the eight
+// "rows" with a factor per k: scale points at the first of the sixteen
 __device__ __forceinline__ LcA lc_a_rows_scaled(const float* p, int ld, const float* scale) {
     const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
-    const float2 x = *reinterpret_cast<const float2*>(p + g * ld + 2 * t), y = *reinterpret_cast<const float2*>(p + (g + 8) * ld + 2 * t);
-    const float2 f = *reinterpret_cast<const float2*>(scale + 2 * t);
-    return LcA{{lc_split(x.x * f.x), lc_split(y.x * f.x), lc_split(x.y * f.y), lc_split(y.y * f.y)}};
+    const float* lo = p + g * ld + 2 * t;
+    const float* hi = lo + 8 * ld;
+    const float2 w = lc_pair(lo), x = lc_pair(hi), y = lc_pair(lo + 8), z = lc_pair(hi + 8);
+    const float2 f = lc_pair(scale + 2 * t), e = lc_pair(scale + 2 * t + 8);
+    return LcA{{lc_split(w.x, f.x, w.y, f.y), lc_split(x.x, f.x, x.y, f.y), lc_split(y.x, e.x, y.y, e.y), lc_split(z.x, e.x, z.y, e.y)}};
 }
 __device__ __forceinline__ LcB lc_b_rows(const float* p, int ld) {
     const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
-    const float2 x = *reinterpret_cast<const float2*>(p + g * ld + 2 * t);
-    return LcB{{lc_split(x.x), lc_split(x.y)}};
+    const float2 x = lc_pair(p + g * ld + 2 * t), y = lc_pair(p + g * ld + 2 * t + 8);
+    return LcB{{lc_split(x.x, x.y), lc_split(y.x, y.y)}};
 }
-// s0, s1: factors of the numbers at k = t and k = t + 4
-__device__ __forceinline__ LcA lc_a_rows4(const float* p, int ld, float s0, float s1) {
-    const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
-    return LcA{{lc_split(p[g * ld + t] * s0), lc_split(p[(g + 8) * ld + t] * s0), lc_split(p[g * ld + t + 4] * s1),
-                lc_split(p[(g + 8) * ld + t + 4] * s1)}};
+// the factors of a thread's four k: scale points at the first of the sixteen
+struct LcScale {
+    float f[4];
+};
+__device__ __forceinline__ LcScale lc_scale(const float* scale) {
+    const int t = threadIdx.x & 3;
+    return LcScale{{scale[t], scale[t + 4], scale[t + 8], scale[t + 12]}};
 }
-__device__ __forceinline__ LcA lc_a_cols(const float* p, int ld, float s0, float s1) {
+__device__ __forceinline__ LcA lc_a_rows4(const float* p, int ld) {
     const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
-    return LcA{{lc_split(p[t * ld + g] * s0), lc_split(p[t * ld + g + 8] * s0), lc_split(p[(t + 4) * ld + g] * s1),
-                lc_split(p[(t + 4) * ld + g + 8] * s1)}};
+    const float* lo = p + g * ld + t;
+    const float* hi = lo + 8 * ld;
+    return LcA{{lc_split(lo[0], lo[4]), lc_split(hi[0], hi[4]), lc_split(lo[8], lo[12]), lc_split(hi[8], hi[12])}};
+}
+__device__ __forceinline__ LcA lc_a_rows4(const float* p, int ld, const LcScale& s) {
+    const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    const float* lo = p + g * ld + t;
+    const float* hi = lo + 8 * ld;
+    return LcA{{lc_split(lo[0], s.f[0], lo[4], s.f[1]), lc_split(hi[0], s.f[0], hi[4], s.f[1]), lc_split(lo[8], s.f[2], lo[12], s.f[3]),
+                lc_split(hi[8], s.f[2], hi[12], s.f[3])}};
+}
+__device__ __forceinline__ LcA lc_a_cols(const float* p, int ld, const LcScale& s) {
+    const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+    const float* q = p + t * ld + g;
+    return LcA{{lc_split(q[0], s.f[0], q[4 * ld], s.f[1]), lc_split(q[8], s.f[0], q[4 * ld + 8], s.f[1]),
+                lc_split(q[8 * ld], s.f[2], q[12 * ld], s.f[3]), lc_split(q[8 * ld + 8], s.f[2], q[12 * ld + 8], s.f[3])}};
 }
 __device__ __forceinline__ LcB lc_b_cols(const float* p, int ld) {
     const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
-    return LcB{{lc_split(p[t * ld + g]), lc_split(p[(t + 4) * ld + g])}};
+    const float* q = p + t * ld + g;
+    return LcB{{lc_split(q[0], q[4 * ld]), lc_split(q[8 * ld], q[12 * ld])}};
 }
 
 // The sums of the decays' logarithms over the chunk's tokens, sb[t] = log gamma_t, by the first two warps; tokens beyond the
@@ -173,41 +251,45 @@ struct LcArgs {
 };
 
 // V^T diag(sr) K of a chunk, [dv, dk], to its place in `states`; k and v stand in shared memory.
-template <int DK, int DV>
+template <int DK, int DV, bool EIGHT = false>
 __device__ __forceinline__ void lc_add_up(const LcArgs& a, int h, int c, const float* sk, const float* sv, const float* sr) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int WM = DV / 32, WN = 8 / WM, NT = DK / WN / 8;      // warps along dv (32 rows each) and dk; tiles of 8 columns per warp
+    constexpr int RUN = NT < 4 ? NT : 4;         // column tiles at a time: more would not fit the registers
     const int m0 = (warp % WM) * 32, n0 = (warp / WM) * (DK / WN);
-    float acc[NT / 2][2][2][4];                  // [pair of column tiles][16 rows][column tile]
-#pragma unroll
-    for (int x = 0; x < NT * 8; ++x) (&acc[0][0][0][0])[x] = 0.0f;
     const int t = lane & 3, g = lane >> 2;
-#pragma unroll 2
-    for (int k0 = 0; k0 < LC_C; k0 += 8) {
-        const float s0 = sr[k0 + t], s1 = sr[k0 + t + 4];
-        LcA fa[2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) fa[i] = lc_a_cols(sv + k0 * LC_LD + m0 + 16 * i, LC_LD, s0, s1);
-#pragma unroll
-        for (int j = 0; j < NT / 2; ++j) {
-            const float* p = sk + k0 * LC_LD + n0 + 16 * j;
-            const LcB fb[2] = {lc_b_cols(p, LC_LD), lc_b_cols(p + 8, LC_LD)};
-            lc_products<2, 2>(acc[j], fa, fb);
-        }
-    }
     float* o = a.states + ((size_t)c * a.H + h) * a.dv * a.dk;
+#pragma unroll 1
+    for (int j0 = 0; j0 < NT; j0 += RUN) {
+        float acc[RUN][2][1][4], low[RUN][2][1][4];      // [column tile][16 rows]
+        lc_zero<RUN * 8>(&acc[0][0][0][0]);
+        lc_zero<RUN * 8>(&low[0][0][0][0]);
+#pragma unroll 1
+        for (int k0 = 0; k0 < LC_C; k0 += 16) {
+            const LcScale scale = lc_scale(sr + k0);
+            LcA fa[2];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+            for (int i = 0; i < 2; ++i) fa[i] = lc_a_cols(sv + k0 * LC_LD + m0 + 16 * i, LC_LD, scale);
 #pragma unroll
-        for (int j = 0; j < NT; ++j) {
-            const int n = n0 + 8 * j + 2 * t;
-            if (n >= a.dk) continue;
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const int m = m0 + 16 * i + g + 8 * half;
-                if (m < a.dv) *reinterpret_cast<float2*>(o + (size_t)m * a.dk + n) = make_float2(acc[j >> 1][i][j & 1][2 * half], acc[j >> 1][i][j & 1][2 * half + 1]);
+            for (int j = 0; j < RUN; ++j) {
+                const LcB fb = lc_b_cols(sk + k0 * LC_LD + n0 + 8 * (j0 + j), LC_LD);
+                lc_products<2, 1, EIGHT>(acc[j], low[j], fa, &fb);
             }
         }
+        lc_add<RUN * 8>(&acc[0][0][0][0], &low[0][0][0][0]);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < RUN; ++j) {
+                const int n = n0 + 8 * (j0 + j) + 2 * t;
+                if (n >= a.dk) continue;
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int m = m0 + 16 * i + g + 8 * half;
+                    if (m < a.dv) *reinterpret_cast<float2*>(o + (size_t)m * a.dk + n) = make_float2(acc[j][i][0][2 * half], acc[j][i][0][2 * half + 1]);
+                }
+            }
+    }
 }
 
 // ---- what a chunk adds to the state, as [dv, dk]: V^T diag(gamma_C / gamma) K -------------------------------------------------
@@ -297,24 +379,28 @@ __global__ void __launch_bounds__(256, 2) lc_output_kernel(LcArgs a, const float
     lc_decays(a.gate, a.head_decay, t0, cnt, a.H, h, sb);
     const int m0 = (warp & 1) * 32, wn = warp >> 1, t = lane & 3, g = lane >> 2;
     constexpr int HALVES = DV / 64;
-    float acc[HALVES][2][2][4];                  // [half of dv][16 rows][8 columns]
-#pragma unroll
-    for (int x = 0; x < HALVES * 16; ++x) (&acc[0][0][0][0])[x] = 0.0f;
+    float acc[HALVES][2][2][4], low[HALVES][2][2][4];      // [half of dv][8 columns][16 rows]
+    lc_zero<HALVES * 16>(&acc[0][0][0][0]);
+    lc_zero<HALVES * 16>(&low[0][0][0][0]);
     if (DV > 64) lc_wait<0>();
     else lc_wait<1>();
     __syncthreads();
-#pragma unroll 2
-    for (int k0 = 0; k0 < DK; k0 += 8) {         // (both halves of S with one reading of q)
+#pragma unroll 1
+    for (int k0 = 0; k0 < DK; k0 += 16) {         // (both halves of S with one reading of q)
         LcA fa[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows(sq + (m0 + 16 * i) * LC_LD + k0, LC_LD);
 #pragma unroll
         for (int b = 0; b < HALVES; ++b) {
-            const float* p = (b == 0 ? sa : su) + wn * 16 * LC_LD + k0;
-            const LcB fb[2] = {lc_b_rows(p, LC_LD), lc_b_rows(p + 8 * LC_LD, LC_LD)};
-            lc_products<2, 2>(acc[b], fa, fb);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const LcB fb = lc_b_rows((b == 0 ? sa : su) + (wn * 16 + 8 * j) * LC_LD + k0, LC_LD);
+                lc_one(acc[b][j], low[b][j], fa, fb);
+            }
         }
     }
+    lc_add<HALVES * 16>(&acc[0][0][0][0], &low[0][0][0][0]);
+    lc_zero<HALVES * 16>(&low[0][0][0][0]);
     __syncthreads();
     lc_load<DK, LC_LD>(sa, a.k + (size_t)t0 * a.ldk + (size_t)kh * a.dk, a.ldk, cnt, a.dk);
     lc_commit();
@@ -333,25 +419,29 @@ __global__ void __launch_bounds__(256, 2) lc_output_kernel(LcArgs a, const float
         for (int b = 0; b < HALVES; ++b)
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                acc[b][i][j][0] *= g0;
-                acc[b][i][j][1] *= g0;
-                acc[b][i][j][2] *= g1;
-                acc[b][i][j][3] *= g1;
+                acc[b][j][i][0] *= g0;
+                acc[b][j][i][1] *= g0;
+                acc[b][j][i][2] *= g1;
+                acc[b][j][i][3] *= g1;
             }
     }
     {   // scores of the rows m0.. and keys 16 wn..: nothing to do above the diagonal
-        float s[2][2][4];
-#pragma unroll
-        for (int x = 0; x < 16; ++x) (&s[0][0][0])[x] = 0.0f;
+        float s[2][2][4], s_low[2][2][4];        // [8 columns][16 rows]
+        lc_zero<16>(&s[0][0][0]);
+        lc_zero<16>(&s_low[0][0][0]);
         if (wn * 16 <= m0 + 31) {
-#pragma unroll 2
-            for (int k0 = 0; k0 < DK; k0 += 8) {
+#pragma unroll 1
+            for (int k0 = 0; k0 < DK; k0 += 16) {
                 LcA fa[2];
 #pragma unroll
                 for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows(sq + (m0 + 16 * i) * LC_LD + k0, LC_LD);
-                const LcB fb[2] = {lc_b_rows(sa + wn * 16 * LC_LD + k0, LC_LD), lc_b_rows(sa + (wn * 16 + 8) * LC_LD + k0, LC_LD)};
-                lc_products<2, 2>(s, fa, fb);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const LcB fb = lc_b_rows(sa + (wn * 16 + 8 * j) * LC_LD + k0, LC_LD);
+                    lc_one(s[j], s_low[j], fa, fb);
+                }
             }
+            lc_add<16>(&s[0][0][0], &s_low[0][0][0]);
         }
         __syncthreads();                         // every warp is through with k
 #pragma unroll
@@ -361,22 +451,26 @@ __global__ void __launch_bounds__(256, 2) lc_output_kernel(LcArgs a, const float
 #pragma unroll
                 for (int x = 0; x < 4; ++x) {
                     const int m = m0 + 16 * i + g + 8 * (x >> 1), n = wn * 16 + 8 * j + 2 * t + (x & 1);
-                    sa[m * LC_LP + n] = n <= m ? s[i][j][x] * lc_exp(sb[m] - sb[n]) : 0.0f;
+                    sa[m * LC_LP + n] = n <= m ? s[j][i][x] * lc_exp(sb[m] - sb[n]) : 0.0f;
                 }
     }
     lc_wait<0>();
     __syncthreads();
-    for (int k0 = 0; k0 < m0 + 32; k0 += 8) {
+    for (int k0 = 0; k0 < m0 + 32; k0 += 16) {
         LcA fa[2];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows4(sa + (m0 + 16 * i) * LC_LP + k0, LC_LP, 1.0f, 1.0f);
+        for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows4(sa + (m0 + 16 * i) * LC_LP + k0, LC_LP);
 #pragma unroll
         for (int b = 0; b < HALVES; ++b) {
             const float* p = su + k0 * LC_LD + 64 * b + wn * 16;
-            const LcB fb[2] = {lc_b_cols(p, LC_LD), lc_b_cols(p + 8, LC_LD)};
-            lc_products<2, 2>(acc[b], fa, fb);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const LcB fb = lc_b_cols(p + 8 * j, LC_LD);
+                lc_one(acc[b][j], low[b][j], fa, fb);
+            }
         }
     }
+    lc_add<HALVES * 16>(&acc[0][0][0][0], &low[0][0][0][0]);
 #pragma unroll
     for (int b = 0; b < HALVES; ++b)
 #pragma unroll
@@ -390,7 +484,7 @@ __global__ void __launch_bounds__(256, 2) lc_output_kernel(LcArgs a, const float
                     const int m = m0 + 16 * i + g + 8 * half;
                     if (m < cnt)
                         *reinterpret_cast<float2*>(a.out + ((size_t)(t0 + m) * a.H + h) * a.dv + n) =
-                            make_float2(acc[b][i][j][2 * half], acc[b][i][j][2 * half + 1]);
+                            make_float2(acc[b][j][i][2 * half], acc[b][j][i][2 * half + 1]);
                 }
             }
 }
@@ -502,18 +596,22 @@ __global__ void __launch_bounds__(256, 2) lc_delta_prepare_kernel(LcArgs a) {
     lc_wait<1>();
     __syncthreads();
     {
-        float s[2][2][4];
-#pragma unroll
-        for (int x = 0; x < 16; ++x) (&s[0][0][0])[x] = 0.0f;
+        float s[2][2][4], s_low[2][2][4];        // [8 columns][16 rows]
+        lc_zero<16>(&s[0][0][0]);
+        lc_zero<16>(&s_low[0][0][0]);
         if (wn * 16 <= m0 + 31) {
-#pragma unroll 2
-            for (int k0 = 0; k0 < DK; k0 += 8) {
+#pragma unroll 1
+            for (int k0 = 0; k0 < DK; k0 += 16) {
                 LcA fa[2];
 #pragma unroll
                 for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows(sk + (m0 + 16 * i) * LC_LD + k0, LC_LD);
-                const LcB fb[2] = {lc_b_rows(sk + wn * 16 * LC_LD + k0, LC_LD), lc_b_rows(sk + (wn * 16 + 8) * LC_LD + k0, LC_LD)};
-                lc_products<2, 2>(s, fa, fb);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const LcB fb = lc_b_rows(sk + (wn * 16 + 8 * j) * LC_LD + k0, LC_LD);
+                    lc_one(s[j], s_low[j], fa, fb);
+                }
             }
+            lc_add<16>(&s[0][0][0], &s_low[0][0][0]);
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i)
@@ -522,7 +620,7 @@ __global__ void __launch_bounds__(256, 2) lc_delta_prepare_kernel(LcArgs a) {
 #pragma unroll
                 for (int x = 0; x < 4; ++x) {
                     const int m = m0 + 16 * i + g + 8 * (x >> 1), n = wn * 16 + 8 * j + 2 * t + (x & 1);
-                    sL[m * LC_LP + n] = n < m ? s[i][j][x] * sbeta[m] * lc_exp(sb[m] - sb[n]) : 0.0f;
+                    sL[m * LC_LP + n] = n < m ? s[j][i][x] * sbeta[m] * lc_exp(sb[m] - sb[n]) : 0.0f;
                 }
     }
     lc_wait<0>();
@@ -531,24 +629,24 @@ __global__ void __launch_bounds__(256, 2) lc_delta_prepare_kernel(LcArgs a) {
     // both products: rows m0 + 16 i (32 per warp pair), columns wn * (COLS / 4)..; T has nothing to the right of its diagonal blocks
     auto product = [&](const float* s, const float* scale, int cols, int width, float* o, size_t ld, auto tiles) {
         constexpr int NT = decltype(tiles)::value;
-        float acc[NT / 2][2][2][4];
-#pragma unroll
-        for (int x = 0; x < NT * 8; ++x) (&acc[0][0][0][0])[x] = 0.0f;
-        for (int k0 = 0; k0 < m0 + 32; k0 += 8) {
-            const float s0 = scale[k0 + t], s1 = scale[k0 + t + 4];
+        float acc[NT][2][4], low[NT][2][4];      // [8 columns][16 rows]
+        lc_zero<NT * 8>(&acc[0][0][0]);
+        lc_zero<NT * 8>(&low[0][0][0]);
+        for (int k0 = 0; k0 < m0 + 32; k0 += 16) {
+            const LcScale f = lc_scale(scale + k0);
             LcA fa[2];
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const bool right = k0 >= m0 + 16 * i + 16;       // scratch: counts as zero
-                fa[i] = right ? LcA{} : lc_a_rows4(sT + (m0 + 16 * i) * LC_LP + k0, LC_LP, s0, s1);
+                fa[i] = right ? LcA{} : lc_a_rows4(sT + (m0 + 16 * i) * LC_LP + k0, LC_LP, f);
             }
 #pragma unroll
-            for (int j = 0; j < NT / 2; ++j) {
-                const float* p = s + k0 * LC_LD + wn * width + 16 * j;
-                const LcB fb[2] = {lc_b_cols(p, LC_LD), lc_b_cols(p + 8, LC_LD)};
-                lc_products<2, 2>(acc[j], fa, fb);
+            for (int j = 0; j < NT; ++j) {
+                const LcB fb = lc_b_cols(s + k0 * LC_LD + wn * width + 8 * j, LC_LD);
+                lc_one(acc[j], low[j], fa, fb);
             }
         }
+        lc_add<NT * 8>(&acc[0][0][0], &low[0][0][0]);
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -558,7 +656,7 @@ __global__ void __launch_bounds__(256, 2) lc_delta_prepare_kernel(LcArgs a) {
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
                     const int m = m0 + 16 * i + g + 8 * half;
-                    if (m < cnt) *reinterpret_cast<float2*>(o + (size_t)m * ld + n) = make_float2(acc[j >> 1][i][j & 1][2 * half], acc[j >> 1][i][j & 1][2 * half + 1]);
+                    if (m < cnt) *reinterpret_cast<float2*>(o + (size_t)m * ld + n) = make_float2(acc[j][i][2 * half], acc[j][i][2 * half + 1]);
                 }
             }
     };
@@ -659,22 +757,23 @@ __global__ void __launch_bounds__(LC_CARRY_THREADS) lc_delta_carry_kernel(LcArgs
         const float* sr = su + LC_C * LU;
         {
             const int m0 = (warp & 3) * 16, part = warp >> 2;
-            float p[1][NT][4];
+            float p[1][NT][4], low[1][NT][4];
+            lc_zero<NT * 4>(&p[0][0][0]);
+            lc_zero<NT * 4>(&low[0][0][0]);
 #pragma unroll
-            for (int x = 0; x < NT * 4; ++x) (&p[0][0][0])[x] = 0.0f;
-#pragma unroll
-            for (int k = 0; k < DK / 4; k += 8) {
+            for (int k = 0; k < DK / 4; k += 16) {
                 const int k0 = part * (DK / 4) + k;
                 const LcA fa = lc_a_rows(sw + m0 * LC_LD + k0, LC_LD);
                 LcB fb[NT];
 #pragma unroll
                 for (int j = 0; j < NT; ++j) {
-                    const float2 x = *reinterpret_cast<const float2*>(sS + (8 * j + g) * LC_LD + k0 + 2 * t);
-                    const float2 y = *reinterpret_cast<const float2*>(sS + (NS + 8 * j + g) * LC_LD + k0 + 2 * t);
-                    fb[j] = LcB{{lc_split(x.x + y.x), lc_split(x.y + y.y)}};
+                    const float* one = sS + (8 * j + g) * LC_LD + k0 + 2 * t;
+                    const float2 x0 = lc_pair(one), y0 = lc_pair(one + NS * LC_LD), x1 = lc_pair(one + 8), y1 = lc_pair(one + NS * LC_LD + 8);
+                    fb[j] = LcB{{lc_split(x0.x + y0.x, x0.y + y0.y), lc_split(x1.x + y1.x, x1.y + y1.y)}};
                 }
-                lc_products<1, NT>(p, &fa, fb);
+                lc_products<1, NT>(p, low, &fa, fb);
             }
+            lc_add<NT * 4>(&p[0][0][0], &low[0][0][0]);
 #pragma unroll
             for (int j = 0; j < NT; ++j)
 #pragma unroll
@@ -687,28 +786,31 @@ __global__ void __launch_bounds__(LC_CARRY_THREADS) lc_delta_carry_kernel(LcArgs
         if (threadIdx.x < LC_C * (NS / 4)) {
             const int row = threadIdx.x / (NS / 4), col = (threadIdx.x % (NS / 4)) * 4;
             float4 u = *reinterpret_cast<const float4*>(su + row * LU + col);
+            float4 x[4];
 #pragma unroll
-            for (int part = 0; part < 4; ++part) {
-                const float4 x = *reinterpret_cast<const float4*>(sp + (part * LC_C + row) * LQ + col);
-                u = make_float4(u.x - x.x, u.y - x.y, u.z - x.z, u.w - x.w);
-            }
+            for (int part = 0; part < 4; ++part) x[part] = *reinterpret_cast<const float4*>(sp + (part * LC_C + row) * LQ + col);
+            u.x -= (x[0].x + x[1].x) + (x[2].x + x[3].x);
+            u.y -= (x[0].y + x[1].y) + (x[2].y + x[3].y);
+            u.z -= (x[0].z + x[1].z) + (x[2].z + x[3].z);
+            u.w -= (x[0].w + x[1].w) + (x[2].w + x[3].w);
             *reinterpret_cast<float4*>(su + row * LU + col) = u;
             if (row < cnt && col < cols) *reinterpret_cast<float4*>(a.u + ((size_t)(t0 + row) * a.H + h) * a.dv + n_base + col) = u;
         }
         __syncthreads();
         if (has_rows) {
-            float p[1][NT][4];
+            float p[1][NT][4], low[1][NT][4];
+            lc_zero<NT * 4>(&p[0][0][0]);
+            lc_zero<NT * 4>(&low[0][0][0]);
 #pragma unroll
-            for (int x = 0; x < NT * 4; ++x) (&p[0][0][0])[x] = 0.0f;
-#pragma unroll
-            for (int k = 0; k < LC_C / 2; k += 8) {
+            for (int k = 0; k < LC_C / 2; k += 16) {
                 const int k0 = side * (LC_C / 2) + k;
-                const LcA fa = lc_a_cols(sk + k0 * LC_LD + s_row, LC_LD, sr[k0 + t], sr[k0 + t + 4]);
+                const LcA fa = lc_a_cols(sk + k0 * LC_LD + s_row, LC_LD, lc_scale(sr + k0));
                 LcB fb[NT];
 #pragma unroll
                 for (int j = 0; j < NT; ++j) fb[j] = lc_b_cols(su + k0 * LU + 8 * j, LU);
-                lc_products<1, NT>(p, &fa, fb);
+                lc_products<1, NT>(p, low, &fa, fb);
             }
+            lc_add<NT * 4>(&p[0][0][0], &low[0][0][0]);
 #pragma unroll
             for (int j = 0; j < NT; ++j)
 #pragma unroll
@@ -773,7 +875,7 @@ __global__ void __launch_bounds__(256, 2) lc_forget_state_kernel(LcArgs a) {
     }
     if (first == 0 && ch < a.dk) a.gain[((size_t)c * a.H + h) * a.dk + ch] = sF[0][ch] * sF[1][ch] * sF[2][ch] * sF[3][ch];
     __syncthreads();
-    lc_add_up<DK, DV>(a, h, c, sf, sv, sr);
+    lc_add_up<DK, DV, true>(a, h, c, sf, sv, sr);
 }
 
 // Two blocks per SM: q (then q', then the scores), f (then k'), and a buffer for S's halves and then v.
@@ -857,20 +959,23 @@ __global__ void __launch_bounds__(256, 2) lc_forget_output_kernel(LcArgs a) {
     }
     const int m0 = (warp & 1) * 32, wn = warp >> 1, t = lane & 3, g = lane >> 2;
     constexpr int HALVES = DV / 64;
-    float acc[HALVES][2][2][4];
-#pragma unroll
-    for (int x = 0; x < HALVES * 16; ++x) (&acc[0][0][0][0])[x] = 0.0f;
+    float acc[HALVES][2][2][4], low[HALVES][2][2][4];      // [half of dv][8 columns][16 rows]
+    lc_zero<HALVES * 16>(&acc[0][0][0][0]);
+    lc_zero<HALVES * 16>(&low[0][0][0][0]);
 #pragma unroll
     for (int b = 0; b < HALVES; ++b) {
         lc_wait<0>();
         __syncthreads();
-#pragma unroll 2
-        for (int k0 = 0; k0 < DK; k0 += 8) {
+#pragma unroll 1
+        for (int k0 = 0; k0 < DK; k0 += 16) {
             LcA fa[2];
 #pragma unroll
             for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows_scaled(sq + (m0 + 16 * i) * LC_LD + k0, LC_LD, &sbefore[m0 / 16 + i][k0]);
-            const LcB fb[2] = {lc_b_rows(sx + wn * 16 * LC_LD + k0, LC_LD), lc_b_rows(sx + (wn * 16 + 8) * LC_LD + k0, LC_LD)};
-            lc_products<2, 2>(acc[b], fa, fb);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const LcB fb = lc_b_rows(sx + (wn * 16 + 8 * j) * LC_LD + k0, LC_LD);
+                lc_one(acc[b][j], low[b][j], fa, fb);
+            }
         }
         __syncthreads();
         if (b + 1 < HALVES) lc_load<DK, LC_LD>(sx, a.dv > 64 ? S + (size_t)64 * a.dk : S, a.dk, a.dv - 64, a.dk);
@@ -878,19 +983,20 @@ __global__ void __launch_bounds__(256, 2) lc_forget_output_kernel(LcArgs a) {
         lc_commit();
     }
     // between the runs: warp w < 6 takes one of the blocks (1,0) (2,0) (2,1) (3,0) (3,1) (3,2)
-    float cross[2][4];
-#pragma unroll
-    for (int x = 0; x < 8; ++x) (&cross[0][0])[x] = 0.0f;
+    float cross[1][2][4], cross_low[1][2][4];
+    lc_zero<8>(&cross[0][0][0]);
+    lc_zero<8>(&cross_low[0][0][0]);
     const int bi = warp == 0 ? 1 : warp < 3 ? 2 : 3, bj = warp == 0 ? 0 : warp < 3 ? warp - 1 : warp - 3;
     if (warp < 6) {
         const float* between = bi - bj == 1 ? sone : bi - bj == 2 ? sF[bi - 1] : smid;
-#pragma unroll 4
-        for (int k0 = 0; k0 < DK; k0 += 8) {
+#pragma unroll 2
+        for (int k0 = 0; k0 < DK; k0 += 16) {
             const LcA fa = lc_a_rows_scaled(sq + bi * LC_RUN * LC_LD + k0, LC_LD, between + k0);
             const float* p = sf + bj * LC_RUN * LC_LD + k0;
             const LcB fb[2] = {lc_b_rows(p, LC_LD), lc_b_rows(p + 8 * LC_LD, LC_LD)};
-            lc_products<1, 2>(&cross, &fa, fb);
+            lc_products<1, 2>(cross, cross_low, &fa, fb);
         }
+        lc_add<8>(&cross[0][0][0], &cross_low[0][0][0]);
     }
     __syncthreads();                             // every warp is through with q': the scores take its place
 #pragma unroll
@@ -900,22 +1006,26 @@ __global__ void __launch_bounds__(256, 2) lc_forget_output_kernel(LcArgs a) {
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int x = 0; x < 4; ++x) sq[(bi * LC_RUN + g + 8 * (x >> 1)) * LC_LP + bj * LC_RUN + 8 * j + 2 * t + (x & 1)] = cross[j][x];
+            for (int x = 0; x < 4; ++x) sq[(bi * LC_RUN + g + 8 * (x >> 1)) * LC_LP + bj * LC_RUN + 8 * j + 2 * t + (x & 1)] = cross[0][j][x];
     }
     lc_wait<0>();
     __syncthreads();
-    for (int k0 = 0; k0 < m0 + 32; k0 += 8) {
+    for (int k0 = 0; k0 < m0 + 32; k0 += 16) {
         LcA fa[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i)              // nothing stands to the right of a row's own run
-            fa[i] = k0 >= m0 + 16 * i + 16 ? LcA{} : lc_a_rows4(sq + (m0 + 16 * i) * LC_LP + k0, LC_LP, 1.0f, 1.0f);
+            fa[i] = k0 >= m0 + 16 * i + 16 ? LcA{} : lc_a_rows4(sq + (m0 + 16 * i) * LC_LP + k0, LC_LP);
 #pragma unroll
         for (int b = 0; b < HALVES; ++b) {
             const float* p = sx + k0 * LC_LD + 64 * b + wn * 16;
-            const LcB fb[2] = {lc_b_cols(p, LC_LD), lc_b_cols(p + 8, LC_LD)};
-            lc_products<2, 2>(acc[b], fa, fb);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const LcB fb = lc_b_cols(p + 8 * j, LC_LD);
+                lc_one(acc[b][j], low[b][j], fa, fb);
+            }
         }
     }
+    lc_add<HALVES * 16>(&acc[0][0][0][0], &low[0][0][0][0]);
 #pragma unroll
     for (int b = 0; b < HALVES; ++b)
 #pragma unroll
@@ -929,7 +1039,7 @@ __global__ void __launch_bounds__(256, 2) lc_forget_output_kernel(LcArgs a) {
                     const int m = m0 + 16 * i + g + 8 * half;
                     if (m < cnt)
                         *reinterpret_cast<float2*>(a.out + ((size_t)(t0 + m) * a.H + h) * a.dv + n) =
-                            make_float2(acc[b][i][j][2 * half], acc[b][i][j][2 * half + 1]);
+                            make_float2(acc[b][j][i][2 * half], acc[b][j][i][2 * half + 1]);
                 }
             }
 }

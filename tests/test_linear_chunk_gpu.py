@@ -68,7 +68,7 @@ def test_products(H, G, dk, dv, delta, decay):
             scale = ref.norm()
             err, was = ((mine - ref).norm() / scale).item(), ((old - ref).norm() / scale).item()
             print(f"err {err:.2e} walk {was:.2e}")
-            # 22 bits of every factor of up to 64 + 128 + 128 products one after the other, each rounded like the walk's: a few 2^-22
+            # up to 64 + 128 + 128 products one after the other, their sums rounded like the walk's: a few 2^-22
             assert err <= max(5e-7, 1.5 * was), (r, err, was)
 
 
