@@ -216,14 +216,18 @@ __device__ __forceinline__ LcB lc_b_cols(const float* p, int ld) {
 }
 
 // The sums of the decays' logarithms over the chunk's tokens, sb[t] = log gamma_t, by the first two warps; tokens beyond the
-// chunk add nothing.  A decay of 0 counts as exp(-200), which no 32-bit number can tell from it.
+// chunk add nothing.  A decay of 0 counts as exp(-200), which no 32-bit number can tell from it; one that is no number (or negative) is
+// NaN here, and so is all that comes after it.
 __device__ __forceinline__ void lc_decays(const float* __restrict__ gate, const float* __restrict__ head_decay, int t0, int cnt, int H, int h,
                                           double* sb) {
     __shared__ double first_half;
     double x = 0.0;
     const int t = threadIdx.x, lane = t & 31;
     if (t < LC_C) {
-        if (t < cnt) x = (double)fmaxf(logf(gate ? gate[(size_t)(t0 + t) * H + h] : head_decay[h]), -200.0f);
+        if (t < cnt) {
+            const float l = logf(gate ? gate[(size_t)(t0 + t) * H + h] : head_decay[h]);
+            x = (double)(l < -200.0f ? -200.0f : l);         // (keeps a NaN, which fmaxf would not)
+        }
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const double up = __shfl_up_sync(0xffffffffu, x, o);

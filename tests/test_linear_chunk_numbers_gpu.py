@@ -92,3 +92,14 @@ def test_very_large_numbers(kind):
     got, want = p.run(True), p.exact()
     for mine, ref in zip(got, want):
         assert torch.isfinite(mine).all() and ((mine.double() - ref).norm() / ref.norm()).item() <= 2e-7
+
+
+@pytest.mark.parametrize("kind", ["plain", "delta"])
+@pytest.mark.parametrize("token", [0, 37, 64, 149])
+def test_a_decay_that_is_no_number(kind, token):
+    """It makes the state one that is no number, as in the walk: not an empty one."""
+    p = Portion(kind, 150)
+    p.gate[token, 1] = float("nan")
+    (out, state), (walk, walked) = p.run(True), p.run(False)
+    assert torch.equal(torch.isnan(out[token:]), torch.isnan(walk[token:])) and torch.equal(torch.isnan(state), torch.isnan(walked))
+    assert torch.isnan(state.view(p.H, -1)[1]).all() and not torch.isnan(state.view(p.H, -1)[[0, 2, 3]]).any()
