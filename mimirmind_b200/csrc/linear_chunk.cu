@@ -50,6 +50,21 @@ __device__ __forceinline__ void lc_load(float* s, const float* __restrict__ p, s
     }
 }
 
+// Whether the 16-byte pieces that this thread itself has brought in with lc_load (and waited for) hold a number that the products turn into a NaN:
+// a NaN, an infinity or one beyond bf16's range.
+template <int COLS, int LD, int THREADS = 256>
+__device__ __forceinline__ bool lc_not_finite(const float* s) {
+    constexpr int Q = COLS / 4;
+    uint32_t top = 0;
+#pragma unroll
+    for (int e = 0; e < 64 * Q / THREADS; ++e) {
+        const int idx = threadIdx.x + e * THREADS;
+        const uint4 v = *reinterpret_cast<const uint4*>(s + (idx / Q) * LD + (idx % Q) * 4);
+        top = max(max(max(v.x & 0x7fffffffu, v.y & 0x7fffffffu), max(v.z & 0x7fffffffu, v.w & 0x7fffffffu)), top);
+    }
+    return top >= 0x7f7f8000u;
+}
+
 // Two numbers as three bf16 pairs each, x = h + m + l: every part is the rest rounded to 8 bits, so the three hold all 24 bits of x
 // (from 3.4e38, bf16's largest number, on x counts as infinite).
 struct LcSplit {
@@ -240,6 +255,29 @@ __device__ __forceinline__ void lc_decays(const float* __restrict__ gate, const 
     __syncthreads();
 }
 __device__ __forceinline__ float lc_exp(double x) { return expf((float)x); }
+
+// acc += scores [64][LC_LP] x values [64][LC_LD] for the warp's rows m0.. and columns, a row's own token and those before it only: a product of tiles
+// multiplies a later token's numbers with zeros, and where they are infinite or NaN that is a NaN.  Taken by chunks that hold such
+// a number, whose outputs before its token stay what they are without it.
+__device__ __noinline__ float lc_causal_sum(float sum, const float* scores, const float* values, int m) {
+    for (int s = 0; s <= m; ++s) sum = fmaf(scores[s], values[s * LC_LD], sum);
+    return sum;
+}
+template <int HALVES>
+__device__ __forceinline__ void lc_causal(float (*acc)[2][2][4], const float* scores, const float* values, int m0, int wn) {
+    const int t = threadIdx.x & 3, g = (threadIdx.x & 31) >> 2;
+#pragma unroll
+    for (int b = 0; b < HALVES; ++b)
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    const int m = m0 + 16 * i + g + 8 * (x >> 1), n = 64 * b + wn * 16 + 8 * j + 2 * t + (x & 1);
+                    acc[b][j][i][x] = lc_causal_sum(acc[b][j][i][x], scores + m * LC_LP, values + n, m);
+                }
+}
 
 struct LcArgs {
     const float *q, *k, *v, *gate, *beta, *head_decay;
@@ -459,8 +497,9 @@ __global__ void __launch_bounds__(256, 2) lc_output_kernel(LcArgs a, const float
                 }
     }
     lc_wait<0>();
-    __syncthreads();
-    for (int k0 = 0; k0 < m0 + 32; k0 += 16) {
+    const bool plain = !__syncthreads_or(lc_not_finite<DV, LC_LD>(su));
+    if (!plain) lc_causal<HALVES>(acc, sa, su, m0, wn);
+    else for (int k0 = 0; k0 < m0 + 32; k0 += 16) {
         LcA fa[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows4(sa + (m0 + 16 * i) * LC_LP + k0, LC_LP);
@@ -588,9 +627,11 @@ __global__ void __launch_bounds__(256, 2) lc_delta_prepare_kernel(LcArgs a) {
     lc_load<DV, LC_LD>(sv, a.v + (size_t)t0 * a.ldv + (size_t)h * a.dv, a.ldv, cnt, a.dv);
     lc_commit();
     lc_decays(a.gate, a.head_decay, t0, cnt, a.H, h, sb);
+    bool odd = false;                            // a NaN or an infinity
     if (threadIdx.x < LC_C) {
         const int t = threadIdx.x;
         const float b = t < cnt ? a.beta[(size_t)(t0 + t) * a.H + h] : 0.0f;
+        odd = !(fabsf(b) < INFINITY && fabs(sb[t]) < INFINITY);
         sbeta[t] = b;
         sbg[t] = b * lc_exp(sb[t]);
         a.ratio[((size_t)c * a.H + h) * LC_C + t] = lc_exp(sb[LC_C - 1] - sb[t]);
@@ -628,7 +669,22 @@ __global__ void __launch_bounds__(256, 2) lc_delta_prepare_kernel(LcArgs a) {
                 }
     }
     lc_wait<0>();
-    __syncthreads();
+    odd |= lc_not_finite<DK, LC_LD>(sk) || lc_not_finite<DV, LC_LD>(sv);
+    if (__syncthreads_or(odd)) {                 // W and U0 by substitution, a column per thread, in place: no row takes part in one before it
+        if (threadIdx.x < DK + DV) {
+            const bool key = threadIdx.x < DK;
+            float* col = key ? sk + threadIdx.x : sv + (threadIdx.x - DK);
+            for (int m = 0; m < LC_C; ++m) {
+                float x = (key ? sbg : sbeta)[m] * col[m * LC_LD];
+                for (int p = 0; p < m; ++p) x = fmaf(-sL[m * LC_LP + p], col[p * LC_LD], x);
+                col[m * LC_LD] = x;
+            }
+        }
+        __syncthreads();
+        for (int idx = threadIdx.x; idx < cnt * a.dk; idx += 256) a.w[((size_t)(t0 + idx / a.dk) * a.H + h) * a.dk + idx % a.dk] = sk[idx / a.dk * LC_LD + idx % a.dk];
+        for (int idx = threadIdx.x; idx < cnt * a.dv; idx += 256) a.u[((size_t)(t0 + idx / a.dv) * a.H + h) * a.dv + idx % a.dv] = sv[idx / a.dv * LC_LD + idx % a.dv];
+        return;
+    }
     lc_invert(sL, sT);
     // both products: rows m0 + 16 i (32 per warp pair), columns wn * (COLS / 4)..; T has nothing to the right of its diagonal blocks
     auto product = [&](const float* s, const float* scale, int cols, int width, float* o, size_t ld, auto tiles) {
@@ -1013,8 +1069,9 @@ __global__ void __launch_bounds__(256, 2) lc_forget_output_kernel(LcArgs a) {
             for (int x = 0; x < 4; ++x) sq[(bi * LC_RUN + g + 8 * (x >> 1)) * LC_LP + bj * LC_RUN + 8 * j + 2 * t + (x & 1)] = cross[0][j][x];
     }
     lc_wait<0>();
-    __syncthreads();
-    for (int k0 = 0; k0 < m0 + 32; k0 += 16) {
+    const bool plain = !__syncthreads_or(lc_not_finite<DV, LC_LD>(sx));
+    if (!plain) lc_causal<HALVES>(acc, sq, sx, m0, wn);
+    else for (int k0 = 0; k0 < m0 + 32; k0 += 16) {
         LcA fa[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i)              // nothing stands to the right of a row's own run

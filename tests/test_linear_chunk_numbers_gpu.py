@@ -103,3 +103,20 @@ def test_a_decay_that_is_no_number(kind, token):
     (out, state), (walk, walked) = p.run(True), p.run(False)
     assert torch.equal(torch.isnan(out[token:]), torch.isnan(walk[token:])) and torch.equal(torch.isnan(state), torch.isnan(walked))
     assert torch.isnan(state.view(p.H, -1)[1]).all() and not torch.isnan(state.view(p.H, -1)[[0, 2, 3]]).any()
+
+
+@pytest.mark.parametrize("kind,what", [(k, w) for k in ("plain", "delta", "forget") for w in ("q", "k", "v", "gate", "beta")
+                                       if not (k == "forget" and w == "gate") and (k == "delta" or w != "beta")])
+@pytest.mark.parametrize("number", [float("nan"), float("inf")])
+@pytest.mark.parametrize("token", [0, 37, 64, 70, 127, 149])
+@pytest.mark.parametrize("dk,dv", [(128, 128), (64, 64)])
+def test_a_number_that_is_none_reaches_later_tokens_only(kind, what, number, token, dk, dv):
+    if number == float("inf") and (what in ("gate", "beta") or (kind == "forget" and what == "k")):
+        pytest.skip("decays and strengths are logistic values: a NaN is the only one that can stand there")
+    p = Portion(kind, 150, dk=dk, dv=dv)
+    clean = p.run(True)[0].clone()
+    getattr(p, what)[token, 5 if what in ("q", "k", "v") else 1] = number
+    (out, state), (walk, walked) = p.run(True), p.run(False)
+    # before the token nothing has changed, but for the order of a chunk's sums
+    assert torch.isfinite(out[:token]).all() and (out[:token] - clean[:token]).norm() <= 1e-6 * clean.norm()
+    assert torch.equal(torch.isfinite(out), torch.isfinite(walk)) and torch.equal(torch.isfinite(state), torch.isfinite(walked))
