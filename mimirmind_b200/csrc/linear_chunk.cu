@@ -728,7 +728,8 @@ __global__ void __launch_bounds__(256, 2) lc_delta_prepare_kernel(LcArgs a) {
 // Bound by the chain of the two products and its barriers, and within it by issuing instructions (splitting the operands is most of
 // them), so 16 warps share the k of each product and a warp makes as many tiles as use its fragments: in the first, warp w has rows
 // 16 (w % 4) of U and a quarter of the key channels, in the second rows 16 (w % 8) of dk and half of the tokens; both have all
-// NS columns.  The quarters meet in a pass over U, the halves never: S is kept as the sum of two, each carried by its own warps.
+// NS columns.  The quarters meet in a pass over U, the halves in the next chunk: S is read as the sum of the first half's numbers, which are
+// carried, and of what the second half has just added (two sums that were carried side by side would grow apart and cancel).
 // The next chunk's W, k and U0 arrive under the current one's products.  64 chunks: 229 us (254 with a tile and half of the k per warp).
 #define LC_CARRY_THREADS 512
 template <int DK, int NS>
@@ -757,7 +758,7 @@ __global__ void __launch_bounds__(LC_CARRY_THREADS) lc_delta_carry_kernel(LcArgs
         if (threadIdx.x < LC_C / 4) lc_cp16(sr + 4 * threadIdx.x, a.ratio + ((size_t)(first + i) * a.H + h) * LC_C + 4 * threadIdx.x, true);
         lc_commit();
     };
-    // the warp's part of S: rows 16 (warp % 8).. of dk (if there are so many), all columns; the second half's part starts from zero
+    // rows 16 (warp % 8).. of dk (if there are so many), all columns: in the first half's warps S, in the second's what they add per chunk
     const int s_row = (warp & 7) * 16;
     const bool has_rows = s_row < DK;
     float S[NT][4];
@@ -842,6 +843,11 @@ __global__ void __launch_bounds__(LC_CARRY_THREADS) lc_delta_carry_kernel(LcArgs
                         make_float2(p[0][j][2 * half], p[0][j][2 * half + 1]);
         }
         to_global(a.states + ((size_t)c * a.H + h) * a.dv * a.dk, true);
+        if (side == 0 && has_rows)
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) S[j][x] += sS[(NS + 8 * j + 2 * t + (x & 1)) * LC_LD + s_row + g + 8 * (x >> 1)];
         __syncthreads();
         if (threadIdx.x < LC_C * (NS / 4)) {
             const int row = threadIdx.x / (NS / 4), col = (threadIdx.x % (NS / 4)) * 4;
@@ -874,7 +880,7 @@ __global__ void __launch_bounds__(LC_CARRY_THREADS) lc_delta_carry_kernel(LcArgs
 #pragma unroll
             for (int j = 0; j < NT; ++j)
 #pragma unroll
-                for (int x = 0; x < 4; ++x) S[j][x] = fmaf(gain, S[j][x], p[0][j][x]);
+                for (int x = 0; x < 4; ++x) S[j][x] = side == 0 ? fmaf(gain, S[j][x], p[0][j][x]) : p[0][j][x];
         }
         to_shared();                             // read by everyone before the pass over U
         t0 = next_t0;

@@ -105,6 +105,14 @@ def test_a_decay_that_is_no_number(kind, token):
     assert torch.isnan(state.view(p.H, -1)[1]).all() and not torch.isnan(state.view(p.H, -1)[[0, 2, 3]]).any()
 
 
+@pytest.mark.parametrize("n", [2048])
+def test_what_a_chunk_writes_and_takes_back(n):
+    p = Portion("delta", n, keys="the same", decay="none")
+    want = p.exact()
+    for mine, walk in zip(errors(p.run(True), want), errors(p.run(False), want)):
+        assert mine <= 1.2 * walk, (mine, walk)
+
+
 @pytest.mark.parametrize("kind,what", [(k, w) for k in ("plain", "delta", "forget") for w in ("q", "k", "v", "gate", "beta")
                                        if not (k == "forget" and w == "gate") and (k == "delta" or w != "beta")])
 @pytest.mark.parametrize("number", [float("nan"), float("inf")])
