@@ -440,8 +440,7 @@ static int launch_attention_f32(const void* q, const void* k_pages, const void* 
                                 cudaStream_t s) {
     const int tile_bytes = (ATT_TILE * (HD + 4) * 3 + 2 * ATT_TILE * HD + ATT_TILE * (ATT_TILE + 4)) * (int)sizeof(float);
     const int token_bytes = (128 * (HD + 4) + 128 * HD + HD + 128) * (int)sizeof(float);
-    if (cudaFuncSetAttribute(attention_tile_f32_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_bytes) != cudaSuccess ||
-        cudaFuncSetAttribute(attention_token_f32_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, token_bytes) != cudaSuccess) {
+    if (!mm_allow_smem<attention_tile_f32_kernel<HD>>(tile_bytes) || !mm_allow_smem<attention_token_f32_kernel<HD>>(token_bytes)) {
         mm_set_last_error("attention: cannot reserve shared memory");
         return MM_ERR_LAUNCH;
     }

@@ -355,7 +355,7 @@ struct PrefillArgs {
 template <int HDK, int HDV, bool CAP, bool FOLLOW>
 static int attention_prefill_launch_as(const PrefillArgs& a, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, cudaStream_t s) {
     constexpr size_t smem = (size_t)(HDK / 64 + 4 + KV_STAGES * (HDK / 64 + HDV / 64)) * HALF_BYTES + sizeof(AttCtl);
-    if (cudaFuncSetAttribute(attention_prefill_tc_kernel<HDK, HDV, CAP, FOLLOW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    if (!mm_allow_smem<attention_prefill_tc_kernel<HDK, HDV, CAP, FOLLOW>>(smem)) {
         mm_set_last_error("attention_prefill_tcgen05: cannot reserve shared memory");
         return MM_ERR_LAUNCH;
     }

@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #define MM_OK 0
 #define MM_ERR_BAD_ARG 1       // a size or combination the kernel refuses
 #define MM_ERR_UNSUPPORTED 2   // valid in principle, not built for this shape/dtype
@@ -184,6 +186,20 @@ static inline void mm_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
+// Allows every launch of `Kernel` up to `bytes` of dynamic shared memory (the most that any of them asks for): once per device, not per launch,
+// where the call would come on top of the launch's own time on the host.
+template <auto Kernel>
+static inline bool mm_allow_smem(size_t bytes) {
+    static std::atomic<unsigned long long> allowed{0};      // a bit per device
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+    if (allowed.load(std::memory_order_acquire) & bit) return true;
+    if (cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
+    allowed.fetch_or(bit, std::memory_order_release);
+    return true;
 }
 
 // ---- programmatic dependent launch --------------------------------------------------------------------------------------

@@ -252,7 +252,7 @@ static int launch_gemv_simt(const void* A, const void* W, const void* bias, int 
                             cudaStream_t s) {
     const size_t smem = (size_t)STAGES * (NB + M) * (KB + 4) * sizeof(float);
     constexpr size_t most = (size_t)STAGES * (NB + SIMT_GEMV_ROWS) * (KB + 4) * sizeof(float);
-    if (cudaFuncSetAttribute(gemv_simt_kernel<NB, KB, STAGES, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) {
+    if (!mm_allow_smem<gemv_simt_kernel<NB, KB, STAGES, R>>(most)) {
         mm_set_last_error("gemm: cannot reserve shared memory");
         return MM_ERR_LAUNCH;
     }
@@ -266,8 +266,7 @@ template <typename TA, typename TW, typename TC, int BM, int BN, int TM, int TN,
 static int launch_simt_tile(const void* A, const void* W, const void* bias, int bias_dtype, void* C, int M, int N, int K, int lda, int ldc,
                             cudaStream_t s) {
     const int smem = 2 * BK * (BM + BN) * (int)sizeof(float);
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(gemm_simt_kernel<TA, TW, TC, BM, BN, TM, TN, BK, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 smem) != cudaSuccess) {
+    if (smem > 48 * 1024 && !mm_allow_smem<gemm_simt_kernel<TA, TW, TC, BM, BN, TM, TN, BK, VEC>>(smem)) {
         mm_set_last_error("gemm: cannot reserve shared memory");
         return MM_ERR_LAUNCH;
     }

@@ -1111,13 +1111,13 @@ __global__ void __launch_bounds__(256, 2) lc_forget_output_kernel(LcArgs a) {
             }
 }
 
-template <typename... A>
-static int lc_launch(void (*kernel)(A...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+template <auto Kernel, typename... A>
+static int lc_launch(dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+    if (smem > 0 && !mm_allow_smem<Kernel>(smem)) {
         mm_set_last_error("linear state chunks: cannot reserve shared memory");
         return MM_ERR_LAUNCH;
     }
-    mm_launch(kernel, grid, dim3(threads), smem, s, args...);
+    mm_launch(Kernel, grid, dim3(threads), smem, s, args...);
     MM_CHECK_LAUNCH();
     return MM_OK;
 }
@@ -1127,20 +1127,20 @@ static int lc_run(const LcArgs& a, int n_requests, cudaStream_t s) {
     const dim3 chunks(a.H, a.n_chunks);
     const size_t tile = LC_C * LC_LD * sizeof(float), square = LC_C * LC_LP * sizeof(float);
     if (a.beta == nullptr) {
-        if (const int rc = lc_launch(lc_state_kernel<DK, DV>, chunks, 256, 2 * tile, s, a)) return rc;
+        if (const int rc = lc_launch<lc_state_kernel<DK, DV>>(chunks, 256, 2 * tile, s, a)) return rc;
         const long long size = (long long)a.H * a.dv * a.dk;
-        if (const int rc = lc_launch(lc_carry_kernel<false>, dim3(ceil_div(size / 4, 256), n_requests), 256, 0, s, a)) return rc;
-        return lc_launch(lc_output_kernel<DK, DV>, chunks, 256, 3 * tile, s, a, a.v, (size_t)a.ldv);
+        if (const int rc = lc_launch<lc_carry_kernel<false>>(dim3(ceil_div(size / 4, 256), n_requests), 256, 0, s, a)) return rc;
+        return lc_launch<lc_output_kernel<DK, DV>>(chunks, 256, 3 * tile, s, a, a.v, (size_t)a.ldv);
     }
-    if (const int rc = lc_launch(lc_delta_prepare_kernel<DK, DV>, chunks, 256, 2 * tile + 2 * square, s, a)) return rc;
+    if (const int rc = lc_launch<lc_delta_prepare_kernel<DK, DV>>(chunks, 256, 2 * tile + 2 * square, s, a)) return rc;
     // columns of S per block: 16 while the blocks then fit the SMs (one each: 186 KB), else 32, whose chain is a little longer
     const bool wide = (long long)ceil_div(a.dv, 16) * a.H * n_requests > 148 && a.dv > 16;
 #define LC_CARRY(NS)                                                                                                                       \
-    lc_launch(lc_delta_carry_kernel<DK, NS>, dim3(ceil_div(a.dv, NS), a.H, n_requests), LC_CARRY_THREADS,                                   \
+    lc_launch<lc_delta_carry_kernel<DK, NS>>(dim3(ceil_div(a.dv, NS), a.H, n_requests), LC_CARRY_THREADS,                                   \
               (size_t)(2 * (2 * LC_C * LC_LD + LC_C * (NS + 8) + LC_C + 4) + 2 * NS * LC_LD + 4 * LC_C * (NS + 4)) * sizeof(float), s, a)
     if (const int rc = wide ? LC_CARRY(32) : LC_CARRY(16)) return rc;
 #undef LC_CARRY
-    return lc_launch(lc_output_kernel<DK, DV>, chunks, 256, 3 * tile, s, a, (const float*)a.u, (size_t)a.H * a.dv);
+    return lc_launch<lc_output_kernel<DK, DV>>(chunks, 256, 3 * tile, s, a, (const float*)a.u, (size_t)a.H * a.dv);
 }
 
 // 1 if the products take these sizes and pointers: heads of up to 128 numbers that are multiples of 4, rows and heads on 16-byte boundaries
@@ -1183,10 +1183,10 @@ template <int DK, int DV>
 static int lc_run_forget(const LcArgs& a, int n_requests, cudaStream_t s) {
     const dim3 chunks(a.H, a.n_chunks);
     const size_t tile = LC_C * LC_LD * sizeof(float);
-    if (const int rc = lc_launch(lc_forget_state_kernel<DK, DV>, chunks, 256, 2 * tile, s, a)) return rc;
+    if (const int rc = lc_launch<lc_forget_state_kernel<DK, DV>>(chunks, 256, 2 * tile, s, a)) return rc;
     const long long size = (long long)a.H * a.dv * a.dk;
-    if (const int rc = lc_launch(lc_carry_kernel<true>, dim3(ceil_div(size / 4, 256), n_requests), 256, 0, s, a)) return rc;
-    return lc_launch(lc_forget_output_kernel<DK, DV>, chunks, 256, 3 * tile, s, a);
+    if (const int rc = lc_launch<lc_carry_kernel<true>>(dim3(ceil_div(size / 4, 256), n_requests), 256, 0, s, a)) return rc;
+    return lc_launch<lc_forget_output_kernel<DK, DV>>(chunks, 256, 3 * tile, s, a);
 }
 
 // The recurrence with a forget gate per key channel: f [tokens, H dk] beside q; gain fp32 [chunks, H, dk]; the rest as above.

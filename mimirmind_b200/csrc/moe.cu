@@ -381,7 +381,7 @@ MM_EXPORT int mm_moe_sort(const void* idx, int n_rows, int E, void* offsets, voi
     int threads = n_rows > 256 ? 1024 : 256;
     while (threads > 128 && (size_t)(2 + threads / 32) * E * sizeof(int32_t) > 100 * 1024) threads /= 2;      // thousands of experts: fewer warps' counts
     const size_t sort_smem = (size_t)(2 + threads / 32) * E * sizeof(int32_t);
-    if (sort_smem > 48 * 1024 && cudaFuncSetAttribute(moe_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sort_smem) != cudaSuccess) {
+    if (sort_smem > 48 * 1024 && !mm_allow_smem<moe_sort_kernel>(100 * 1024)) {
         mm_set_last_error("moe sort: cannot reserve shared memory");
         return MM_ERR_LAUNCH;
     }

@@ -882,7 +882,7 @@ MM_EXPORT int mm_sample_rows(const void* logits, void* out, int R, int V, const 
     const size_t room = (R * ranks <= sms ? 200 * 1024 : 112 * 1024) - sizeof(SampleShared);
     const int cache_floats = (size_t)chunk * sizeof(float) <= room ? chunk : 0;
     const size_t smem = sizeof(SampleShared) + (size_t)cache_floats * sizeof(float);
-    if (cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess) {
+    if (!mm_allow_smem<sample_rows_kernel>(200 * 1024)) {
         mm_set_last_error("sample: cannot reserve shared memory");
         return MM_ERR_LAUNCH;
     }

@@ -138,3 +138,14 @@ def test_no_further_from_64_bits_than_the_kernel_before(dk, dv, form, spread, mo
         errs.append(((out.double() - want).norm() / want.norm()).item())
     print(form, spread, dk, dv, "%.3e %.3e" % tuple(errs))
     assert errs[0] <= 1.002 * errs[1]
+
+
+def test_shared_memory_is_reserved_once():
+    """Not on every launch: the host's time is what bounds a layer over a short prompt."""
+    from torch.profiler import ProfilerActivity, profile
+    q, k, v, table = setting(128, 64, "window")
+    attend(q, k, v, table, 128, 64, "window")
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as seen:
+        attend(q, k, v, table, 128, 64, "window")
+    names = [e.key for e in seen.key_averages()]
+    assert any("Launch" in n for n in names) and not any("FuncSetAttribute" in n for n in names)
