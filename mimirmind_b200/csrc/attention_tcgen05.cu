@@ -13,18 +13,17 @@
 //                         the 128-byte-swizzled K-major layout the tensor core reads
 //     O[g] += P V         tcgen05.mma 128x128x16 x 8, V read MN-major (as stored: keys x head dim), accumulated
 //                         in tensor memory over all key tiles of the group
-// O is rescaled lazily: probabilities are taken relative to a reference maximum that is only moved (and O, in
+// With equal sizes and no options O is rescaled lazily: probabilities are taken relative to a reference maximum that is only moved (and O, in
 // tensor memory, multiplied by the matching factor with tcgen05.ld / tcgen05.st) when the row's maximum has grown
 // by more than 2^8 since; until then P may exceed 1 by that factor, which bf16 and the fp32 sums hold easily.
 // After the first few tiles a row's maximum rarely grows that much, so the threads neither read nor scale O per
-// tile.  S and P are double-buffered: while the softmax threads work on tile t the tensor core already computes S
+// tile.  The other forms (FOLLOW) move it with every new maximum, which keeps the largest probability exact.  S and P are double-buffered: while the softmax threads work on tile t the tensor core already computes S
 // of tile t+1 and adds P V of tile t-1.
 // Warp 1 issues Q K^T, warp 11 issues P V (a single issuing thread, waiting on the barriers of both products in
 // turn, was what bound the kernel); warp 0 = TMA producer for keys (and Q), warp 10 = TMA producer for values: every lane fetches one half of one
 // page, so the 16 to 32 small copies of a tile are issued at once (one thread issuing them in turn was the
 // bottleneck of the whole kernel); warp 1 = MMA issuer and tensor-memory owner; warps 2..9 = softmax and output.  Same formula as the other attention kernels (reference src/compute/Attention.cpp:43-94).
-// Warp 0 requests Q and the first key tile before the CTA's set-up barrier (tensor-memory allocation, zeroing of the value
-// ring), which nothing of that needs.
+// Warp 0 requests Q and the first key tile before the CTA's set-up barrier (tensor-memory allocation), which nothing of that needs.
 // The keys a query sees may also be its own run of tokens, and the first tokens of the sequence beside either (KeyMask): the walk over
 // key tiles then starts with the kept tokens' tiles.  A head's output may be multiplied by the logistic of a number per token.
 // All mbarrier waits are bounded; on a time-out the kernel frees its tensor memory, sets `err`
