@@ -24,8 +24,14 @@
 #define FIXED_ONE 1099511627776.0f  // 2^40
 
 __device__ __forceinline__ uint32_t order_key(float v) {
+    // (u | 0x80000000 would be compiled to a negation of the absolute value, which does not keep a NaN's bits)
     const uint32_t u = __float_as_uint(v);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+    return u ^ ((uint32_t)((int32_t)u >> 31) | 0x80000000u);
+}
+// The key among masses: a NaN counts as one of the best for top-k, but stands below all positive logits where masses are added up.
+__device__ __forceinline__ uint32_t mass_key(float v) {
+    const uint32_t key = order_key(v);
+    return key > 0xff800000u ? 0x7fffffffu : key;
 }
 
 // splitmix64 finaliser over (seed, counter): a stateless stream of 64-bit numbers
@@ -162,48 +168,112 @@ MM_EXPORT int mm_argmax_rows_split(const void* logits, void* out, void* part_val
 // reading.
 //
 // Top-k, top-p and the draw each look for one element of the same order (logit descending, index ascending): the first
-// whose cumulative count or mass exceeds a target.  One pass over the row makes mass and count per eighth of a nat
-// below the maximum (256 bins), from which all three find the bin of their element; the few elements of that bin
-// (divided by 256 once more if they are more than DRAW_LIST) are put into a list in the first CTA's shared memory,
-// which finds the element there.  So a row is read once from memory and once or twice more per search from the copy
-// of the slice in shared memory (or L2), where a radix select over all elements took four passes per search and a
-// weight's exponential in each.  Masses are added in 32-bit halves of 20 bits: shared memory adds 32-bit numbers by
-// itself, 64-bit ones by compare and swap.  32 rows of 152,064 logits with top-p: 303 us before, 55 us now.
+// whose cumulative count or mass exceeds a target.  A row is read once from memory, 16 bytes a load, and kept in shared memory:
+//   1. mass and count per eighth of a nat below the maximum (256 bins), in 16 copies that the lanes of a warp share out: a
+//      warp's additions then hardly ever meet in a bank.  Masses in halves of 20 bits: shared memory adds 32-bit numbers by
+//      itself, 64-bit ones by compare and swap.
+//   2. From these each search's bin is known, or a short range of bins: top-p's target depends on what top-k keeps and the
+//      draw's on what top-p keeps, which lies between the sums before and after a bin; all steps are monotone.
+//   3. If more than DRAW_LIST numbers lie in these bins: the same once more with 1/2048 of a nat, over their numbers only.
+//   4. The numbers of the bins go into a list, and the first CTA finds all three elements there.
+// Bound by instructions (an exponential, three additions in shared memory and some 30 more per number, 75 numbers a thread) and
+// by four or five exchanges of the cluster.  With a pass, two cluster barriers and a list for each search, and copies of the
+// bins by warp, 32 rows of 152,064 logits with top-p took 62 us, this takes 44 (with 1.5 as temperature, where the cut
+// lies among most of the row, 77 and 46; both from HBM).  The numbers in registers instead of shared memory, unrolled, took twice as long as
+// before: 76 copies of a pass are more instructions than their cache holds.  So did bins of two nats in a column per thread,
+// without atomics: what is saved there is lost on the second pass that they need.
 // Rows with a NaN or an infinite maximum, and searches that end in more than DRAW_LIST logits within 1/2048 nat, take
-// the radix select.
+// the radix select, four passes per search over the slice.
 #define DRAW_THREADS 512
 #define DRAW_WARPS (DRAW_THREADS / 32)
-#define DRAW_COPIES 8                              // histograms of a CTA: two warps share one
-#define DRAW_SEGMENT (DRAW_COPIES * 4064)          // elements counted before the 32-bit sums are emptied: 2 warps x 2032 each, at most 2^20 an element
+#define DRAW_COPIES 8                              // the radix select's histograms of a CTA: two warps share one
+#define DRAW_LANES 16                              // copies of the bins: two lanes of a warp share one
 #define DRAW_LIST 2048
-#define DRAW_SCALE 8.0f                            // bins per nat
+#define DRAW_NEAR 512                              // numbers that a warp keeps the places of
+#define DRAW_SLOTS 4                               // bins that are cut finer at once
+#define DRAW_FINE (DRAW_SLOTS * 256)
+#define DRAW_FEW 128                               // elements among which every one is compared with every other
+#define DRAW_LO_MAX 3800                           // numbers of one bin whose low and high halves 32 bits hold: at most 2^20 e^(1/16) each
+#define DRAW_ROOM 38016                            // numbers of a slice kept in shared memory beside the rest: 227 KB together
+#define DRAW_SLICE_MAX (DRAW_LANES * DRAW_LO_MAX)  // numbers of a slice that the sums have room for
 #define SAMPLE_MAX_CLUSTER 8
 
-struct DrawHist {
-    uint32_t lo[DRAW_COPIES][256], hi[DRAW_COPIES][256], ct[DRAW_COPIES][256];
+struct BinPlace {
+    unsigned long long before, carry;              // the mass of the bins before it, what is left of the target
+    unsigned long long upto;                       // the mass including it
+    int bin, sub;                                  // sub: -1 without the finer bins
+    uint32_t count;                                // numbers in it
+};
+struct BinTable {                                  // 256 bins: mass, count and their sums up to and including a bin
+    unsigned long long mass[256], upto[256];
+    uint32_t ct[256], upto_ct[256];
 };
 
-struct SampleShared {
+struct alignas(16) SampleShared {
     union {
-        DrawHist h;
-        unsigned long long list[DRAW_LIST];        // (order key << 32) | index
-        unsigned long long whist[DRAW_COPIES][256];   // the radix select's
+        struct {
+            uint32_t lo[257][DRAW_LANES], hi[257][DRAW_LANES], ct[257][DRAW_LANES];
+        } hist;
+        struct {
+            union {
+                struct {
+                    uint32_t lo[DRAW_FINE], hi[DRAW_FINE];
+                    unsigned long long pub[DRAW_FINE];             // the masses as published
+                };
+                unsigned long long own[DRAW_LIST];                 // then this CTA's candidates
+                unsigned long long sublist[DRAW_LIST];             // then, in the first CTA, those of one bin
+            };
+            union {
+                uint32_t ct[DRAW_FINE];                            // published
+                struct {
+                    uint32_t lo[256], hi[256], ct[256];
+                } cut;                                             // then a cut within the list
+            };
+            BinTable tab[DRAW_SLOTS];                              // the cluster's
+        } fine;
+        unsigned long long whist[DRAW_COPIES][256];                // the radix select's
         int counts[DRAW_THREADS];
     };
-    unsigned long long pub[2][256 + 4];            // what this CTA publishes: a histogram, or scalars in [256..]
-    uint32_t pub_ct[2][256];
-    unsigned long long tot[256], tot1[256];        // the cluster's histogram; the one of the first level
-    uint32_t tot_ct[256], tot1_ct[256];
+    union {
+        unsigned short near[DRAW_WARPS][DRAW_NEAR];                // places in the slice of the numbers of the bins that hold places, by warp
+        unsigned long long list[DRAW_LIST];        // then, in the first CTA, the cluster's candidates: (order key << 32) | index
+    };
+    BinTable tab;                                  // the cluster's bins
+    union {
+        uint32_t pub_ct[256];
+        unsigned long long few_w[DRAW_FEW];        // masses of a bin's candidates
+    };
+    union {
+        struct {
+            unsigned long long pub[2][256 + 4];    // what this CTA publishes: masses, or scalars in [256..]
+            unsigned long long tot[256];           // of the radix select: the cluster's histogram
+        };
+        BinTable cut_tab;                          // of a cut within the list
+    };
     unsigned long long warp_part[DRAW_WARPS];
     unsigned long long carry, before;              // what is left of the target inside the chosen bin; the mass of the bins before it
+    unsigned long long found_mass;
+    BinPlace place[2];
+    float want[3][2];                              // where the searches may end, in 1/2048 nat below the maximum: from, up to
+    uint32_t found_key, found_index, found_tie;
     uint32_t chosen, chosen_ct;
-    uint32_t list_n;
+    uint32_t mask[8];                              // the bins that hold these places
+    int slot_bin[DRAW_SLOTS];                      // those that are cut finer
+    unsigned char slot_of[256], marked[257];       // a bin's slot + 1 (0: not cut); 1 for a bin that held places at first
+    uint32_t n_list, list_n, few_n, too_many, is_fine;
     uint32_t range[2];
     int result;
 };
+static_assert(sizeof(SampleShared) % 16 == 0 && sizeof(SampleShared) + DRAW_ROOM * sizeof(float) <= 227 * 1024, "beyond a CTA's shared memory");
+
+// This CTA's.  Functions that are called rather than inlined take it from here: a pointer that is passed to them would make every access of theirs,
+// the atomic ones above all, one to an address of unknown kind.
+__device__ __forceinline__ SampleShared* draw_shared() {
+    extern __shared__ __align__(16) unsigned char sample_smem[];
+    return reinterpret_cast<SampleShared*>(sample_smem);
+}
 
 struct ClusterCtx {
-    SampleShared* sh;
     const float* vals;                             // this CTA's slice: its copy in shared memory, or the row itself
     int vals_begin;                                // index of vals[0] in the row
     uint32_t rank, n_ranks;
@@ -267,8 +337,8 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v)
 
 // Every CTA's value is reduced over its threads and published; returns the sum (or the maximum) over the cluster, the
 // same in every thread of every CTA.
-__device__ unsigned long long cluster_combine(ClusterCtx& c, unsigned long long mine, bool take_max) {
-    SampleShared* sh = c.sh;
+__device__ __noinline__ unsigned long long cluster_combine(ClusterCtx& c, unsigned long long mine, bool take_max) {
+    SampleShared* sh = draw_shared();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     mine = take_max ? warp_max_u64(mine) : warp_sum_u64(mine);
     __syncthreads();
@@ -294,136 +364,113 @@ __device__ __forceinline__ unsigned long long weight_of(float logit, float inv_t
     const float p = expf(logit * inv_t - max_scaled);
     return (unsigned long long)(p * FIXED_ONE);
 }
+// The same of a plain row, whose weights are below 2^41, in halves of 20 bits (and what is above): by sums that cut off what lies below the integer.
+struct Halves {
+    uint32_t low, high;
+};
+__device__ __forceinline__ Halves weight_halves(float logit, float inv_t, float max_scaled) {
+    const float p = expf(__fmaf_rn(logit, inv_t, -max_scaled));
+    const float high = __fmaf_rz(p, 1048576.0f, 8388608.0f);
+    const float low = __fadd_rz(__fmaf_rn(high - 8388608.0f, -1048576.0f, p * FIXED_ONE), 8388608.0f);
+    return Halves{__float_as_uint(low) & 0x7fffffu, __float_as_uint(high) & 0x7fffffu};
+}
+__device__ __forceinline__ unsigned long long weight_below(float logit, float inv_t, float max_scaled) {
+    const Halves w = weight_halves(logit, inv_t, max_scaled);
+    return ((unsigned long long)w.high << 20) + w.low;
+}
 __device__ __forceinline__ float logit_of_key(uint32_t key) {
     return __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
 }
 
-// The bin (in ascending order of bins) in which the cumulative weight, counts or masses, exceeds `target`, by the first
-// warp: left in chosen, with its count in chosen_ct, what is left of the target in carry and the mass before it in
-// `before`.  A target at or beyond the total (rounding at the tail) takes the last bin that holds anything.
-__device__ void pick_bin(SampleShared* sh, const unsigned long long* mass, const uint32_t* count, bool by_count, unsigned long long target) {
+// The bin of tot (in ascending order of bins) in which the cumulative weight exceeds `target`, by the first warp: left in
+// chosen, with what is left of the target in carry.  A target at or beyond the total (rounding at the tail) takes the last bin
+// that holds anything.
+__device__ __noinline__ void pick_bin(unsigned long long target) {
+    SampleShared* sh = draw_shared();
     __syncthreads();
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
-        unsigned long long h[8], m[8], mine = 0ull, mine_m = 0ull;
+        unsigned long long h[8], mine = 0ull;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            m[j] = mass[8 * lane + j];
-            h[j] = by_count ? (unsigned long long)count[8 * lane + j] : m[j];
+            h[j] = sh->tot[8 * lane + j];
             mine += h[j];
-            mine_m += m[j];
         }
-        unsigned long long incl = mine, incl_m = mine_m;
+        unsigned long long incl = mine;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, o), up_m = __shfl_up_sync(0xffffffffu, incl_m, o);
-            if (lane >= o) {
-                incl += up;
-                incl_m += up_m;
-            }
+            const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
         }
-        unsigned long long cum = incl - mine, cum_m = incl_m - mine_m, rem = 0ull, before = 0ull, last_rem = 0ull, last_before = 0ull;
+        unsigned long long cum = incl - mine, rem = 0ull, last_rem = 0ull;
         int chosen = -1, last = -1;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             if (chosen < 0 && h[j] && target < cum + h[j]) {
                 chosen = 8 * lane + j;
                 rem = target - cum;
-                before = cum_m;
             }
             if (h[j]) {
                 last = 8 * lane + j;
                 last_rem = h[j] - 1ull;
-                last_before = cum_m;
             }
             cum += h[j];
-            cum_m += m[j];
         }
         const uint32_t found = __ballot_sync(0xffffffffu, chosen >= 0), any = __ballot_sync(0xffffffffu, last >= 0);
         const int owner = found ? __ffs(found) - 1 : any ? 31 - __clz(any) : 0;
         if (lane == owner) {
-            const int bin = found ? chosen : last < 0 ? 0 : last;
-            sh->chosen = (uint32_t)bin;
-            sh->chosen_ct = count[bin];
+            sh->chosen = (uint32_t)(found ? chosen : last < 0 ? 0 : last);
             sh->carry = found ? rem : last_rem;
-            sh->before = found ? before : last_before;
         }
     }
     __syncthreads();
 }
 
-// bins of the two levels of a plain row; monotone in the logit (a product, a sum and a conversion, each rounded, are)
+// The sums of a table, by one warp: eight rows of 32 bins side by side.
+__device__ __noinline__ void sum_table(uint32_t offset) {     // of the table within SampleShared
+    BinTable* t = reinterpret_cast<BinTable*>(reinterpret_cast<unsigned char*>(draw_shared()) + offset);
+    const int lane = threadIdx.x & 31;
+    unsigned long long m[8], carry = 0ull;
+    uint32_t n[8], carry_ct = 0u;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        m[j] = t->mass[32 * j + lane];
+        n[j] = t->ct[32 * j + lane];
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const unsigned long long up = __shfl_up_sync(0xffffffffu, m[j], o);
+            const uint32_t up_ct = __shfl_up_sync(0xffffffffu, n[j], o);
+            if (lane >= o) {
+                m[j] += up;
+                n[j] += up_ct;
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        t->upto[32 * j + lane] = m[j] + carry;
+        t->upto_ct[32 * j + lane] = n[j] + carry_ct;
+        carry += __shfl_sync(0xffffffffu, m[j], 31);
+        carry_ct += __shfl_sync(0xffffffffu, n[j], 31);
+    }
+}
+
+// Bins of a plain row, monotone in the logit (a rounded product and sum, a scaling and limits are): 65536 of 1/2048 nat below the
+// maximum, the last one without an end; 256 of them are a bin of the first level.
 struct DrawBins {
     float inv_t, max_scaled;
-    __device__ __forceinline__ float place(float v) const { return __fmul_rn(__fmaf_rn(-v, inv_t, max_scaled), DRAW_SCALE); }
-    __device__ __forceinline__ int first(float v) const { return (int)fmaxf(fminf(place(v), 255.0f), 0.0f); }
-    // within bin b of the first level
-    __device__ __forceinline__ int second(float v, int b) const { return (int)fmaxf(fminf((place(v) - (float)b) * 256.0f, 255.0f), 0.0f); }
+    __device__ __forceinline__ float place(float v) const { return fmaxf(fminf(2048.0f * __fmaf_rn(-v, inv_t, max_scaled), 65535.0f), 0.0f); }
+    // The bin of the first level, 0 to 256 (256 is the end of bin 255), as the low bits of the result: powers of two scale exactly and the limits
+    // come with the sum, so this is two instructions.  inv_t and max_scaled divided by 32.
+    static __device__ __forceinline__ uint32_t first_bits(float v, float inv_t32, float max_scaled32) {
+        return __float_as_uint(__fmaf_rz(__saturatef(__fmaf_rn(-v, inv_t32, max_scaled32)), 256.0f, 8388608.0f));
+    }
+    // the integer part, from the low bits of a sum that cuts the rest off
+    __device__ __forceinline__ int of(float v) const { return (int)(__float_as_uint(__fadd_rz(place(v), 8388608.0f)) & 65535u); }
 };
-
-// Mass and count of every bin over the cluster, in tot and tot_ct.  bin(v): 0..255, or below 0 for an element that is left out.
-template <class Bin>
-__device__ void draw_hist(ClusterCtx& c, int begin, int end, float inv_t, float max_scaled, Bin bin) {
-    SampleShared* sh = c.sh;
-    uint32_t* flat = &sh->h.lo[0][0];
-    const int copy = (threadIdx.x >> 5) % DRAW_COPIES;
-    unsigned long long mass = 0ull;
-    uint32_t count = 0u;
-    for (int seg = begin; seg == begin || seg < end; seg += DRAW_SEGMENT) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < 3 * DRAW_COPIES * 256; i += DRAW_THREADS) flat[i] = 0u;
-        __syncthreads();
-        const int stop = min(end, seg + DRAW_SEGMENT);
-        for (int i = seg + (int)threadIdx.x; i < stop; i += 4 * DRAW_THREADS) {
-            float v[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int j = i + u * DRAW_THREADS;
-                v[u] = j < stop ? c.vals[j - c.vals_begin] : 0.0f;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (i + u * DRAW_THREADS >= stop) continue;
-                const int at = bin(v[u]);
-                if (at < 0) continue;
-                const unsigned long long w = weight_of(v[u], inv_t, max_scaled);
-                const uint32_t low = (uint32_t)w & 0xfffffu, high = (uint32_t)(w >> 20);
-                if (low) atomicAdd(&sh->h.lo[copy][at], low);
-                if (high) atomicAdd(&sh->h.hi[copy][at], high);
-                atomicAdd(&sh->h.ct[copy][at], 1u);
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x < 256) {
-            unsigned long long low = 0ull, high = 0ull;
-#pragma unroll
-            for (int k = 0; k < DRAW_COPIES; ++k) {
-                low += sh->h.lo[k][threadIdx.x];
-                high += sh->h.hi[k][threadIdx.x];
-                count += sh->h.ct[k][threadIdx.x];
-            }
-            mass += low + (high << 20);
-        }
-    }
-    const uint32_t b = c.round & 1;
-    if (threadIdx.x < 256) {
-        sh->pub[b][threadIdx.x] = mass;
-        sh->pub_ct[b][threadIdx.x] = count;
-    }
-    __syncthreads();
-    sample_cluster_sync();
-    if (threadIdx.x < 256) {
-        unsigned long long sum = 0ull, v[SAMPLE_MAX_CLUSTER];
-        ld_all_peers_u64(&sh->pub[b][threadIdx.x], c.n_ranks, v);
-#pragma unroll
-        for (uint32_t r = 0; r < SAMPLE_MAX_CLUSTER; ++r) sum += v[r];
-        sh->tot[threadIdx.x] = sum;
-    } else {
-        sh->tot_ct[threadIdx.x - 256] = sum_all_peers_u32(&sh->pub_ct[b][threadIdx.x - 256], c.n_ranks);
-    }
-    ++c.round;
-    __syncthreads();
-}
 
 // Candidates are the elements with key >= floor_key.  In the order (key descending, index ascending) find the
 // first element whose cumulative weight exceeds `target`.  Weight is 1 when `by_count`, else the fixed-point
@@ -431,23 +478,23 @@ __device__ void draw_hist(ClusterCtx& c, int begin, int end, float inv_t, float 
 struct SelectResult {
     uint32_t key;
     unsigned long long tie_rank;
-    unsigned long long mass;      // of the elements with this key or a larger one (by draw_select only)
-    int token;                    // the element itself, if it is known (by draw_select only), else -1
 };
 
-__device__ SelectResult radix_select(ClusterCtx& c, int begin, int end, float inv_t, float max_scaled, uint32_t floor_key, bool by_count,
+__device__ __noinline__ SelectResult radix_select(ClusterCtx& c, int begin, int end, float inv_t, float max_scaled, uint32_t floor_key, bool by_count,
                                      unsigned long long target) {
-    SampleShared* sh = c.sh;
-    const int copy = (threadIdx.x >> 5) % DRAW_COPIES;
+    SampleShared* sh = draw_shared();
+    const float* vals = c.vals;                    // (not read anew after every store)
+    const int vals_begin = c.vals_begin, copy = (threadIdx.x >> 5) % DRAW_COPIES;
     uint32_t prefix = 0;
     for (int pass = 0; pass < 4; ++pass) {
         const int shift = 24 - 8 * pass;
         __syncthreads();
         for (int i = threadIdx.x; i < DRAW_COPIES * 256; i += DRAW_THREADS) (&sh->whist[0][0])[i] = 0ull;
         __syncthreads();
+#pragma unroll 4
         for (int i = begin + (int)threadIdx.x; i < end; i += DRAW_THREADS) {
-            const float v = c.vals[i - c.vals_begin];
-            const uint32_t key = order_key(v);
+            const float v = vals[i - vals_begin];
+            const uint32_t key = by_count ? order_key(v) : mass_key(v);
             if (key < floor_key) continue;
             if (pass > 0 && (key >> (shift + 8)) != prefix) continue;
             const unsigned long long w = by_count ? 1ull : weight_of(v, inv_t, max_scaled);
@@ -469,10 +516,9 @@ __device__ SelectResult radix_select(ClusterCtx& c, int begin, int end, float in
 #pragma unroll
             for (uint32_t r = 0; r < SAMPLE_MAX_CLUSTER; ++r) sum += v[r];
             sh->tot[threadIdx.x] = sum;
-            sh->tot_ct[threadIdx.x] = 0u;
         }
         ++c.round;
-        pick_bin(sh, sh->tot, sh->tot_ct, false, target);
+        pick_bin(target);
         prefix = (prefix << 8) | (255u - sh->chosen);
         target = sh->carry;
     }
@@ -481,25 +527,80 @@ __device__ SelectResult radix_select(ClusterCtx& c, int begin, int end, float in
     // all elements with this key have the same logit, hence the same weight
     const unsigned long long w = by_count ? 1ull : weight_of(logit_of_key(prefix), inv_t, max_scaled);
     r.tie_rank = w ? target / w : 0ull;
-    r.mass = 0ull;
-    r.token = -1;
     return r;
 }
 
-__device__ unsigned long long kept_mass(ClusterCtx& c, int begin, int end, float inv_t, float max_scaled, uint32_t floor_key) {
+__device__ __noinline__ unsigned long long kept_mass(ClusterCtx& c, int begin, int end, float inv_t, float max_scaled, uint32_t floor_key) {
     unsigned long long local = 0;
+    const float* vals = c.vals;
+    const int vals_begin = c.vals_begin;
+#pragma unroll 4
     for (int i = begin + (int)threadIdx.x; i < end; i += DRAW_THREADS) {
-        const float v = c.vals[i - c.vals_begin];
-        if (order_key(v) >= floor_key) local += weight_of(v, inv_t, max_scaled);
+        const float v = vals[i - vals_begin];
+        if (mass_key(v) >= floor_key) local += weight_of(v, inv_t, max_scaled);
     }
     return cluster_combine(c, local, false);
 }
 
-// The search within the list, by the CTA that holds it: entries in registers, ranges of keys cut into 256 bins until all
-// entries left have one key, then the same over their indices.  Leaves key, tie rank, mass and index in pub[b][0..3].
-__device__ void search_list(ClusterCtx& c, int n, bool by_count, unsigned long long target, unsigned long long before, float inv_t,
-                            float max_scaled, uint32_t b) {
-    SampleShared* sh = c.sh;
+// The bin of a table whose cumulative weight first exceeds `target` (at most the total: beyond it the last element is meant), by
+// threads 0 to 255 of those that call it: the thread whose bin it is gets true.
+__device__ __forceinline__ bool in_bin(const BinTable* t, int i, bool by_count, unsigned long long target, unsigned long long& carry) {
+    const unsigned long long whole = by_count ? (unsigned long long)t->upto_ct[255] : t->upto[255];
+    if (target >= whole) target = whole - 1ull;
+    const unsigned long long upto = by_count ? (unsigned long long)t->upto_ct[i] : t->upto[i], own = by_count ? (unsigned long long)t->ct[i] : t->mass[i];
+    carry = target - (upto - own);
+    return target < upto && target >= upto - own;
+}
+
+// Bins of two targets, by the whole block, in sh->place: bins of the first level, cut finer where that is at hand.
+__device__ __noinline__ void pick_places(bool by_count, unsigned long long target0, unsigned long long target1) {
+    SampleShared* sh = draw_shared();
+    const int i = threadIdx.x & 255, j = threadIdx.x >> 8;
+    const unsigned long long target = j ? target1 : target0;
+    static_assert(DRAW_THREADS == 512, "a half of the block per target");
+    unsigned long long carry;
+    __syncthreads();
+    if (in_bin(&sh->tab, i, by_count, target, carry)) sh->place[j] = BinPlace{sh->tab.upto[i] - sh->tab.mass[i], carry, sh->tab.upto[i], i, -1, sh->tab.ct[i]};
+    __syncthreads();
+    if (!sh->is_fine) return;
+    const int bin = sh->place[j].bin;
+    const unsigned long long before = sh->place[j].before, rest = sh->place[j].carry;
+    int slot = -1;
+#pragma unroll
+    for (int k = 0; k < DRAW_SLOTS; ++k)
+        if (sh->slot_bin[k] == bin) slot = k;
+    __syncthreads();
+    if (slot >= 0) {
+        const BinTable* t = &sh->fine.tab[slot];
+        if (in_bin(t, i, by_count, rest, carry)) sh->place[j] = BinPlace{before + t->upto[i] - t->mass[i], carry, before + t->upto[i], bin, i, t->ct[i]};
+    }
+    __syncthreads();
+}
+
+// The same within 256 bins that this CTA filled in sh->cut: place[0] gets the bin as `sub`, its masses after `before`.
+__device__ __noinline__ void pick_cut(bool by_count, unsigned long long target, unsigned long long before) {
+    SampleShared* sh = draw_shared();
+    auto& cut = sh->fine.cut;
+    __syncthreads();
+    if (threadIdx.x < 256) {
+        sh->cut_tab.mass[threadIdx.x] = (unsigned long long)cut.lo[threadIdx.x] + ((unsigned long long)cut.hi[threadIdx.x] << 20);
+        sh->cut_tab.ct[threadIdx.x] = cut.ct[threadIdx.x];
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) sum_table(offsetof(SampleShared, cut_tab));
+    __syncthreads();
+    unsigned long long carry;
+    const int i = threadIdx.x & 255;
+    if (threadIdx.x < 256 && in_bin(&sh->cut_tab, i, by_count, target, carry))
+        sh->place[0] = BinPlace{before + sh->cut_tab.upto[i] - sh->cut_tab.mass[i], carry, before + sh->cut_tab.upto[i], sh->place[0].bin, i, sh->cut_tab.ct[i]};
+    __syncthreads();
+}
+
+// The search within one bin's entries (sublist) where they are more than DRAW_FEW, by the CTA that holds them: entries in registers, ranges of
+// keys cut into 256 bins until all entries left have one key, then the same over their indices.  The result in the found_ fields.
+__device__ __noinline__ void search_list(int n, bool by_count, unsigned long long target, unsigned long long before, float inv_t,
+                                         float max_scaled) {
+    SampleShared* sh = draw_shared();
     constexpr int PER = DRAW_LIST / DRAW_THREADS;
     unsigned long long e[PER];
     bool in[PER];
@@ -508,7 +609,7 @@ __device__ void search_list(ClusterCtx& c, int n, bool by_count, unsigned long l
     for (int u = 0; u < PER; ++u) {
         const int i = threadIdx.x + u * DRAW_THREADS;
         in[u] = i < n;
-        e[u] = in[u] ? sh->list[i] : 0ull;
+        e[u] = in[u] ? sh->fine.sublist[i] : 0ull;
         if (in[u]) {
             lo = min(lo, (uint32_t)(e[u] >> 32));
             hi = max(hi, (uint32_t)(e[u] >> 32));
@@ -531,154 +632,199 @@ __device__ void search_list(ClusterCtx& c, int n, bool by_count, unsigned long l
         lo = sh->range[0];
         hi = sh->range[1];
     };
-    auto narrow = [&](bool counted, bool by_index) {   // one round: the bin of the target among the entries that are in
-        const uint32_t span = hi - lo;
-        const int width = 32 - __clz(span), s = width > 8 ? width - 8 : 0;
+    block_range();
+    int left = n;
+    bool by_index = false;
+    unsigned long long w = 0ull, tie = 0ull;
+    uint32_t key = 0u;
+#pragma unroll 1
+    while (true) {                                 // ends: every round leaves a range at most 1/128 as wide, or one key, then one index
+        if (lo == hi && by_index) break;
+        if (lo == hi) {
+            key = lo;
+            w = weight_of(logit_of_key(key), inv_t, max_scaled);
+            tie = by_count ? target : (w ? target / w : 0ull);
+            if (tie >= (unsigned long long)left) tie = (unsigned long long)left - 1ull;
+            target = tie;                          // the tie-th smallest index
+            by_index = by_count = true;
+            lo = 0xffffffffu;
+            hi = 0u;
+#pragma unroll
+            for (int u = 0; u < PER; ++u)
+                if (in[u]) {
+                    lo = min(lo, (uint32_t)e[u]);
+                    hi = max(hi, (uint32_t)e[u]);
+                }
+            block_range();
+            continue;
+        }
+        const uint32_t old_hi = hi, old_lo = lo;
+        const int width = 32 - __clz(hi - lo), s = width > 8 ? width - 8 : 0;
+        auto& cut = sh->fine.cut;
         __syncthreads();
-        for (int i = threadIdx.x; i < 256; i += DRAW_THREADS) sh->h.lo[0][i] = sh->h.hi[0][i] = sh->h.ct[0][i] = 0u;
+        if (threadIdx.x < 256) cut.lo[threadIdx.x] = cut.hi[threadIdx.x] = cut.ct[threadIdx.x] = 0u;
         __syncthreads();
+        uint32_t at[PER];
 #pragma unroll
         for (int u = 0; u < PER; ++u) {
+            at[u] = by_index ? ((uint32_t)e[u] - old_lo) >> s : (old_hi - (uint32_t)(e[u] >> 32)) >> s;
             if (!in[u]) continue;
-            const uint32_t x = by_index ? (uint32_t)e[u] : (uint32_t)(e[u] >> 32);
-            const uint32_t at = by_index ? (x - lo) >> s : (hi - x) >> s;
-            if (!by_index) {
-                const unsigned long long w = weight_of(logit_of_key(x), inv_t, max_scaled);
-                const uint32_t low = (uint32_t)w & 0xfffffu, high = (uint32_t)(w >> 20);
-                if (low) atomicAdd(&sh->h.lo[0][at], low);
-                if (high) atomicAdd(&sh->h.hi[0][at], high);
-            }
-            atomicAdd(&sh->h.ct[0][at], 1u);
+            const unsigned long long m = by_index ? 0ull : weight_of(logit_of_key((uint32_t)(e[u] >> 32)), inv_t, max_scaled);
+            atomicAdd(&cut.lo[at[u]], (uint32_t)m & 0xfffffu);
+            atomicAdd(&cut.hi[at[u]], (uint32_t)(m >> 20));
+            atomicAdd(&cut.ct[at[u]], 1u);
         }
-        __syncthreads();
-        if (threadIdx.x < 256) {
-            sh->tot[threadIdx.x] = (unsigned long long)sh->h.lo[0][threadIdx.x] + ((unsigned long long)sh->h.hi[0][threadIdx.x] << 20);
-            sh->tot_ct[threadIdx.x] = sh->h.ct[0][threadIdx.x];
+        pick_cut(by_count, target, before);
+        const uint32_t bin = (uint32_t)sh->place[0].sub;
+        target = sh->place[0].carry;
+        if (!by_index) {
+            before = sh->place[0].before;
+            left = (int)sh->place[0].count;
         }
-        pick_bin(sh, sh->tot, sh->tot_ct, counted, target);
-        const uint32_t bin = sh->chosen;
-        target = sh->carry;
         lo = 0xffffffffu;
-        const uint32_t old_hi = hi, old_lo = by_index ? old_hi - span : 0u;
         hi = 0u;
 #pragma unroll
         for (int u = 0; u < PER; ++u) {
-            if (!in[u]) continue;
-            const uint32_t x = by_index ? (uint32_t)e[u] : (uint32_t)(e[u] >> 32);
-            in[u] = (by_index ? (x - old_lo) >> s : (old_hi - x) >> s) == bin;
+            in[u] = in[u] && at[u] == bin;
             if (in[u]) {
+                const uint32_t x = by_index ? (uint32_t)e[u] : (uint32_t)(e[u] >> 32);
                 lo = min(lo, x);
                 hi = max(hi, x);
             }
         }
         block_range();
-    };
-    block_range();
-    int left = n;
-    while (lo != hi) {                             // ends: every round leaves a range at most 1/128 as wide, or one key
-        narrow(by_count, false);
-        before += sh->before;
-        left = (int)sh->chosen_ct;
-        __syncthreads();
-    }
-    const uint32_t key = lo;
-    const unsigned long long w = weight_of(logit_of_key(key), inv_t, max_scaled);
-    unsigned long long tie = by_count ? target : (w ? target / w : 0ull);
-    if (tie >= (unsigned long long)left) tie = (unsigned long long)left - 1ull;
-    // the tie-th smallest index
-    target = tie;
-    lo = 0xffffffffu;
-    hi = 0u;
-#pragma unroll
-    for (int u = 0; u < PER; ++u)
-        if (in[u]) {
-            lo = min(lo, (uint32_t)e[u]);
-            hi = max(hi, (uint32_t)e[u]);
-        }
-    block_range();
-    while (lo != hi) {
-        narrow(true, true);
-        __syncthreads();
     }
     if (threadIdx.x == 0) {
-        sh->pub[b][0] = key;
-        sh->pub[b][1] = tie;
-        sh->pub[b][2] = before + w * (unsigned long long)left;
-        sh->pub[b][3] = lo;
+        sh->found_key = key;
+        sh->found_tie = (uint32_t)tie;
+        sh->found_mass = before + w * (unsigned long long)left;
+        sh->found_index = lo;
     }
 }
 
-// The element of a plain row (see the top of this part); tot1 and tot1_ct hold the first level's bins.
-__device__ SelectResult draw_select(ClusterCtx& c, int begin, int end, const DrawBins& bins, uint32_t floor_key, bool by_count,
-                                    unsigned long long target) {
-    SampleShared* sh = c.sh;
-    const unsigned long long whole_target = target;
-    pick_bin(sh, sh->tot1, sh->tot1_ct, by_count, target);
-    const int b1 = (int)sh->chosen;
-    int b2 = -1, n = (int)sh->chosen_ct;
-    unsigned long long before = sh->before;
-    target = sh->carry;
-    if (n > DRAW_LIST) {
-        draw_hist(c, begin, end, bins.inv_t, bins.max_scaled, [&](float v) { return bins.first(v) == b1 ? bins.second(v, b1) : -1; });
-        pick_bin(sh, sh->tot, sh->tot_ct, by_count, target);
-        b2 = (int)sh->chosen;
-        n = (int)sh->chosen_ct;
-        before += sh->before;
-        target = sh->carry;
-    }
-    if (n > DRAW_LIST) {                           // (nearly) equal logits
-        SelectResult r = radix_select(c, begin, end, bins.inv_t, bins.max_scaled, floor_key, by_count, whole_target);
-        r.mass = kept_mass(c, begin, end, bins.inv_t, bins.max_scaled, r.key);
-        return r;
-    }
-    // every CTA puts its elements of the bin into the first one's list
-    const uint32_t counter = peer_address(&sh->list_n, 0u), list = peer_address(&sh->list[0], 0u);
-    const int lane = threadIdx.x & 31;
-    for (int i = begin + (int)threadIdx.x; __any_sync(0xffffffffu, i < end); i += 4 * DRAW_THREADS) {
-        float v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int j = i + u * DRAW_THREADS;
-            v[u] = j < end ? c.vals[j - c.vals_begin] : 0.0f;
+__device__ __forceinline__ unsigned long long top_p_need(float P, unsigned long long total) {
+    unsigned long long need = (unsigned long long)ceil((double)P * (double)total);
+    if (need < 1ull) need = 1ull;
+    return need > total ? total : need;
+}
+__device__ __forceinline__ unsigned long long draw_target(float u, unsigned long long total) {
+    const unsigned long long target = (unsigned long long)((double)u * (double)total);
+    return target >= total ? total - 1ull : target;
+}
+
+// Where the row's searches may end, by the whole block, in sh->want.
+__device__ __noinline__ void search_places(int V, int k, float P, float u) {
+    SampleShared* sh = draw_shared();
+    unsigned long long lo = sh->tab.upto[255], hi = lo;            // what top-k keeps, then what top-p keeps: between these
+#pragma unroll 1
+    for (int s = 0; s < 3; ++s) {                                  // top-k, top-p, the draw
+        if (!(s == 0 ? k > 0 && k < V : s == 1 ? P > 0.0f && P < 1.0f : true)) {
+            if (threadIdx.x < 2) sh->want[s][threadIdx.x] = threadIdx.x ? 0.0f : INFINITY;
+            continue;
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int j = i + u * DRAW_THREADS;
-            const bool mine = j < end && bins.first(v[u]) == b1 && (b2 < 0 || bins.second(v[u], b1) == b2);
-            const uint32_t all = __ballot_sync(0xffffffffu, mine);
-            if (!all) continue;
-            uint32_t at = 0u;
-            if (lane == __ffs(all) - 1)
-                asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], %2;\n" : "=r"(at) : "r"(counter), "r"((uint32_t)__popc(all)) : "memory");
-            at = __shfl_sync(0xffffffffu, at, __ffs(all) - 1) + (uint32_t)__popc(all & ((1u << lane) - 1u));
-            if (mine && at < DRAW_LIST) {
-                const unsigned long long entry = ((unsigned long long)order_key(v[u]) << 32) | (uint32_t)j;
-                asm volatile("st.shared::cluster.u64 [%0], %1;\n" ::"r"(list + 8u * at), "l"(entry) : "memory");
-            }
+        unsigned long long t0 = (unsigned long long)(k - 1), t1 = t0;
+        if (s == 1) {
+            lo = top_p_need(P, lo);
+            t0 = lo - 1ull;
+            t1 = top_p_need(P, hi) - 1ull;
+        } else if (s == 2) {
+            t0 = draw_target(u, lo);
+            t1 = draw_target(u, hi);
+        }
+        pick_places(s == 0, t0, t1);
+        if (threadIdx.x < 2) {
+            const int bin = sh->place[threadIdx.x].bin, sub = sh->place[threadIdx.x].sub;
+            sh->want[s][threadIdx.x] = (float)(256 * bin + (threadIdx.x ? (sub < 0 ? 256 : sub + 1) : (sub < 0 ? 0 : sub)));
+        }
+        if (s == 0) {
+            lo = max(sh->place[0].before, 1ull);
+            hi = max(sh->place[0].upto, 1ull);
+        } else if (s == 1) {
+            hi = max(min(hi, sh->place[1].upto), lo);
         }
     }
     __syncthreads();
-    sample_cluster_sync();
-    const uint32_t b = c.round & 1;
-    if (c.rank == 0) {
-        search_list(c, n, by_count, target, before, bins.inv_t, bins.max_scaled, b);
-        if (threadIdx.x == 0) sh->list_n = 0u;
+}
+__device__ __forceinline__ bool wanted(const SampleShared* sh, float from, float upto) {   // does any of the places lie in [from, upto)
+    bool in = false;
+#pragma unroll
+    for (int s = 0; s < 3; ++s) in |= sh->want[s][0] < upto && sh->want[s][1] > from;
+    return in;
+}
+
+// One search within the list, by the whole first CTA; the result in the found_ fields.
+__device__ __noinline__ void search_bins(const DrawBins bins, bool by_count, unsigned long long target) {
+    SampleShared* sh = draw_shared();
+    pick_places(by_count, target, target);
+    const int n = (int)sh->n_list, bin = sh->place[0].bin;
+    if (sh->place[0].sub < 0 && sh->place[0].count > DRAW_FEW) {   // one cut into 256 leaves few
+        auto& cut = sh->fine.cut;
+        const unsigned long long rest = sh->place[0].carry, before = sh->place[0].before;
+        if (threadIdx.x < 256) cut.lo[threadIdx.x] = cut.hi[threadIdx.x] = cut.ct[threadIdx.x] = 0u;
         __syncthreads();
+        for (int i = threadIdx.x; i < n; i += DRAW_THREADS) {
+            const float v = logit_of_key((uint32_t)(sh->list[i] >> 32));
+            const int at = bins.of(v);
+            if (at >> 8 != bin) continue;
+            const unsigned long long w = weight_below(v, bins.inv_t, bins.max_scaled);
+            atomicAdd(&cut.lo[at & 255], (uint32_t)w & 0xfffffu);
+            atomicAdd(&cut.hi[at & 255], (uint32_t)(w >> 20));
+            atomicAdd(&cut.ct[at & 255], 1u);
+        }
+        pick_cut(by_count, rest, before);
     }
-    sample_cluster_sync();
-    SelectResult r;
-    r.key = (uint32_t)ld_peer_u64(&sh->pub[b][0], 0u);
-    r.tie_rank = ld_peer_u64(&sh->pub[b][1], 0u);
-    r.mass = ld_peer_u64(&sh->pub[b][2], 0u);
-    r.token = (int)ld_peer_u64(&sh->pub[b][3], 0u);
-    ++c.round;
-    return r;
+    const int sub = sh->place[0].sub;
+    if (threadIdx.x == 0) sh->few_n = 0u;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += DRAW_THREADS) {
+        const unsigned long long e = sh->list[i];
+        const int at = bins.of(logit_of_key((uint32_t)(e >> 32)));
+        if (at >> 8 == bin && (sub < 0 || (at & 255) == sub)) sh->fine.sublist[atomicAdd(&sh->few_n, 1u)] = e;
+    }
+    __syncthreads();
+    const int m = (int)sh->few_n;
+    if (m > DRAW_FEW) {
+        search_list(m, by_count, sh->place[0].carry, sh->place[0].before, bins.inv_t, bins.max_scaled);
+        __syncthreads();
+        return;
+    }
+    const unsigned long long e = (int)threadIdx.x < m ? sh->fine.sublist[threadIdx.x] : 0ull;
+    const uint32_t key = (uint32_t)(e >> 32), index = (uint32_t)e;
+    const unsigned long long w = weight_below(logit_of_key(key), bins.inv_t, bins.max_scaled);
+    if ((int)threadIdx.x < m) sh->few_w[threadIdx.x] = w;
+    __syncthreads();
+    if ((int)threadIdx.x < m) {
+        unsigned long long above = 0ull;           // mass, or count, of the entries with larger keys
+        unsigned long long above_m = 0ull;
+        uint32_t same = 0u, same_before = 0u;
+#pragma unroll 4
+        for (int i = 0; i < m; ++i) {
+            const unsigned long long o = sh->fine.sublist[i];
+            const uint32_t okey = (uint32_t)(o >> 32);
+            if (okey > key) {
+                above_m += sh->few_w[i];
+                above += by_count ? 1ull : sh->few_w[i];
+            }
+            if (okey == key) {
+                ++same;
+                if ((uint32_t)o < index) ++same_before;
+            }
+        }
+        const unsigned long long one = by_count ? 1ull : w, carry = sh->place[0].carry;
+        if (carry >= above && carry < above + one * same && (carry - above) / one == same_before) {
+            sh->found_key = key;
+            sh->found_index = index;
+            sh->found_tie = same_before;
+            sh->found_mass = sh->place[0].before + above_m + w * same;
+        }
+    }
+    __syncthreads();
 }
 
 // Index of the (rank)-th element, by ascending index, whose key equals `key`; written to out_token by the thread
-// that owns it.  Returns nothing: if no element has the key, rank 0's thread 0 writes `fallback`.
-__device__ void write_nth_with_key(ClusterCtx& c, int begin, int end, uint32_t key, unsigned long long rank, int fallback, int32_t* out_token) {
-    SampleShared* sh = c.sh;
+// that owns it.  False, in every thread of the cluster, if no element has the key.
+__device__ __noinline__ bool write_nth_with_key(ClusterCtx& c, int begin, int end, uint32_t key, unsigned long long rank, int32_t* out_token) {
+    SampleShared* sh = draw_shared();
     const int len = end - begin;
     const int sub = (len + DRAW_THREADS - 1) / DRAW_THREADS;
     const int lo = begin + min(len, (int)threadIdx.x * sub), hi = begin + min(len, ((int)threadIdx.x + 1) * sub);
@@ -707,13 +853,10 @@ __device__ void write_nth_with_key(ClusterCtx& c, int begin, int end, uint32_t k
         total += v[r];
     }
     ++c.round;
-    if (total == 0ull) {
-        if (c.rank == 0 && threadIdx.x == 0) *out_token = fallback;
-        return;
-    }
+    if (total == 0ull) return false;
     if (rank >= total) rank = total - 1ull;
     const unsigned long long here = sh->pub[b][256];
-    if (rank < before || rank >= before + here) return;           // another CTA's slice holds it
+    if (rank < before || rank >= before + here) return true;      // another CTA's slice holds it
     rank -= before;
     if (threadIdx.x == 0) {
         unsigned long long seen = 0ull;
@@ -741,128 +884,369 @@ __device__ void write_nth_with_key(ClusterCtx& c, int begin, int end, uint32_t k
                 ++seen;
             }
     }
+    return true;
 }
 
 __global__ void __launch_bounds__(DRAW_THREADS, 2)
 sample_rows_kernel(const float* __restrict__ logits, int32_t* __restrict__ out, int V,
                    const float* __restrict__ temperature, const int32_t* __restrict__ top_k,
                    const float* __restrict__ top_p, const unsigned long long* __restrict__ seeds,
-                   const unsigned long long* __restrict__ counters, int cache_floats) {
+                   const unsigned long long* __restrict__ counters, int chunk, int vec) {
     extern __shared__ __align__(16) unsigned char sample_smem[];
     ClusterCtx c;
-    c.sh = reinterpret_cast<SampleShared*>(sample_smem);
+    SampleShared* sh = draw_shared();
     c.rank = blockIdx.x;                                           // the cluster spans x
     c.n_ranks = gridDim.x;
     c.round = 0;
-    const int r = blockIdx.y;
+    const int r = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float* row = logits + (size_t)r * V;
     const float T = temperature[r];
     const int k = top_k[r];
     const float P = top_p[r];
-    const int chunk = (V + (int)c.n_ranks - 1) / (int)c.n_ranks;
-    const int begin = min(V, (int)c.rank * chunk), end = min(V, begin + chunk);
-    if (threadIdx.x == 0) c.sh->list_n = 0u;                       // before the first cluster barrier
-
-    // maximum and its lowest index: (order key, ~index) packed so that the larger number is the better pair;
-    // NaN takes no part; a row without any number gives index 0
-    // The slice is read from global memory once, eight loads in flight per thread, and kept in shared memory if it
-    // fits (`cache_floats` > 0): the passes below then read it from there.
-    float* cache = reinterpret_cast<float*>(sample_smem + sizeof(SampleShared));
-    const bool cached = cache_floats >= end - begin;
-    unsigned long long best = 0ull;
+    const int begin = min(V, (int)c.rank * chunk), end = min(V, begin + chunk), len = end - begin;
+    const int quads = (len + 3) / 4;
+    const bool cached = chunk <= DRAW_ROOM;
+    // the q-th four numbers of the slice from memory; what lies beyond its end is -inf
+    auto from_row = [&](int q) {
+        float4 w = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        const float* at = row + begin + 4 * q;
+        if (vec) return 4 * q < len ? __ldg(reinterpret_cast<const float4*>(at)) : w;
+        if (4 * q < len) w.x = __ldg(at);
+        if (4 * q + 1 < len) w.y = __ldg(at + 1);
+        if (4 * q + 2 < len) w.z = __ldg(at + 2);
+        if (4 * q + 3 < len) w.w = __ldg(at + 3);
+        return w;
+    };
+    float4* kept = reinterpret_cast<float4*>(sample_smem + sizeof(SampleShared));
+    c.vals = cached ? reinterpret_cast<const float*>(kept) : row;
+    c.vals_begin = cached ? begin : 0;
+    if (tid == 0) sh->list_n = sh->too_many = 0u;
+    // the maximum; NaN takes no part.  Eight loads of 16 bytes a thread are under way together
+    float top = NAN;
     bool has_nan = false;
-    for (int i = begin + (int)threadIdx.x; i < end; i += 8 * DRAW_THREADS) {
-        float v[8];
+    for (int q0 = tid; q0 < quads; q0 += 8 * DRAW_THREADS) {
+        float4 w[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int j = i + u * DRAW_THREADS;
-            v[u] = j < end ? row[j] : -INFINITY;
-        }
+        for (int j = 0; j < 8; ++j) w[j] = from_row(q0 + j * DRAW_THREADS);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const int j = i + u * DRAW_THREADS;
-            if (j >= end) continue;
-            if (cached) cache[j - begin] = v[u];
-            if (v[u] != v[u]) {
-                has_nan = true;
-                continue;
-            }
-            const unsigned long long packed = ((unsigned long long)order_key(v[u]) << 32) | (uint32_t)(~(uint32_t)j);
-            best = packed > best ? packed : best;
+        for (int j = 0; j < 8; ++j) {
+            const int q = q0 + j * DRAW_THREADS;
+            if (q >= quads) break;
+            if (cached) kept[q] = w[j];
+            top = fmaxf(fmaxf(top, fmaxf(w[j].x, w[j].y)), fmaxf(w[j].z, w[j].w));
+            has_nan |= w[j].x != w[j].x || w[j].y != w[j].y || w[j].z != w[j].z || w[j].w != w[j].w;
         }
     }
-    c.vals = cached ? cache : row;
-    c.vals_begin = cached ? begin : 0;
-    best = cluster_combine(c, best, true);
-    const int best_index = best ? (int)(~(uint32_t)(best & 0xffffffffull)) : 0;
+    for (int i = tid; i < (int)(sizeof(sh->hist) / 16); i += DRAW_THREADS) reinterpret_cast<uint4*>(&sh->hist)[i] = make_uint4(0u, 0u, 0u, 0u);
+    {
+        const uint32_t best = __reduce_max_sync(0xffffffffu, top != top ? 0u : order_key(top));
+        has_nan = __any_sync(0xffffffffu, has_nan);
+        if (lane == 0) sh->warp_part[warp] = ((unsigned long long)best << 1) | (has_nan ? 1ull : 0ull);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const unsigned long long p = lane < DRAW_WARPS ? sh->warp_part[lane] : 0ull;
+        const uint32_t best = __reduce_max_sync(0xffffffffu, (uint32_t)(p >> 1));
+        const bool any = __any_sync(0xffffffffu, (p & 1ull) != 0ull);
+        if (lane == 0) sh->pub[0][256] = ((unsigned long long)best << 1) | (any ? 1ull : 0ull);
+    }
+    sample_cluster_sync();
+    uint32_t best = 0u;
+    bool nan_in_row = false;
+    {
+        unsigned long long p[SAMPLE_MAX_CLUSTER];
+        ld_all_peers_u64(&sh->pub[0][256], c.n_ranks, p);
+#pragma unroll
+        for (uint32_t i = 0; i < SAMPLE_MAX_CLUSTER; ++i) {
+            best = max(best, (uint32_t)(p[i] >> 1));
+            nan_in_row |= (p[i] & 1ull) != 0ull;
+        }
+    }
+    ++c.round;
     // (every path below ends with a cluster barrier: no CTA may exit while a peer still reads its shared memory)
-    if (T <= 0.0f || k == 1 || best == 0ull) {
-        if (c.rank == 0 && threadIdx.x == 0) out[r] = best_index;
+    auto quad = [&](int q) { return cached ? kept[q] : from_row(q); };
+    // the lowest index of the maximum; a row without any number gives index 0
+    auto write_best = [&]() {
+        unsigned long long first = 0ull;
+        const float top_logit = logit_of_key(best);
+        for (int q = tid; q < quads && first == 0ull && best != 0u; q += DRAW_THREADS) {
+            const float4 four = quad(q);
+            const float x[4] = {four.x, four.y, four.z, four.w};
+            if (!(fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3])) >= top_logit)) continue;
+#pragma unroll
+            for (int j = 3; j >= 0; --j)
+                if (__float_as_uint(x[j]) == __float_as_uint(top_logit) && 4 * q + j < len) first = (uint32_t)~(uint32_t)(begin + 4 * q + j);
+        }
+        first = cluster_combine(c, first, true);
+        if (c.rank == 0 && tid == 0) out[r] = first ? (int)~(uint32_t)first : 0;
         sample_cluster_sync();
+    };
+    if (T <= 0.0f || k == 1 || best == 0u) {
+        write_best();
         return;
     }
-    const float max_logit = logit_of_key((uint32_t)(best >> 32));
+    const float max_logit = logit_of_key(best);
     const float inv_t = 1.0f / T;
     const float max_scaled = max_logit * inv_t;
-    // At or beyond 2^16 the rounding of max_scaled lets weights of the largest logits exceed FIXED_ONE by more than the 32-bit sums
-    // of the histograms have room for; NaN and infinities are not below it.
-    const bool plain = cluster_combine(c, has_nan ? 1ull : 0ull, true) == 0ull && fabsf(max_scaled) < 65536.0f && isfinite(inv_t) && inv_t > 0.0f;
-    const DrawBins bins{inv_t, max_scaled};
-
-    // top-k: everything at or above the k-th largest logit stays
-    uint32_t floor_key = 0;
-    unsigned long long total;
+    const uint64_t bits = mix64(seeds[r], counters[r]);
+    const float u = (float)(bits >> 40) * (1.0f / 16777216.0f);  // 24 bits → [0,1)
+    // Below 2^21 max_scaled is off by 1/16 at most, so that no weight exceeds FIXED_ONE e^(1/16) and the sums of the bins have room; NaN and
+    // infinities are not below it.
+    const bool plain = !nan_in_row && fabsf(max_scaled) < 2097152.0f && isfinite(inv_t) && inv_t > 0.0f && chunk <= DRAW_SLICE_MAX;
     if (plain) {
-        draw_hist(c, begin, end, inv_t, max_scaled, [&](float v) { return bins.first(v); });
-        if (threadIdx.x < 256) {
-            c.sh->tot1[threadIdx.x] = c.sh->tot[threadIdx.x];
-            c.sh->tot1_ct[threadIdx.x] = c.sh->tot_ct[threadIdx.x];
+        const DrawBins bins{inv_t, max_scaled};
+        const float inv_t32 = inv_t * 0.03125f, max_scaled32 = max_scaled * 0.03125f;
+        // a bin's word for this lane: 64 bytes a bin, the exponent of first_bits shifted out by the start
+        const uint32_t cell = (uint32_t)__cvta_generic_to_shared(&sh->hist.lo[0][tid % DRAW_LANES]) - (0x4b000000u * 64u);
+        constexpr uint32_t HI = sizeof(sh->hist.lo), CT = 2 * sizeof(sh->hist.lo);
+#pragma unroll 2
+        for (int q = tid; q < quads; q += DRAW_THREADS) {
+            const float4 four = quad(q);
+            const float x[4] = {four.x, four.y, four.z, four.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const Halves w = weight_halves(x[j], inv_t, max_scaled);
+                const uint32_t at = DrawBins::first_bits(x[j], inv_t32, max_scaled32) * 64u + cell;
+                asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(at), "r"(w.low) : "memory");
+                if (w.high) asm volatile("red.shared.add.u32 [%0+%2], %1;" ::"r"(at), "r"(w.high), "n"(HI) : "memory");
+                asm volatile("red.shared.add.u32 [%0+%2], %1;" ::"r"(at), "r"(1u), "n"(CT) : "memory");
+            }
         }
         __syncthreads();
-        if (k > 0 && k < V) {
-            const SelectResult s = draw_select(c, begin, end, bins, 0u, true, (unsigned long long)(k - 1));
-            floor_key = s.key;
-            total = s.mass;
-        } else {
-            total = 0ull;
+        if (tid < 256) {
+            unsigned long long low = 0ull, high = 0ull;
+            uint32_t count = 0u;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) total += c.sh->tot1[(threadIdx.x & 31) + 32 * i];
-            total = warp_sum_u64(total);
+            for (int i = 0; i < DRAW_LANES; ++i) {                 // (from another copy on in every lane: no two in one bank)
+                const int copy_i = (i + tid) % DRAW_LANES;
+                low += sh->hist.lo[tid][copy_i];
+                high += sh->hist.hi[tid][copy_i];
+                count += sh->hist.ct[tid][copy_i];
+                if (tid == 255) {
+                    low += sh->hist.lo[256][copy_i];
+                    high += sh->hist.hi[256][copy_i];
+                    count += sh->hist.ct[256][copy_i];
+                }
+            }
+            sh->pub[1][tid] = low + (high << 20);
+            sh->pub_ct[tid] = tid == 255 ? count - (uint32_t)(4 * quads - len) : count;
         }
-    } else {
-        if (k > 0 && k < V) floor_key = radix_select(c, begin, end, inv_t, max_scaled, 0u, true, (unsigned long long)(k - 1)).key;
-        total = kept_mass(c, begin, end, inv_t, max_scaled, floor_key);
-    }
-    if (total == 0ull) {  // numerical underflow: the reference falls back to the best candidate
-        if (c.rank == 0 && threadIdx.x == 0) out[r] = best_index;
         sample_cluster_sync();
+        if (tid < 256) {
+            unsigned long long p[SAMPLE_MAX_CLUSTER], mass = 0ull;
+            ld_all_peers_u64(&sh->pub[1][tid], c.n_ranks, p);
+#pragma unroll
+            for (uint32_t i = 0; i < SAMPLE_MAX_CLUSTER; ++i) mass += p[i];
+            sh->tab.mass[tid] = mass;
+        } else {
+            sh->tab.ct[tid - 256] = sum_all_peers_u32(&sh->pub_ct[tid - 256], c.n_ranks);
+        }
+        if (tid < DRAW_SLOTS) sh->slot_bin[tid] = -1;
+        if (tid == 0) sh->is_fine = 0u;
+        __syncthreads();
+        if (warp == 0) sum_table(offsetof(SampleShared, tab));
+        __syncthreads();
+        bool fits = false, listed = false;
+        int slots = 0;
+        uint32_t n_near = 0u;
+        // every number of the bins that hold places, as of the first round: from the warp's list, or from the slice if that has overflowed
+        auto each_near = [&](auto use) {
+            if (listed) {
+                for (uint32_t i = lane; i < n_near; i += 32) {
+                    const int at = sh->near[warp][i];
+                    use(c.vals[at + begin - c.vals_begin], at);
+                }
+            } else {
+                for (int i = tid; i < len; i += DRAW_THREADS) {
+                    const float y = c.vals[i + begin - c.vals_begin];
+                    if (sh->marked[min(bins.of(y) >> 8, 255)]) use(y, i);
+                }
+            }
+        };
+        auto& f = sh->fine;
+        for (int round = 0;; ++round) {
+            if (tid == 0) sh->n_list = 0u;
+            search_places(V, k, P, u);
+            // how many numbers lie in these places; which bins they are
+            if (warp < 8) {
+                const bool in = wanted(sh, 256.0f * (float)tid, 256.0f * (float)(tid + 1));
+                bool cut = false;
+#pragma unroll
+                for (int i = 0; i < DRAW_SLOTS; ++i) cut |= sh->slot_bin[i] == tid;
+                const uint32_t all = __ballot_sync(0xffffffffu, in), n = __reduce_add_sync(0xffffffffu, in && !cut ? sh->tab.ct[tid] : 0u);
+                const uint32_t open = __ballot_sync(0xffffffffu, in && !cut);
+                if (lane == 0) {
+                    sh->mask[warp] = all;
+                    if (n) atomicAdd(&sh->n_list, n);
+                    sh->warp_part[warp] = open;
+                }
+            }
+            for (int i = tid; i < 256 * slots; i += DRAW_THREADS) {
+                const float at = (float)(256 * sh->slot_bin[i >> 8] + (i & 255));
+                const uint32_t n = f.tab[i >> 8].ct[i & 255];
+                if (n && wanted(sh, at, at + 1.0f)) atomicAdd(&sh->n_list, n);
+            }
+            __syncthreads();
+            if (round == 0) {
+                // the numbers of these bins, from the slice; a quarter of a warp's words has none nearer than the last of the bins
+                if (tid < 256) sh->marked[tid] = (unsigned char)((sh->mask[warp] >> lane) & 1u);
+                if (tid == 256) sh->marked[256] = (unsigned char)(sh->mask[7] >> 31);
+                int last = 0;
+#pragma unroll
+                for (int w = 0; w < 8; ++w)
+                    if (sh->mask[w]) last = 32 * w + 31 - __clz(sh->mask[w]);
+                const float nearer = last == 255 ? INFINITY : (float)(last + 1) / 256.0f;
+                const uint32_t mark = (uint32_t)__cvta_generic_to_shared(&sh->marked[0]) - 0x4b000000u;
+                __syncthreads();
+#pragma unroll 1
+                for (int q0 = warp * 32; q0 < quads; q0 += DRAW_THREADS) {
+                    const int q = q0 + lane;
+                    const float4 four = q < quads ? quad(q) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+                    const float x[4] = {four.x, four.y, four.z, four.w};
+                    if (!__any_sync(0xffffffffu, __saturatef(__fmaf_rn(-fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3])), inv_t32, max_scaled32)) < nearer)) continue;
+                    uint32_t m[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        asm volatile("ld.shared.u8 %0, [%1];" : "=r"(m[j]) : "r"(DrawBins::first_bits(x[j], inv_t32, max_scaled32) + mark) : "memory");
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const bool in = m[j] != 0u && 4 * q + j < len;
+                        const uint32_t all = __ballot_sync(0xffffffffu, in);
+                        const uint32_t at = n_near + (uint32_t)__popc(all & ((1u << lane) - 1u));
+                        if (in && at < DRAW_NEAR) sh->near[warp][at] = (unsigned short)(4 * q + j);
+                        n_near += (uint32_t)__popc(all);
+                    }
+                }
+                listed = !__syncthreads_or(n_near > DRAW_NEAR);
+            }
+            fits = sh->n_list <= DRAW_LIST;
+            if (fits || round == 2) break;
+            int n_bins = 0, before = 0;
+            bool open = false;
+            const int only = k > 0 && k < V ? (int)sh->want[0][0] >> 8 : -1;   // of too many bins, top-k's own: the others are fewer once its place is known
+#pragma unroll
+            for (int w = 0; w < 8; ++w) {
+                const uint32_t m = sh->mask[w];
+                if (w < warp) before += __popc(m);
+                if (w == warp) before += __popc(m & ((1u << lane) - 1u));
+                n_bins += __popc(m);
+                open |= sh->warp_part[w] != 0ull;
+            }
+            if (!open || (n_bins > DRAW_SLOTS && (only < 0 || round > 0))) break;     // (nearly) equal logits, or masses of many bins in doubt
+            const bool all_bins = n_bins <= DRAW_SLOTS;
+            slots = all_bins ? n_bins : 1;
+            __syncthreads();
+            if (tid < DRAW_SLOTS) sh->slot_bin[tid] = -1;
+            if (tid < 256) sh->slot_of[tid] = 0;
+            __syncthreads();
+            if (warp < 8 && (all_bins ? ((sh->mask[warp] >> lane) & 1u) != 0u : tid == only)) {
+                const int slot = all_bins ? before : 0;
+                sh->slot_bin[slot] = tid;
+                sh->slot_of[tid] = (unsigned char)(slot + 1);
+            }
+            for (int i = tid; i < 256 * slots; i += DRAW_THREADS) f.lo[i] = f.hi[i] = f.ct[i] = 0u;
+            __syncthreads();
+            each_near([&](float y, int) {
+                const int at = bins.of(y), slot = (int)sh->slot_of[at >> 8] - 1, i = 256 * slot + (at & 255);
+                if (slot < 0) return;
+                const Halves w = weight_halves(y, inv_t, max_scaled);
+                atomicAdd(&f.lo[i], w.low);
+                if (w.high) atomicAdd(&f.hi[i], w.high);
+                atomicAdd(&f.ct[i], 1u);
+            });
+            __syncthreads();
+            for (int i = tid; i < 256 * slots; i += DRAW_THREADS) f.pub[i] = (unsigned long long)f.lo[i] + ((unsigned long long)f.hi[i] << 20);
+            sample_cluster_sync();
+            for (int i = tid; i < 256 * slots; i += DRAW_THREADS) {
+                unsigned long long p[SAMPLE_MAX_CLUSTER], mass = 0ull;
+                ld_all_peers_u64(&f.pub[i], c.n_ranks, p);
+#pragma unroll
+                for (uint32_t j = 0; j < SAMPLE_MAX_CLUSTER; ++j) mass += p[j];
+                const uint32_t count = sum_all_peers_u32(&f.ct[i], c.n_ranks);
+                f.tab[i >> 8].mass[i & 255] = mass;
+                f.tab[i >> 8].ct[i & 255] = count;
+                if (count > DRAW_LO_MAX) sh->too_many = 1u;        // (nearly) equal logits: 32 bits may not have held the low halves
+            }
+            if (tid == 0) sh->is_fine = 1u;
+            __syncthreads();
+            if (warp < slots) sum_table((uint32_t)(offsetof(SampleShared, fine.tab) + warp * sizeof(BinTable)));
+            __syncthreads();
+            if (sh->too_many != 0u) break;
+            sample_cluster_sync();                                 // the peers have read this CTA's sums
+        }
+        if (fits) {
+            const float a0 = sh->want[0][0], a1 = sh->want[0][1], b0 = sh->want[1][0], b1 = sh->want[1][1], c0 = sh->want[2][0], c1 = sh->want[2][1];
+            unsigned long long* own = f.own;                       // (beside the warps' lists, which take the place of the cluster's)
+            each_near([&](float y, int i) {
+                const float place = bins.place(y);
+                if (!((place >= a0 && place < a1) || (place >= b0 && place < b1) || (place >= c0 && place < c1))) return;
+                const uint32_t at = atomicAdd(&sh->list_n, 1u);
+                if (at < DRAW_LIST) own[at] = ((unsigned long long)order_key(y) << 32) | (uint32_t)(begin + i);
+            });
+            sample_cluster_sync();
+            if (c.rank != 0) {
+                sample_cluster_sync();                             // until the first CTA has the lists
+                return;
+            }
+            uint32_t held[SAMPLE_MAX_CLUSTER];
+#pragma unroll
+            for (uint32_t i = 0; i < SAMPLE_MAX_CLUSTER; ++i) {
+                held[i] = 0u;
+                if (i < c.n_ranks) asm volatile("ld.shared::cluster.u32 %0, [%1];\n" : "=r"(held[i]) : "r"(peer_address(&sh->list_n, i)) : "memory");
+            }
+            unsigned long long e[SAMPLE_MAX_CLUSTER];
+#pragma unroll
+            for (uint32_t i = 0; i < SAMPLE_MAX_CLUSTER; ++i)
+                if (tid < (int)held[i]) e[i] = ld_peer_u64(&f.own[tid], i);
+            uint32_t at = 0u;
+#pragma unroll
+            for (uint32_t i = 0; i < SAMPLE_MAX_CLUSTER; ++i) {    // (n_list of them in all, at most DRAW_LIST)
+                if (tid < (int)held[i]) sh->list[at + tid] = e[i];
+                for (uint32_t j = tid + DRAW_THREADS; j < held[i]; j += DRAW_THREADS) sh->list[at + j] = ld_peer_u64(&f.own[j], i);
+                at += held[i];
+            }
+            asm volatile("barrier.cluster.arrive.release;\n" ::: "memory");
+            // the three searches, one after the other
+            uint32_t floor_key = 0u;
+            unsigned long long total = sh->tab.upto[255];
+            if (k > 0 && k < V) {
+                search_bins(bins, true, (unsigned long long)(k - 1));
+                floor_key = sh->found_key;
+                total = sh->found_mass;
+            }
+            if (P > 0.0f && P < 1.0f) {                            // the smallest prefix whose cumulative share reaches P
+                search_bins(bins, false, top_p_need(P, total) - 1ull);
+                if (sh->found_key > floor_key) {
+                    floor_key = sh->found_key;
+                    total = sh->found_mass;
+                }
+            }
+            search_bins(bins, false, draw_target(u, total));
+            if (tid == 0) out[r] = (int)sh->found_index;
+            asm volatile("barrier.cluster.wait.acquire;\n" ::: "memory");
+            return;
+        }
+        sample_cluster_sync();                                     // the radix select's sums take the place of what peers may be reading
+    }
+    // every other row: radix selects over the slice
+    // top-k: everything at or above the k-th largest logit stays
+    uint32_t floor_key = 0;
+    if (k > 0 && k < V) floor_key = radix_select(c, begin, end, inv_t, max_scaled, 0u, true, (unsigned long long)(k - 1)).key;
+    unsigned long long total = kept_mass(c, begin, end, inv_t, max_scaled, floor_key);
+    if (total == 0ull) {  // numerical underflow: the reference falls back to the best candidate
+        write_best();
         return;
     }
     // top-p: the smallest prefix whose cumulative share reaches P
     if (P > 0.0f && P < 1.0f) {
-        unsigned long long need = (unsigned long long)ceil((double)P * (double)total);
-        if (need < 1ull) need = 1ull;
-        if (need > total) need = total;
-        const SelectResult s = plain ? draw_select(c, begin, end, bins, floor_key, false, need - 1ull)
-                                     : radix_select(c, begin, end, inv_t, max_scaled, floor_key, false, need - 1ull);
-        if (s.key > floor_key) {
-            floor_key = s.key;
-            total = plain ? s.mass : kept_mass(c, begin, end, inv_t, max_scaled, floor_key);
-        } else if (!plain) {
-            total = kept_mass(c, begin, end, inv_t, max_scaled, floor_key);
-        }
+        const SelectResult s = radix_select(c, begin, end, inv_t, max_scaled, floor_key, false, top_p_need(P, total) - 1ull);
+        if (s.key > floor_key) floor_key = s.key;
+        total = kept_mass(c, begin, end, inv_t, max_scaled, floor_key);
     }
-    // the draw
-    const uint64_t bits = mix64(seeds[r], counters[r]);
-    const float u = (float)(bits >> 40) * (1.0f / 16777216.0f);  // 24 bits → [0,1)
-    unsigned long long target = (unsigned long long)((double)u * (double)total);
-    if (target >= total) target = total - 1ull;
-    const SelectResult s = plain ? draw_select(c, begin, end, bins, floor_key, false, target)
-                                 : radix_select(c, begin, end, inv_t, max_scaled, floor_key, false, target);
-    if (s.token >= 0) {
-        if (c.rank == 0 && threadIdx.x == 0) out[r] = s.token;
-    } else {
-        write_nth_with_key(c, begin, end, s.key, s.tie_rank, best_index, &out[r]);
+    const SelectResult s = radix_select(c, begin, end, inv_t, max_scaled, floor_key, false, draw_target(u, total));
+    if (!write_nth_with_key(c, begin, end, s.key, s.tie_rank, &out[r])) {
+        write_best();
+        return;
     }
     sample_cluster_sync();
 }
@@ -871,18 +1255,17 @@ MM_EXPORT int mm_sample_rows(const void* logits, void* out, int R, int V, const 
                              const void* top_p, const void* seeds, const void* counters, void* stream) {
     MM_REQUIRE(R >= 0 && R <= 65535 && V > 0, "sample: bad sizes");
     if (R == 0) return MM_OK;
-    // a wide row is shared by a cluster of CTAs (a power of two: other sizes place badly); a narrow one is one CTA's
+    // A row is shared by a cluster of CTAs (a power of two: other sizes place badly): enough that their shared memory holds a copy of it, more
+    // while the launch leaves SMs idle and a slice keeps 4096 numbers.
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     int ranks = 1;
-    while (ranks < SAMPLE_MAX_CLUSTER && V / (ranks * 2) >= 4096 && (ranks == 1 || R * ranks * 2 <= 2 * sms)) ranks *= 2;   // one wave of two CTAs per SM
-    // a copy of the CTA's slice in shared memory if it fits: beside another CTA's, or with an SM to itself while every CTA of the launch has one
-    const int chunk = (V + ranks - 1) / ranks;
-    const size_t room = (R * ranks <= sms ? 200 * 1024 : 112 * 1024) - sizeof(SampleShared);
-    const int cache_floats = (size_t)chunk * sizeof(float) <= room ? chunk : 0;
-    const size_t smem = sizeof(SampleShared) + (size_t)cache_floats * sizeof(float);
-    if (!mm_allow_smem<sample_rows_kernel>(200 * 1024)) {
+    while (ranks < SAMPLE_MAX_CLUSTER && ((V + ranks - 1) / ranks > DRAW_ROOM || (V / (ranks * 2) >= 4096 && (long long)R * ranks * 2 <= sms))) ranks *= 2;
+    const int vec = V % 4 == 0 && reinterpret_cast<uintptr_t>(logits) % 16 == 0;
+    const int chunk = ((V + ranks - 1) / ranks + 3) / 4 * 4;
+    const size_t smem = sizeof(SampleShared) + (chunk <= DRAW_ROOM ? (size_t)chunk * sizeof(float) : 0);
+    if (!mm_allow_smem<sample_rows_kernel>(sizeof(SampleShared) + DRAW_ROOM * sizeof(float))) {
         mm_set_last_error("sample: cannot reserve shared memory");
         return MM_ERR_LAUNCH;
     }
@@ -900,7 +1283,7 @@ MM_EXPORT int mm_sample_rows(const void* logits, void* out, int R, int V, const 
     cfg.numAttrs = ranks > 1 ? 1 : 0;
     cudaLaunchKernelEx(&cfg, sample_rows_kernel, (const float*)logits, (int32_t*)out, V, (const float*)temperature,
                        (const int32_t*)top_k, (const float*)top_p, (const unsigned long long*)seeds,
-                       (const unsigned long long*)counters, cache_floats);
+                       (const unsigned long long*)counters, chunk, vec);
     MM_CHECK_LAUNCH();
     return MM_OK;
 }

@@ -96,3 +96,30 @@ def test_equal_logits_at_a_very_low_temperature(R, V, T):
     for r in range(R):          # equal weights: the share of token i is [i, i+1) / V; u has 24 or more bits, the product rounds once
         u = plain.uniform_from(int(seeds[r]), int(counters[r]))
         assert abs(got[r] - u * V) <= 1.0 + 1e-6 * V, (r, T, got[r], u * V)
+
+
+@pytest.mark.parametrize("R,V,scale,T,k,p,shift", [
+    (6, 152064, 2.0, 0.8, 0, 0.95, 0),       # the bins of the cut and the draw hold less than a list, or a little more
+    (4, 152064, 2.0, 1.5, 0, 0.9, 0),        # ... several lists: the bins are cut finer
+    (3, 152064, 2.0, 8.0, 0, 0.9, 0),        # ... and more of them than a warp keeps
+    (4, 152064, 2.0, 1.5, 5000, 0.95, 0),    # top-k's own bin leaves the others' places in doubt
+    (40, 152061, 2.0, 1.0, 0, 0.95, 0),      # rows that start off 16 bytes
+    (40, 65536, 2.0, 1.0, 300, 0.99, 1),     # ... and a first row that does
+    (5, 8 * 38016, 2.0, 0.7, 0, 0.9, 0),     # the widest row whose slices are kept in shared memory
+    (3, 8 * 38016 + 4, 2.0, 0.7, 0, 0.9, 0),
+    (2, 8 * 65024 + 4, 2.0, 0.7, 0, 0.9, 0),   # beyond what the sums of the bins hold
+])
+def test_draws_where_the_search_changes_its_way(R, V, scale, T, k, p, shift):
+    from mimirmind_b200.kernels import ops
+    rng = np.random.RandomState(V % 991 + k)
+    logits = (scale * rng.randn(R, V)).astype(np.float32)
+    for r in range(R):
+        logits[r, rng.choice(V, 24, replace=False)] += 10 * rng.rand(24).astype(np.float32)
+    full = lambda v, dt: torch.full((R,), v, dtype=dt, device=DEV)           # noqa: E731
+    seeds = rng.randint(1, 2 ** 31, size=R)
+    buf = torch.empty(R * V + shift, device=DEV)
+    x = buf[shift:].view(R, V)
+    x.copy_(torch.tensor(logits))
+    got = ops.sample_rows(x, full(T, torch.float32), full(k, torch.int32), full(p, torch.float32), torch.tensor(seeds, device=DEV), full(3, torch.int64)).cpu().tolist()
+    for r in list(range(R))[:6]:
+        check(logits[r], T, k, p, plain.uniform_from(int(seeds[r]), 3), got[r])
