@@ -17,8 +17,7 @@
 // larger of the nine partial products, added up in 32 bits (Henry, Tang and Heinecke 2019).  Error against 64 bits, of outputs and states over 300 to 4,096 tokens: where many tokens
 // add up (decays near 1) 0.7e-7 to 1.4e-7, half of the 32-bit walk's; where a state forgets half of itself per token, so that the
 // walk has little left to round, 0.6e-7 to 1.2e-7 (the walk: 0.4e-7 to 0.9e-7).  With two tf32 numbers (22 bits) and three products it was
-// 1.0e-7 to 2.4e-7 in both, for kernels 5 to 8 % shorter (4,096 tokens with the delta rule: chain 219 us, now 238, preparation 82 and 87, outputs 99 and
-// 108).  The FMA units, whose tiles are held up by shared-memory reads, take twice as long.
+// 1.0e-7 to 2.4e-7 in both, for kernels 5 to 8 % shorter.  The FMA units, whose tiles are held up by shared-memory reads, take twice as long.
 // Ratios of decays are exponentials of differences of the logarithms' sums, which are kept in 64 bits: quotients of products of
 // the decays themselves would underflow within a chunk (0.2 a token), differences of 32-bit sums lose what lies close together.
 #include "common.cuh"
@@ -230,6 +229,102 @@ __device__ __forceinline__ LcB lc_b_cols(const float* p, int ld) {
     return LcB{{lc_split(q[0], q[4 * ld]), lc_split(q[8 * ld], q[12 * ld])}};
 }
 
+// ---- operands split once, by the block: three planes of bf16 in shared memory --------------------------------------------------
+// A tile [rows][COLS] as its parts h, m and l, each [rows][COLS + 8] in bf16: rows 16 bytes off a multiple of 128, so that ldmatrix, which
+// reads eight rows' 16 bytes, meets every bank once.  Split while it is brought in, an operand costs its eleven instructions per two
+// numbers once and not in every warp that multiplies with it.
+template <int COLS>
+__host__ __device__ constexpr int lc_plane(int rows) { return rows * (COLS + 8) * 2; }        // bytes of one of the three
+__device__ __forceinline__ void lc_sts64(uint32_t to, uint32_t x, uint32_t y) { asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(to), "r"(x), "r"(y) : "memory"); }
+__device__ __forceinline__ void lc_sts32(uint32_t to, uint32_t x) { asm volatile("st.shared.b32 [%0], %1;" ::"r"(to), "r"(x) : "memory"); }
+__device__ __forceinline__ void lc_put4(uint32_t to, int plane, const LcSplit& x, const LcSplit& y) {
+    lc_sts64(to, x.h, y.h);
+    lc_sts64(to + plane, x.m, y.m);
+    lc_sts64(to + 2 * plane, x.l, y.l);
+}
+__device__ __forceinline__ uint32_t lc_top(const float4& v) {             // (see lc_not_finite)
+    const uint32_t a = __float_as_uint(v.x) & 0x7fffffffu, b = __float_as_uint(v.y) & 0x7fffffffu, c = __float_as_uint(v.z) & 0x7fffffffu,
+                   d = __float_as_uint(v.w) & 0x7fffffffu;
+    return max(max(a, b), max(c, d));
+}
+// A thread's 16-byte pieces of rows [0, 64) x columns [0, COLS) of a matrix of `rows` x `cols` numbers, zeros beyond; and these as planes.
+template <int COLS>
+struct LcTile {
+    static constexpr int Q = COLS / 4, N = 64 * Q / 256;
+    float4 v[N];
+    __device__ __forceinline__ void load(const float* __restrict__ p, size_t ld, int rows, int cols) {
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+            const int idx = threadIdx.x + e * 256, r = idx / Q, c = (idx % Q) * 4;
+            v[e] = r < rows && c < cols ? __ldg(reinterpret_cast<const float4*>(p + (size_t)r * ld + c)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    }
+    __device__ __forceinline__ void to_planes(uint32_t planes) const {
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+            const int idx = threadIdx.x + e * 256, r = idx / Q, c = (idx % Q) * 4;
+            lc_put4(planes + (r * (COLS + 8) + c) * 2, lc_plane<COLS>(64), lc_split(v[e].x, v[e].y), lc_split(v[e].z, v[e].w));
+        }
+    }
+    __device__ __forceinline__ void to_floats(float* s) const {            // [64][LC_LD]
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+            const int idx = threadIdx.x + e * 256;
+            *reinterpret_cast<float4*>(s + (idx / Q) * LC_LD + (idx % Q) * 4) = v[e];
+        }
+    }
+    __device__ __forceinline__ bool not_finite() const {
+        uint32_t top = 0u;
+#pragma unroll
+        for (int e = 0; e < N; ++e) top = max(top, lc_top(v[e]));
+        return top >= 0x7f7f8000u;
+    }
+};
+__device__ __forceinline__ void lc_ldsm(uint32_t at, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(at) : "memory");
+}
+__device__ __forceinline__ void lc_ldsm_t(uint32_t at, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(at) : "memory");
+}
+// Fragments of sixteen k from planes with rows of LD numbers; `at` is the address of the sub-tile's first number in plane h.
+// a_mk: the operand stands as [m][k]; a_km: as [k][m]; b2_nk and b2_kn: two tiles of eight columns, [n][k] and [k][n].
+template <int LD>
+__device__ __forceinline__ LcA lc_a_mk(uint32_t at, int plane) {
+    const int lane = threadIdx.x & 31;
+    at += (((lane & 7) + (lane & 8)) * LD + (lane & 16) / 2) * 2;
+    LcA r;
+    lc_ldsm(at, r.x[0].h, r.x[1].h, r.x[2].h, r.x[3].h);
+    lc_ldsm(at + plane, r.x[0].m, r.x[1].m, r.x[2].m, r.x[3].m);
+    lc_ldsm(at + 2 * plane, r.x[0].l, r.x[1].l, r.x[2].l, r.x[3].l);
+    return r;
+}
+template <int LD>
+__device__ __forceinline__ LcA lc_a_km(uint32_t at, int plane) {
+    const int lane = threadIdx.x & 31;
+    at += (((lane & 7) + (lane & 16) / 2) * LD + (lane & 8)) * 2;
+    LcA r;
+    lc_ldsm_t(at, r.x[0].h, r.x[1].h, r.x[2].h, r.x[3].h);
+    lc_ldsm_t(at + plane, r.x[0].m, r.x[1].m, r.x[2].m, r.x[3].m);
+    lc_ldsm_t(at + 2 * plane, r.x[0].l, r.x[1].l, r.x[2].l, r.x[3].l);
+    return r;
+}
+template <int LD>
+__device__ __forceinline__ void lc_b2_nk(uint32_t at, int plane, LcB* b) {
+    const int lane = threadIdx.x & 31;
+    at += (((lane & 7) + (lane & 16) / 2) * LD + (lane & 8)) * 2;
+    lc_ldsm(at, b[0].x[0].h, b[0].x[1].h, b[1].x[0].h, b[1].x[1].h);
+    lc_ldsm(at + plane, b[0].x[0].m, b[0].x[1].m, b[1].x[0].m, b[1].x[1].m);
+    lc_ldsm(at + 2 * plane, b[0].x[0].l, b[0].x[1].l, b[1].x[0].l, b[1].x[1].l);
+}
+template <int LD>
+__device__ __forceinline__ void lc_b2_kn(uint32_t at, int plane, LcB* b) {
+    const int lane = threadIdx.x & 31;
+    at += (((lane & 7) + (lane & 8)) * LD + (lane & 16) / 2) * 2;
+    lc_ldsm_t(at, b[0].x[0].h, b[0].x[1].h, b[1].x[0].h, b[1].x[1].h);
+    lc_ldsm_t(at + plane, b[0].x[0].m, b[0].x[1].m, b[1].x[0].m, b[1].x[1].m);
+    lc_ldsm_t(at + 2 * plane, b[0].x[0].l, b[0].x[1].l, b[1].x[0].l, b[1].x[1].l);
+}
+
 // The sums of the decays' logarithms over the chunk's tokens, sb[t] = log gamma_t, by the first two warps; tokens beyond the
 // chunk add nothing.  A decay of 0 counts as exp(-200), which no 32-bit number can tell from it; one that is no number (or negative) is
 // NaN here, and so is all that comes after it.
@@ -263,20 +358,27 @@ __device__ __noinline__ float lc_causal_sum(float sum, const float* scores, cons
     for (int s = 0; s <= m; ++s) sum = fmaf(scores[s], values[s * LC_LD], sum);
     return sum;
 }
-template <int HALVES>
-__device__ __forceinline__ void lc_causal(float (*acc)[2][2][4], const float* scores, const float* values, int m0, int wn) {
+// acc [16 rows][8 columns] of a warp's 32 rows and sixteen columns
+__device__ __forceinline__ void lc_causal(float (*acc)[2][4], const float* scores, const float* values, int m0, int wn) {
     const int t = threadIdx.x & 3, g = (threadIdx.x & 31) >> 2;
 #pragma unroll
-    for (int b = 0; b < HALVES; ++b)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
+        for (int j = 0; j < 2; ++j)
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
+            for (int x = 0; x < 4; ++x) {
+                const int m = m0 + 16 * i + g + 8 * (x >> 1), n = wn * 16 + 8 * j + 2 * t + (x & 1);
+                acc[i][j][x] = lc_causal_sum(acc[i][j][x], scores + m * LC_LP, values + n, m);
+            }
+}
+
+__device__ __forceinline__ void lc_causal_cols(float (*acc)[2][4], const float* scores, const float* values, int m0, int wn) {     // acc [8 columns][16 rows]
+    float r[2][2][4];
 #pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                    const int m = m0 + 16 * i + g + 8 * (x >> 1), n = 64 * b + wn * 16 + 8 * j + 2 * t + (x & 1);
-                    acc[b][j][i][x] = lc_causal_sum(acc[b][j][i][x], scores + m * LC_LP, values + n, m);
-                }
+    for (int x = 0; x < 16; ++x) r[(x >> 2) & 1][x >> 3][x & 3] = acc[x >> 3][(x >> 2) & 1][x & 3];
+    lc_causal(r, scores, values, m0, wn);
+#pragma unroll
+    for (int x = 0; x < 16; ++x) acc[x >> 3][(x >> 2) & 1][x & 3] = r[(x >> 2) & 1][x >> 3][x & 3];
 }
 
 struct LcArgs {
@@ -398,62 +500,54 @@ __global__ void __launch_bounds__(256) lc_carry_kernel(LcArgs a) {
 }
 
 // ---- the outputs of a chunk: diag(gamma) Q S + (Q K^T, decayed and masked) U --------------------------------------------------
-// Two blocks per SM (104 KB each): q, and two buffers, first for the halves of S, then for k (later the decayed scores) and u.  Bound by the
-// tensor cores and by issuing what splits their operands.
+// Two blocks per SM (104 KB each): the planes of q (then of the scores) and of one other operand: S's first 64 rows (of dv), its others, k, u.
+// A warp has 32 tokens and sixteen columns of each half of dv.  Bound by the tensor cores (mma.sync: 8.2 cycles for 16 x 8 x 16 per
+// quarter of an SM, 59 us of 153 for 3,000 tokens, 32 heads of 128 x 128); with fragments split by every warp that needs them 164 us.
 template <int DK, int DV>
 __global__ void __launch_bounds__(256, 2) lc_output_kernel(LcArgs a, const float* __restrict__ values, size_t ldu) {
     extern __shared__ __align__(16) float lc_smem[];
-    float* sq = lc_smem;                         // [64][LC_LD]
-    float* sa = sq + LC_C * LC_LD;               // S's first 64 rows (of dv), then k, then the scores [64][LC_LP]
-    float* su = sa + LC_C * LC_LD;               // S's other rows, then u
+    constexpr int WIDE = DK > DV ? DK : DV, PK = lc_plane<DK>(64), PV = lc_plane<DV>(64), PS = lc_plane<64>(64), HALVES = DV / 64;
+    const uint32_t pq = (uint32_t)__cvta_generic_to_shared(lc_smem), px = pq + 3 * PK;
+    float* fx = lc_smem + LC_C * LC_LP;          // (a chunk that holds a NaN or an infinity: the scores and u as they are)
+    static_assert(3 * PK + 3 * lc_plane<WIDE>(64) >= (LC_C * LC_LP + LC_C * LC_LD) * 4, "they fit");
     __shared__ double sb[LC_C];
     const int h = blockIdx.x, c = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = a.chunk_meta[4 * c], cnt = a.chunk_meta[4 * c + 1];
     const int kh = h / (a.H / a.G);
     const float* S = a.states + ((size_t)c * a.H + h) * a.dv * a.dk;
-    const float* up = values + (size_t)t0 * ldu + (size_t)h * a.dv;
-    lc_load<DK, LC_LD>(sq, a.q + (size_t)t0 * a.ldq + (size_t)kh * a.dk, a.ldq, cnt, a.dk);
-    lc_load<DK, LC_LD>(sa, S, a.dk, min(64, a.dv), a.dk);
-    lc_commit();
-    if (DV > 64) lc_load<DK, LC_LD>(su, a.dv > 64 ? S + (size_t)64 * a.dk : S, a.dk, a.dv - 64, a.dk);
-    else lc_load<DV, LC_LD>(su, up, ldu, cnt, a.dv);
-    lc_commit();
-    lc_decays(a.gate, a.head_decay, t0, cnt, a.H, h, sb);
+    {
+        LcTile<DK> tq, ts;
+        tq.load(a.q + (size_t)t0 * a.ldq + (size_t)kh * a.dk, a.ldq, cnt, a.dk);
+        ts.load(S, a.dk, min(64, a.dv), a.dk);
+        lc_decays(a.gate, a.head_decay, t0, cnt, a.H, h, sb);
+        tq.to_planes(pq);
+        ts.to_planes(px);
+    }
     const int m0 = (warp & 1) * 32, wn = warp >> 1, t = lane & 3, g = lane >> 2;
-    constexpr int HALVES = DV / 64;
-    float acc[HALVES][2][2][4], low[HALVES][2][2][4];      // [half of dv][8 columns][16 rows]
+    float acc[HALVES][2][2][4];                  // [half of dv][16 rows][8 columns]
     lc_zero<HALVES * 16>(&acc[0][0][0][0]);
-    lc_zero<HALVES * 16>(&low[0][0][0][0]);
-    if (DV > 64) lc_wait<0>();
-    else lc_wait<1>();
     __syncthreads();
-#pragma unroll 1
-    for (int k0 = 0; k0 < DK; k0 += 16) {         // (both halves of S with one reading of q)
-        LcA fa[2];
 #pragma unroll
-        for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows(sq + (m0 + 16 * i) * LC_LD + k0, LC_LD);
+    for (int b = 0; b < HALVES; ++b) {
+        float low[2][2][4];
+        lc_zero<16>(&low[0][0][0]);
+#pragma unroll 2
+        for (int k0 = 0; k0 < DK; k0 += 16) {
+            LcA fa[2];
+            LcB fb[2];
 #pragma unroll
-        for (int b = 0; b < HALVES; ++b) {
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const LcB fb = lc_b_rows((b == 0 ? sa : su) + (wn * 16 + 8 * j) * LC_LD + k0, LC_LD);
-                lc_one(acc[b][j], low[b][j], fa, fb);
-            }
+            for (int i = 0; i < 2; ++i) fa[i] = lc_a_mk<DK + 8>(pq + ((m0 + 16 * i) * (DK + 8) + k0) * 2, PK);
+            lc_b2_nk<DK + 8>(px + (wn * 16 * (DK + 8) + k0) * 2, PK, fb);
+            lc_products<2, 2>(acc[b], low, fa, fb);
         }
+        lc_add<16>(&acc[b][0][0][0], &low[0][0][0]);
+        __syncthreads();
+        LcTile<DK> next;
+        if (b + 1 < HALVES) next.load(a.dv > 64 ? S + (size_t)64 * a.dk : S, a.dk, a.dv - 64, a.dk);
+        else next.load(a.k + (size_t)t0 * a.ldk + (size_t)kh * a.dk, a.ldk, cnt, a.dk);
+        next.to_planes(px);
+        __syncthreads();
     }
-    lc_add<HALVES * 16>(&acc[0][0][0][0], &low[0][0][0][0]);
-    lc_zero<HALVES * 16>(&low[0][0][0][0]);
-    __syncthreads();
-    lc_load<DK, LC_LD>(sa, a.k + (size_t)t0 * a.ldk + (size_t)kh * a.dk, a.ldk, cnt, a.dk);
-    lc_commit();
-    if (DV > 64) {
-        lc_load<DV, LC_LD>(su, up, ldu, cnt, a.dv);
-        lc_commit();
-        lc_wait<1>();
-    } else {
-        lc_wait<0>();
-    }
-    __syncthreads();
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const float g0 = lc_exp(sb[m0 + 16 * i + g]), g1 = lc_exp(sb[m0 + 16 * i + g + 8]);
@@ -461,59 +555,81 @@ __global__ void __launch_bounds__(256, 2) lc_output_kernel(LcArgs a, const float
         for (int b = 0; b < HALVES; ++b)
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                acc[b][j][i][0] *= g0;
-                acc[b][j][i][1] *= g0;
-                acc[b][j][i][2] *= g1;
-                acc[b][j][i][3] *= g1;
+                acc[b][i][j][0] *= g0;
+                acc[b][i][j][1] *= g0;
+                acc[b][i][j][2] *= g1;
+                acc[b][i][j][3] *= g1;
             }
     }
-    {   // scores of the rows m0.. and keys 16 wn..: nothing to do above the diagonal
-        float s[2][2][4], s_low[2][2][4];        // [8 columns][16 rows]
-        lc_zero<16>(&s[0][0][0]);
-        lc_zero<16>(&s_low[0][0][0]);
+    // scores of the rows m0.. and keys 16 wn..: nothing to do above the diagonal
+    float sc[2][2][4];                           // [16 rows][8 columns]
+    {
+        float low[2][2][4];
+        lc_zero<16>(&sc[0][0][0]);
+        lc_zero<16>(&low[0][0][0]);
         if (wn * 16 <= m0 + 31) {
-#pragma unroll 1
+#pragma unroll 2
             for (int k0 = 0; k0 < DK; k0 += 16) {
                 LcA fa[2];
+                LcB fb[2];
 #pragma unroll
-                for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows(sq + (m0 + 16 * i) * LC_LD + k0, LC_LD);
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const LcB fb = lc_b_rows(sa + (wn * 16 + 8 * j) * LC_LD + k0, LC_LD);
-                    lc_one(s[j], s_low[j], fa, fb);
-                }
+                for (int i = 0; i < 2; ++i) fa[i] = lc_a_mk<DK + 8>(pq + ((m0 + 16 * i) * (DK + 8) + k0) * 2, PK);
+                lc_b2_nk<DK + 8>(px + (wn * 16 * (DK + 8) + k0) * 2, PK, fb);
+                lc_products<2, 2>(sc, low, fa, fb);
             }
-            lc_add<16>(&s[0][0][0], &s_low[0][0][0]);
-        }
-        __syncthreads();                         // every warp is through with k
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-#pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                    const int m = m0 + 16 * i + g + 8 * (x >> 1), n = wn * 16 + 8 * j + 2 * t + (x & 1);
-                    sa[m * LC_LP + n] = n <= m ? s[j][i][x] * lc_exp(sb[m] - sb[n]) : 0.0f;
-                }
-    }
-    lc_wait<0>();
-    const bool plain = !__syncthreads_or(lc_not_finite<DV, LC_LD>(su));
-    if (!plain) lc_causal<HALVES>(acc, sa, su, m0, wn);
-    else for (int k0 = 0; k0 < m0 + 32; k0 += 16) {
-        LcA fa[2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) fa[i] = lc_a_rows4(sa + (m0 + 16 * i) * LC_LP + k0, LC_LP);
-#pragma unroll
-        for (int b = 0; b < HALVES; ++b) {
-            const float* p = su + k0 * LC_LD + 64 * b + wn * 16;
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const LcB fb = lc_b_cols(p + 8 * j, LC_LD);
-                lc_one(acc[b][j], low[b][j], fa, fb);
-            }
+            lc_add<16>(&sc[0][0][0], &low[0][0][0]);
         }
     }
-    lc_add<HALVES * 16>(&acc[0][0][0][0], &low[0][0][0][0]);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const int m = m0 + 16 * i + g + 8 * (x >> 1), n = wn * 16 + 8 * j + 2 * t + (x & 1);
+                sc[i][j][x] = n <= m ? sc[i][j][x] * lc_exp(sb[m] - sb[n]) : 0.0f;
+            }
+    LcTile<DV> tu;
+    tu.load(values + (size_t)t0 * ldu + (size_t)h * a.dv, ldu, cnt, a.dv);
+    const bool plain = !__syncthreads_or(tu.not_finite());      // ... and every warp is through with q and k
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int m = m0 + 16 * i + g + 8 * half, n = wn * 16 + 8 * j + 2 * t;
+                if (plain) {
+                    const LcSplit p = lc_split(sc[i][j][2 * half], sc[i][j][2 * half + 1]);
+                    const uint32_t to = pq + (m * 72 + n) * 2;
+                    lc_sts32(to, p.h);
+                    lc_sts32(to + PS, p.m);
+                    lc_sts32(to + 2 * PS, p.l);
+                } else {
+                    *reinterpret_cast<float2*>(lc_smem + m * LC_LP + n) = make_float2(sc[i][j][2 * half], sc[i][j][2 * half + 1]);
+                }
+            }
+    if (plain) tu.to_planes(px);
+    else tu.to_floats(fx);
+    __syncthreads();
+#pragma unroll
+    for (int b = 0; b < HALVES; ++b) {
+        if (!plain) {
+            lc_causal(acc[b], lc_smem, fx + 64 * b, m0, wn);
+            continue;
+        }
+        float low[2][2][4];
+        lc_zero<16>(&low[0][0][0]);
+        for (int k0 = 0; k0 < m0 + 32; k0 += 16) {
+            LcA fa[2];
+            LcB fb[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) fa[i] = lc_a_mk<72>(pq + ((m0 + 16 * i) * 72 + k0) * 2, PS);
+            lc_b2_kn<DV + 8>(px + (k0 * (DV + 8) + 64 * b + wn * 16) * 2, PV, fb);
+            lc_products<2, 2>(acc[b], low, fa, fb);
+        }
+        lc_add<16>(&acc[b][0][0][0], &low[0][0][0]);
+    }
 #pragma unroll
     for (int b = 0; b < HALVES; ++b)
 #pragma unroll
@@ -527,7 +643,7 @@ __global__ void __launch_bounds__(256, 2) lc_output_kernel(LcArgs a, const float
                     const int m = m0 + 16 * i + g + 8 * half;
                     if (m < cnt)
                         *reinterpret_cast<float2*>(a.out + ((size_t)(t0 + m) * a.H + h) * a.dv + n) =
-                            make_float2(acc[b][j][i][2 * half], acc[b][j][i][2 * half + 1]);
+                            make_float2(acc[b][i][j][2 * half], acc[b][i][j][2 * half + 1]);
                 }
             }
 }
@@ -1076,7 +1192,10 @@ __global__ void __launch_bounds__(256, 2) lc_forget_output_kernel(LcArgs a) {
     }
     lc_wait<0>();
     const bool plain = !__syncthreads_or(lc_not_finite<DV, LC_LD>(sx));
-    if (!plain) lc_causal<HALVES>(acc, sq, sx, m0, wn);
+    if (!plain) {
+#pragma unroll
+        for (int b = 0; b < HALVES; ++b) lc_causal_cols(acc[b], sq, sx + 64 * b, m0, wn);
+    }
     else for (int k0 = 0; k0 < m0 + 32; k0 += 16) {
         LcA fa[2];
 #pragma unroll
@@ -1126,11 +1245,12 @@ template <int DK, int DV>
 static int lc_run(const LcArgs& a, int n_requests, cudaStream_t s) {
     const dim3 chunks(a.H, a.n_chunks);
     const size_t tile = LC_C * LC_LD * sizeof(float), square = LC_C * LC_LP * sizeof(float);
+    const size_t planes = 3 * lc_plane<DK>(64) + 3 * lc_plane<(DK > DV ? DK : DV)>(64);
     if (a.beta == nullptr) {
         if (const int rc = lc_launch<lc_state_kernel<DK, DV>>(chunks, 256, 2 * tile, s, a)) return rc;
         const long long size = (long long)a.H * a.dv * a.dk;
         if (const int rc = lc_launch<lc_carry_kernel<false>>(dim3(ceil_div(size / 4, 256), n_requests), 256, 0, s, a)) return rc;
-        return lc_launch<lc_output_kernel<DK, DV>>(chunks, 256, 3 * tile, s, a, a.v, (size_t)a.ldv);
+        return lc_launch<lc_output_kernel<DK, DV>>(chunks, 256, planes, s, a, a.v, (size_t)a.ldv);
     }
     if (const int rc = lc_launch<lc_delta_prepare_kernel<DK, DV>>(chunks, 256, 2 * tile + 2 * square, s, a)) return rc;
     // columns of S per block: 16 while the blocks then fit the SMs (one each: 186 KB), else 32, whose chain is a little longer
@@ -1140,7 +1260,7 @@ static int lc_run(const LcArgs& a, int n_requests, cudaStream_t s) {
               (size_t)(2 * (2 * LC_C * LC_LD + LC_C * (NS + 8) + LC_C + 4) + 2 * NS * LC_LD + 4 * LC_C * (NS + 4)) * sizeof(float), s, a)
     if (const int rc = wide ? LC_CARRY(32) : LC_CARRY(16)) return rc;
 #undef LC_CARRY
-    return lc_launch<lc_output_kernel<DK, DV>>(chunks, 256, 3 * tile, s, a, (const float*)a.u, (size_t)a.H * a.dv);
+    return lc_launch<lc_output_kernel<DK, DV>>(chunks, 256, planes, s, a, (const float*)a.u, (size_t)a.H * a.dv);
 }
 
 // 1 if the products take these sizes and pointers: heads of up to 128 numbers that are multiples of 4, rows and heads on 16-byte boundaries
