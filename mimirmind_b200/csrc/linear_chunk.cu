@@ -390,8 +390,8 @@ struct LcArgs {
     int n_chunks, H, G, dk, dv;
     float *states;       // [chunks, H, dv, dk]: what a chunk adds, then what it starts from
     float *gain;         // [chunks, H]: gamma_C
-    float *ratio;        // [chunks, H, 64]: gamma_C / gamma_t (delta rule)
-    float *w, *u;        // [tokens, H dk], [tokens, H dv] (delta rule)
+    uint4* frag;         // fragments of W and of K' per chunk and head (delta rule, see lc_delta_prepare_kernel)
+    float* u;            // [tokens, H dv] (delta rule)
 };
 
 // V^T diag(sr) K of a chunk, [dv, dk], to its place in `states`; k and v stand in shared memory.
@@ -725,7 +725,20 @@ __device__ __forceinline__ void lc_invert(const float* __restrict__ L, float* __
     __syncthreads();
 }
 
-// W = T diag(beta gamma) K, U0 = T diag(beta) V of a chunk, and the decays that the carry needs.  Bound by the tensor cores.
+// W = T diag(beta gamma) K, U0 = T diag(beta) V of a chunk, and what else the chain needs: its gain, and W and K' = diag(gamma_C / gamma) K as the
+// fragments that the chain's warps multiply, split and in the order of their lanes: a 16-byte word per lane and part, for W by rows of
+// 16 tokens and steps of sixteen channels, for K' by eight channels and 32 tokens.  (A product's result has the places of the next one's
+// first operand, so W goes out as it comes.)  Bound by the tensor cores.
+template <int DK>
+struct LcFrag {
+    static constexpr int W = 4 * (DK / 16) * 3 * 32, K = (DK / 8) * 2 * 3 * 32, SIZE = W + K;      // words
+};
+__device__ __forceinline__ void lc_put_frag(uint4* to, const LcSplit& x, const LcSplit& y, const LcSplit& z, const LcSplit& w) {
+    const int lane = threadIdx.x & 31;
+    to[lane] = make_uint4(x.h, y.h, z.h, w.h);
+    to[32 + lane] = make_uint4(x.m, y.m, z.m, w.m);
+    to[64 + lane] = make_uint4(x.l, y.l, z.l, w.l);
+}
 template <int DK, int DV>
 __global__ void __launch_bounds__(256, 2) lc_delta_prepare_kernel(LcArgs a) {
     extern __shared__ __align__(16) float lc_smem[];
@@ -734,7 +747,7 @@ __global__ void __launch_bounds__(256, 2) lc_delta_prepare_kernel(LcArgs a) {
     float* sL = sv + LC_C * LC_LD;               // [64][LC_LP]
     float* sT = sL + LC_C * LC_LP;               // [64][LC_LP]
     __shared__ double sb[LC_C];
-    __shared__ float sbeta[LC_C], sbg[LC_C];
+    __shared__ float sbeta[LC_C], sbg[LC_C], sr[LC_C];
     const int h = blockIdx.x, c = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = a.chunk_meta[4 * c], cnt = a.chunk_meta[4 * c + 1];
     const int kh = h / (a.H / a.G);
@@ -750,12 +763,24 @@ __global__ void __launch_bounds__(256, 2) lc_delta_prepare_kernel(LcArgs a) {
         odd = !(fabsf(b) < INFINITY && fabs(sb[t]) < INFINITY);
         sbeta[t] = b;
         sbg[t] = b * lc_exp(sb[t]);
-        a.ratio[((size_t)c * a.H + h) * LC_C + t] = lc_exp(sb[LC_C - 1] - sb[t]);
+        sr[t] = lc_exp(sb[LC_C - 1] - sb[t]);
         if (t == 0) a.gain[(size_t)c * a.H + h] = lc_exp(sb[LC_C - 1]);
     }
     const int m0 = (warp & 1) * 32, wn = warp >> 1, t = lane & 3, g = lane >> 2;
+    uint4* fw = a.frag + ((size_t)c * a.H + h) * LcFrag<DK>::SIZE;
+    uint4* fk = fw + LcFrag<DK>::W;
     lc_wait<1>();
     __syncthreads();
+    for (int item = warp; item < DK / 8 * 2; item += 8) {       // K': eight channels and 32 tokens
+        LcSplit x[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int row = (item & 1) * 32 + 8 * e + 2 * t;
+            const float* p = sk + row * LC_LD + (item >> 1) * 8 + g;
+            x[e] = lc_split(p[0], sr[row], p[LC_LD], sr[row + 1]);
+        }
+        lc_put_frag(fk + item * 96, x[0], x[1], x[2], x[3]);
+    }
     {
         float s[2][2][4], s_low[2][2][4];        // [8 columns][16 rows]
         lc_zero<16>(&s[0][0][0]);
@@ -797,13 +822,17 @@ __global__ void __launch_bounds__(256, 2) lc_delta_prepare_kernel(LcArgs a) {
             }
         }
         __syncthreads();
-        for (int idx = threadIdx.x; idx < cnt * a.dk; idx += 256) a.w[((size_t)(t0 + idx / a.dk) * a.H + h) * a.dk + idx % a.dk] = sk[idx / a.dk * LC_LD + idx % a.dk];
+        for (int item = warp; item < 4 * (DK / 16); item += 8) {
+            const float* p = sk + (item / (DK / 16) * 16 + g) * LC_LD + item % (DK / 16) * 16 + 2 * t;
+            lc_put_frag(fw + item * 96, lc_split(p[0], p[1]), lc_split(p[8 * LC_LD], p[8 * LC_LD + 1]), lc_split(p[8], p[9]),
+                        lc_split(p[8 * LC_LD + 8], p[8 * LC_LD + 9]));
+        }
         for (int idx = threadIdx.x; idx < cnt * a.dv; idx += 256) a.u[((size_t)(t0 + idx / a.dv) * a.H + h) * a.dv + idx % a.dv] = sv[idx / a.dv * LC_LD + idx % a.dv];
         return;
     }
     lc_invert(sL, sT);
     // both products: rows m0 + 16 i (32 per warp pair), columns wn * (COLS / 4)..; T has nothing to the right of its diagonal blocks
-    auto product = [&](const float* s, const float* scale, int cols, int width, float* o, size_t ld, auto tiles) {
+    auto product = [&](const float* s, const float* scale, int cols, int width, float* o, size_t ld, auto tiles, auto as_fragments) {
         constexpr int NT = decltype(tiles)::value;
         float acc[NT][2][4], low[NT][2][4];      // [8 columns][16 rows]
         lc_zero<NT * 8>(&acc[0][0][0]);
@@ -823,6 +852,15 @@ __global__ void __launch_bounds__(256, 2) lc_delta_prepare_kernel(LcArgs a) {
             }
         }
         lc_add<NT * 8>(&acc[0][0][0], &low[0][0][0]);
+        if constexpr (decltype(as_fragments)::value) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < NT; j += 2)
+                    lc_put_frag(fw + ((m0 / 16 + i) * (DK / 16) + (wn * width + 8 * j) / 16) * 96, lc_split(acc[j][i][0], acc[j][i][1]), lc_split(acc[j][i][2], acc[j][i][3]),
+                                lc_split(acc[j + 1][i][0], acc[j + 1][i][1]), lc_split(acc[j + 1][i][2], acc[j + 1][i][3]));
+            return;
+        }
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
@@ -836,176 +874,165 @@ __global__ void __launch_bounds__(256, 2) lc_delta_prepare_kernel(LcArgs a) {
                 }
             }
     };
-    product(sk, sbg, a.dk, DK / 4, a.w + ((size_t)t0 * a.H + h) * a.dk, (size_t)a.H * a.dk, std::integral_constant<int, DK / 32>{});
-    product(sv, sbeta, a.dv, DV / 4, a.u + ((size_t)t0 * a.H + h) * a.dv, (size_t)a.H * a.dv, std::integral_constant<int, DV / 32>{});
+    product(sk, sbg, a.dk, DK / 4, nullptr, 0, std::integral_constant<int, DK / 32>{}, std::true_type{});
+    product(sv, sbeta, a.dv, DV / 4, a.u + ((size_t)t0 * a.H + h) * a.dv, (size_t)a.H * a.dv, std::integral_constant<int, DV / 32>{}, std::false_type{});
 }
 
-// U = U0 - W S and S' = gamma_C S + K^T diag(gamma_C / gamma) U, chunk after chunk, for NS columns of one head's S per block.
-// Bound by the chain of the two products and its barriers, and within it by issuing instructions (splitting the operands is most of
-// them), so 16 warps share the k of each product and a warp makes as many tiles as use its fragments: in the first, warp w has rows
-// 16 (w % 4) of U and a quarter of the key channels, in the second rows 16 (w % 8) of dk and half of the tokens; both have all
-// NS columns.  The quarters meet in a pass over U, the halves in the next chunk: S is read as the sum of the first half's numbers, which are
-// carried, and of what the second half has just added (two sums that were carried side by side would grow apart and cancel).
-// The next chunk's W, k and U0 arrive under the current one's products.  64 chunks: 229 us (254 with a tile and half of the k per warp).
+// U = U0 - W S and S' = gamma_C S + K'^T U, chunk after chunk, for sixteen columns of one head's S per block: a chain of two products per chunk.
+// W and K' come as fragments straight into the registers of the warps that multiply them, the next chunk's while the current one is worked on;
+// S and U are split by the threads that make them and pass through shared memory as planes.  In the first product warp w has rows 16 (w % 4)
+// of U and a quarter of the key channels; the quarters meet in a pass over U.  In the second warp w has eight key channels of
+// S^T = U^T K' and all sixteen columns: S stays in its registers.
+// Bound by the tensor cores (24 products of 16 x 8 x 16 per warp and half of a chunk), what they read from shared memory, three barriers, and
+// the fragments' way from L2 (96 KB per block and chunk): 64 chunks take 179 us.  Warps that split all that they multiply took 238; with W
+// and K' split by eight more warps into planes in shared memory 206, bound by the reads and writes there.
 #define LC_CARRY_THREADS 512
-template <int DK, int NS>
-__global__ void __launch_bounds__(LC_CARRY_THREADS) lc_delta_carry_kernel(LcArgs a) {
-    constexpr int LU = NS + 8, LQ = NS + 4, TILE = 2 * LC_C * LC_LD + LC_C * LU + LC_C + 4, NT = NS / 8;
+template <int DK>
+struct LcCarryShared {
+    static constexpr int PS = lc_plane<DK>(16), PU = lc_plane<16>(64), LQ = 20;
+    // bytes: the planes of S^T [16][dk] and U [64][16], the quarters of W S
+    static constexpr int S = 0, U = S + 3 * PS, SUM = U + 3 * PU, SIZE = SUM + 4 * LC_C * LQ * 4;
+};
+template <int DK>
+__global__ void __launch_bounds__(LC_CARRY_THREADS, 1) lc_delta_carry_kernel(LcArgs a) {
+    using M = LcCarryShared<DK>;
     extern __shared__ __align__(16) float lc_smem[];
-    float* sS = lc_smem + 2 * TILE;              // [2][NS][LC_LD]: the two parts of S
-    float* sp = sS + 2 * NS * LC_LD;             // [4][64][LQ]: the quarters of W S
-    const int h = blockIdx.y, r = blockIdx.z, n_base = blockIdx.x * NS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t = lane & 3, g = lane >> 2, kh = h / (a.H / a.G), side = warp >> 3;
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(lc_smem);
+    const int h = blockIdx.y, r = blockIdx.z, n_base = blockIdx.x * 16, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int first = a.req_chunks[2 * r], count = a.req_chunks[2 * r + 1];
     if (count <= 0) return;
-    const int cols = min(NS, a.dv - n_base);
-    auto fill = [&](int i, int t0, int cnt) {
-        float* sw = lc_smem + (i & 1) * TILE;
-        float* sk = sw + LC_C * LC_LD;
-        float* su = sk + LC_C * LC_LD;
-        float* sr = su + LC_C * LU;
-        lc_load<DK, LC_LD, LC_CARRY_THREADS>(sw, a.w + ((size_t)t0 * a.H + h) * a.dk, (size_t)a.H * a.dk, cnt, a.dk);
-        lc_load<DK, LC_LD, LC_CARRY_THREADS>(sk, a.k + (size_t)t0 * a.ldk + (size_t)kh * a.dk, a.ldk, cnt, a.dk);
-        if (threadIdx.x < LC_C * (NS / 4)) {     // (NS <= 32)
-            const int row = threadIdx.x / (NS / 4), col = (threadIdx.x % (NS / 4)) * 4;
-            const bool in = row < cnt && col < cols;
-            lc_cp16(su + row * LU + col, a.u + (in ? ((size_t)(t0 + row) * a.H + h) * a.dv + n_base + col : 0), in);
-        }
-        if (threadIdx.x < LC_C / 4) lc_cp16(sr + 4 * threadIdx.x, a.ratio + ((size_t)(first + i) * a.H + h) * LC_C + 4 * threadIdx.x, true);
-        lc_commit();
+    const int t = lane & 3, g = lane >> 2;
+    // fragments: the warp's steps of W, its channels of K'
+    constexpr int STEPS = DK / 64;
+    const bool has = warp * 8 < DK;
+    uint4 fw[STEPS][3], fk[2][3];
+    auto load_w = [&](int c) {
+        const uint4* p = a.frag + ((size_t)c * a.H + h) * LcFrag<DK>::SIZE + ((warp & 3) * (DK / 16) + (warp >> 2) * STEPS) * 96 + lane;
+#pragma unroll
+        for (int e = 0; e < STEPS; ++e)
+#pragma unroll
+            for (int part = 0; part < 3; ++part) fw[e][part] = __ldg(p + (e * 3 + part) * 32);
     };
-    // rows 16 (warp % 8).. of dk (if there are so many), all columns: in the first half's warps S, in the second's what they add per chunk
-    const int s_row = (warp & 7) * 16;
-    const bool has_rows = s_row < DK;
-    float S[NT][4];
+    auto load_k = [&](int c) {
+        const uint4* p = a.frag + ((size_t)c * a.H + h) * LcFrag<DK>::SIZE + LcFrag<DK>::W + warp * 192 + lane;
+        if (has)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+                for (int part = 0; part < 3; ++part) fk[e][part] = __ldg(p + (e * 3 + part) * 32);
+    };
+    // S^T of key channels 8 warp.. (if there are so many): rows g and g + 8 of the sixteen columns, channels 2t and 2t + 1
+    const int m = warp * 8 + 2 * t;
+    float S[4];
+    float* st = a.state + (size_t)a.slots[r] * a.state_stride + (size_t)h * a.dv * a.dk;
     {
         const bool fresh = a.positions[a.chunk_meta[4 * first]] == 0;
-        const float* st = a.state + (size_t)a.slots[r] * a.state_stride + (size_t)h * a.dv * a.dk;
 #pragma unroll
-        for (int j = 0; j < NT; ++j)
-#pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                const int m = s_row + g + 8 * (x >> 1), n = n_base + 8 * j + 2 * t + (x & 1);
-                S[j][x] = (side == 0 && !fresh && has_rows && m < a.dk && n < a.dv) ? st[(size_t)n * a.dk + m] : 0.0f;
-            }
+        for (int x = 0; x < 4; ++x) {
+            const int n = n_base + g + 8 * (x >> 1);
+            S[x] = (!fresh && has && m + (x & 1) < a.dk && n < a.dv) ? st[(size_t)n * a.dk + m + (x & 1)] : 0.0f;
+        }
     }
-    auto to_shared = [&]() {
-        if (!has_rows) return;
+    auto to_planes = [&]() {
+        if (!has) return;
 #pragma unroll
-        for (int j = 0; j < NT; ++j)
-#pragma unroll
-            for (int x = 0; x < 4; ++x) sS[(side * NS + 8 * j + 2 * t + (x & 1)) * LC_LD + s_row + g + 8 * (x >> 1)] = S[j][x];
-    };
-    auto to_global = [&](float* __restrict__ to, bool vec) {     // the sum of the two parts, as [dv, dk]
-        for (int idx = threadIdx.x; idx < NS * (DK / 4); idx += LC_CARRY_THREADS) {
-            const int n = idx / (DK / 4), m = (idx % (DK / 4)) * 4;
-            if (n >= cols || m >= a.dk) continue;
-            const float4 x = *reinterpret_cast<const float4*>(sS + n * LC_LD + m), y = *reinterpret_cast<const float4*>(sS + (NS + n) * LC_LD + m);
-            float* p = to + (size_t)(n_base + n) * a.dk + m;
-            if (vec) {
-                *reinterpret_cast<float4*>(p) = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
-            } else {
-                p[0] = x.x + y.x;
-                p[1] = x.y + y.y;
-                p[2] = x.z + y.z;
-                p[3] = x.w + y.w;
-            }
+        for (int half = 0; half < 2; ++half) {
+            const LcSplit x = lc_split(S[2 * half], S[2 * half + 1]);
+            const uint32_t to = base + M::S + ((g + 8 * half) * (DK + 8) + m) * 2;
+            lc_sts32(to, x.h);
+            lc_sts32(to + M::PS, x.m);
+            lc_sts32(to + 2 * M::PS, x.l);
         }
     };
+    // the pass over U: a thread's row and two columns
+    const int row = threadIdx.x >> 3, col = (threadIdx.x & 7) * 2;
+    float* sum = lc_smem + M::SUM / 4;
+    auto u_place = [&](int t0) { return a.u + ((size_t)(t0 + row) * a.H + h) * a.dv + n_base + col; };
+    load_w(first);
+    load_k(first);
+    to_planes();
     int t0 = a.chunk_meta[4 * first], cnt = a.chunk_meta[4 * first + 1];
-    float gain = a.gain[(size_t)first * a.H + h];
-    fill(0, t0, cnt);
-    to_shared();
     for (int i = 0; i < count; ++i) {
         const int c = first + i;
+        const bool mine = row < cnt && n_base + col < a.dv;
+        const float gain = __ldg(a.gain + (size_t)c * a.H + h);
+        float2 u = mine ? *reinterpret_cast<const float2*>(u_place(t0)) : make_float2(0.0f, 0.0f);
         int next_t0 = 0, next_cnt = 0;
-        float next_gain = 0.0f;
         if (i + 1 < count) {
             next_t0 = a.chunk_meta[4 * (c + 1)];
             next_cnt = a.chunk_meta[4 * (c + 1) + 1];
-            next_gain = a.gain[(size_t)(c + 1) * a.H + h];
         }
-        lc_wait<0>();                            // the chunk's tiles, on their way since the chunk before
-        __syncthreads();                         // ... and S; nobody still reads the other tiles
-        if (i + 1 < count) fill(i + 1, next_t0, next_cnt);
-        const float* sw = lc_smem + (i & 1) * TILE;
-        const float* sk = sw + LC_C * LC_LD;
-        float* su = const_cast<float*>(sk) + LC_C * LC_LD;
-        const float* sr = su + LC_C * LU;
+        __syncthreads();                         // S's planes
         {
             const int m0 = (warp & 3) * 16, part = warp >> 2;
-            float p[1][NT][4], low[1][NT][4];
-            lc_zero<NT * 4>(&p[0][0][0]);
-            lc_zero<NT * 4>(&low[0][0][0]);
+            float p[1][2][4], low[1][2][4];
+            lc_zero<8>(&p[0][0][0]);
+            lc_zero<8>(&low[0][0][0]);
 #pragma unroll
-            for (int k = 0; k < DK / 4; k += 16) {
-                const int k0 = part * (DK / 4) + k;
-                const LcA fa = lc_a_rows(sw + m0 * LC_LD + k0, LC_LD);
-                LcB fb[NT];
-#pragma unroll
-                for (int j = 0; j < NT; ++j) {
-                    const float* one = sS + (8 * j + g) * LC_LD + k0 + 2 * t;
-                    const float2 x0 = lc_pair(one), y0 = lc_pair(one + NS * LC_LD), x1 = lc_pair(one + 8), y1 = lc_pair(one + NS * LC_LD + 8);
-                    fb[j] = LcB{{lc_split(x0.x + y0.x, x0.y + y0.y), lc_split(x1.x + y1.x, x1.y + y1.y)}};
-                }
-                lc_products<1, NT>(p, low, &fa, fb);
+            for (int e = 0; e < STEPS; ++e) {
+                const int k0 = (part * STEPS + e) * 16;
+                const LcA fa = {{{fw[e][0].x, fw[e][1].x, fw[e][2].x}, {fw[e][0].y, fw[e][1].y, fw[e][2].y}, {fw[e][0].z, fw[e][1].z, fw[e][2].z},
+                                 {fw[e][0].w, fw[e][1].w, fw[e][2].w}}};
+                LcB fb[2];
+                lc_b2_nk<DK + 8>(base + M::S + k0 * 2, M::PS, fb);
+                lc_products<1, 2>(p, low, &fa, fb);
             }
-            lc_add<NT * 4>(&p[0][0][0], &low[0][0][0]);
+            if (i + 1 < count) load_w(c + 1);
+            lc_add<8>(&p[0][0][0], &low[0][0][0]);
 #pragma unroll
-            for (int j = 0; j < NT; ++j)
+            for (int j = 0; j < 2; ++j)
 #pragma unroll
                 for (int half = 0; half < 2; ++half)
-                    *reinterpret_cast<float2*>(sp + (part * LC_C + m0 + g + 8 * half) * LQ + 8 * j + 2 * t) =
-                        make_float2(p[0][j][2 * half], p[0][j][2 * half + 1]);
+                    *reinterpret_cast<float2*>(sum + (part * LC_C + m0 + g + 8 * half) * M::LQ + 8 * j + 2 * t) = make_float2(p[0][j][2 * half], p[0][j][2 * half + 1]);
         }
-        to_global(a.states + ((size_t)c * a.H + h) * a.dv * a.dk, true);
-        if (side == 0 && has_rows)
+        {   // what the chunk starts from, as [dv, dk]
+            float* o = a.states + ((size_t)c * a.H + h) * a.dv * a.dk;
 #pragma unroll
-            for (int j = 0; j < NT; ++j)
+            for (int half = 0; half < 2; ++half) {
+                const int n = n_base + g + 8 * half;
+                if (has && m < a.dk && n < a.dv) *reinterpret_cast<float2*>(o + (size_t)n * a.dk + m) = make_float2(S[2 * half], S[2 * half + 1]);
+            }
+        }
+        __syncthreads();                         // the quarters
+        {
+            float2 x[4];
 #pragma unroll
-                for (int x = 0; x < 4; ++x) S[j][x] += sS[(NS + 8 * j + 2 * t + (x & 1)) * LC_LD + s_row + g + 8 * (x >> 1)];
-        __syncthreads();
-        if (threadIdx.x < LC_C * (NS / 4)) {
-            const int row = threadIdx.x / (NS / 4), col = (threadIdx.x % (NS / 4)) * 4;
-            float4 u = *reinterpret_cast<const float4*>(su + row * LU + col);
-            float4 x[4];
-#pragma unroll
-            for (int part = 0; part < 4; ++part) x[part] = *reinterpret_cast<const float4*>(sp + (part * LC_C + row) * LQ + col);
+            for (int part = 0; part < 4; ++part) x[part] = *reinterpret_cast<const float2*>(sum + (part * LC_C + row) * M::LQ + col);
             u.x -= (x[0].x + x[1].x) + (x[2].x + x[3].x);
             u.y -= (x[0].y + x[1].y) + (x[2].y + x[3].y);
-            u.z -= (x[0].z + x[1].z) + (x[2].z + x[3].z);
-            u.w -= (x[0].w + x[1].w) + (x[2].w + x[3].w);
-            *reinterpret_cast<float4*>(su + row * LU + col) = u;
-            if (row < cnt && col < cols) *reinterpret_cast<float4*>(a.u + ((size_t)(t0 + row) * a.H + h) * a.dv + n_base + col) = u;
+            if (mine) *reinterpret_cast<float2*>(u_place(t0)) = u;
+            const LcSplit y = lc_split(u.x, u.y);
+            const uint32_t to = base + M::U + (row * 24 + col) * 2;
+            lc_sts32(to, y.h);
+            lc_sts32(to + M::PU, y.m);
+            lc_sts32(to + 2 * M::PU, y.l);
         }
-        __syncthreads();
-        if (has_rows) {
-            float p[1][NT][4], low[1][NT][4];
-            lc_zero<NT * 4>(&p[0][0][0]);
-            lc_zero<NT * 4>(&low[0][0][0]);
+        __syncthreads();                         // U's planes
+        if (has) {
+            float p[1][1][4], low[1][1][4];
+            lc_zero<4>(&p[0][0][0]);
+            lc_zero<4>(&low[0][0][0]);
 #pragma unroll
-            for (int k = 0; k < LC_C / 2; k += 16) {
-                const int k0 = side * (LC_C / 2) + k;
-                const LcA fa = lc_a_cols(sk + k0 * LC_LD + s_row, LC_LD, lc_scale(sr + k0));
-                LcB fb[NT];
-#pragma unroll
-                for (int j = 0; j < NT; ++j) fb[j] = lc_b_cols(su + k0 * LU + 8 * j, LU);
-                lc_products<1, NT>(p, low, &fa, fb);
+            for (int step = 0; step < 4; ++step) {
+                const LcA fa = lc_a_km<24>(base + M::U + 16 * step * 24 * 2, M::PU);
+                const uint4* f = fk[step >> 1];
+                const LcB fb = step & 1 ? LcB{{{f[0].z, f[1].z, f[2].z}, {f[0].w, f[1].w, f[2].w}}} : LcB{{{f[0].x, f[1].x, f[2].x}, {f[0].y, f[1].y, f[2].y}}};
+                lc_products<1, 1>(p, low, &fa, &fb);
             }
-            lc_add<NT * 4>(&p[0][0][0], &low[0][0][0]);
+            if (i + 1 < count) load_k(c + 1);
+            lc_add<4>(&p[0][0][0], &low[0][0][0]);
 #pragma unroll
-            for (int j = 0; j < NT; ++j)
-#pragma unroll
-                for (int x = 0; x < 4; ++x) S[j][x] = side == 0 ? fmaf(gain, S[j][x], p[0][j][x]) : p[0][j][x];
+            for (int x = 0; x < 4; ++x) S[x] = fmaf(gain, S[x], p[0][0][x]);
         }
-        to_shared();                             // read by everyone before the pass over U
+        to_planes();                             // (read by all before the second barrier)
         t0 = next_t0;
         cnt = next_cnt;
-        gain = next_gain;
     }
-    __syncthreads();
-    float* st = a.state + (size_t)a.slots[r] * a.state_stride + (size_t)h * a.dv * a.dk;
-    to_global(st, ((uintptr_t)st & 15) == 0);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+        const int n = n_base + g + 8 * (x >> 1);
+        if (has && m + (x & 1) < a.dk && n < a.dv) st[(size_t)n * a.dk + m + (x & 1)] = S[x];
+    }
 }
 
 // ---- a forget gate per key channel (csrc/linear_state.cu): k_t = 1 - f_t, S_t = diag(f_t) S_(t-1) + k_t v_t^T -------------------------
@@ -1253,13 +1280,7 @@ static int lc_run(const LcArgs& a, int n_requests, cudaStream_t s) {
         return lc_launch<lc_output_kernel<DK, DV>>(chunks, 256, planes, s, a, a.v, (size_t)a.ldv);
     }
     if (const int rc = lc_launch<lc_delta_prepare_kernel<DK, DV>>(chunks, 256, 2 * tile + 2 * square, s, a)) return rc;
-    // columns of S per block: 16 while the blocks then fit the SMs (one each: 186 KB), else 32, whose chain is a little longer
-    const bool wide = (long long)ceil_div(a.dv, 16) * a.H * n_requests > 148 && a.dv > 16;
-#define LC_CARRY(NS)                                                                                                                       \
-    lc_launch<lc_delta_carry_kernel<DK, NS>>(dim3(ceil_div(a.dv, NS), a.H, n_requests), LC_CARRY_THREADS,                                   \
-              (size_t)(2 * (2 * LC_C * LC_LD + LC_C * (NS + 8) + LC_C + 4) + 2 * NS * LC_LD + 4 * LC_C * (NS + 4)) * sizeof(float), s, a)
-    if (const int rc = wide ? LC_CARRY(32) : LC_CARRY(16)) return rc;
-#undef LC_CARRY
+    if (const int rc = lc_launch<lc_delta_carry_kernel<DK>>(dim3(ceil_div(a.dv, 16), a.H, n_requests), LC_CARRY_THREADS, LcCarryShared<DK>::SIZE, s, a)) return rc;
     return lc_launch<lc_output_kernel<DK, DV>>(chunks, 256, planes, s, a, (const float*)a.u, (size_t)a.H * a.dv);
 }
 
@@ -1272,17 +1293,17 @@ MM_EXPORT int mm_linear_chunk_supported(const void* q, const void* k, const void
 
 // q, k, v, gate, beta (null: no delta rule), head_decay, out, state as for the walk (decays positive or zero); chunk_meta [chunks, 4] =
 // (first token, tokens <= 64, request, .), req_chunks [requests, 2] = (first chunk, chunks).  Scratch, fp32: states [chunks, H, dv, dk], gain
-// [chunks, H], and with beta ratio [chunks, H, 64], w [tokens, H, dk], u [tokens, H, dv].
+// [chunks, H], and with beta frag [chunks, H, 12288] (24576 numbers for dk > 64), u [tokens, H, dv].
 MM_EXPORT int mm_linear_chunk(const void* q, const void* k, const void* v, int ldq, int ldk, int ldv, const void* gate, const void* beta,
                               const void* head_decay, void* out, void* state, long long state_stride, const void* chunk_meta,
                               const void* req_chunks, const void* slots, const void* positions, int n_requests, int n_chunks, int H, int Gq,
-                              int dk, int dv, void* states, void* gain, void* ratio, void* w, void* u, void* stream) {
+                              int dk, int dv, void* states, void* gain, void* frag, void* u, void* stream) {
     MM_REQUIRE(H > 0 && Gq > 0 && H % Gq == 0, "linear state chunks: heads must be a positive multiple of the q/k heads");
     MM_REQUIRE(mm_linear_chunk_supported(q, k, v, ldq, ldk, ldv, state, state_stride, dk, dv), "linear state chunks: sizes or pointers that the products do not take");
     MM_REQUIRE(gate != nullptr || head_decay != nullptr, "linear state: a decay per token or per head is needed");
     MM_REQUIRE(out && slots && positions && chunk_meta && req_chunks && states && gain, "linear state chunks: the lists and the scratch are needed");
-    MM_REQUIRE(beta == nullptr || (ratio && w && u), "linear state chunks: the delta rule needs its scratch");
-    MM_REQUIRE((((uintptr_t)out | (uintptr_t)states | (uintptr_t)ratio | (uintptr_t)w | (uintptr_t)u) & 15) == 0, "linear state chunks: the scratch starts on 16-byte boundaries");
+    MM_REQUIRE(beta == nullptr || (frag && u), "linear state chunks: the delta rule needs its scratch");
+    MM_REQUIRE((((uintptr_t)out | (uintptr_t)states | (uintptr_t)frag | (uintptr_t)u) & 15) == 0, "linear state chunks: the scratch starts on 16-byte boundaries");
     MM_REQUIRE(n_chunks <= 65535 && n_requests <= 65535, "linear state chunks: too many chunks or requests");
     if (n_requests <= 0 || n_chunks <= 0) return MM_OK;
     LcArgs a;
@@ -1293,7 +1314,7 @@ MM_EXPORT int mm_linear_chunk(const void* q, const void* k, const void* v, int l
     a.chunk_meta = (const int32_t*)chunk_meta; a.req_chunks = (const int32_t*)req_chunks;
     a.slots = (const int32_t*)slots; a.positions = (const int32_t*)positions;
     a.n_chunks = n_chunks; a.H = H; a.G = Gq; a.dk = dk; a.dv = dv;
-    a.states = (float*)states; a.gain = (float*)gain; a.ratio = (float*)ratio; a.w = (float*)w; a.u = (float*)u;
+    a.states = (float*)states; a.gain = (float*)gain; a.frag = (uint4*)frag; a.u = (float*)u;
     cudaStream_t s = (cudaStream_t)stream;
     if (dk <= 64) return dv <= 64 ? lc_run<64, 64>(a, n_requests, s) : lc_run<64, 128>(a, n_requests, s);
     return dv <= 64 ? lc_run<128, 64>(a, n_requests, s) : lc_run<128, 128>(a, n_requests, s);

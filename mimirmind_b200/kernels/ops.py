@@ -1179,16 +1179,16 @@ def linear_state_products(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, sta
         _need(t, what, torch.int32)
     n_chunks, n_req = chunk_meta.shape[0], req_chunks.shape[0]
     out = _rows_for(out, n, heads * dv, q)
-    # states [chunks, heads, dv, dk], gain [chunks, heads], with the delta rule ratio [chunks, heads, 64], w [n, heads, dk], u [n, heads, dv]
+    # states [chunks, heads, dv, dk], gain [chunks, heads], with the delta rule fragments of two operands in three 16-bit parts, u [n, heads, dv]
     sizes = [n_chunks * heads * dv * dk, n_chunks * heads]
     if beta is not None:
-        sizes += [n_chunks * heads * LINEAR_CHUNK, n * heads * dk, n * heads * dv]
+        sizes += [n_chunks * heads * LINEAR_CHUNK * (64 if dk <= 64 else 128) * 3, n * heads * dv]
     _kept, parts = _scratch(sizes, q.device)
-    states, gain, ratio, w, u = parts + [None] * (5 - len(parts))
+    states, gain, frag, u = parts + [None] * (4 - len(parts))
     check(_lib.load().mm_linear_chunk(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0), _ptr(gate), _ptr(beta),
                                       _ptr(head_decay), out.data_ptr(), state.data_ptr(), state.stride(0), chunk_meta.data_ptr(),
                                       req_chunks.data_ptr(), slots.data_ptr(), positions.data_ptr(), n_req, n_chunks, heads, qk_heads, dk, dv,
-                                      states, gain, ratio, w, u, _stream()), "linear_chunk")
+                                      states, gain, frag, u, _stream()), "linear_chunk")
     return out
 
 
