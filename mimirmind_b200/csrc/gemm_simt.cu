@@ -1,5 +1,5 @@
-// C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]) on the fp32 FMA units: the matrix product of the
-// true 32-bit path, and the any-shape fallback of the bfloat16 path.
+// C[M,N] = A[M,K] * W[N,K]^T (+ bias[N]) on the fp32 FMA units: the any-shape product of the true 32-bit path
+// (its layers' weights go to gemm_split_tcgen05.cu) and the fallback of the bfloat16 path.
 //
 // The reference computes Y[m,n] = sum_k X[m,k] * W[n,k] with W stored [N_out, K_in]
 // (src/compute/Matmul.cpp:54-65) and adds a bias per output column
@@ -7,6 +7,7 @@
 // ascending order by one thread, so its value does not depend on M, on the row's place
 // in the batch, on the tile it falls into, or on which of the two kernels below made it.
 #include "common.cuh"
+#include "gemm_split.h"
 
 // ---------------------------------------------------------------------------------------------------------------
 // tiles: a thread owns TM x TN outputs
@@ -16,8 +17,8 @@
 // of both operands are on their way from global memory into registers meanwhile (two buffers, one barrier per BK).
 // A buffer is [k][row]; a row's place is turned by (k / 4 % 8) * 4, so that the scattered stores of a warp (8 runs of k x 4
 // rows) fall into 32 different banks and four neighbouring rows still are one 16-byte word.
-// 64 x 64 outputs of 128 threads (8 x 4 each): 509 x 9,728 x 896 in 236 us (37.6 TFLOP/s; 4 x 4 a thread with scalar loads,
-// the form before: 477), 509 x 896 x 4,864, a single block per SM, in 176 us (before: 685).  Larger tiles (128 x 64, 128 x 128 of
+// 64 x 64 outputs of 128 threads (8 x 4 each): 37.6 TFLOP/s where they fill the GPU (509 x 9,728 x 896 in 236 us, 4 x 4 a thread with
+// scalar loads 477).  Larger tiles (128 x 64, 128 x 128 of
 // 8 x 8) gain nothing where they fill the GPU and lose a factor of 2 and 3 where they do not; fp32 FMAs alone: 10 % slower.
 template <typename T, bool VEC>
 __device__ __forceinline__ float4 simt_load4(const T* __restrict__ p, bool row_ok, int k, int K) {     // VEC: one aligned load, K % 4 == 0
@@ -164,8 +165,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_simt_kernel(const 
 // STAGES buffers; thread (c, g) of the 128 owns column c and the rows g, g + 128/NB, ... of A, R of them, and adds up k in
 // order.  A row of a buffer is padded by 16 bytes: the eight threads of a quarter warp read eight different bank groups.
 // 4 rows: 151,936 x 896 (545 MB) in 104 us with 128 rows of W per block, where a number of W is read once from shared memory (142 us with 32,
-// where each of 4 row groups reads it; 64-row tiles, the form before: 879); 896 x 4,864, 8 rows per block so that most SMs have one, in
-// 21 us (before: 755), of which the chain of 4,864 dependent additions is 10.
+// where each of 4 row groups reads it; 64-row tiles, the form before: 879).
 #define SIMT_GEMV_ROWS 16
 
 __device__ __forceinline__ void simt_cp16(void* smem, const void* gmem, bool in) {
@@ -302,6 +302,7 @@ MM_EXPORT int mm_gemm_simt(const void* A, int a_dtype, const void* W, int w_dtyp
     cudaStream_t s = (cudaStream_t)stream;
     typedef __nv_bfloat16 bf;
     const int key = a_dtype * 4 + w_dtype * 2 + c_dtype;
+    if (key == 0 && gemm_split_takes(W, N, K)) return gemm_split((const float*)A, (const float*)W, bias, bias_dtype, (float*)C, M, N, K, lda, ldc, s);
     if (key == 0 && M <= SIMT_GEMV_ROWS && K % 4 == 0 && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0) {
 #define SIMT_GEMV(NB, KB, STAGES, R) return launch_gemv_simt<NB, KB, STAGES, R>(A, W, bias, bias_dtype, C, M, N, K, lda, ldc, s)
         // as many rows of W per block as still leave every SM a few blocks

@@ -214,7 +214,9 @@ def attention_generic(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Ten
 
 
 def gemm_simt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor) -> torch.Tensor:
-    """out[M,N] = a[M,K] @ w[N,K]^T (+ bias) on the fp32 FMA units, k summed in ascending order."""
+    """out[M,N] = a[M,K] @ w[N,K]^T (+ bias) in 32 bits: on the fp32 FMA units, k summed in ascending order, or, fp32 throughout with layer-sized
+    weights, on the tensor cores from three bfloat16 parts of every number (``gemm_split_tcgen05.cu``).  Which follows from the weights: a row's bits
+    do not depend on M."""
     _need(a, "gemm a")
     _need(w, "gemm w")
     _need(out, "gemm out")

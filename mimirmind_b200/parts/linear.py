@@ -4,8 +4,8 @@ The reference computes ``Y[m,n] = Σ_k X[m,k]·W[n,k]`` (src/compute/Matmul.cpp:
 on CUDA, picks a kernel by weight type and M, with cuBLASLt as its bf16 library path
 (src/compute/cuda/GpuMatmul.cpp:786-884, 1095-1430).  Here the choice is by dtype only:
 
-* fp32 activations or fp32 weights → this library's fp32-FMA kernel (true 32-bit, each
-  output summed over k in ascending order, independent of the batch);
+* fp32 activations or fp32 weights → this library's 32-bit product (FMAs over k in ascending
+  order, or tensor cores over three-part numbers; each output independent of the batch);
 * bf16 × bf16 → the tensor-core route chosen by :mod:`mimirmind_b200.kernels.matmul_bf16`.
 """
 from __future__ import annotations

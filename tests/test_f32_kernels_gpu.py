@@ -28,6 +28,53 @@ def test_product(M, N, K):
         assert torch.equal(one[0], out[m])
 
 
+# rows and tokens around the tiles of 16 and 128 rows and of 8, 16, 32, 64 and 128 tokens; k in one, two, four and eight parts, whole steps of 64 and not
+@pytest.mark.parametrize("N,K", [(128, 128), (131, 260), (200, 644), (257, 1540), (1000, 2052)])
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16, 17, 33, 64, 65, 129, 300])
+def test_product_of_split_numbers(M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(M * N + K)
+    a, w, b = (torch.randn(s, generator=g, device=DEV) for s in ((M, K), (N, K), (N,)))
+    a *= torch.exp2(torch.randint(-12, 13, (M, K), generator=g, device=DEV))
+    loose = torch.empty(M * K + 1, device=DEV)[1:].view(M, K).copy_(a)          # rows off the 16-byte boundaries
+    out, two = torch.empty((M, N), device=DEV), torch.empty((M, N), device=DEV)
+    ops().gemm_simt(a, w, b, out)
+    ref, size = a.double() @ w.double().T + b.double(), a.double().abs() @ w.double().abs().T + b.double().abs()
+    # K / 16 rounded additions, two dozen roundings of whole sums beside them (the parts, what is cut off sixteen terms of one sum), and five sums of K / 16 steps of
+    # 2^-7 of the size
+    assert ((out - ref).abs() <= (K / 16 + 24 + 5 * K / 16 / 128) * 2.0 ** -24 * size).all()
+    ops().gemm_simt(loose, w, b, two)
+    assert torch.equal(two, out)
+    for m in {0, M // 2, M - 1}:                # alone: the kernel for a few rows
+        one = torch.empty((1, N), device=DEV)
+        ops().gemm_simt(a[m:m + 1].contiguous(), w, b, one)
+        assert torch.equal(one[0], out[m])
+
+
+@pytest.mark.parametrize("M", [5, 12, 40, 150])
+def test_product_of_numbers_that_cannot_be_split(M):
+    """An infinity, a NaN, a number beyond bf16's largest and sums that overflow: what 32-bit FMAs over k in order give, and nothing beside them changes."""
+    N, K = 260, 520
+    g = torch.Generator(device=DEV).manual_seed(M)
+    a, w = (torch.randn(s, generator=g, device=DEV) for s in ((M, K), (N, K)))
+    clean = torch.empty((M, N), device=DEV)
+    ops().gemm_simt(a, w, None, clean)
+    a[1, 3], a[2, 500], a[3, 17], w[130, 7], w[259, 519], w[5] = float("inf"), float("nan"), 3.4e38, float("-inf"), 3.4e38, 0.0
+    a[4] = 3e38                                 # sums that overflow
+    out = torch.empty((M, N), device=DEV)
+    ops().gemm_simt(a, w, None, out)
+    rows, cols = [1, 2, 3, 4], [130, 259, 5]
+    keep = torch.ones((M, N), dtype=torch.bool, device=DEV)
+    keep[rows] = False
+    keep[:, cols] = False
+    assert torch.equal(out[keep], clean[keep])
+    narrow = torch.empty((M, 96), device=DEV)   # the product by FMAs: fewer than 128 rows of weights
+    for n0 in (0, 96, 164):
+        ops().gemm_simt(a, w[n0:n0 + 96].contiguous(), None, narrow)
+        got = out[:, n0:n0 + 96]
+        assert torch.equal(torch.isnan(got), torch.isnan(narrow)) and torch.equal(torch.isinf(got), torch.isinf(narrow))
+        assert torch.equal(got[torch.isinf(got)], narrow[torch.isinf(narrow)])
+
+
 @pytest.mark.parametrize("M,N,K", [(3, 70, 96), (40, 130, 100), (300, 257, 36)])
 @pytest.mark.parametrize("ta,tw,tc", [(torch.bfloat16, torch.float32, torch.bfloat16), (torch.float32, torch.bfloat16, torch.float32)])
 def test_product_of_mixed_types(M, N, K, ta, tw, tc):
