@@ -267,7 +267,7 @@ struct Options {
     int tma_decode_stages = 3;
     int target_ctas = 2 * 148;        // decode CTAs wanted
     int use_cluster_merge = 1;
-    int cluster_max_wanted = 12;
+    int cluster_max_wanted = 12, cluster_max_tiles = 48;
     int fixed_split = 0;              // > 0: cut keys by absolute position into splits of this length
     int gemv_max_rows = 8;
     int skinny_max_rows = 64;

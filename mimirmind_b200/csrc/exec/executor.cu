@@ -953,7 +953,7 @@ MMX_EXPORT int mmx_option(const char* name, int value) {
         int* p;
     } table[] = {{"prefill_min", &o.prefill_min}, {"use_tcgen05_prefill", &o.use_tcgen05_prefill}, {"use_tma_decode", &o.use_tma_decode},
                  {"tma_decode_stages", &o.tma_decode_stages}, {"target_ctas", &o.target_ctas}, {"use_cluster_merge", &o.use_cluster_merge},
-                 {"cluster_max_wanted", &o.cluster_max_wanted}, {"fixed_split", &o.fixed_split}, {"gemv_max_rows", &o.gemv_max_rows},
+                 {"cluster_max_wanted", &o.cluster_max_wanted}, {"cluster_max_tiles", &o.cluster_max_tiles}, {"fixed_split", &o.fixed_split}, {"gemv_max_rows", &o.gemv_max_rows},
                  {"skinny_max_rows", &o.skinny_max_rows}, {"tcgen05_swiglu_min_rows", &o.tcgen05_swiglu_min_rows},
                  {"tcgen05_pair_min_rows", &o.tcgen05_pair_min_rows}, {"use_side_stream", &o.use_side_stream}};
     for (auto& t : table)

@@ -107,11 +107,12 @@ void choose_split(int n_items, int G, int max_kv_len, int head_dim, int page_siz
     p.cluster = false;
     const int ctas = std::max(1, n_items * G);
     if (ctas >= o.target_ctas / 2) return;      // one CTA per SM or more already: a split would only add the merge pass
-    const int wanted = std::max(1, std::min(o.target_ctas / ctas, (max_kv_len + 63) / 64));
+    const int tiles = (max_kv_len + 63) / 64, wanted = std::max(1, std::min(o.target_ctas / ctas, tiles));
     if (o.use_tma_decode && o.use_cluster_merge && (head_dim == 64 || head_dim == 128) && tma_page(page_size) && wanted >= 2) {
         int size = 1;
         while (size * 2 <= std::min(wanted, 8)) size *= 2;
-        if ((wanted >= 8 || 4 * size >= 3 * wanted) && wanted <= o.cluster_max_wanted && ctas <= cluster_capacity(head_dim, size)) {
+        if (wanted == tiles && tiles < 8 && 4 * size < 3 * wanted) size *= 2;      // a tile for each split: rather an empty CTA than a merge launch
+        if ((wanted >= 8 || 4 * size >= 3 * wanted) && (wanted <= o.cluster_max_wanted || tiles <= o.cluster_max_tiles) && ctas <= cluster_capacity(head_dim, size)) {
             p.max_splits = size;
             p.cluster = true;
             return;

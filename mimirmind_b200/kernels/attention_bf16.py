@@ -26,7 +26,9 @@ USE_TMA_DECODE = True   # decode attention with a TMA producer warp (page sizes 
 TMA_DECODE_STAGES = 3
 TARGET_CTAS = 2 * 148  # decode CTAs wanted (measured: 2 per SM beat 1 and 4 at batch 8; batch 64 is best unsplit)
 USE_CLUSTER_MERGE = True   # up to 8 splits per token: one thread-block cluster merges them through shared memory
-CLUSTER_MAX_WANTED = 12    # ... preferred over more splits and a merge launch when up to this many were wanted
+CLUSTER_MAX_WANTED = 12    # ... preferred over more splits and a merge launch when up to this many were wanted,
+CLUSTER_MAX_TILES = 48     # or when its eight CTAs have at most six tiles of 64 keys each (whole decode steps of two layers, cluster and merge launch, us: 1 request
+#                            at 1,000 keys, 2 KV heads 139 and 149, 4 KV heads 400 and 408; 2 requests at 3,000 157 and 159, 407 and 415; at 8,000 170 and 166, 435 and 426)
 FIXED_SPLIT = None     # tests set a split length in keys to cut by absolute position instead
 
 _declared = False
@@ -78,22 +80,28 @@ def cluster_capacity(head_dim: int, size: int) -> int:
     return _cluster_capacity[key]
 
 
-def choose_split(n_items: int, num_kv_heads: int, max_kv_len: int, head_dim: int = 0, page_size: int = 0):
+def choose_split(n_items: int, num_kv_heads: int, max_kv_len: int, head_dim: int = 0, page_size: int = 0, max_tiles: Optional[int] = None):
     """(split_len, max_splits, cluster) for the decode kernel.  split_len 0: every token's key range is cut evenly
     into at most max_splits pieces of whole 64-key tiles, so the grid is full whatever the lengths.  cluster: the
-    splits of a token are one thread-block cluster and merge themselves."""
+    splits of a token are one thread-block cluster and merge themselves.  max_tiles: instead of CLUSTER_MAX_TILES."""
     if FIXED_SPLIT:
         return FIXED_SPLIT, max(1, -(-max_kv_len // FIXED_SPLIT)), False
     ctas = max(1, n_items * num_kv_heads)
     if ctas >= TARGET_CTAS // 2:
         return 0, 1, False       # one CTA per SM or more already: a split would only add the merge pass
     # never more CTAs than are resident at once (two per SM): a second, nearly empty wave costs a whole pass
-    wanted = max(1, min(TARGET_CTAS // ctas, -(-max_kv_len // 64)))
+    tiles = -(-max_kv_len // 64)
+    wanted = max(1, min(TARGET_CTAS // ctas, tiles))
     # Clusters of 2, 4 or 8 place well on the GPU (measured: 3 and 6 do not), and only as many as are resident at
     # once.  Worth a few splits less (12 -> 8 measured faster), not half of them (6 -> 4, 3 -> 2 measured slower).
     if USE_TMA_DECODE and USE_CLUSTER_MERGE and head_dim in (64, 128) and page_size in (8, 16, 32, 64) and wanted >= 2:
         size = 1 << (min(wanted, 8).bit_length() - 1)
-        if (wanted >= 8 or 4 * size >= 3 * wanted) and wanted <= CLUSTER_MAX_WANTED and ctas <= cluster_capacity(head_dim, size):
+        # Where the keys are what there is little of, a tile for each split, the next size up: a CTA of the cluster stays empty, but the
+        # merge launch goes (a step of 1 token, 2 KV heads, at 131 keys: 134 us instead of 142, at 380 134 and 143).
+        if wanted == tiles < 8 and 4 * size < 3 * wanted:
+            size *= 2
+        few = wanted <= CLUSTER_MAX_WANTED or tiles <= (CLUSTER_MAX_TILES if max_tiles is None else max_tiles)
+        if (wanted >= 8 or 4 * size >= 3 * wanted) and few and ctas <= cluster_capacity(head_dim, size):
             return 0, size, True
     return 0, wanted, False
 

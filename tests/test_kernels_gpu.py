@@ -377,6 +377,19 @@ def test_attention_decode_cluster_merge(H, G, hd, ps, n, size, window):
     assert np.abs(out2.float().cpu().numpy() - out.float().cpu().numpy()).max() <= 2 ** -7 * np.abs(ref).max()
 
 
+@pytest.mark.parametrize("H,G,hd", [(14, 2, 64), (28, 4, 128)])
+@pytest.mark.parametrize("keys,size", [(129, 4), (192, 4), (193, 4), (257, 4), (321, 8), (448, 8), (449, 8), (833, 8), (3072, 8), (3073, 0)])
+def test_attention_decode_few_requests_as_clusters(H, G, hd, keys, size):
+    """Steps of two requests where keys are short of splits (CTAs without a tile), and long ones with up to six tiles a CTA; beyond that the
+    merge kernel.  One request is shorter than the step's longest."""
+    rng = np.random.RandomState(keys)
+    case = make_attention_case(rng, H, G, hd, 16, [keys, keys // 2], [1, 1], torch.bfloat16)
+    ref = attention_reference(case, 0)
+    out, plan = run_bf16_attention(case, H, G, hd, 16, 0)
+    assert plan.cluster == (size > 0) and (plan.max_splits == size if size else plan.max_splits > 12)
+    assert np.abs(out.float().cpu().numpy().reshape(ref.shape) - ref).max() <= 2.5 * 2 ** -8 * np.abs(ref).max()
+
+
 @pytest.mark.parametrize("n_keys", [4096, 8192])
 @pytest.mark.parametrize("far", ["first tile", "page edge"])
 def test_attention_over_thousands_of_keys(n_keys, far):
