@@ -597,7 +597,7 @@ bool gemm_split_takes(const void* W, int N, int K) { return K % 4 == 0 && ((uint
 int gemm_split(const float* A, const float* W, const void* bias, int bias_dtype, float* C, int M, int N, int K, int lda, int ldc, cudaStream_t s) {
     const SplitArgs g{A, W, bias, C, bias_dtype, M, N, K, lda, ldc, gemm_split_parts(K), 1, lda % 4 == 0 && ((uintptr_t)A & 15) == 0};
     if (M <= FEW) return M <= 8 ? launch_few<1>(g, s) : launch_few<2>(g, s);
-    // The tile and the parts' place that take the least time: rounds of one CTA per SM, each with a start (8 us with the first loads and the end) and
+    // The tile and the parts' place that take the least time: rounds of one CTA per SM (clusters of 4 find room for 132 CTAs, of 8 for 120), each with a start (8 us with the first loads and the end) and
     // a time per 64 k that was measured for each tile, and 2 us where a cluster's results meet.  Within 15 % of what is measured
     // for 17 to 1,024 tokens of 896 to 9,728 rows.
     constexpr int TILES[3] = {32, 64, 128}, STEP_NS[3] = {1030, 1220, 1700};
@@ -607,7 +607,8 @@ int gemm_split(const float* A, const float* W, const void* bias, int bias_dtype,
     for (int i = 0; i < 3; ++i) {
         for (const int r : {1, g.parts}) {
             const long long ctas = (long long)ceil_div(M, TILES[i]) * ceil_div(N, 128) * r;
-            const long long ns = (ctas + 147) / 148 * (8000 + (long long)ceil_div(steps, r) * STEP_NS[i]) + (r > 1 ? 2000 : 0);
+            const int room = r == 8 ? 120 : r == 4 ? 132 : 148;
+            const long long ns = (ctas + room - 1) / room * (8000 + (long long)ceil_div(steps, r) * STEP_NS[i]) + (r > 1 ? 2000 : 0);
             if (best < 0 || ns < best) {
                 best = ns;
                 nt = TILES[i];
