@@ -113,11 +113,12 @@ __device__ __forceinline__ long long att_offset(const int32_t* __restrict__ tabl
 }
 
 // A tile of 32 rows of one head, 128 threads: thread (ty, tx) owns the scores of rows 2 ty, 2 ty + 1 and keys tx, tx + 8, tx + 16, tx + 24 of
-// a chunk, and the outputs of the same rows in the columns 32 g + 4 tx...  Bound by the FMA units and the shared-memory reads that
-// feed them; the next chunk's keys and values arrive under the current one, their places looked up two chunks ahead.
+// a chunk, and the outputs of the same rows in the columns 32 g + 4 tx...  Bound by the chain of chunks and the latency of the
+// shared-memory reads that feed the FMA units (a warp per scheduler at most tiles; one row a thread and eight warps read half as much again: 66 us), so what
+// is multiplied next is read while the current numbers are multiplied; the next chunk's keys and values arrive under the current one, their places looked up two chunks ahead.
 // The chunk's sum is added up in the order of a warp's butterfly over the key's place in the chunk: 16, 8 apart within a
 // thread, 4, 2, 1 apart between the eight threads of a row.  Keys that a row does not see are skipped, not multiplied by zero.
-// 509 tokens, 14 heads of 64: 62 us (a warp per token and head, the plain form: 820).
+// 509 tokens, 14 heads of 64: 51 us (without the reads ahead 59; a warp per token and head, the plain form: 820).
 template <int HD>
 __global__ void __launch_bounds__(128) attention_tile_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_pages,
                                                                  const float* __restrict__ v_pages, float* __restrict__ out,
@@ -207,22 +208,27 @@ __global__ void __launch_bounds__(128) attention_tile_f32_kernel(const float* __
             for (int i = 0; i < RP; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) s[i][j] = 0.0f;
-#pragma unroll 8
-            for (int d = 0; d < HD; d += 4) {
-                float4 a[RP], b[4];
+            // the numbers of the next four columns are read while the current ones are multiplied
+            auto scores = [&](float4* a, float4* b, int d) {
 #pragma unroll
                 for (int i = 0; i < RP; ++i) a[i] = *reinterpret_cast<const float4*>(sq + (ty * RP + i) * LD + d);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(kb + (tx + 8 * j) * LD + d);
+            };
+            float4 qa[2][RP], ka[2][4];
+            scores(qa[0], ka[0], 0);
 #pragma unroll
-                for (int i = 0; i < RP; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        s[i][j] = fmaf(a[i].x, b[j].x, s[i][j]);
-                        s[i][j] = fmaf(a[i].y, b[j].y, s[i][j]);
-                        s[i][j] = fmaf(a[i].z, b[j].z, s[i][j]);
-                        s[i][j] = fmaf(a[i].w, b[j].w, s[i][j]);
-                    }
+            for (int d = 0; d < HD; d += 4) {
+                const int u = (d >> 2) & 1;
+                if (d + 4 < HD) scores(qa[u ^ 1], ka[u ^ 1], d + 4);
+#define ATT_SCORE(C)                                       \
+    _Pragma("unroll") for (int i = 0; i < RP; ++i)         \
+        _Pragma("unroll") for (int j = 0; j < 4; ++j) s[i][j] = fmaf(qa[u][i].C, ka[u][j].C, s[i][j])
+                ATT_SCORE(x);
+                ATT_SCORE(y);
+                ATT_SCORE(z);
+                ATT_SCORE(w);
+#undef ATT_SCORE
             }
             bool whole = true;                   // every row of the warp's sees every key of the chunk
 #pragma unroll
@@ -260,16 +266,23 @@ __global__ void __launch_bounds__(128) attention_tile_f32_kernel(const float* __
             whole = __all_sync(0xffffffffu, whole);
             __syncwarp();                        // a row's probabilities are written and read by the same eight threads
             if (whole) {
-#pragma unroll 2
+                auto values = [&](float4* v, int j) {
+#pragma unroll
+                    for (int a = 0; a < CG; ++a) v[a] = *reinterpret_cast<const float4*>(vb + j * HD + a * 32 + tx * 4);
+                };
+                float4 va[2][CG];
+                values(va[0], 0);
+#pragma unroll
                 for (int j = 0; j < 32; j += 4) {
                     float4 p[RP];
 #pragma unroll
                     for (int i = 0; i < RP; ++i) p[i] = *reinterpret_cast<const float4*>(sp + (ty * RP + i) * LP + j);
 #pragma unroll
-                    for (int jj = 0; jj < 4; ++jj)
+                    for (int jj = 0; jj < 4; ++jj) {
+                        if (j + jj + 1 < 32) values(va[(jj + 1) & 1], j + jj + 1);
 #pragma unroll
                         for (int a = 0; a < CG; ++a) {
-                            const float4 v = *reinterpret_cast<const float4*>(vb + (j + jj) * HD + a * 32 + tx * 4);
+                            const float4 v = va[jj & 1][a];
 #pragma unroll
                             for (int i = 0; i < RP; ++i) {
                                 const float pj = jj == 0 ? p[i].x : jj == 1 ? p[i].y : jj == 2 ? p[i].z : p[i].w;
@@ -279,6 +292,7 @@ __global__ void __launch_bounds__(128) attention_tile_f32_kernel(const float* __
                                 acc[i][4 * a + 3] = fmaf(pj, v.w, acc[i][4 * a + 3]);
                             }
                         }
+                    }
                 }
             } else {
 #pragma unroll 4
