@@ -300,7 +300,7 @@ Rows linear(Step& st, Arena& mem, const Rows& x, const Tensor& W, int out_dtype,
         }
         return out;
     }
-    check_kernel(mm_gemm_simt(x.ptr, x.dtype, W.ptr, W.dtype, nullptr, F32, out.ptr, out_dtype, m, n, k, k, n, s), "gemm_simt");
+    check_kernel(mm_gemm_simt(x.ptr, x.dtype, W.ptr, W.dtype, nullptr, F32, out.ptr, out_dtype, m, n, k, k, n, st.err, s), "gemm_simt");
     return out;
 }
 

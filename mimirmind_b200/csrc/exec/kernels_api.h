@@ -28,7 +28,7 @@ int mm_slot_mapping(const void* positions, const void* token_req, const void* bl
 
 // matrix products
 int mm_gemm_simt(const void* A, int a_dtype, const void* W, int w_dtype, const void* bias, int bias_dtype, void* C, int c_dtype,
-                 int M, int N, int K, int lda, int ldc, void* stream);
+                 int M, int N, int K, int lda, int ldc, void* err, void* stream);
 int mm_gemv_bf16(const void* W, const void* x, const void* bias, int bias_dtype, void* out, int out_dtype, int M, int N, int K,
                  int ldx, int ldo, int rt, int ks, int swiglu, const void* in_ss, int in_tiles, int in_dim, float in_eps,
                  void* stream);

@@ -295,14 +295,15 @@ static int launch_gemm_simt(const void* A, const void* W, const void* bias, int 
 #undef SIMT_TILE
 }
 
+// err: device int set to 1 when a bounded wait of the tensor-core form ran out (may be null)
 MM_EXPORT int mm_gemm_simt(const void* A, int a_dtype, const void* W, int w_dtype, const void* bias, int bias_dtype,
-                           void* C, int c_dtype, int M, int N, int K, int lda, int ldc, void* stream) {
+                           void* C, int c_dtype, int M, int N, int K, int lda, int ldc, void* err, void* stream) {
     MM_REQUIRE(M >= 0 && N > 0 && K > 0 && lda >= K && ldc >= N, "gemm: bad sizes");
     if (M == 0) return MM_OK;
     cudaStream_t s = (cudaStream_t)stream;
     typedef __nv_bfloat16 bf;
     const int key = a_dtype * 4 + w_dtype * 2 + c_dtype;
-    if (key == 0 && gemm_split_takes(W, N, K)) return gemm_split((const float*)A, (const float*)W, bias, bias_dtype, (float*)C, M, N, K, lda, ldc, s);
+    if (key == 0 && gemm_split_takes(W, N, K)) return gemm_split((const float*)A, (const float*)W, bias, bias_dtype, (float*)C, M, N, K, lda, ldc, (int*)err, s);
     if (key == 0 && M <= SIMT_GEMV_ROWS && K % 4 == 0 && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0) {
 #define SIMT_GEMV(NB, KB, STAGES, R) return launch_gemv_simt<NB, KB, STAGES, R>(A, W, bias, bias_dtype, C, M, N, K, lda, ldc, s)
         // as many rows of W per block as still leave every SM a few blocks

@@ -11,6 +11,7 @@
 // in order, the parts' results in order.  The tile's size along the tokens and whether the parts are walked by one CTA or shared out over a
 // cluster do not change a bit, so a row's value depends neither on M nor on what stands beside it.  A result that is not finite (an
 // operand was not, or rounds to infinity in bf16, or a sum overflowed) is made again by 32-bit FMAs over k in ascending order.
+// All waits are bounded; when one runs out the CTA gives its tensor memory back, sets `err` and makes its whole tile again like that.
 //
 // A CTA works on 128 rows of W (M of the instruction) x NT tokens (its N), 64 k a step:
 //   warps 0..7    bring both operands' 64 k in as fp32 (asynchronous copies that a thread later reads back itself, or registers), split them and
@@ -51,6 +52,8 @@ struct SplitArgs {
     float* C;
     int bias_dtype, M, N, K, lda, ldc, parts, ranks;
     bool a_words;            // rows of A stand on 16-byte boundaries
+    int* err;
+    int give_up;             // 1: as if a wait had run out from the start, so that none is tried more than once
 };
 
 __device__ __forceinline__ uint32_t gs_round2(float x, float y) {
@@ -105,7 +108,9 @@ __device__ __forceinline__ void gs_st8(uint32_t at, const float* v) {
                  "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])) : "memory");
 }
 // A bounded wait that sleeps in the barrier (up to 20 us a try, so under 2 s in all): seventeen warps that poll instead keep the
-// stores of the planes waiting.
+// stores of the planes waiting.  False when it ran out, here or in another warp; the lanes of a warp may see the one or the other, and what
+// follows is for whole warps, so no lane leaves its way for it: the summing warps stop after a vote, the others walk on to their ends
+// without waiting for more than a try.  The tile is made again then.
 __device__ __forceinline__ bool gs_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
     for (int it = 0; it < 100000; ++it) {
         uint32_t ok;
@@ -175,7 +180,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const Spli
         mbar_init(smem_u32(&ctl.sum_empty), SUM_WARPS);
         mbar_init(smem_u32(&ctl.low_full), 1);
         mbar_init(smem_u32(&ctl.low_empty), SUM_WARPS);
-        ctl.abort_flag = 0;
+        ctl.abort_flag = g.give_up;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -227,7 +232,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const Spli
         for (int i = 0; i < S::RING; ++i) fetch(first + i);
         for (int step = first; step < last; ++step) {
             const int it = step - first, s = it & 1;
-            if (!gs_wait(smem_u32(&ctl.empty[s]), ((it >> 1) & 1) ^ 1, abort_flag)) break;
+            gs_wait(smem_u32(&ctl.empty[s]), ((it >> 1) & 1) ^ 1, abort_flag);
             asm volatile("cp.async.wait_group %0;\n" ::"n"(S::RING - 1) : "memory");
             const uint32_t to = planes + s * S::STAGE + place;
             const float4* held = reinterpret_cast<const float4*>(smem_raw + (ring - smem_u32(smem_raw)) + it % S::RING * S::RING_BYTES) + tid;
@@ -264,7 +269,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const Spli
             const int count = 4 / HB * (part_begin(p + 1) - part_begin(p));
 #pragma unroll 1
             for (int c = 0; c < count; ++c, ++group) {
-                if (!gs_wait(smem_u32(&ctl.sum_full), group & 1, abort_flag)) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, gs_wait(smem_u32(&ctl.sum_full), group & 1, abort_flag))) { ok = false; break; }
                 tc_fence_after();
 #pragma unroll
                 for (int b = 0; b < HB; ++b)
@@ -279,7 +284,7 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const Spli
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&ctl.sum_empty));
             }
-            if (!ok || !gs_wait(smem_u32(&ctl.low_full), (p - p_begin) & 1, abort_flag)) { ok = false; break; }
+            if (!ok || !__all_sync(0xffffffffu, gs_wait(smem_u32(&ctl.low_full), (p - p_begin) & 1, abort_flag))) { ok = false; break; }
             tc_fence_after();
 #pragma unroll
             for (int j = 0; j < CH; j += LD) {
@@ -306,32 +311,27 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const Spli
 #pragma unroll
         for (int i = 0; i < CH; ++i)
             asm volatile("st.shared.f32 [%0], %1;" ::"r"(planes + ((half * CH + i) * 128 + quarter * 32 + lane) * 4), "f"(acc[i]) : "memory");
-        if (!ok)                                 // a wait ran out: made again below
-#pragma unroll 1
-            for (int i = 0; i < CH; ++i)
-                asm volatile("st.shared.b32 [%0], %1;" ::"r"(planes + ((half * CH + i) * 128 + quarter * 32 + lane) * 4), "r"(0x7fffffff) : "memory");
     } else {
         // ---- products: the warp walks along together, so that the operands' places stay in uniform registers, one thread issues ----
         constexpr uint32_t idesc = idesc_bf16(128, NT, false);
         const uint32_t base = __shfl_sync(0xffffffffu, tmem, 0), low = base + HB * NT;
-        bool ok = true;
         int group = 0;
-        for (int p = p_begin; p < p_end && ok; ++p) {
+        for (int p = p_begin; p < p_end; ++p) {
             const int begin = part_begin(p), end = part_begin(p + 1);
-            for (int step = begin; step < end && ok; ++step) {
+            for (int step = begin; step < end; ++step) {
                 const int it = step - first, s = it & 1;
-                if (!gs_wait(smem_u32(&ctl.full[s]), (it >> 1) & 1, abort_flag)) ok = false;
+                gs_wait(smem_u32(&ctl.full[s]), (it >> 1) & 1, abort_flag);
                 const uint32_t at = planes + s * S::STAGE, xat = at + 3 * W_PLANE;
                 const uint64_t wh = smem_desc_sw128(at, 16, 1024), xh = smem_desc_sw128(xat, 16, 1024);
                 constexpr uint64_t WP = W_PLANE >> 4, XP = S::X_PLANE >> 4;           // the next plane
 #pragma unroll
                 for (int k0 = 0; k0 < 4; k0 += HB, ++group) {
                     const bool fresh = step == begin && k0 == 0;
-                    if (ok && !gs_wait(smem_u32(&ctl.sum_empty), (group & 1) ^ 1, abort_flag)) ok = false;
+                    gs_wait(smem_u32(&ctl.sum_empty), (group & 1) ^ 1, abort_flag);
                     // the part before has been read
-                    if (ok && fresh && !gs_wait(smem_u32(&ctl.low_empty), ((p - p_begin) & 1) ^ 1, abort_flag)) ok = false;
+                    if (fresh) gs_wait(smem_u32(&ctl.low_empty), ((p - p_begin) & 1) ^ 1, abort_flag);
                     tc_fence_after();
-                    if (gs_elect() && ok) {
+                    if (gs_elect()) {
 #pragma unroll
                         for (int k = k0; k < k0 + HB; ++k) gs_umma(base + (k - k0) * NT, wh + 2 * k, xh + 2 * k, idesc, 0u);   // 32 bytes along the swizzled rows
                         umma_commit(smem_u32(&ctl.sum_full));
@@ -362,6 +362,11 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const Spli
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (*abort_flag) {                           // (every role is through: the flag is settled and nobody else writes to the planes)
+        if (tid == 0 && g.err != nullptr) atomicExch(g.err, 1);
+        for (int i = tid; i < NT * 128; i += SPLIT_THREADS) asm volatile("st.shared.b32 [%0], %1;" ::"r"(planes + i * 4), "r"(0x7fffffff) : "memory");
+        __syncthreads();                         // the tile holds no number: all of it is made again below
+    }
     // before the cluster's barrier: a CTA of another launch may be waiting for it where this cluster's next CTA is to wait for that one's
     if (warp == 16) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::COLS) : "memory");
     if (g.ranks > 1) gs_cluster_sync();
@@ -555,6 +560,10 @@ int gemm_split_parts(int K) {
     return steps >= 24 ? 8 : steps >= 10 ? 4 : steps >= 4 ? 2 : 1;
 }
 
+SplitArgs split_args(const float* A, const float* W, const void* bias, int bias_dtype, float* C, int M, int N, int K, int lda, int ldc, int* err, int give_up) {
+    return SplitArgs{A, W, bias, C, bias_dtype, M, N, K, lda, ldc, gemm_split_parts(K), 1, lda % 4 == 0 && ((uintptr_t)A & 15) == 0, err, give_up};
+}
+
 template <int NT>
 int launch_split(SplitArgs g, int ranks, cudaStream_t s) {
     g.ranks = ranks;
@@ -581,6 +590,7 @@ int launch_split(SplitArgs g, int ranks, cudaStream_t s) {
 
 int launch_split(const SplitArgs& g, int nt, int ranks, cudaStream_t s) {
     switch (nt) {
+        case FEW: return g.M <= 8 ? launch_few<1>(g, s) : launch_few<2>(g, s);
         case 32: return launch_split<32>(g, ranks, s);
         case 64: return launch_split<64>(g, ranks, s);
         default: return launch_split<128>(g, ranks, s);
@@ -594,9 +604,10 @@ int launch_split(const SplitArgs& g, int nt, int ranks, cudaStream_t s) {
 // (131 x 260 for one token: 4 us by FMAs, 6 here).
 bool gemm_split_takes(const void* W, int N, int K) { return K % 4 == 0 && ((uintptr_t)W & 15) == 0 && N >= 128 && N <= 65536 && K >= 128; }
 
-int gemm_split(const float* A, const float* W, const void* bias, int bias_dtype, float* C, int M, int N, int K, int lda, int ldc, cudaStream_t s) {
-    const SplitArgs g{A, W, bias, C, bias_dtype, M, N, K, lda, ldc, gemm_split_parts(K), 1, lda % 4 == 0 && ((uintptr_t)A & 15) == 0};
-    if (M <= FEW) return M <= 8 ? launch_few<1>(g, s) : launch_few<2>(g, s);
+int gemm_split(const float* A, const float* W, const void* bias, int bias_dtype, float* C, int M, int N, int K, int lda, int ldc, int* err,
+               cudaStream_t s) {
+    const SplitArgs g = split_args(A, W, bias, bias_dtype, C, M, N, K, lda, ldc, err, 0);
+    if (M <= FEW) return launch_split(g, FEW, 1, s);
     // The tile and the parts' place that take the least time: rounds of one CTA per SM (clusters of 4 find room for 132 CTAs, of 8 for 120), each with a start (8 us with the first loads and the end) and
     // a time per 64 k that was measured for each tile, and 2 us where a cluster's results meet.  Within 15 % of what is measured
     // for 17 to 1,024 tokens of 896 to 9,728 rows.
@@ -617,4 +628,15 @@ int gemm_split(const float* A, const float* W, const void* bias, int bias_dtype,
         }
     }
     return launch_split(g, nt, ranks, s);
+}
+
+// The same product in a form of the caller's choice, which does not change a bit: tiles of `tile` tokens (16: the kernel for up to
+// so many; 32, 64 or 128), the parts of k one after the other or in a cluster.  `give_up`: 1 as if a wait of the tiles' kernel had run out at its
+// start.
+MM_EXPORT int mm_gemm_split(const void* A, const void* W, const void* bias, int bias_dtype, void* C, int M, int N, int K, int lda, int ldc, int tile,
+                            int side_by_side, int give_up, void* err, void* stream) {
+    MM_REQUIRE(M > 0 && N > 0 && K > 0 && lda >= K && ldc >= N && gemm_split_takes(W, N, K), "gemm_split: bad sizes");
+    MM_REQUIRE((tile == FEW && M <= FEW) || tile == 32 || tile == 64 || tile == 128, "gemm_split: no such tile");
+    const SplitArgs g = split_args((const float*)A, (const float*)W, bias, bias_dtype, (float*)C, M, N, K, lda, ldc, (int*)err, give_up);
+    return launch_split(g, tile, side_by_side ? g.parts : 1, (cudaStream_t)stream);
 }

@@ -230,7 +230,29 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ou
             raise KernelError("gemm: bias shape mismatch")
     check(_lib.load().mm_gemm_simt(a.data_ptr(), dtype_code(a.dtype), w.data_ptr(), dtype_code(w.dtype), _ptr(bias),
                                    dtype_code(bias.dtype) if bias is not None else F32, out.data_ptr(),
-                                   dtype_code(out.dtype), m, n, k, k, n, _stream()), "gemm_simt")
+                                   dtype_code(out.dtype), m, n, k, k, n, tcgen05_error_flag(out.device).data_ptr(), _stream()), "gemm_simt")
+    return out
+
+
+def gemm_split(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, tile: int, side_by_side: bool, give_up: bool = False) -> torch.Tensor:
+    """The tensor-core form of ``gemm_simt`` (fp32 throughout, rows of ``a`` and ``out`` at any stride) in tiles of ``tile`` tokens: 16 (up to 16 tokens), 32, 64 or 128, the parts
+    of k one after the other in a block or ``side_by_side`` in a cluster.  Every form gives the same bits.  ``give_up``: as if a wait of the tiles'
+    kernel had run out at its start: none is tried more than once, the error flag is set and the result is made again by FMAs."""
+    m, k = a.shape
+    n = w.shape[0]
+    _need(w, "gemm w", torch.float32)
+    for t, what, cols in ((a, "a", k), (out, "out", n)):
+        if t.dtype != torch.float32 or not t.is_cuda or t.shape != (m, cols) or t.stride(1) != 1:
+            raise KernelError(f"gemm {what}: fp32 rows with unit column stride are needed")
+    if w.shape != (n, k):
+        raise KernelError("gemm: shape mismatch")
+    if bias is not None:
+        _need(bias, "gemm bias")
+        if bias.shape != (n,):
+            raise KernelError("gemm: bias shape mismatch")
+    check(_lib.load().mm_gemm_split(a.data_ptr(), w.data_ptr(), _ptr(bias), dtype_code(bias.dtype) if bias is not None else F32, out.data_ptr(), m, n, k,
+                                    a.stride(0), out.stride(0), int(tile), int(bool(side_by_side)), int(bool(give_up)), tcgen05_error_flag(a.device).data_ptr(),
+                                    _stream()), "gemm_split")
     return out
 
 

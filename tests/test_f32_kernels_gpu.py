@@ -75,6 +75,32 @@ def test_product_of_numbers_that_cannot_be_split(M):
         assert torch.equal(got[torch.isinf(got)], narrow[torch.isinf(narrow)])
 
 
+@pytest.mark.parametrize("tile", [32, 64, 128])
+@pytest.mark.parametrize("side_by_side", [False, True])
+@pytest.mark.parametrize("M,N,K", [(40, 130, 128), (150, 260, 1540)])
+def test_product_whose_waits_run_out(tile, side_by_side, M, N, K):
+    """As if a wait had run out at the start: the kernel returns, the error flag is set and the result is what FMAs over k in order give, to the bit.
+    The next product is as if nothing had been."""
+    g = torch.Generator(device=DEV).manual_seed(M + tile)
+    a, w, b = (torch.randn(s, generator=g, device=DEV) for s in ((M, K), (N, K), (N,)))
+    whole, gone, again, narrow = (torch.empty((M, N), device=DEV) for _ in range(4))
+    flag = ops().tcgen05_error_flag(a.device)
+    ops().gemm_split(a, w, b, whole, tile, side_by_side)
+    assert int(flag.item()) == 0
+    try:
+        ops().gemm_split(a, w, b, gone, tile, side_by_side, give_up=True)
+        assert int(flag.item()) == 1
+    finally:
+        flag.zero_()
+    ops().gemm_split(a, w, b, again, tile, side_by_side)
+    assert int(flag.item()) == 0 and torch.equal(again, whole)
+    for n0 in range(0, N, 65):                  # the product by FMAs: fewer than 128 rows of weights
+        part = torch.empty((M, min(65, N - n0)), device=DEV)
+        ops().gemm_simt(a, w[n0:n0 + 65].contiguous(), b[n0:n0 + 65].contiguous(), part)
+        narrow[:, n0:n0 + 65] = part
+    assert torch.equal(gone, narrow)
+
+
 @pytest.mark.parametrize("M,N,K", [(3, 70, 96), (40, 130, 100), (300, 257, 36)])
 @pytest.mark.parametrize("ta,tw,tc", [(torch.bfloat16, torch.float32, torch.bfloat16), (torch.float32, torch.bfloat16, torch.float32)])
 def test_product_of_mixed_types(M, N, K, ta, tw, tc):
