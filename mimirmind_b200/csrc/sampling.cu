@@ -459,15 +459,16 @@ __device__ __noinline__ void sum_table(uint32_t offset) {     // of the table wi
 }
 
 // Bins of a plain row, monotone in the logit (a rounded product and sum, a scaling and limits are): 65536 of 1/2048 nat below the
-// maximum, the last one without an end; 256 of them are a bin of the first level.
+// maximum, the last one without an end; 256 of them are a bin of the first level.  Both come from one rounded number, the distance from the maximum
+// in 32 nats, by powers of two, so that a logit's bin of the first level holds its finer one whatever the temperature (near 1e38
+// inv_t / 32 is below the normal numbers and not what inv_t is).
 struct DrawBins {
-    float inv_t, max_scaled;
-    __device__ __forceinline__ float place(float v) const { return fmaxf(fminf(2048.0f * __fmaf_rn(-v, inv_t, max_scaled), 65535.0f), 0.0f); }
-    // The bin of the first level, 0 to 256 (256 is the end of bin 255), as the low bits of the result: powers of two scale exactly and the limits
-    // come with the sum, so this is two instructions.  inv_t and max_scaled divided by 32.
-    static __device__ __forceinline__ uint32_t first_bits(float v, float inv_t32, float max_scaled32) {
-        return __float_as_uint(__fmaf_rz(__saturatef(__fmaf_rn(-v, inv_t32, max_scaled32)), 256.0f, 8388608.0f));
-    }
+    float inv_t, max_scaled, inv_t32, max_scaled32;                // as they are, and divided by 32
+    __device__ __forceinline__ float below(float v) const { return __saturatef(__fmaf_rn(-v, inv_t32, max_scaled32)); }
+    __device__ __forceinline__ float place(float v) const { return fminf(65536.0f * below(v), 65535.0f); }
+    // The bin of the first level, 0 to 256 (256 is the end of bin 255), as the low bits of the result: the limits come with the sum, so this is
+    // two instructions.
+    __device__ __forceinline__ uint32_t first_bits(float v) const { return __float_as_uint(__fmaf_rz(below(v), 256.0f, 8388608.0f)); }
     // the integer part, from the low bits of a sum that cuts the rest off
     __device__ __forceinline__ int of(float v) const { return (int)(__float_as_uint(__fadd_rz(place(v), 8388608.0f)) & 65535u); }
 };
@@ -994,8 +995,7 @@ sample_rows_kernel(const float* __restrict__ logits, int32_t* __restrict__ out, 
     // infinities are not below it.
     const bool plain = !nan_in_row && fabsf(max_scaled) < 2097152.0f && isfinite(inv_t) && inv_t > 0.0f && chunk <= DRAW_SLICE_MAX;
     if (plain) {
-        const DrawBins bins{inv_t, max_scaled};
-        const float inv_t32 = inv_t * 0.03125f, max_scaled32 = max_scaled * 0.03125f;
+        const DrawBins bins{inv_t, max_scaled, inv_t * 0.03125f, max_scaled * 0.03125f};
         // a bin's word for this lane: 64 bytes a bin, the exponent of first_bits shifted out by the start
         const uint32_t cell = (uint32_t)__cvta_generic_to_shared(&sh->hist.lo[0][tid % DRAW_LANES]) - (0x4b000000u * 64u);
         constexpr uint32_t HI = sizeof(sh->hist.lo), CT = 2 * sizeof(sh->hist.lo);
@@ -1006,7 +1006,7 @@ sample_rows_kernel(const float* __restrict__ logits, int32_t* __restrict__ out, 
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const Halves w = weight_halves(x[j], inv_t, max_scaled);
-                const uint32_t at = DrawBins::first_bits(x[j], inv_t32, max_scaled32) * 64u + cell;
+                const uint32_t at = bins.first_bits(x[j]) * 64u + cell;
                 asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(at), "r"(w.low) : "memory");
                 if (w.high) asm volatile("red.shared.add.u32 [%0+%2], %1;" ::"r"(at), "r"(w.high), "n"(HI) : "memory");
                 asm volatile("red.shared.add.u32 [%0+%2], %1;" ::"r"(at), "r"(1u), "n"(CT) : "memory");
@@ -1103,11 +1103,11 @@ sample_rows_kernel(const float* __restrict__ logits, int32_t* __restrict__ out, 
                     const int q = q0 + lane;
                     const float4 four = q < quads ? quad(q) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
                     const float x[4] = {four.x, four.y, four.z, four.w};
-                    if (!__any_sync(0xffffffffu, __saturatef(__fmaf_rn(-fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3])), inv_t32, max_scaled32)) < nearer)) continue;
+                    if (!__any_sync(0xffffffffu, bins.below(fmaxf(fmaxf(x[0], x[1]), fmaxf(x[2], x[3]))) < nearer)) continue;
                     uint32_t m[4];
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
-                        asm volatile("ld.shared.u8 %0, [%1];" : "=r"(m[j]) : "r"(DrawBins::first_bits(x[j], inv_t32, max_scaled32) + mark) : "memory");
+                        asm volatile("ld.shared.u8 %0, [%1];" : "=r"(m[j]) : "r"(bins.first_bits(x[j]) + mark) : "memory");
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const bool in = m[j] != 0u && 4 * q + j < len;

@@ -123,3 +123,19 @@ def test_draws_where_the_search_changes_its_way(R, V, scale, T, k, p, shift):
     got = ops.sample_rows(x, full(T, torch.float32), full(k, torch.int32), full(p, torch.float32), torch.tensor(seeds, device=DEV), full(3, torch.int64)).cpu().tolist()
     for r in list(range(R))[:6]:
         check(logits[r], T, k, p, plain.uniform_from(int(seeds[r]), 3), got[r])
+
+
+@pytest.mark.parametrize("T", [1e36, 1e38, 3e38])
+@pytest.mark.parametrize("k,p", [(0, 0.9), (40000, 1.0)])
+def test_temperatures_whose_reciprocal_is_below_the_normal_numbers(T, k, p):
+    """The first bins and the finer ones have to agree on every logit where 1 / (32 T) has fewer than 24 bits."""
+    from mimirmind_b200.kernels import ops
+    R, V = 6, 152064
+    rng = np.random.RandomState(int(np.log10(T)) + k)
+    logits = (rng.uniform(-1.0, 1.0, size=(R, V)) * min(3.3e38, 4.0 * T)).astype(np.float32)
+    seeds = rng.randint(1, 2 ** 31, size=R)
+    full = lambda v, dt: torch.full((R,), v, dtype=dt, device=DEV)           # noqa: E731
+    got = ops.sample_rows(torch.tensor(logits, device=DEV), full(T, torch.float32), full(k, torch.int32), full(p, torch.float32),
+                          torch.tensor(seeds, device=DEV), full(3, torch.int64)).cpu().tolist()
+    for r in range(R):
+        check(logits[r], float(np.float32(T)), k, p, plain.uniform_from(int(seeds[r]), 3), got[r])
