@@ -2,15 +2,16 @@
 // the weights of layers (see gemm_split_takes).
 //
 // Every number is split into three bf16 numbers, which hold all of its 24 bits, and a product is the sum of the six larger of the nine partial
-// products (Henry, Tang and Heinecke 2019).  The tensor core cuts off what falls below 2^-24 of a sum's largest term instead of rounding, so
+// products (Henry, Tang and Heinecke 2019).  bf16 ends at 2^-133, so the numbers are multiplied by 2^16 before (the third part of a
+// number below 2^-110 would be cut off otherwise) and the results by 2^-32 in the end, which changes no bit of what both ways hold.  The tensor core cuts off what falls below 2^-24 of a sum's largest term instead of rounding, so
 // the largest partial products, which have 16 bits, are summed there sixteen k at a time from zero and added up beyond that by rounded additions;
-// the five others, 2^-8 of them, stay on the tensor core for a part of k.  Error against 64 bits, of normal numbers, in 1e-7 of the result's size (2-norm):
+// the five others, 2^-8 of them, stay on the tensor core for a part of k.  Error against 64 bits in 1e-7 of the result's size (2-norm):
 // 0.87 for K = 896, 1.30 for 4,864 and 2.4 for 18,944, where FMAs over k in ascending order have 5.3, 12.5 and 25.
 //
 // Which sums are made, and in which order, follows from K alone: k is cut into up to eight parts (gemm_split_parts), a part's sums are added up
 // in order, the parts' results in order.  The tile's size along the tokens and whether the parts are walked by one CTA or shared out over a
 // cluster do not change a bit, so a row's value depends neither on M nor on what stands beside it.  A result that is not finite (an
-// operand was not, or rounds to infinity in bf16, or a sum overflowed) is made again by 32-bit FMAs over k in ascending order.
+// operand was not, or is 2^112 or more, or a sum reached 2^96) is made again by 64-bit FMAs over k in ascending order.
 // All waits are bounded; when one runs out the CTA gives its tensor memory back, sets `err` and makes its whole tile again like that.
 //
 // A CTA works on 128 rows of W (M of the instruction) x NT tokens (its N), 64 k a step:
@@ -66,8 +67,17 @@ __device__ __forceinline__ void gs_rest(float& x, float& y, uint32_t part) {
     y = __fsub_rn(y, __uint_as_float(part & 0xffff0000u));
 }
 __device__ __forceinline__ void gs_store8(uint32_t at, uint32_t x, uint32_t y) { asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"(x), "r"(y) : "memory"); }
+// What is split is 2^16 times the number: see the header.
+constexpr float GS_UP = 65536.0f, GS_DOWN = 1.0f / (65536.0f * 65536.0f);
+__device__ __forceinline__ void gs_up2(float& x, float& y) {
+    uint64_t v;
+    asm("{\n\t.reg .b64 u;\n\tmov.b64 %0, {%1, %2};\n\tmov.b64 u, {%3, %3};\n\tmul.rn.f32x2 %0, %0, u;\n\t}" : "=&l"(v) : "f"(x), "f"(y), "f"(GS_UP));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+}
 // four consecutive k of a row as the three planes
 __device__ __forceinline__ void gs_split4(uint32_t at, int plane, float4 v) {
+    gs_up2(v.x, v.y);
+    gs_up2(v.z, v.w);
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
         const uint32_t a = gs_round2(v.x, v.y), b = gs_round2(v.z, v.w);
@@ -140,10 +150,14 @@ __device__ __forceinline__ void gs_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
+// The result by 64-bit FMAs over k in order; a sum that 32 bits round to infinity is one from there on, as it is by 32-bit FMAs.
 __device__ __noinline__ float gs_again(const float* __restrict__ a, const float* __restrict__ w, int K) {
-    float s = 0.0f;
-    for (int k = 0; k < K; ++k) s = fmaf(a[k], w[k], s);
-    return s;
+    double s = 0.0;
+    for (int k = 0; k < K; ++k) {
+        s = fma((double)a[k], (double)w[k], s);
+        if (fabs(s) >= 3.4028235677973366e38) s = copysign((double)INFINITY, s);      // 2^128 - 2^103
+    }
+    return (float)s;
 }
 
 struct SplitCtl {
@@ -392,7 +406,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const Spli
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
             if (n + x >= g.N) continue;
-            if (!isfinite(v[x])) v[x] = gs_again(g.A + (size_t)m * g.lda, g.W + (size_t)(n + x) * g.K, g.K);
+            if (isfinite(v[x])) v[x] *= GS_DOWN;
+            else v[x] = gs_again(g.A + (size_t)m * g.lda, g.W + (size_t)(n + x) * g.K, g.K);
             if (g.bias) v[x] += g.bias_dtype == MM_F32 ? ((const float*)g.bias)[n + x] : __bfloat162float(((const __nv_bfloat16*)g.bias)[n + x]);
         }
         float* c = g.C + (size_t)m * g.ldc + n;
@@ -428,6 +443,7 @@ __device__ __forceinline__ void gs_parts(const float2* v, uint32_t (*out)[N]) {
 #pragma unroll
     for (int i = 0; i < N; ++i) {
         float x = v[i].x, y = v[i].y;
+        gs_up2(x, y);
 #pragma unroll
         for (int p = 0; p < 3; ++p) {
             out[p][i] = gs_round2(x, y);
@@ -527,7 +543,8 @@ __global__ void __launch_bounds__(256, NJ == 1 ? 2 : 1) gemv_split_kernel(const 
         float v = sums[first][m][c % 16];
 #pragma unroll
         for (int p = 1; p < PARTS; ++p) v += sums[first + p][m][c % 16];
-        if (!isfinite(v)) v = gs_again(g.A + (size_t)m * g.lda, g.W + (size_t)n * g.K, g.K);
+        if (isfinite(v)) v *= GS_DOWN;
+        else v = gs_again(g.A + (size_t)m * g.lda, g.W + (size_t)n * g.K, g.K);
         if (g.bias) v += g.bias_dtype == MM_F32 ? ((const float*)g.bias)[n] : __bfloat162float(((const __nv_bfloat16*)g.bias)[n]);
         g.C[(size_t)m * g.ldc + n] = v;
     }

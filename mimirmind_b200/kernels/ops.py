@@ -237,7 +237,7 @@ def gemm_simt(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ou
 def gemm_split(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, tile: int, side_by_side: bool, give_up: bool = False) -> torch.Tensor:
     """The tensor-core form of ``gemm_simt`` (fp32 throughout, rows of ``a`` and ``out`` at any stride) in tiles of ``tile`` tokens: 16 (up to 16 tokens), 32, 64 or 128, the parts
     of k one after the other in a block or ``side_by_side`` in a cluster.  Every form gives the same bits.  ``give_up``: as if a wait of the tiles'
-    kernel had run out at its start: none is tried more than once, the error flag is set and the result is made again by FMAs."""
+    kernel had run out at its start: none is tried more than once, the error flag is set and the result is made again by 64-bit FMAs."""
     m, k = a.shape
     n = w.shape[0]
     _need(w, "gemm w", torch.float32)

@@ -75,15 +75,33 @@ def test_product_of_numbers_that_cannot_be_split(M):
         assert torch.equal(got[torch.isinf(got)], narrow[torch.isinf(narrow)])
 
 
+@pytest.mark.parametrize("M", [4, 12, 40, 150])
+@pytest.mark.parametrize("a_exp,w_exp", [(-112, 0), (-120, 0), (-125, 20), (-140, 100), (0, -120), (-70, -70), (90, 0), (100, 20), (60, 60)])
+def test_product_of_small_and_large_numbers(M, a_exp, w_exp):
+    """Operands near either end of the exponents: as exact as in the middle, up to the subnormal result's own rounding."""
+    N, K = 200, 640
+    g = torch.Generator(device=DEV).manual_seed(M)
+    a, w = torch.randn((M, K), generator=g, device=DEV), torch.randn((N, K), generator=g, device=DEV)
+    a, w = (torch.ldexp(x.double(), torch.tensor(e, device=DEV)).float() for x, e in ((a, a_exp), (w, w_exp)))
+    out = torch.empty((M, N), device=DEV)
+    ops().gemm_simt(a, w, None, out)
+    ref, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    # as in test_product_of_split_numbers
+    assert ((out - ref).abs() <= (K / 16 + 24 + 5 * K / 16 / 128) * 2.0 ** -24 * size + 2.0 ** -150).all()
+    # n = K / 16 rounded additions to a sum that grows like the root of their number, each off by an ulp / sqrt(12), at most 2^-23 / sqrt(12) of it
+    # (2-norms): together 2^-24 sqrt(n / 6) of the result.  By FMAs over k, n = K, it would be four times as much
+    assert (out - ref).norm() <= (K / 16 / 6) ** 0.5 * 2.0 ** -24 * ref.norm() + 2.0 ** -150 * (M * N) ** 0.5
+
+
 @pytest.mark.parametrize("tile", [32, 64, 128])
 @pytest.mark.parametrize("side_by_side", [False, True])
 @pytest.mark.parametrize("M,N,K", [(40, 130, 128), (150, 260, 1540)])
 def test_product_whose_waits_run_out(tile, side_by_side, M, N, K):
-    """As if a wait had run out at the start: the kernel returns, the error flag is set and the result is what FMAs over k in order give, to the bit.
+    """As if a wait had run out at the start: the kernel returns, the error flag is set and the result is a sum in 64 bits.
     The next product is as if nothing had been."""
     g = torch.Generator(device=DEV).manual_seed(M + tile)
     a, w, b = (torch.randn(s, generator=g, device=DEV) for s in ((M, K), (N, K), (N,)))
-    whole, gone, again, narrow = (torch.empty((M, N), device=DEV) for _ in range(4))
+    whole, gone, again = (torch.empty((M, N), device=DEV) for _ in range(3))
     flag = ops().tcgen05_error_flag(a.device)
     ops().gemm_split(a, w, b, whole, tile, side_by_side)
     assert int(flag.item()) == 0
@@ -94,11 +112,8 @@ def test_product_whose_waits_run_out(tile, side_by_side, M, N, K):
         flag.zero_()
     ops().gemm_split(a, w, b, again, tile, side_by_side)
     assert int(flag.item()) == 0 and torch.equal(again, whole)
-    for n0 in range(0, N, 65):                  # the product by FMAs: fewer than 128 rows of weights
-        part = torch.empty((M, min(65, N - n0)), device=DEV)
-        ops().gemm_simt(a, w[n0:n0 + 65].contiguous(), b[n0:n0 + 65].contiguous(), part)
-        narrow[:, n0:n0 + 65] = part
-    assert torch.equal(gone, narrow)
+    ref, size = a.double() @ w.double().T + b.double(), a.double().abs() @ w.double().abs().T + b.double().abs()
+    assert ((gone - ref).abs() <= 2.0 ** -23 * size).all()           # rounded to 32 bits, and the bias added in 32 bits
 
 
 @pytest.mark.parametrize("M,N,K", [(3, 70, 96), (40, 130, 100), (300, 257, 36)])
