@@ -11,7 +11,7 @@
 // Which sums are made, and in which order, follows from K alone: k is cut into up to eight parts (gemm_split_parts), a part's sums are added up
 // in order, the parts' results in order.  The tile's size along the tokens and whether the parts are walked by one CTA or shared out over a
 // cluster do not change a bit, so a row's value depends neither on M nor on what stands beside it.  A result that is not finite (an
-// operand was not, or is 2^112 or more, or a sum reached 2^96) is made again by 64-bit FMAs over k in ascending order.
+// operand was not, or is 2^112 or more, or a sum reached 2^96) is made again by FMAs over k in ascending order (gs_again).
 // All waits are bounded; when one runs out the CTA gives its tensor memory back, sets `err` and makes its whole tile again like that.
 //
 // A CTA works on 128 rows of W (M of the instruction) x NT tokens (its N), 64 k a step:
@@ -150,14 +150,60 @@ __device__ __forceinline__ void gs_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
-// The result by 64-bit FMAs over k in order; a sum that 32 bits round to infinity is one from there on, as it is by 32-bit FMAs.
-__device__ __noinline__ float gs_again(const float* __restrict__ a, const float* __restrict__ w, int K) {
+// A result that the tensor cores have not given as a number: what 32-bit FMAs over k in order make of it, or, where that is a number (of 2^96 or
+// more), 64-bit ones.  gs_again: a token's with ROWS rows of W (`rows` of them there), sixteen k of all rows on their way together, and no further
+// once none of them is a number, which nothing changes.  A thread does it for itself, so it takes long where it takes many: 509 x 9,728 x 896
+// with a NaN early in every row 211 us (what a state that has gone wrong brings, in every product from there on; one number and one k at a time it was
+// 26,100), with an infinity in every row 10,000, with all results from 2^96 on 20,100.
+__device__ __forceinline__ float gs_again64(const float* __restrict__ a, const float* __restrict__ w, int K) {
     double s = 0.0;
-    for (int k = 0; k < K; ++k) {
-        s = fma((double)a[k], (double)w[k], s);
-        if (fabs(s) >= 3.4028235677973366e38) s = copysign((double)INFINITY, s);      // 2^128 - 2^103
+#pragma unroll 2
+    for (int k = 0; k < K; k += 4) {
+        const float4 y = __ldg(reinterpret_cast<const float4*>(w + k));
+        s = fma((double)a[k], (double)y.x, s);
+        s = fma((double)a[k + 1], (double)y.y, s);
+        s = fma((double)a[k + 2], (double)y.z, s);
+        s = fma((double)a[k + 3], (double)y.w, s);
     }
     return (float)s;
+}
+template <int ROWS>
+__device__ __noinline__ float4 gs_again(const float* __restrict__ a, const float* __restrict__ w, int K, int rows, bool a_words) {
+    const float* p[ROWS];
+    float s[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) {
+        p[r] = w + (r < rows ? (size_t)r * K : 0);
+        s[r] = 0.0f;
+    }
+    for (int k0 = 0; k0 < K; k0 += 16) {
+        float4 x[4], y[ROWS][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int k = k0 + 4 * i < K ? k0 + 4 * i : k0;
+            x[i] = a_words ? __ldg(reinterpret_cast<const float4*>(a + k)) : make_float4(a[k], a[k + 1], a[k + 2], a[k + 3]);
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) y[r][i] = __ldg(reinterpret_cast<const float4*>(p[r] + k));
+        }
+        bool number = false;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (k0 + 4 * i < K) {
+                    s[r] = fmaf(x[i].x, y[r][i].x, s[r]);
+                    s[r] = fmaf(x[i].y, y[r][i].y, s[r]);
+                    s[r] = fmaf(x[i].z, y[r][i].z, s[r]);
+                    s[r] = fmaf(x[i].w, y[r][i].w, s[r]);
+                }
+            number |= s[r] == s[r];
+        }
+        if (!number) break;
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r)
+        if (isfinite(s[r])) s[r] = gs_again64(a, p[r], K);
+    return make_float4(s[0], s[ROWS > 1 ? 1 : 0], s[ROWS > 2 ? 2 : 0], s[ROWS > 3 ? 3 : 0]);
 }
 
 struct SplitCtl {
@@ -403,11 +449,13 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const Spli
             }
             v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
         }
+        const bool finite[4] = {isfinite(v[0]), isfinite(v[1]), isfinite(v[2]), isfinite(v[3])};
+        float4 made = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (!(finite[0] && finite[1] && finite[2] && finite[3])) made = gs_again<4>(g.A + (size_t)m * g.lda, g.W + (size_t)n * g.K, g.K, g.N - n, g.a_words);
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
             if (n + x >= g.N) continue;
-            if (isfinite(v[x])) v[x] *= GS_DOWN;
-            else v[x] = gs_again(g.A + (size_t)m * g.lda, g.W + (size_t)(n + x) * g.K, g.K);
+            v[x] = finite[x] ? v[x] * GS_DOWN : x == 0 ? made.x : x == 1 ? made.y : x == 2 ? made.z : made.w;
             if (g.bias) v[x] += g.bias_dtype == MM_F32 ? ((const float*)g.bias)[n + x] : __bfloat162float(((const __nv_bfloat16*)g.bias)[n + x]);
         }
         float* c = g.C + (size_t)m * g.ldc + n;
@@ -544,7 +592,7 @@ __global__ void __launch_bounds__(256, NJ == 1 ? 2 : 1) gemv_split_kernel(const 
 #pragma unroll
         for (int p = 1; p < PARTS; ++p) v += sums[first + p][m][c % 16];
         if (isfinite(v)) v *= GS_DOWN;
-        else v = gs_again(g.A + (size_t)m * g.lda, g.W + (size_t)n * g.K, g.K);
+        else v = gs_again<1>(g.A + (size_t)m * g.lda, g.W + (size_t)n * g.K, g.K, 1, g.a_words).x;
         if (g.bias) v += g.bias_dtype == MM_F32 ? ((const float*)g.bias)[n] : __bfloat162float(((const __nv_bfloat16*)g.bias)[n]);
         g.C[(size_t)m * g.ldc + n] = v;
     }

@@ -93,6 +93,30 @@ def test_product_of_small_and_large_numbers(M, a_exp, w_exp):
     assert (out - ref).norm() <= (K / 16 / 6) ** 0.5 * 2.0 ** -24 * ref.norm() + 2.0 ** -150 * (M * N) ** 0.5
 
 
+@pytest.mark.parametrize("M", [4, 300])
+def test_product_of_rows_that_are_no_numbers_is_not_slow(M):
+    """What a state that has gone wrong brings into every product after it: a NaN in every row.  Number by number it took some two hundred times as long
+    as other rows; twice as long is what it takes."""
+    N, K = 4096, 896
+    g = torch.Generator(device=DEV).manual_seed(M)
+    w, out, times = torch.randn((N, K), generator=g, device=DEV), torch.empty((M, N), device=DEV), []
+    for bad in (False, True):
+        a = torch.randn((M, K), generator=g, device=DEV)
+        if bad:
+            a[:, 5] = float("nan")
+        taken = []
+        for _ in range(8):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            ops().gemm_simt(a, w, None, out)
+            end.record()
+            end.synchronize()
+            taken.append(start.elapsed_time(end))
+        times.append(sorted(taken)[2])
+        assert bool(torch.isnan(out).all()) == bad
+    assert times[1] <= 10 * times[0], times
+
+
 @pytest.mark.parametrize("tile", [32, 64, 128])
 @pytest.mark.parametrize("side_by_side", [False, True])
 @pytest.mark.parametrize("M,N,K", [(40, 130, 128), (150, 260, 1540)])
