@@ -195,7 +195,7 @@ MM_EXPORT int mm_argmax_rows_split(const void* logits, void* out, void* part_val
 #define DRAW_FEW 128                               // elements among which every one is compared with every other
 #define DRAW_LO_MAX 3800                           // numbers of one bin whose low and high halves 32 bits hold: at most 2^20 e^(1/16) each
 #define DRAW_ROOM 38016                            // numbers of a slice kept in shared memory beside the rest: 227 KB together
-#define DRAW_SLICE_MAX (DRAW_LANES * DRAW_LO_MAX)  // numbers of a slice that the sums have room for
+#define DRAW_SEGMENT (DRAW_LANES * DRAW_LO_MAX)    // numbers that the bins' sums have room for: longer slices go in segments
 #define SAMPLE_MAX_CLUSTER 8
 
 struct BinPlace {
@@ -472,6 +472,81 @@ struct DrawBins {
     // the integer part, from the low bits of a sum that cuts the rest off
     __device__ __forceinline__ int of(float v) const { return (int)(__float_as_uint(__fadd_rz(place(v), 8388608.0f)) & 65535u); }
 };
+
+// the q-th four numbers of a slice from memory; what lies beyond its end is -inf
+__device__ __forceinline__ float4 slice_quad(const float* __restrict__ slice, int len, int vec, int q) {
+    float4 w = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+    const float* at = slice + 4 * q;
+    if (vec) return 4 * q < len ? __ldg(reinterpret_cast<const float4*>(at)) : w;
+    if (4 * q < len) w.x = __ldg(at);
+    if (4 * q + 1 < len) w.y = __ldg(at + 1);
+    if (4 * q + 2 < len) w.z = __ldg(at + 2);
+    if (4 * q + 3 < len) w.w = __ldg(at + 3);
+    return w;
+}
+// four numbers of a plain row into this lane's copy of the bins of the first level
+__device__ __forceinline__ void add_to_bins(const float4& four, const DrawBins& bins) {
+    SampleShared* sh = draw_shared();
+    // a bin's word for this lane: 64 bytes a bin, the exponent of first_bits shifted out by the start
+    const uint32_t cell = (uint32_t)__cvta_generic_to_shared(&sh->hist.lo[0][threadIdx.x % DRAW_LANES]) - (0x4b000000u * 64u);
+    constexpr uint32_t HI = sizeof(sh->hist.lo), CT = 2 * sizeof(sh->hist.lo);
+    const float x[4] = {four.x, four.y, four.z, four.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const Halves w = weight_halves(x[j], bins.inv_t, bins.max_scaled);
+        const uint32_t at = bins.first_bits(x[j]) * 64u + cell;
+        asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(at), "r"(w.low) : "memory");
+        if (w.high) asm volatile("red.shared.add.u32 [%0+%2], %1;" ::"r"(at), "r"(w.high), "n"(HI) : "memory");
+        asm volatile("red.shared.add.u32 [%0+%2], %1;" ::"r"(at), "r"(1u), "n"(CT) : "memory");
+    }
+}
+// mass and count of a bin over its copies
+__device__ __forceinline__ unsigned long long bin_sums(int bin, uint32_t& count) {
+    SampleShared* sh = draw_shared();
+    unsigned long long low = 0ull, high = 0ull;
+    count = 0u;
+#pragma unroll
+    for (int i = 0; i < DRAW_LANES; ++i) {                         // (from another copy on in every lane: no two in one bank)
+        const int copy_i = (i + bin) % DRAW_LANES;
+        low += sh->hist.lo[bin][copy_i];
+        high += sh->hist.hi[bin][copy_i];
+        count += sh->hist.ct[bin][copy_i];
+        if (bin == 255) {
+            low += sh->hist.lo[256][copy_i];
+            high += sh->hist.hi[256][copy_i];
+            count += sh->hist.ct[256][copy_i];
+        }
+    }
+    return low + (high << 20);
+}
+// A slice of more numbers than the bins' 32-bit sums have room for: segment by segment through them, the sums of all but the last in `tab` and the bins
+// empty again for that one; returns its first four.  (2 rows of 486,720 logits with top-p, two segments: 104 us; by radix selects 480.)
+__device__ __noinline__ int early_segments(const float* __restrict__ slice, int len, int vec, const DrawBins bins) {
+    SampleShared* sh = draw_shared();
+    constexpr int STEP = DRAW_SEGMENT / 4;
+    const int quads = (len + 3) / 4;
+    unsigned long long mass = 0ull;
+    uint32_t count = 0u;
+    int q0 = 0;
+    for (; q0 + STEP < quads; q0 += STEP) {
+#pragma unroll 4
+        for (int q = q0 + (int)threadIdx.x; q < q0 + STEP; q += DRAW_THREADS) add_to_bins(slice_quad(slice, len, vec, q), bins);
+        __syncthreads();
+        if (threadIdx.x < 256) {
+            uint32_t n;
+            mass += bin_sums(threadIdx.x, n);
+            count += n;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < (int)(sizeof(sh->hist) / 16); i += DRAW_THREADS) reinterpret_cast<uint4*>(&sh->hist)[i] = make_uint4(0u, 0u, 0u, 0u);
+        __syncthreads();
+    }
+    if (threadIdx.x < 256) {                                       // (read again by the same thread)
+        sh->tab.mass[threadIdx.x] = mass;
+        sh->tab.ct[threadIdx.x] = count;
+    }
+    return q0;
+}
 
 // Candidates are the elements with key >= floor_key.  In the order (key descending, index ascending) find the
 // first element whose cumulative weight exceeds `target`.  Weight is 1 when `by_count`, else the fixed-point
@@ -907,17 +982,7 @@ sample_rows_kernel(const float* __restrict__ logits, int32_t* __restrict__ out, 
     const int begin = min(V, (int)c.rank * chunk), end = min(V, begin + chunk), len = end - begin;
     const int quads = (len + 3) / 4;
     const bool cached = chunk <= DRAW_ROOM;
-    // the q-th four numbers of the slice from memory; what lies beyond its end is -inf
-    auto from_row = [&](int q) {
-        float4 w = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
-        const float* at = row + begin + 4 * q;
-        if (vec) return 4 * q < len ? __ldg(reinterpret_cast<const float4*>(at)) : w;
-        if (4 * q < len) w.x = __ldg(at);
-        if (4 * q + 1 < len) w.y = __ldg(at + 1);
-        if (4 * q + 2 < len) w.z = __ldg(at + 2);
-        if (4 * q + 3 < len) w.w = __ldg(at + 3);
-        return w;
-    };
+    auto from_row = [&](int q) { return slice_quad(row + begin, len, vec, q); };
     float4* kept = reinterpret_cast<float4*>(sample_smem + sizeof(SampleShared));
     c.vals = cached ? reinterpret_cast<const float*>(kept) : row;
     c.vals_begin = cached ? begin : 0;
@@ -993,42 +1058,22 @@ sample_rows_kernel(const float* __restrict__ logits, int32_t* __restrict__ out, 
     const float u = (float)(bits >> 40) * (1.0f / 16777216.0f);  // 24 bits → [0,1)
     // Below 2^21 max_scaled is off by 1/16 at most, so that no weight exceeds FIXED_ONE e^(1/16) and the sums of the bins have room; NaN and
     // infinities are not below it.
-    const bool plain = !nan_in_row && fabsf(max_scaled) < 2097152.0f && isfinite(inv_t) && inv_t > 0.0f && chunk <= DRAW_SLICE_MAX;
+    const bool plain = !nan_in_row && fabsf(max_scaled) < 2097152.0f && isfinite(inv_t) && inv_t > 0.0f;
     if (plain) {
         const DrawBins bins{inv_t, max_scaled, inv_t * 0.03125f, max_scaled * 0.03125f};
-        // a bin's word for this lane: 64 bytes a bin, the exponent of first_bits shifted out by the start
-        const uint32_t cell = (uint32_t)__cvta_generic_to_shared(&sh->hist.lo[0][tid % DRAW_LANES]) - (0x4b000000u * 64u);
-        constexpr uint32_t HI = sizeof(sh->hist.lo), CT = 2 * sizeof(sh->hist.lo);
+        // slices of more than 60,800 numbers: all segments but the last, their sums in `tab`
+        const int q_first = len > DRAW_SEGMENT ? early_segments(row + begin, len, vec, bins) : 0;
 #pragma unroll 2
-        for (int q = tid; q < quads; q += DRAW_THREADS) {
-            const float4 four = quad(q);
-            const float x[4] = {four.x, four.y, four.z, four.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const Halves w = weight_halves(x[j], inv_t, max_scaled);
-                const uint32_t at = bins.first_bits(x[j]) * 64u + cell;
-                asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(at), "r"(w.low) : "memory");
-                if (w.high) asm volatile("red.shared.add.u32 [%0+%2], %1;" ::"r"(at), "r"(w.high), "n"(HI) : "memory");
-                asm volatile("red.shared.add.u32 [%0+%2], %1;" ::"r"(at), "r"(1u), "n"(CT) : "memory");
-            }
-        }
+        for (int q = q_first + tid; q < quads; q += DRAW_THREADS) add_to_bins(quad(q), bins);
         __syncthreads();
         if (tid < 256) {
-            unsigned long long low = 0ull, high = 0ull;
-            uint32_t count = 0u;
-#pragma unroll
-            for (int i = 0; i < DRAW_LANES; ++i) {                 // (from another copy on in every lane: no two in one bank)
-                const int copy_i = (i + tid) % DRAW_LANES;
-                low += sh->hist.lo[tid][copy_i];
-                high += sh->hist.hi[tid][copy_i];
-                count += sh->hist.ct[tid][copy_i];
-                if (tid == 255) {
-                    low += sh->hist.lo[256][copy_i];
-                    high += sh->hist.hi[256][copy_i];
-                    count += sh->hist.ct[256][copy_i];
-                }
+            uint32_t count;
+            unsigned long long mass = bin_sums(tid, count);
+            if (q_first > 0) {
+                mass += sh->tab.mass[tid];
+                count += sh->tab.ct[tid];
             }
-            sh->pub[1][tid] = low + (high << 20);
+            sh->pub[1][tid] = mass;
             sh->pub_ct[tid] = tid == 255 ? count - (uint32_t)(4 * quads - len) : count;
         }
         sample_cluster_sync();
@@ -1099,7 +1144,7 @@ sample_rows_kernel(const float* __restrict__ logits, int32_t* __restrict__ out, 
                 const uint32_t mark = (uint32_t)__cvta_generic_to_shared(&sh->marked[0]) - 0x4b000000u;
                 __syncthreads();
 #pragma unroll 1
-                for (int q0 = warp * 32; q0 < quads; q0 += DRAW_THREADS) {
+                for (int q0 = warp * 32; q0 < quads && len <= DRAW_SEGMENT; q0 += DRAW_THREADS) {      // (the lists hold places in 16 bits)
                     const int q = q0 + lane;
                     const float4 four = q < quads ? quad(q) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
                     const float x[4] = {four.x, four.y, four.z, four.w};
@@ -1117,7 +1162,7 @@ sample_rows_kernel(const float* __restrict__ logits, int32_t* __restrict__ out, 
                         n_near += (uint32_t)__popc(all);
                     }
                 }
-                listed = !__syncthreads_or(n_near > DRAW_NEAR);
+                listed = !__syncthreads_or(n_near > DRAW_NEAR) && len <= DRAW_SEGMENT;
             }
             fits = sh->n_list <= DRAW_LIST;
             if (fits || round == 2) break;

@@ -139,3 +139,38 @@ def test_temperatures_whose_reciprocal_is_below_the_normal_numbers(T, k, p):
                           torch.tensor(seeds, device=DEV), full(3, torch.int64)).cpu().tolist()
     for r in range(R):
         check(logits[r], float(np.float32(T)), k, p, plain.uniform_from(int(seeds[r]), 3), got[r])
+
+
+def test_wide_rows_are_not_slow():
+    """A row of more numbers than the bins' 32-bit sums have room for goes through them in segments; without them it took eight to nine times
+    as long as a row that is a little shorter."""
+    from mimirmind_b200.kernels import ops
+    times = []
+    for V in (8 * 60800, 8 * 60800 + 320):
+        x = 2 * torch.randn((2, V), device=DEV)
+        full = lambda v, dt: torch.full((2,), v, dtype=dt, device=DEV)       # noqa: E731
+        args = [full(0.8, torch.float32), full(0, torch.int32), full(0.95, torch.float32), full(5, torch.int64), torch.arange(2, device=DEV)]
+        taken = []
+        for _ in range(8):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            ops.sample_rows(x, *args)
+            end.record()
+            end.synchronize()
+            taken.append(start.elapsed_time(end))
+        times.append(sorted(taken)[2])
+    assert times[1] <= 4 * times[0], times
+
+
+@pytest.mark.parametrize("R,V,scale,T,k,p", [(2, 8 * 60800 + 4, 2.0, 0.7, 0, 0.9), (2, 1000003, 2.0, 0.8, 50, 0.95), (3, 1000000, 0.5, 1.5, 0, 0.9),
+                                             (2, 2 * 8 * 60800 + 4, 3.0, 0.3, 0, 1.0), (1, 700000, 0.0, 1.0, 0, 1.0)])
+def test_draws_from_rows_in_segments(R, V, scale, T, k, p):
+    from mimirmind_b200.kernels import ops
+    rng = np.random.RandomState(V % 991 + k)
+    logits = (1.0 + scale * rng.randn(R, V)).astype(np.float32)
+    full = lambda v, dt: torch.full((R,), v, dtype=dt, device=DEV)           # noqa: E731
+    seeds = rng.randint(1, 2 ** 31, size=R)
+    got = ops.sample_rows(torch.tensor(logits, device=DEV), full(T, torch.float32), full(k, torch.int32), full(p, torch.float32),
+                          torch.tensor(seeds, device=DEV), full(3, torch.int64)).cpu().tolist()
+    for r in range(R):
+        check(logits[r], T, k, p, plain.uniform_from(int(seeds[r]), 3), got[r])
