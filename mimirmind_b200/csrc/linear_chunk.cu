@@ -901,27 +901,28 @@ __global__ void __launch_bounds__(256, 2) lc_delta_prepare_kernel(LcArgs a) {
     product(sv, sbeta, a.dv, DV / 4, a.u + ((size_t)t0 * a.H + h) * a.dv, (size_t)a.H * a.dv, std::integral_constant<int, DV / 32>{}, std::false_type{});
 }
 
-// U = U0 - W S and S' = gamma_C S + K'^T U, chunk after chunk, for sixteen columns of one head's S per block: a chain of two products per chunk.
+// U = U0 - W S and S' = gamma_C S + K'^T U, chunk after chunk, for 16 NG columns of one head's S per block: a chain of two products per chunk.
 // W and K' come as fragments straight into the registers of the warps that multiply them, the next chunk's while the current one is worked on;
 // S and U are split by the threads that make them and pass through shared memory as planes.  In the first product warp w has rows 16 (w % 4)
 // of U and a quarter of the key channels; the quarters meet in a pass over U.  In the second warp w has eight key channels of
-// S^T = U^T K' and all sixteen columns: S stays in its registers.
+// S^T = U^T K' and all columns: S stays in its registers.
 // Bound by the tensor cores (24 products of 16 x 8 x 16 per warp and half of a chunk), what they read from shared memory, three barriers, and
 // the fragments' way from L2 (96 KB per block and chunk): 64 chunks take 179 us.  Warps that split all that they multiply took 238; with W
 // and K' split by eight more warps into planes in shared memory 206, bound by the reads and writes there.
 #define LC_CARRY_THREADS 512
-template <int DK>
+template <int DK, int NG>
 struct LcCarryShared {
-    static constexpr int PS = lc_plane<DK>(16), PU = lc_plane<16>(64), LQ = 20;
-    // bytes: the planes of S^T [16][dk] and U [64][16], the quarters of W S
+    static constexpr int NS = 16 * NG, PS = lc_plane<DK>(NS), PU = lc_plane<NS>(64), LQ = NS + 4;
+    // bytes: the planes of S^T [NS][dk] and U [64][NS], the quarters of W S
     static constexpr int S = 0, U = S + 3 * PS, SUM = U + 3 * PU, SIZE = SUM + 4 * LC_C * LQ * 4;
 };
-template <int DK>
+template <int DK, int NG>
 __global__ void __launch_bounds__(LC_CARRY_THREADS, 1) lc_delta_carry_kernel(LcArgs a) {
-    using M = LcCarryShared<DK>;
+    using M = LcCarryShared<DK, NG>;
+    constexpr int NS = M::NS;
     extern __shared__ __align__(16) float lc_smem[];
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(lc_smem);
-    const int h = blockIdx.y, r = blockIdx.z, n_base = blockIdx.x * 16, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int h = blockIdx.y, r = blockIdx.z, n_base = blockIdx.x * NS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int first = a.req_chunks[2 * r], count = a.req_chunks[2 * r + 1];
     if (count <= 0) return;
     const int t = lane & 3, g = lane >> 2;
@@ -944,42 +945,48 @@ __global__ void __launch_bounds__(LC_CARRY_THREADS, 1) lc_delta_carry_kernel(LcA
 #pragma unroll
                 for (int part = 0; part < 3; ++part) fk[e][part] = __ldg(p + (e * 3 + part) * 32);
     };
-    // S^T of key channels 8 warp.. (if there are so many): rows g and g + 8 of the sixteen columns, channels 2t and 2t + 1
+    // S^T of key channels 8 warp.. (if there are so many): of every sixteen columns rows g and g + 8, channels 2t and 2t + 1
     const int m = warp * 8 + 2 * t;
-    float S[4];
+    float S[NG][4];
     float* st = a.state + (size_t)a.slots[r] * a.state_stride + (size_t)h * a.dv * a.dk;
     {
         const bool fresh = a.positions[a.chunk_meta[4 * first]] == 0;
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-            const int n = n_base + g + 8 * (x >> 1);
-            S[x] = (!fresh && has && m + (x & 1) < a.dk && n < a.dv) ? st[(size_t)n * a.dk + m + (x & 1)] : 0.0f;
-        }
+        for (int b = 0; b < NG; ++b)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const int n = n_base + 16 * b + g + 8 * (x >> 1);
+                S[b][x] = (!fresh && has && m + (x & 1) < a.dk && n < a.dv) ? st[(size_t)n * a.dk + m + (x & 1)] : 0.0f;
+            }
     }
     auto to_planes = [&]() {
         if (!has) return;
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const LcSplit x = lc_split(S[2 * half], S[2 * half + 1]);
-            const uint32_t to = base + M::S + ((g + 8 * half) * (DK + 8) + m) * 2;
-            lc_sts32(to, x.h);
-            lc_sts32(to + M::PS, x.m);
-            lc_sts32(to + 2 * M::PS, x.l);
-        }
+        for (int b = 0; b < NG; ++b)
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const LcSplit x = lc_split(S[b][2 * half], S[b][2 * half + 1]);
+                const uint32_t to = base + M::S + ((16 * b + g + 8 * half) * (DK + 8) + m) * 2;
+                lc_sts32(to, x.h);
+                lc_sts32(to + M::PS, x.m);
+                lc_sts32(to + 2 * M::PS, x.l);
+            }
     };
-    // the pass over U: a thread's row and two columns
+    // the pass over U: a thread's row and two of every sixteen columns
     const int row = threadIdx.x >> 3, col = (threadIdx.x & 7) * 2;
     float* sum = lc_smem + M::SUM / 4;
-    auto u_place = [&](int t0) { return a.u + ((size_t)(t0 + row) * a.H + h) * a.dv + n_base + col; };
+    auto u_place = [&](int t0, int b) { return a.u + ((size_t)(t0 + row) * a.H + h) * a.dv + n_base + 16 * b + col; };
     load_w(first);
     load_k(first);
     to_planes();
     int t0 = a.chunk_meta[4 * first], cnt = a.chunk_meta[4 * first + 1];
     for (int i = 0; i < count; ++i) {
         const int c = first + i;
-        const bool mine = row < cnt && n_base + col < a.dv;
         const float gain = __ldg(a.gain + (size_t)c * a.H + h);
-        float2 u = mine ? *reinterpret_cast<const float2*>(u_place(t0)) : make_float2(0.0f, 0.0f);
+        float2 u[NG];
+#pragma unroll
+        for (int b = 0; b < NG; ++b)
+            u[b] = row < cnt && n_base + 16 * b + col < a.dv ? *reinterpret_cast<const float2*>(u_place(t0, b)) : make_float2(0.0f, 0.0f);
         int next_t0 = 0, next_cnt = 0;
         if (i + 1 < count) {
             next_t0 = a.chunk_meta[4 * (c + 1)];
@@ -988,22 +995,23 @@ __global__ void __launch_bounds__(LC_CARRY_THREADS, 1) lc_delta_carry_kernel(LcA
         __syncthreads();                         // S's planes
         {
             const int m0 = (warp & 3) * 16, part = warp >> 2;
-            float p[1][2][4], low[1][2][4];
-            lc_zero<8>(&p[0][0][0]);
-            lc_zero<8>(&low[0][0][0]);
+            float p[1][2 * NG][4], low[1][2 * NG][4];
+            lc_zero<8 * NG>(&p[0][0][0]);
+            lc_zero<8 * NG>(&low[0][0][0]);
 #pragma unroll
             for (int e = 0; e < STEPS; ++e) {
                 const int k0 = (part * STEPS + e) * 16;
                 const LcA fa = {{{fw[e][0].x, fw[e][1].x, fw[e][2].x}, {fw[e][0].y, fw[e][1].y, fw[e][2].y}, {fw[e][0].z, fw[e][1].z, fw[e][2].z},
                                  {fw[e][0].w, fw[e][1].w, fw[e][2].w}}};
-                LcB fb[2];
-                lc_b2_nk<DK + 8>(base + M::S + k0 * 2, M::PS, fb);
-                lc_products<1, 2>(p, low, &fa, fb);
+                LcB fb[2 * NG];
+#pragma unroll
+                for (int b = 0; b < NG; ++b) lc_b2_nk<DK + 8>(base + M::S + (16 * b * (DK + 8) + k0) * 2, M::PS, fb + 2 * b);
+                lc_products<1, 2 * NG>(p, low, &fa, fb);
             }
             if (i + 1 < count) load_w(c + 1);
-            lc_add<8>(&p[0][0][0], &low[0][0][0]);
+            lc_add<8 * NG>(&p[0][0][0], &low[0][0][0]);
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
+            for (int j = 0; j < 2 * NG; ++j)
 #pragma unroll
                 for (int half = 0; half < 2; ++half)
                     *reinterpret_cast<float2*>(sum + (part * LC_C + m0 + g + 8 * half) * M::LQ + 8 * j + 2 * t) = make_float2(p[0][j][2 * half], p[0][j][2 * half + 1]);
@@ -1011,51 +1019,60 @@ __global__ void __launch_bounds__(LC_CARRY_THREADS, 1) lc_delta_carry_kernel(LcA
         {   // what the chunk starts from, as [dv, dk]
             float* o = a.states + ((size_t)c * a.H + h) * a.dv * a.dk;
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const int n = n_base + g + 8 * half;
-                if (has && m < a.dk && n < a.dv) *reinterpret_cast<float2*>(o + (size_t)n * a.dk + m) = make_float2(S[2 * half], S[2 * half + 1]);
-            }
+            for (int b = 0; b < NG; ++b)
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int n = n_base + 16 * b + g + 8 * half;
+                    if (has && m < a.dk && n < a.dv) *reinterpret_cast<float2*>(o + (size_t)n * a.dk + m) = make_float2(S[b][2 * half], S[b][2 * half + 1]);
+                }
         }
         __syncthreads();                         // the quarters
-        {
+#pragma unroll
+        for (int b = 0; b < NG; ++b) {
             float2 x[4];
 #pragma unroll
-            for (int part = 0; part < 4; ++part) x[part] = *reinterpret_cast<const float2*>(sum + (part * LC_C + row) * M::LQ + col);
-            u.x -= (x[0].x + x[1].x) + (x[2].x + x[3].x);
-            u.y -= (x[0].y + x[1].y) + (x[2].y + x[3].y);
-            if (mine) *reinterpret_cast<float2*>(u_place(t0)) = u;
-            const LcSplit y = lc_split(u.x, u.y);
-            const uint32_t to = base + M::U + (row * 24 + col) * 2;
+            for (int part = 0; part < 4; ++part) x[part] = *reinterpret_cast<const float2*>(sum + (part * LC_C + row) * M::LQ + 16 * b + col);
+            u[b].x -= (x[0].x + x[1].x) + (x[2].x + x[3].x);
+            u[b].y -= (x[0].y + x[1].y) + (x[2].y + x[3].y);
+            if (row < cnt && n_base + 16 * b + col < a.dv) *reinterpret_cast<float2*>(u_place(t0, b)) = u[b];
+            const LcSplit y = lc_split(u[b].x, u[b].y);
+            const uint32_t to = base + M::U + (row * (NS + 8) + 16 * b + col) * 2;
             lc_sts32(to, y.h);
             lc_sts32(to + M::PU, y.m);
             lc_sts32(to + 2 * M::PU, y.l);
         }
         __syncthreads();                         // U's planes
         if (has) {
-            float p[1][1][4], low[1][1][4];
-            lc_zero<4>(&p[0][0][0]);
-            lc_zero<4>(&low[0][0][0]);
+            float p[NG][1][4], low[NG][1][4];
+            lc_zero<4 * NG>(&p[0][0][0]);
+            lc_zero<4 * NG>(&low[0][0][0]);
 #pragma unroll
             for (int step = 0; step < 4; ++step) {
-                const LcA fa = lc_a_km<24>(base + M::U + 16 * step * 24 * 2, M::PU);
+                LcA fa[NG];
+#pragma unroll
+                for (int b = 0; b < NG; ++b) fa[b] = lc_a_km<NS + 8>(base + M::U + (16 * step * (NS + 8) + 16 * b) * 2, M::PU);
                 const uint4* f = fk[step >> 1];
                 const LcB fb = step & 1 ? LcB{{{f[0].z, f[1].z, f[2].z}, {f[0].w, f[1].w, f[2].w}}} : LcB{{{f[0].x, f[1].x, f[2].x}, {f[0].y, f[1].y, f[2].y}}};
-                lc_products<1, 1>(p, low, &fa, &fb);
+                lc_products<NG, 1>(p, low, fa, &fb);
             }
             if (i + 1 < count) load_k(c + 1);
-            lc_add<4>(&p[0][0][0], &low[0][0][0]);
+            lc_add<4 * NG>(&p[0][0][0], &low[0][0][0]);
 #pragma unroll
-            for (int x = 0; x < 4; ++x) S[x] = fmaf(gain, S[x], p[0][0][x]);
+            for (int b = 0; b < NG; ++b)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) S[b][x] = fmaf(gain, S[b][x], p[b][0][x]);
         }
         to_planes();                             // (read by all before the second barrier)
         t0 = next_t0;
         cnt = next_cnt;
     }
 #pragma unroll
-    for (int x = 0; x < 4; ++x) {
-        const int n = n_base + g + 8 * (x >> 1);
-        if (has && m + (x & 1) < a.dk && n < a.dv) st[(size_t)n * a.dk + m + (x & 1)] = S[x];
-    }
+    for (int b = 0; b < NG; ++b)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const int n = n_base + 16 * b + g + 8 * (x >> 1);
+            if (has && m + (x & 1) < a.dk && n < a.dv) st[(size_t)n * a.dk + m + (x & 1)] = S[b][x];
+        }
 }
 
 // ---- a forget gate per key channel (csrc/linear_state.cu): k_t = 1 - f_t, S_t = diag(f_t) S_(t-1) + k_t v_t^T -------------------------
@@ -1303,7 +1320,13 @@ static int lc_run(const LcArgs& a, int n_requests, cudaStream_t s) {
         return lc_launch<lc_output_kernel<DK, DV>>(chunks, 256, planes, s, a, a.v, (size_t)a.ldv);
     }
     if (const int rc = lc_launch<lc_delta_prepare_kernel<DK, DV>>(chunks, 256, 2 * tile + 2 * square, s, a)) return rc;
-    if (const int rc = lc_launch<lc_delta_carry_kernel<DK>>(dim3(ceil_div(a.dv, 16), a.H, n_requests), LC_CARRY_THREADS, LcCarryShared<DK>::SIZE, s, a)) return rc;
+    // Columns of S per block: sixteen, or 32 where that saves so many rounds of one block per SM that they make up for a chunk's time, which is 1.5 (dk 64)
+    // to 1.6 times as long.  1,024 tokens, us with 16 and with 32 columns: 32 heads of 64 x 64, one portion (1 round and 1) 88 and 103, two (2, 1) 177 and
+    // 162, four (4, 2) 342 and 308; 48 heads of 128 x 128 (3, 2) 291 and 304, 32 heads, two portions (4, 2) 376 and 345.
+    const long long narrow = ceil_div((long long)ceil_div(a.dv, 16) * a.H * n_requests, 148), wide = ceil_div((long long)ceil_div(a.dv, 32) * a.H * n_requests, 148);
+#define LC_CARRY(NG) lc_launch<lc_delta_carry_kernel<DK, NG>>(dim3(ceil_div(a.dv, 16 * NG), a.H, n_requests), LC_CARRY_THREADS, LcCarryShared<DK, NG>::SIZE, s, a)
+    if (const int rc = 10 * narrow > 16 * wide ? LC_CARRY(2) : LC_CARRY(1)) return rc;
+#undef LC_CARRY
     return lc_launch<lc_output_kernel<DK, DV>>(chunks, 256, planes, s, a, (const float*)a.u, (size_t)a.H * a.dv);
 }
 

@@ -72,6 +72,40 @@ def test_products(H, G, dk, dv, delta, decay):
             assert err <= max(5e-7, 1.5 * was), (r, err, was)
 
 
+@pytest.mark.parametrize("H,dk,dv", [(148, 64, 20), (148, 100, 32), (74, 128, 100), (160, 48, 64)])
+def test_blocks_of_32_columns(H, dk, dv):
+    """So many heads that a block of the delta rule's chain takes 32 columns of a state: the bits of a few heads alone, whose blocks take sixteen."""
+    from mimirmind_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(H + dv)
+    lens, begin = [150, 64, 3], [0, 7, 0]
+    n = sum(lens)
+    rnd = lambda *s: torch.randn(s, generator=gen, device=DEV)                       # noqa: E731
+    unit = lambda t: t / t.norm(dim=-1, keepdim=True)                                # noqa: E731
+    q, k, v = rnd(n, H, dk) * dk ** -0.5, unit(rnd(n, H, dk) + rnd(1, H, dk)), rnd(n, H, dv)
+    gate, beta = 0.8 + 0.2 * torch.rand((n, H), generator=gen, device=DEV), torch.rand((n, H), generator=gen, device=DEV)
+    before = rnd(3, H, dv, dk)
+    meta, per, s = [], [], 0
+    for r, m in enumerate(lens):
+        per.append([len(meta), -(-m // 64)])
+        meta += [[s + o, min(64, m - o), r, 0] for o in range(0, m, 64)]
+        s += m
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)                   # noqa: E731
+    pos = torch.cat([torch.arange(b, b + m, dtype=torch.int32, device=DEV) for b, m in zip(begin, lens)])
+
+    def run(heads):
+        state = before[:, heads].reshape(3, -1).contiguous()
+        flat = lambda t: t[:, heads].reshape(n, -1).contiguous()                     # noqa: E731
+        h = len(heads)
+        out = ops.linear_state_products(flat(q), flat(k), flat(v), state, i32(meta), i32(per), i32([0, 1, 2]), pos, h, h, dk, dv,
+                                        gate=gate[:, heads].contiguous(), beta=beta[:, heads].contiguous())
+        return out.view(n, h, dv), state.view(3, h, dv, dk)
+
+    out, state = run(list(range(H)))
+    few = [0, 1, H // 2, H - 1]
+    some, kept = run(few)
+    assert torch.isfinite(out).all() and torch.equal(out[:, few], some) and torch.equal(state[:, few], kept)
+
+
 @pytest.mark.parametrize("H,dk,dv", [(4, 128, 64), (2, 128, 128), (3, 64, 64), (5, 36, 100)])
 @pytest.mark.parametrize("gates", ["near 1", "wide", "near 0"])
 def test_forget_gate_products(H, dk, dv, gates):
