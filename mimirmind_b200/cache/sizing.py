@@ -42,11 +42,12 @@ def step_bytes_per_token(spec: ModelSpec, layer_tensor_shapes: Sequence[Sequence
     return 2 * 4 * spec.hidden_size + 2 * element_bytes * widest
 
 
-def step_reserve_bytes(spec: ModelSpec, layer_tensor_shapes, element_bytes: int, token_budget: int, max_active: int) -> int:
+def step_reserve_bytes(spec: ModelSpec, layer_tensor_shapes, element_bytes: int, token_budget: int, max_active: int, scratch_bytes: int = 0) -> int:
     """What is kept free for a step of ``token_budget + max_active`` tokens: activations, logits of every active
-    request (three copies: the step's, the sampler's, a captured graph's) and 128 MiB for library workspaces."""
+    request (three copies: the step's, the sampler's, a captured graph's), what a layer keeps beside its rows (``scratch_bytes``) and 128 MiB for library
+    workspaces."""
     tokens = token_budget + max_active
-    return tokens * step_bytes_per_token(spec, layer_tensor_shapes, element_bytes) + 3 * 4 * max_active * spec.vocab_size + (128 << 20)
+    return tokens * step_bytes_per_token(spec, layer_tensor_shapes, element_bytes) + 3 * 4 * max_active * spec.vocab_size + scratch_bytes + (128 << 20)
 
 
 def pool_tokens(free_bytes: int, fraction: float, reserve_bytes: int, bytes_per_token: int, page_size: int, max_context: int,

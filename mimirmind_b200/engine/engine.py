@@ -76,11 +76,12 @@ class Engine:
         (the weights are loaded), less what a step of ``token_budget`` tokens needs, at most
         ``max_context x max_active`` tokens."""
         from ..cache import sizing
-        from ..weights.store import layer_tensor_shapes
+        from ..weights.store import layer_scratch_bytes, layer_tensor_shapes
         esz = 4 if model.rt.dtype == torch.float32 else 2
         shapes = layer_tensor_shapes(model.spec)
         free, _total = torch.cuda.mem_get_info(model.rt.device)
-        return sizing.pool_tokens(free, fraction, sizing.step_reserve_bytes(model.spec, shapes, esz, token_budget, max_active),
+        scratch = layer_scratch_bytes(model.spec, token_budget + max_active, max_active, esz)
+        return sizing.pool_tokens(free, fraction, sizing.step_reserve_bytes(model.spec, shapes, esz, token_budget, max_active, scratch),
                                   sizing.cache_bytes_per_token(model.cache_groups(), esz), page_size, max_context, max_active)
 
     def set_diagnostics(self, parity_dump: str = "", trace_decode_file: str = "") -> None:

@@ -1169,6 +1169,16 @@ def linear_state_chunked(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, stat
 LINEAR_CHUNK = 64      # tokens per chunk of linear_state_products
 
 
+def linear_state_scratch(n_chunks: int, n_tokens: int, heads: int, dk: int, dv: int, delta: bool, per_channel: bool = False) -> list:
+    """fp32 numbers of the arrays that the products over chunks keep beside their results: states [chunks, heads, dv, dk], gain [chunks,
+    heads] or per key channel; with the delta rule the fragments of two operands in three 16-bit parts, whole chunks of keys of 64 or 128 numbers (98 KB a chunk and
+    head of 128: the operand alone, in 32 bits, would be 33), and u [tokens, heads, dv]."""
+    sizes = [n_chunks * heads * dv * dk, n_chunks * heads * (dk if per_channel else 1)]
+    if delta:
+        sizes += [n_chunks * heads * LINEAR_CHUNK * (64 if dk <= 64 else 128) * 3, n_tokens * heads * dv]
+    return sizes
+
+
 def linear_state_products_supported(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, dk: int, dv: int) -> bool:
     """True if ``linear_state_products`` takes these rows: heads of up to 128 numbers in multiples of 4, 16-byte boundaries."""
     return bool(_lib.load().mm_linear_chunk_supported(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0),
@@ -1203,11 +1213,7 @@ def linear_state_products(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, sta
         _need(t, what, torch.int32)
     n_chunks, n_req = chunk_meta.shape[0], req_chunks.shape[0]
     out = _rows_for(out, n, heads * dv, q)
-    # states [chunks, heads, dv, dk], gain [chunks, heads], with the delta rule fragments of two operands in three 16-bit parts, u [n, heads, dv]
-    sizes = [n_chunks * heads * dv * dk, n_chunks * heads]
-    if beta is not None:
-        sizes += [n_chunks * heads * LINEAR_CHUNK * (64 if dk <= 64 else 128) * 3, n * heads * dv]
-    _kept, parts = _scratch(sizes, q.device)
+    _kept, parts = _scratch(linear_state_scratch(n_chunks, n, heads, dk, dv, beta is not None), q.device)
     states, gain, frag, u = parts + [None] * (4 - len(parts))
     check(_lib.load().mm_linear_chunk(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0), _ptr(gate), _ptr(beta),
                                       _ptr(head_decay), out.data_ptr(), state.data_ptr(), state.stride(0), chunk_meta.data_ptr(),
@@ -1787,7 +1793,7 @@ def forget_gate_products(q: torch.Tensor, f: torch.Tensor, v: torch.Tensor, stat
         _need(t, what, torch.int32)
     n_chunks, n_req = chunk_meta.shape[0], req_chunks.shape[0]
     out = _rows_for(out, n, heads * dv, q)
-    _kept, (states, gain) = _scratch([n_chunks * heads * dv * dk, n_chunks * heads * dk], q.device)
+    _kept, (states, gain) = _scratch(linear_state_scratch(n_chunks, n, heads, dk, dv, False, per_channel=True), q.device)
     check(_lib.load().mm_forget_gate_chunk(q.data_ptr(), f.data_ptr(), v.data_ptr(), q.stride(0), f.stride(0), v.stride(0), out.data_ptr(),
                                            state.data_ptr(), state.stride(0), chunk_meta.data_ptr(), req_chunks.data_ptr(), slots.data_ptr(),
                                            positions.data_ptr(), n_req, n_chunks, int(heads), int(dk), int(dv), states, gain,

@@ -223,6 +223,12 @@ class Part:
     def tensor_specs(cls, spec: PartSpec, prefix: str) -> List[TensorSpec]:
         return []
 
+    @classmethod
+    def scratch_bytes(cls, spec: PartSpec, n_tokens: int, n_requests: int, element_bytes: int) -> int:
+        """What ``forward`` keeps on the device beside its rows in a step of ``n_tokens`` over ``n_requests``, at the most (for
+        sizing the cache)."""
+        return 0
+
     def __init__(self, spec: PartSpec, weights: WeightView, rt: Runtime):
         self.spec = spec
         self.rt = rt

@@ -99,6 +99,16 @@ class LinearStateMixer(Mixer):
             out.append(TensorSpec(prefix + spec["out_weight"], (dv if spec.get("out_norm", "head") == "head" else H * dv,), role="norm"))
         return out
 
+    @classmethod
+    def scratch_bytes(cls, spec: PartSpec, n_tokens: int, n_requests: int, element_bytes: int) -> int:
+        """Of the chunks' states, gains and operands; a request's last chunk may hold few tokens.  float32 runs walk."""
+        if element_bytes == 4 or n_tokens < CHUNKED_FROM:
+            return 0
+        H, dk, dv = int(spec["heads"]), int(spec["key_dim"]), int(spec["value_dim"])
+        chunks = n_tokens // min(CHUNK, ops.LINEAR_CHUNK) + n_requests
+        per_channel = spec["decay"] == "forget_gate"
+        return 4 * sum(ops.linear_state_scratch(chunks, n_tokens, H, dk, dv, bool(spec.get("delta")), per_channel))
+
     def __init__(self, spec: PartSpec, weights: WeightView, rt: Runtime):
         super().__init__(spec, weights, rt)
         self.hidden, self.heads, self.qk_heads = int(spec["hidden"]), int(spec["heads"]), int(spec["qk_heads"])

@@ -37,6 +37,10 @@ class ParallelMixers(Mixer):
                 out.append(TensorSpec(prefix + spec[side + "_out"], (spec["hidden"],), role="norm"))
         return out
 
+    @classmethod
+    def scratch_bytes(cls, spec: PartSpec, n_tokens: int, n_requests: int, element_bytes: int) -> int:
+        return sum(MIXERS.get(spec[side].kind).scratch_bytes(spec[side], n_tokens, n_requests, element_bytes) for side in ("left", "right"))
+
     def __init__(self, spec: PartSpec, weights: WeightView, rt: Runtime):
         super().__init__(spec, weights, rt)
         self.hidden = int(spec["hidden"])

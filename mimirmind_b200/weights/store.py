@@ -66,6 +66,13 @@ def layer_tensor_shapes(spec: ModelSpec):
     return out
 
 
+def layer_scratch_bytes(spec: ModelSpec, n_tokens: int, n_requests: int, element_bytes: int) -> int:
+    """What a step's parts keep beside their rows, at the most (one part of one layer runs at a time)."""
+    parts = [(reg.get(part.kind), part) for layer in spec.layers for reg, part in ((MIXERS, layer.mixer), (FEED_FORWARDS, layer.feed_forward))]
+    parts += [(part_class(extra), extra) for layer in spec.layers for extra in layer.extras.values()]
+    return max((cls.scratch_bytes(part, n_tokens, n_requests, element_bytes) for cls, part in parts), default=0)
+
+
 def _storage_dtype(t: torch.Tensor, run_dtype: torch.dtype) -> torch.dtype:
     if not t.dtype.is_floating_point:
         return torch.int32

@@ -3,12 +3,13 @@ from types import SimpleNamespace
 
 import pytest
 
+import domelix_util as domelix
 from conftest import TINY
 from mimirmind_b200.cache import sizing
 from mimirmind_b200.cache.manager import GroupSpec
 from mimirmind_b200.config.engine_config import EngineConfigError, parse_engine_config
 from mimirmind_b200.registry import get_architecture
-from mimirmind_b200.weights.store import layer_tensor_shapes
+from mimirmind_b200.weights.store import layer_scratch_bytes, layer_tensor_shapes
 
 GIB = 1 << 30
 
@@ -46,6 +47,24 @@ def test_step_reserve_grows_with_the_budget_and_the_widest_layer():
     small = sizing.step_reserve_bytes(spec, shapes, 2, 64, 4)
     large = sizing.step_reserve_bytes(spec, shapes, 2, 512, 4)
     assert large - small == (512 - 64) * per_token
+
+
+@pytest.mark.parametrize("layers,per_chunk,per_token", [
+    # numbers a chunk of 64 tokens keeps per head of the layer that keeps most (a state, a decay, the operands' fragments), and a token
+    ([domelix.delta(16, 4, 128, 128, 4), domelix.retention(8, 64, 64, [0.9] * 8)], 16 * (128 * 128 + 1 + 3 * 64 * 128), 16 * 128),
+    ([domelix.delta(4, 4, 68, 64, 4)], 4 * (68 * 64 + 1 + 3 * 64 * 128), 4 * 64),
+    ([domelix.parallel((4, 2, 24, 16, 0.3, 37, 10), (3, 16, 8, (0.5, 0.9, 0.99)))], 3 * (16 * 8 + 1), 0),
+])
+def test_step_reserve_counts_what_matrix_states_keep_per_chunk(layers, per_chunk, per_token):
+    arch = get_architecture("Domelix")
+    spec = arch.build_spec(arch.parse_config(domelix.config(101, 64, 1e-5, layers), "test"))
+    tokens, requests = 4096, 8
+    scratch = layer_scratch_bytes(spec, tokens, requests, 2)
+    assert scratch == 4 * ((tokens // 64 + requests) * per_chunk + tokens * per_token)
+    shapes = layer_tensor_shapes(spec)
+    assert sizing.step_reserve_bytes(spec, shapes, 2, 4088, 8, scratch) - sizing.step_reserve_bytes(spec, shapes, 2, 4088, 8) == scratch
+    assert layer_scratch_bytes(spec, tokens, requests, 4) == 0           # float32 runs walk token by token
+    assert layer_scratch_bytes(spec, 200, requests, 2) == 0              # ... and so do short steps
 
 
 def test_engine_config_takes_the_fraction():
