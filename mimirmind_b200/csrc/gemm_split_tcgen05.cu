@@ -664,10 +664,20 @@ int launch_split(const SplitArgs& g, int nt, int ranks, cudaStream_t s) {
 
 }  // namespace
 
+static bool gemm_split_can(const void* W, int K) { return K % 4 == 0 && ((uintptr_t)W & 15) == 0; }
+
 // By the weights alone, never by M.  Not the products whose weights are mostly streamed, a head's 151,936 rows: there a few tokens' sums by FMAs
-// read them faster (545 MB for 4 tokens 121 us from memory, 127 here), and many tokens are rare.  Under 128 rows or k the fixed costs decide
-// (131 x 260 for one token: 4 us by FMAs, 6 here).
-bool gemm_split_takes(const void* W, int N, int K) { return K % 4 == 0 && ((uintptr_t)W & 15) == 0 && N >= 128 && N <= 65536 && K >= 128; }
+// read them faster (545 MB for 4 tokens 121 us from memory, 127 here), and many tokens are rare.  Nor small weights, where the fixed costs of the split decide for
+// a few tokens, which is what most steps have, and prompts gain little.  us for 1, 4, 8, 64 and 1,024 tokens, weights from memory, by FMAs and here:
+//   512 x 256     2.8  2.9  2.9  11  11      3.8  4.1  4.3  7.7  10        4,864 x 256   3.7  4.6  5.6  12   67      4.5  4.8  5.1  9.6  42
+//   1,024 x 512   3.8  4.2  4.4  22  30      5.8  6.2  6.4  9.8  15        9,728 x 128   3.3  5.1  5.8  9.5  62      4.6  5.5  6.0  8.7  49
+//   2,048 x 512   4.3  5.2  5.8  22  58      6.0  6.3  6.7  10   22        128 x 640     3.7  3.9  4.0  22   24      4.6  4.8  5.2  8.6  9.1
+//   1,024 x 896   5.2  5.7  6.0  38  50      5.9  6.1  6.4  10   25        128 x 2,048   8.5  8.9  9.4  70   78      5.6  5.9  6.2  10   16
+// So k of ten steps and more, which go in four or eight parts, or 1.2 million numbers: a few tokens lose a quarter at the most there, many take half
+// as long or less.
+bool gemm_split_takes(const void* W, int N, int K) {
+    return gemm_split_can(W, K) && N >= 128 && N <= 65536 && K >= 128 && (K > 9 * 64 || (long long)N * K >= 1200000);
+}
 
 int gemm_split(const float* A, const float* W, const void* bias, int bias_dtype, float* C, int M, int N, int K, int lda, int ldc, int* err,
                cudaStream_t s) {
@@ -700,7 +710,7 @@ int gemm_split(const float* A, const float* W, const void* bias, int bias_dtype,
 // start.
 MM_EXPORT int mm_gemm_split(const void* A, const void* W, const void* bias, int bias_dtype, void* C, int M, int N, int K, int lda, int ldc, int tile,
                             int side_by_side, int give_up, void* err, void* stream) {
-    MM_REQUIRE(M > 0 && N > 0 && K > 0 && lda >= K && ldc >= N && gemm_split_takes(W, N, K), "gemm_split: bad sizes");
+    MM_REQUIRE(M > 0 && N > 0 && K > 0 && lda >= K && ldc >= N && gemm_split_can(W, K), "gemm_split: bad sizes");
     MM_REQUIRE((tile == FEW && M <= FEW) || tile == 32 || tile == 64 || tile == 128, "gemm_split: no such tile");
     const SplitArgs g = split_args((const float*)A, (const float*)W, bias, bias_dtype, (float*)C, M, N, K, lda, ldc, (int*)err, give_up);
     return launch_split(g, tile, side_by_side ? g.parts : 1, (cudaStream_t)stream);

@@ -93,6 +93,19 @@ def test_product_of_small_and_large_numbers(M, a_exp, w_exp):
     assert (out - ref).norm() <= (K / 16 / 6) ** 0.5 * 2.0 ** -24 * ref.norm() + 2.0 ** -150 * (M * N) ** 0.5
 
 
+@pytest.mark.parametrize("N,K,split", [(131, 260, False), (512, 576, False), (1024, 256, False), (2048, 512, False), (128, 580, True), (2344, 512, True), (200, 640, True)])
+def test_which_weights_are_split(N, K, split):
+    """Small ones are not, for any number of tokens: their products by FMAs are the bits of narrow pieces of the weights, which always go that way."""
+    g = torch.Generator(device=DEV).manual_seed(N + K)
+    w = torch.randn((N, K), generator=g, device=DEV)
+    for M in (1, 8, 16, 40, 200):
+        a = torch.randn((M, K), generator=g, device=DEV)
+        out, part = torch.empty((M, N), device=DEV), torch.empty((M, 96), device=DEV)
+        ops().gemm_simt(a, w, None, out)
+        ops().gemm_simt(a, w[:96].contiguous(), None, part)
+        assert torch.equal(out[:, :96], part) != split
+
+
 @pytest.mark.parametrize("M", [4, 300])
 def test_product_of_rows_that_are_no_numbers_is_not_slow(M):
     """What a state that has gone wrong brings into every product after it: a NaN in every row.  Number by number it took some two hundred times as long
