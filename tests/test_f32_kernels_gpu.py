@@ -50,6 +50,90 @@ def test_product_of_split_numbers(M, N, K):
         assert torch.equal(one[0], out[m])
 
 
+def split_forms(a, w, b):
+    """The product in every form of the kernels for split numbers, by name."""
+    out = {}
+    for tile in (16, 32, 64, 128):
+        for side_by_side in (False, True):
+            if tile > 16 or (a.shape[0] <= 16 and not side_by_side):
+                y = torch.empty((a.shape[0], w.shape[0]), device=DEV)
+                out[tile, side_by_side] = ops().gemm_split(a, w, b, y, tile, side_by_side)
+    return out
+
+
+# k in one, two, four and eight parts, whole steps of 64 and not: walked by one block, whose sums of the parts before wait in tensor memory, or by one each
+@pytest.mark.parametrize("N,K", [(128, 128), (131, 260), (200, 644), (257, 1540), (1000, 2052)])
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 33, 65, 130, 300])
+def test_forms_of_the_split_product(M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(M * N + K)
+    a, w, b = (torch.randn(s, generator=g, device=DEV) for s in ((M, K), (N, K), (N,)))
+    forms = split_forms(a, w, b)
+    out = forms[32, False]
+    for name, y in forms.items():
+        assert torch.equal(y, out), name
+    ref = a.double() @ w.double().T + b.double()
+    # K / 16 rounded additions to a part's sum and a few to the whole, each off by an ulp / sqrt(12), at most 2^-23 / sqrt(12) of a sum that grows like the root of
+    # their number.  A partial product that half of the steps leave out is 4e-7 (the parts in the middle) and more
+    assert (out - ref).norm() <= ((K / 16 + 8) / 6) ** 0.5 * 2.0 ** -24 * ref.norm()
+    loose = torch.empty((M, K + 3), device=DEV)[:, :K].copy_(a)                 # rows off the 16-byte boundaries
+    wide = torch.full((M, N + 5), 7.0, device=DEV)
+    for tile in (16, 32, 64, 128):
+        if tile > 16 or M <= 16:
+            ops().gemm_split(loose, w, b, wide[:, :N], tile, tile == 64)
+            assert torch.equal(wide[:, :N], out) and (wide[:, N:] == 7.0).all()
+
+
+@pytest.mark.parametrize("numbers", ["powers", "cancelling", "small", "subnormal", "one large"])
+@pytest.mark.parametrize("N,K", [(160, 644), (130, 1664)])
+def test_bits_of_a_row_do_not_depend_on_the_others(numbers, N, K):
+    """mma.sync for a few tokens and tcgen05.mma for more add sixteen products up to the same bits.  No document says so: it is what
+    they do, for operands far apart as well."""
+    g = torch.Generator(device=DEV).manual_seed(K)
+    rnd = lambda *s: torch.randn(s, generator=g, device=DEV)                         # noqa: E731
+    powers = lambda top, *s: torch.exp2(torch.randint(-top, top + 1, s, generator=g, device=DEV).float())     # noqa: E731
+    a, w = rnd(130, K), rnd(N, K)
+    if numbers == "powers":
+        a, w = a * powers(30, 130, K), w * powers(30, N, K)
+    elif numbers == "cancelling":               # pairs that take each other away but for the last bits
+        a[:, 1::2], w[:, 1::2] = -a[:, ::2] * (1 + 2.0 ** -20 * rnd(130, K // 2)), w[:, ::2]
+    elif numbers == "small":
+        a, w = a * 2.0 ** -118, w * powers(20, N, K)
+    elif numbers == "subnormal":
+        a, w = a * 2.0 ** -126 * powers(10, 130, K).clamp(max=1.0), w * 2.0 ** 40
+    else:
+        a[:, ::97] *= 2.0 ** 40
+    for M in (1, 7, 16, 17, 130):
+        forms = split_forms(a[:M].contiguous(), w, None)
+        if M == 1:
+            first = forms[16, False]
+        for name, y in forms.items():
+            assert torch.isfinite(y).all() and torch.equal(y, forms[32, False]), (M, name)
+            assert torch.equal(y[:1], first), (M, name)
+    ref, size = a.double() @ w.double().T, a.double().abs() @ w.double().abs().T
+    assert ((y - ref).abs() <= (K / 16 + 24 + 5 * K / 16 / 128) * 2.0 ** -24 * size + 2.0 ** -150).all()      # as in test_product_of_split_numbers
+
+
+@pytest.mark.parametrize("M", [5, 12, 40, 150])
+def test_split_product_of_numbers_that_cannot_be_split(M):
+    """As below, in every form: what 32-bit FMAs over k in order give, and nothing beside them changes."""
+    N, K = 140, 520
+    g = torch.Generator(device=DEV).manual_seed(M)
+    a, w = (torch.randn(s, generator=g, device=DEV) for s in ((M, K), (N, K)))
+    clean = split_forms(a, w, None)[32, False]
+    a[1, 3], a[2, 500], a[3, 17], w[130, 7], w[139, 519], w[5] = float("inf"), float("nan"), 3.4e38, float("-inf"), 3.4e38, 0.0
+    a[4] = 3e38                                 # sums that overflow
+    keep = torch.ones((M, N), dtype=torch.bool, device=DEV)
+    keep[1:5] = False
+    keep[:, [5, 130, 139]] = False
+    narrow = torch.empty((M, N), device=DEV)    # by FMAs
+    for n0 in (0, 70):
+        narrow[:, n0:n0 + 70] = ops().gemm_simt(a, w[n0:n0 + 70].contiguous(), None, torch.empty((M, 70), device=DEV))
+    for name, out in split_forms(a, w, None).items():
+        assert torch.equal(out[keep], clean[keep]), name
+        assert torch.equal(torch.isnan(out), torch.isnan(narrow)) and torch.equal(torch.isinf(out), torch.isinf(narrow)), name
+        assert torch.equal(out[torch.isinf(out)], narrow[torch.isinf(narrow)]), name
+
+
 @pytest.mark.parametrize("M", [5, 12, 40, 150])
 def test_product_of_numbers_that_cannot_be_split(M):
     """An infinity, a NaN, a number beyond bf16's largest and sums that overflow: what 32-bit FMAs over k in order give, and nothing beside them changes."""
