@@ -50,6 +50,18 @@ def test_product_of_split_numbers(M, N, K):
         assert torch.equal(one[0], out[m])
 
 
+@pytest.mark.parametrize("M,N,K", [(1000, 512, 516), (4900, 100, 260), (5000, 16, 2048), (37, 4864, 200), (9, 4864, 252), (3, 40000, 64)])
+def test_product_of_weights_that_are_not_split(M, N, K):
+    """Tiles of 64 rows with steps of 32 and of 64, of 32 rows, and the kernels that stream the weights, each against a row alone."""
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    a, w, b = (torch.randn(s, generator=g, device=DEV) for s in ((M, K), (N, K), (N,)))
+    out = ops().gemm_simt(a, w, b, torch.empty((M, N), device=DEV))
+    ref, size = a.double() @ w.double().T + b.double(), a.double().abs() @ w.double().abs().T + b.double().abs()
+    assert ((out - ref).abs() <= (K + 1) * 2.0 ** -24 * size).all()             # as in test_product
+    for m in {0, M // 2, M - 1}:
+        assert torch.equal(ops().gemm_simt(a[m:m + 1].contiguous(), w, b, torch.empty((1, N), device=DEV))[0], out[m])
+
+
 def split_forms(a, w, b):
     """The product in every form of the kernels for split numbers, by name."""
     out = {}
@@ -73,7 +85,7 @@ def test_forms_of_the_split_product(M, N, K):
         assert torch.equal(y, out), name
     ref = a.double() @ w.double().T + b.double()
     # K / 16 rounded additions to a part's sum and a few to the whole, each off by an ulp / sqrt(12), at most 2^-23 / sqrt(12) of a sum that grows like the root of
-    # their number.  A partial product that half of the steps leave out is 4e-7 (the parts in the middle) and more
+    # their number.  A partial product that half of the steps leave out is 1.7e-6 of it
     assert (out - ref).norm() <= ((K / 16 + 8) / 6) ** 0.5 * 2.0 ** -24 * ref.norm()
     loose = torch.empty((M, K + 3), device=DEV)[:, :K].copy_(a)                 # rows off the 16-byte boundaries
     wide = torch.full((M, N + 5), 7.0, device=DEV)
