@@ -17,7 +17,7 @@
 // of both operands are on their way from global memory into registers meanwhile (two buffers, one barrier per BK).
 // A buffer is [k][row]; a row's place is turned by (k / 4 % 8) * 4, so that the scattered stores of a warp (8 runs of k x 4
 // rows) fall into 32 different banks and four neighbouring rows still are one 16-byte word.
-// 64 x 64 outputs of 128 threads (8 x 4 each): 37.6 TFLOP/s where they fill the GPU (509 x 9,728 x 896 in 236 us, 4 x 4 a thread with
+// 64 x 64 outputs of 128 threads (8 x 4 each): 40.9 TFLOP/s where they fill the GPU (509 x 9,728 x 896 in 217 us, 4 x 4 a thread with
 // scalar loads 477).  Larger tiles (128 x 64, 128 x 128 of
 // 8 x 8) gain nothing where they fill the GPU and lose a factor of 2 and 3 where they do not; fp32 FMAs alone: 10 % slower.
 template <typename T, bool VEC>
@@ -283,9 +283,9 @@ static int launch_gemm_simt(const void* A, const void* W, const void* bias, int 
 #define SIMT_TILE(BM, TM, BK)                                                                                                            \
     return vec ? launch_simt_tile<TA, TW, TC, BM, 64, TM, 4, BK, true>(A, W, bias, bias_dtype, C, M, N, K, lda, ldc, s)                    \
                : launch_simt_tile<TA, TW, TC, BM, 64, TM, 4, BK, false>(A, W, bias, bias_dtype, C, M, N, K, lda, ldc, s)
-    // 32-row tiles where they put fewer rows on the busiest SM (or M does not fill 64): 100 x 1,152 x 896 25.9 us against 33.1; where both
-    // put the same, 64 rows are ahead (509 x 896 x 4,864 on zeros: 161 against 177 us).  With at most two blocks per SM there is no other
-    // block to fill the barriers, and the deeper step pays (142 against 161 us; with more blocks 210 against 199).
+    // 32-row tiles where they put fewer rows on the busiest SM (or M does not fill 64): 100 x 1,152 x 512 15.1 us against 17.0; where both
+    // put the same, 64 rows are ahead (1,000 x 512 x 512 17.7 against 21.4, 5,000 x 64 x 2,048 61.7 against 80.9).  With at most two blocks per SM there is
+    // no other block to fill the barriers, and the deeper step pays (17.7 against 30.8, 61.7 against 116.7; with more blocks 4,000 x 1,024 x 512 97.5 and 96.9).
     const long long rounds64 = ceil_div(ceil_div(M, 64) * (long long)ceil_div(N, 64), 148);
     const long long rounds32 = ceil_div(ceil_div(M, 32) * (long long)ceil_div(N, 64), 148);
     if (M <= 32 * 65535 && (M <= 32 || rounds32 * 32 * 10 <= rounds64 * 64 * 8)) SIMT_TILE(32, 4, 32);

@@ -3,14 +3,16 @@
 //
 // Every number is split into three bf16 numbers, which hold all of its 24 bits, and a product is the sum of the six larger of the nine partial
 // products (Henry, Tang and Heinecke 2019).  bf16 ends at 2^-133, so the numbers are multiplied by 2^16 before (the third part of a
-// number below 2^-110 would be cut off otherwise) and the results by 2^-32 in the end, which changes no bit of what both ways hold.  The tensor core cuts off what falls below 2^-24 of a sum's largest term instead of rounding, so
-// the largest partial products, which have 16 bits, are summed there sixteen k at a time from zero and added up beyond that by rounded additions;
+// number below 2^-110 would be cut off otherwise) and the results by 2^-32 in the end, which changes no bit of what both ways hold.  The
+// tensor core cuts off what falls below 2^-24 of a sum's largest term instead of rounding, so the largest partial products, which have 16 bits, are summed there sixteen k at a time from zero and added up beyond that by rounded additions;
 // the five others, 2^-8 of them, stay on the tensor core for a part of k.  Error against 64 bits in 1e-7 of the result's size (2-norm):
 // 0.87 for K = 896, 1.30 for 4,864 and 2.4 for 18,944, where FMAs over k in ascending order have 5.3, 12.5 and 25.
 //
 // Which sums are made, and in which order, follows from K alone: k is cut into up to eight parts (gemm_split_parts), a part's sums are added up
 // in order, the parts' results in order.  The tile's size along the tokens and whether the parts are walked by one CTA or shared out over a
-// cluster do not change a bit, so a row's value depends neither on M nor on what stands beside it.  A result that is not finite (an
+// cluster do not change a bit, so a row's value depends neither on M nor on what stands beside it.  (For up to 16 tokens that rests on mma.sync
+// and tcgen05.mma adding sixteen products up to the same bits.  They do, as far as the tests look, with operands up to 2^60 apart; no document
+// says that they have to.)  A result that is not finite (an
 // operand was not, or is 2^112 or more, or a sum reached 2^96) is made again by FMAs over k in ascending order (gs_again).
 // All waits are bounded; when one runs out the CTA gives its tensor memory back, sets `err` and makes its whole tile again like that.
 //
@@ -19,9 +21,10 @@
 //                 write the three planes of each in the 128-byte swizzle;
 //   warp 16       one thread issues tcgen05.mma: per sixteen k the largest products into one of HB buffers, the five others onto `low`;
 //   warps 8..15   read each buffer back and add it up (32 rows and half of the tokens a warp).
-// Bound by shared memory: a step of 128 tokens reads 192 KB of it for the tensor core and writes 96 KB of planes.
-// Three tiles of 128 tokens, one after the other on an SM, take 509 x 9,728 x 896 in 101 us (88 TFLOP/s of 32-bit products; by FMAs: 220); 509 x 896 x 4,864, eight
-// CTAs to a tile, 53 (FMAs: 144).  The issuing warp walks along converged and elects its thread: with one lane in a branch of
+// Bound by nothing that is full: 1,024 x 9,728 x 896, 608 tiles of 128 tokens on 148 SMs, keeps an SM at work for 79 % of the time (the fifth round holds 16
+// tiles), and then its issue slots are busy for 63 % (splitting and summing), shared memory for 48 % (a step reads 192 KB of it for the tensor core
+// and writes 96 KB of planes), the tensor cores for less; the rest goes into what the roles hand over.  From graphs of 20 launches, us: 509 x 9,728 x 896 95.8 (93 TFLOP/s of
+// 32-bit products; by FMAs 217), 1,024 x 9,728 x 896 159 (397), 509 x 896 x 4,864, eight CTAs to a tile, 51.7 (142).  The issuing warp walks along converged and elects its thread: with one lane in a branch of
 // its own a product took 170 clocks to issue instead of the 39 (16 tokens) to 64 (128) that it runs.
 #include "tcgen05.cuh"
 #include "gemm_split.h"
@@ -477,8 +480,8 @@ __global__ void __launch_bounds__(SPLIT_THREADS, 1) gemm_split_kernel(const Spli
 // tensor memory, no planes and no hand-over between warps, and there are enough of them to fill the GPU.  A warp takes one part of k of one tile (eight
 // warps: 8 / PARTS tiles) and splits both operands' fragments in registers, DEPTH sixteens of k on their way from memory; the
 // parts' results meet in shared memory.  Bound by the chain of dependent products (five per sixteen k) and the first loads' latency.
-// Weights from memory, 4 tokens: 896 x 896 10.3 us (by FMAs in order 10.5), 9,728 x 896 18.8 (20.7), 896 x 4,864 16.4 (24.6), 3,584 x 18,944 71 (160),
-// 37,888 x 3,584 113 (128).  Fragments loaded straight into registers took half as long again: eight cache lines to an eight-byte load.
+// Weights from memory, single launches, 4 tokens: 896 x 896 10.3 us (by FMAs in order 10.5), 9,728 x 896 18.8 (20.7), 896 x 4,864 16.4 (24.6), 3,584 x 18,944 71
+// (160), 37,888 x 3,584 113 (128); 12 tokens: 9,728 x 896 28.7 (34.8), 896 x 4,864 20.6 (28.8), but 896 x 896 12.3 (10.3).  Fragments loaded straight into registers took half as long again: eight cache lines to an eight-byte load.
 constexpr int FEW = 16;                       // tokens
 
 __device__ __forceinline__ void gs_mma(float* c, const uint32_t* a, const uint32_t* b) {

@@ -13,8 +13,8 @@
 //   plain:  lc_state (what each chunk adds), lc_carry over the chunks per number of the state, lc_output;
 //   delta:  lc_delta_prepare (T, W, U0 per chunk), lc_delta_carry (U and S', chunk after chunk), lc_output with u for v.
 // A token costs dk dv multiply-adds three to four times as in the token-by-token walk, but as tiles of 16 x 8 x 16 on the tensor
-// cores (mma.sync): every operand is split into three bf16 numbers, which hold all of its 24 bits, and the product is the sum of the six
-// larger of the nine partial products, added up in 32 bits (Henry, Tang and Heinecke 2019).  Error against 64 bits, of outputs and states over 300 to 4,096 tokens: where many tokens
+// cores (mma.sync): every operand is split into three bf16 numbers, which hold all of its 24 bits (of numbers below 2^-110 fewer: bf16 ends at
+// 2^-133), and the product is the sum of the six larger of the nine partial products, added up in 32 bits (Henry, Tang and Heinecke 2019).  Error against 64 bits, of outputs and states over 300 to 4,096 tokens: where many tokens
 // add up (decays near 1) 0.7e-7 to 1.4e-7, half of the 32-bit walk's; where a state forgets half of itself per token, so that the
 // walk has little left to round, 0.6e-7 to 1.2e-7 (the walk: 0.4e-7 to 0.9e-7).  With two tf32 numbers (22 bits) and three products it was
 // 1.0e-7 to 2.4e-7 in both, for kernels 5 to 8 % shorter.  The FMA units, whose tiles are held up by shared-memory reads, take twice as long.

@@ -166,7 +166,8 @@ def paged_sink_attention(q, cache, out, ctx, num_heads: int, num_kv_heads: int, 
             # equal key and value sizes of 64 or 128: the TMA decode kernel of the plain attention, in the forms that
             # finish a row inside the kernel (one split, or the splits of a token as one cluster)
             keys = visible_keys(window, chunk, keep, ctx.max_kv_len)
-            # (more than 12 tiles: here the other kernel merges its splits itself: a layer of 1 request at 2,000 keys 14.8 us there, 15.7 as a cluster)
+            # (more than 12 tiles: here the other kernel merges its splits itself.  1 request, 4 KV heads of 128, us there and as a cluster: 9.3 and 9.9 at 2,000
+            # keys, 10.6 and 11.8 at 3,000; up to 1,500 the cluster would be ahead, 9.3 and 9.0, at 900 10.5 and 8.2.  Up to seven tiles, 130 and 440 keys: 7.2 and 6.6, 9.7 and 7.2)
             _len, max_splits, cluster = attention_bf16.choose_split(n_items, num_kv_heads, keys, key_dim, cache.page_size, max_tiles=0)
             if cluster or max_splits == 1:
                 tma = (max_splits, cluster)

@@ -28,7 +28,8 @@ TARGET_CTAS = 2 * 148  # decode CTAs wanted (measured: 2 per SM beat 1 and 4 at 
 USE_CLUSTER_MERGE = True   # up to 8 splits per token: one thread-block cluster merges them through shared memory
 CLUSTER_MAX_WANTED = 12    # ... preferred over more splits and a merge launch when up to this many were wanted,
 CLUSTER_MAX_TILES = 48     # or when its eight CTAs have at most six tiles of 64 keys each (whole decode steps of two layers, cluster and merge launch, us: 1 request
-#                            at 1,000 keys, 2 KV heads 139 and 149, 4 KV heads 400 and 408; 2 requests at 3,000 157 and 159, 407 and 415; at 8,000 170 and 166, 435 and 426)
+#                            at 3,000 keys, 2 KV heads 158 and 164, 4 KV heads 432 and 439; 2 requests 168 and 177, 440 and 446.  Between 48 and 80 tiles the two
+#                            are close: 1 request at 4,000 keys 169 and 173, 443 and 446, at 5,200 172 and 175, 450 and 446; at 8,000 170 and 166, 435 and 426)
 FIXED_SPLIT = None     # tests set a split length in keys to cut by absolute position instead
 
 _declared = False

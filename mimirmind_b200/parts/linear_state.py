@@ -46,8 +46,8 @@ from .linear import linear
 CHUNK = 64                   # tokens per chunk of the three-pass walk
 CHUNKED_FROM = 256           # a step whose longest portion has at least this many tokens goes chunk by chunk (not in float32)
 # In such a step the portions of at least PRODUCTS_FROM tokens are cut into chunks for the products and the others are walked.  32 heads of
-# 128x128, us: 16 portions of 64 tokens 178 as products, 203 walked, of 128 tokens 330 and 370, one of 64 tokens 56 and 37; 200 portions of
-# one token 2600 and 250, which is why they are kept apart (a chunk costs the same whatever it holds).
+# 128x128, us: 16 portions of 64 tokens 128 as products, 187 walked, of 128 tokens 243 and 354, one of 64 tokens 40 and 27, of 128 40 and 45; 200 portions
+# of one token 1707 and 205, which is why they are kept apart (a chunk costs the same whatever it holds).
 PRODUCTS_FROM = 128
 CONV_BY_TOKEN_FROM = 32      # a step whose longest portion has at least this many tokens runs the convolution per (token, channel)
 
@@ -56,9 +56,11 @@ def delta_by_products(lens, heads: int, dk: int, dv: int) -> bool:
     """Estimates, in us, from times measured with 8 to 64 heads of 64x64, 64x128 and 128x128 and 1 to 16 portions of 256 and 512 tokens:
     a walk's token takes 0.22 (dk 64) to 0.30 (dk 128) after the one before it, and 0.0021, 0.0040 or 0.0064 per head of a full device
     (a portion's state as much as six tokens); in the products it takes 0.0027, 0.0037 or 0.0053 per head.  One portion of 512 tokens, 32
-    heads of 128x128: 135 by products, 190 walked; 16 of 256: 717 and 811; of 64x64, 4 portions of 512: 199 and 182, so that is walked;
-    512 tokens beside 200 portions of one: about 385 and 361, walked.  Below 320 tokens and 8192 x 128 x 128 numbers the launches of the
-    products count for more: a layer with 16 heads took 165 by products for 256 tokens, 147 walked, one with 32 heads 147 and 171."""
+    heads of 128x128: 99 by products, 174 walked; 16 of 256: 652 and 791; of 64x64, 4 portions of 512: 173 and 170, so that is walked;
+    512 tokens beside 200 portions of one: 362 and 299, walked.  Below 320 tokens and 8192 x 128 x 128 numbers the launches of the
+    products count for more: a layer with 16 heads took 118 by products for 256 tokens, 114 walked, one with 32 heads 131 and 156.  The products have
+    become faster than the estimate near its line: 2 portions of 512, 32 heads of 64x64, are walked in 123, by products it would be 94; a
+    layer with 16 heads of 128x128 and 300 tokens takes 127 and would take 119."""
     inside = [n for n in lens if n >= CHUNKED_FROM]
     if not inside or sum((n + ops.LINEAR_CHUNK - 1) // ops.LINEAR_CHUNK for n in inside) > 65535:
         return False
